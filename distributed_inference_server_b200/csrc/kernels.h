@@ -23,6 +23,10 @@ cudaError_t launch_sample(const float *logits, long long ld, int T, int V, const
                           const float *top_p, const unsigned long long *seeds, const unsigned long long *steps,
                           uint32_t *out_tokens, int vocab_offset, float *out_val, float *out_sumexp, float *out_logprob,
                           cudaStream_t st);
+constexpr int kSampleClusterMaxV = 262144;  // 8 CTAs x 512 threads x 64 logits (k_sample.cu)
+cudaError_t launch_sample_cluster(const float *logits, long long ld, int T, int V, const float *temperature, const float *top_p,
+                                  const unsigned long long *seeds, const unsigned long long *steps, uint32_t *out, int vocab_offset,
+                                  float *out_val, float *out_sumexp, float *out_logprob, cudaStream_t st);
 cudaError_t launch_argmax_merge(const float *cand_val, const uint32_t *cand_tok, const float *cand_sum, int tp, int T,
                                 uint32_t *out, float *out_logprob, cudaStream_t st);
 cudaError_t launch_synth_bf16(uint16_t *dst, size_t n, unsigned long long seed, int kind, int layer, float amp,

@@ -991,7 +991,6 @@ int Engine::init_stack(const dis_engine_config *c, const dis_stack_config *sc) {
   }
   seqs.resize((size_t)max_batch);
   slot_stamp.assign((size_t)max_batch, 0);
-  if (const char *g = getenv("DIS_SAMPLER")) sampler_buckets = strcmp(g, "bisect") != 0;
   ENG_CUDA(cudaDeviceSynchronize());
   return DIS_OK;
 }
@@ -1998,11 +1997,6 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   const unsigned long long *seed = mt.d<unsigned long long>(mt.o_seed), *step = mt.d<unsigned long long>(mt.o_step);
   float *d_logprob = reinterpret_cast<float *>(M.d_out + M.max_rows);
   kl++;
-  if (!all_greedy && sampler_buckets) {
-    TpSampPeers solo{};
-    solo.rank = 0; solo.tp = 1; solo.cap_rows = M.max_rows;
-    return launch_tp_sample(solo, M.logits, M.c.vocab, R, M.c.vocab, temp, topp, seed, step, nullptr, 0, M.d_out, d_logprob, stream);
-  }
   return launch_sample(M.logits, M.c.vocab, R, M.c.vocab, temp, topp, seed, step, M.d_out, 0, nullptr, nullptr, d_logprob, stream);
 }
 

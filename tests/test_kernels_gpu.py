@@ -440,6 +440,44 @@ def test_sampler_top_p_matches_oracle(T, V):
             assert got[t] == int(np.argmax(lg[t]))
 
 
+@pytest.mark.parametrize("V,ld", [(1, 1), (3, 7), (130, 131), (16384, 16384), (16385, 16388), (65536, 65537), (131073, 131076),
+                                  (262144, 262144), (262145, 262145)])
+def test_sampler_row_sizes(V, ld):
+    """Rows at the edges of the cluster sampler's register sizes (16384 logits per float4 of a thread), rows that do not start on 16
+    bytes, and one row more than it takes: draws of the oracle, argmax and log-probability against float64; a second call repeats
+    the first bit for bit.  A draw may differ where u * kept is within fp32 noise of an edge: at most one of the rows."""
+    T = 6
+    rng = np.random.default_rng(V)
+    full = np.full((T, ld), 1e9, np.float32)  # the padding behind a row must not be read as logits
+    lg = (rng.standard_normal((T, V)) * 2.0).astype(np.float32)
+    if V > 100:
+        lg[:, 17] = -np.inf
+    full[:, :V] = lg
+    temps = np.array([0.0, 0.7, 1.0, 1.3, 0.9, 0.0], np.float32)
+    tps = np.array([0.5, 0.5, 0.9, 1.0, 0.05, 1.0], np.float32)
+    seeds, steps = rng.integers(0, 2 ** 40, T).astype(np.uint64), rng.integers(0, 100, T).astype(np.uint64)
+    dl, dt, dp = dev_f32(full), dev_f32(temps), dev_f32(tps)
+    ds, dst = (torch.from_numpy(a.view(np.int64)).to(DEV) for a in (seeds, steps))
+    runs = []
+    for _ in range(2):
+        out, lp = G.zeros(T, dtype=torch.int32, device=DEV), G.zeros(T, dtype=torch.float32, device=DEV)
+        check(lib().dis_k_sample(ptr(dl), ld, T, V, ptr(dt), ptr(dp), ptr(ds), ptr(dst), ptr(out), ptr(lp), None))
+        sync()
+        runs.append((out.cpu().numpy(), lp.cpu().numpy()))
+    assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
+    got, lp = runs[0]
+    off = 0
+    for t in range(T):
+        z = lg[t].astype(np.float64) / (float(temps[t]) if temps[t] > 0 else 1.0)
+        want = z[got[t]] - (np.log(np.exp(z - z.max()).sum()) + z.max())
+        assert abs(float(lp[t]) - want) <= 1e-4 * max(1.0, abs(want)), (t, float(lp[t]), want)
+        if temps[t] == 0:
+            assert got[t] == int(np.argmax(lg[t]))
+        else:
+            off += got[t] != O.sample(lg[t], float(temps[t]), float(tps[t]), int(seeds[t]), int(steps[t]))[0]
+    assert off <= 1, off
+
+
 @pytest.mark.parametrize("tp,T,V", [(1, 48, 4099), (1, 32, 128256), (2, 48, 4100), (3, 20, 4098), (4, 24, 128256), (8, 16, 128256)],
                          ids=["single-rank-ragged-vocab", "single-rank-llama3-vocab", "tp2-small-vocab", "tp3-small-vocab",
                               "tp4-llama3-vocab", "tp8-llama3-vocab"])
