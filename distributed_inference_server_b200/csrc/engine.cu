@@ -213,7 +213,7 @@ int Engine::init(const dis_engine_config *c) {
   seqs.resize((size_t)max_batch);
   slot_stamp.assign((size_t)max_batch, 0);
   use_pdl = !(c->flags & DIS_FLAG_NO_PDL);
-  pf_block = attn_prefill_block_tokens(nh_l, nkv_l, m.head_dim);
+  pf_block = attn_prefill_full_block(nh_l, nkv_l, m.head_dim);
   pf_tc = attn_prefill_uses_tc(nh_l, nkv_l, m.head_dim);
   if (const char *g = getenv("DIS_GEMM_PERSIST")) use_persist = atoi(g) != 0;
   if (const char *g = getenv("DIS_GEMV_MAX_T")) gemv_max_t = std::max(0, std::min(kGemvMaxT, atoi(g)));

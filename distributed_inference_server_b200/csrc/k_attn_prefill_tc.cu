@@ -3,19 +3,13 @@
 // No reference counterpart (the reference has no tensor code at all).
 //
 // One CTA = (query block, kv head).  A query block is up to QT = 128 / G consecutive tokens of one sequence
-// (G = query heads per kv head: 32 tokens for Llama-3-8B's 4:1 GQA, 16 for 70B's 8:1); its G heads x QT tokens
+// (G = query heads per kv head: 32 tokens for Llama-3-8B's 4:1 GQA, 16 for 70B's and TinyLlama's 8:1); its G heads x QT tokens
 // are the 128 rows (= 128 TMEM lanes) of every MMA, row = head * QT + token, so K and V are fetched once per
-// 128 query rows instead of once per 64 as in the mma.sync kernel (k_attn_paged.cu), and the QK^T / PV
-// products run at tcgen05 rate instead of through ldmatrix + mma.sync.
+// 128 query rows and the QK^T / PV products run at tcgen05 rate instead of through ldmatrix + mma.sync
+// (k_attn_paged.cu).  Tensor- and exponential-bound: 4 * rows * keys * d flop and rows * keys exponentials per (block, kv head).
 //
-//   warp 0      TMA producer: 64-key K/V tiles (128B-swizzled boxes out of the page pool) into a 3-stage ring
-//   warp 1      one thread issues the MMAs:   S_j   = Q   K_j^T   M128 N64  K16 x 8   (A, B K-major)       -> TMEM S[j&1]
-//                                             O_j   = P_j V_j     M128 N128 K16 x 4   (B = V, MN-major)    -> TMEM O[j&1]
-//   warps 2-5   one thread per row: S_j from TMEM, scale, causal mask, running max / sum (no shuffles: a thread
-//               owns a whole row), P_j = exp2(s - m) as bf16 into shared memory (the A operand of the PV MMA),
-//               then O_{j-1} from TMEM into the fp32 accumulator it keeps in registers: acc = acc * corr + O_{j-1}
-// S, P and O are double-buffered, so the tensor pipe computes S_{j+1} while the softmax of tile j runs and
-// P_j V_j while the row threads fold O_{j-1}.  Tensor-bound: 4 * rows * keys * 128 flop per (block, kv head).
+// Heads of 128: attn_prefill_tc2_kernel, one softmax group per CTA, P through shared memory.  Heads of 64:
+// attn_prefill_tc3_kernel, two softmax groups per CTA on alternate key tiles, P in TMEM.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -28,14 +22,10 @@ namespace dis {
 
 constexpr int kPfThreads = 192;
 constexpr int kPfTile = 64;    // keys per stage
-constexpr int kPfStages = 3;
 constexpr int kPfD = 128;
 constexpr int kPfHalf = kPfTile * 128;                  // one [64 keys][64 dims] block, 8 KB
-constexpr int kPfStageBytes = 4 * kPfHalf;               // K halves + V halves, 32 KB
 constexpr int kPfQBytes = 2 * 128 * 128;                 // Q: two [128 rows][64 dims] halves, 32 KB
 constexpr int kPfPBytes = 128 * 128;                     // P: [128 rows][64 keys] bf16, 16 KB
-constexpr int kPfSmemBytes = kPfQBytes + kPfStages * kPfStageBytes + 2 * kPfPBytes + 256 + 1024;
-constexpr int kPfTmemCols = 512;                         // S0 | S1 (64 each) | O0 | O1 (128 each)
 
 // shared-memory matrix descriptor, MN-major operand, 128B swizzle: element (mn, k) lives at
 //   (mn % 64) * 2 + (mn / 64) * LBO + (k % 8) * 128 + (k / 8) * SBO   -- the [keys][dims] V tile as TMA stores it
@@ -50,225 +40,14 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-template <int G>
-__global__ void __launch_bounds__(kPfThreads, 1)
-attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const uint16_t *__restrict__ q,
-                       const int *__restrict__ page_table, int max_pages, const int *__restrict__ qb_tok0,
-                       const int *__restrict__ qb_len, const int *__restrict__ qb_pos0, const int *__restrict__ qb_ptrow,
-                       uint16_t *__restrict__ out, int n_heads, int n_kv, int page_shift) {
-  constexpr int QT = 128 / G;  // tokens per query block
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t q_base = smem_base;
-  const uint32_t kv_base = q_base + kPfQBytes;
-  const uint32_t p_base = kv_base + kPfStages * kPfStageBytes;
-  const uint32_t bar_base = p_base + 2 * kPfPBytes;
-  auto kv_full = [&](int s) { return bar_base + 8u * s; };
-  auto kv_empty = [&](int s) { return bar_base + 8u * (kPfStages + s); };
-  auto s_full = [&](int b) { return bar_base + 8u * (2 * kPfStages + b); };
-  auto p_full = [&](int b) { return bar_base + 8u * (2 * kPfStages + 2 + b); };
-  auto o_full = [&](int b) { return bar_base + 8u * (2 * kPfStages + 4 + b); };
-  const uint32_t tmem_slot = bar_base + 8u * (2 * kPfStages + 6);
-
-  const int qb = blockIdx.x, kvh = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&kv_map);
-    for (int s = 0; s < kPfStages; s++) { mbar_init(kv_full(s), 1); mbar_init(kv_empty(s), 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(s_full(b), 1); mbar_init(p_full(b), 128); mbar_init(o_full(b), 1); }
-    fence_barrier_init();
-    fence_proxy_async();
-  }
-  if (warp == 1) tmem_alloc<kPfTmemCols>(tmem_slot);
-  pdl_launch_dependents();
-  pdl_wait();  // q and this chunk's K/V rows come from the previous kernels
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  uint32_t tmem_base;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-
-  const int tok0 = qb_tok0[qb], len = qb_len[qb], pos0 = qb_pos0[qb];
-  const int *pt = page_table + (size_t)qb_ptrow[qb] * max_pages;
-  const int page_size = 1 << page_shift;
-  const int box_rows = min(page_size, kPfTile);
-  const int end = pos0 + len;  // keys [0, end)
-  const int n_tiles = (end + kPfTile - 1) / kPfTile;
-
-  // ---- Q tile: row = head * QT + token, K-major, 128B swizzle (rows of padding tokens are zero)
-  if (warp >= 2) {
-    const int row = (warp & 3) * 32 + lane;
-    const int hl = row / QT, t = row % QT;
-    const uint4 *src = reinterpret_cast<const uint4 *>(q + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * kPfD);
-#pragma unroll
-    for (int c = 0; c < 16; c++) {
-      const uint4 v = t < len ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-      const uint32_t off = (uint32_t)(c >> 3) * (128 * 128) + (uint32_t)(row >> 3) * 1024 + (uint32_t)(row & 7) * 128 +
-                           (uint32_t)(((c & 7) ^ (row & 7)) << 4);
-      *reinterpret_cast<uint4 *>(smem + off) = v;
-    }
-    fence_proxy_async();
-  }
-  __syncthreads();
-
-  if (warp == 0) {
-    // ===== TMA producer =====
-    if (lane == 0) {
-      for (int tile = 0; tile < n_tiles; tile++) {
-        const int stage = tile % kPfStages;
-        if (tile >= kPfStages) mbar_wait(kv_empty(stage), (uint32_t)(tile / kPfStages - 1) & 1u);
-        const uint32_t sbase = kv_base + stage * kPfStageBytes;
-        mbar_expect_tx(kv_full(stage), kPfStageBytes);
-        for (int r = 0; r < kPfTile; r += box_rows) {
-          const int pos = tile * kPfTile + r;
-          const long long page = pt[min(pos >> page_shift, max_pages - 1)];
-          const long long krow = row0 + ((page * 2 + 0) * n_kv + kvh) * page_size + (pos & (page_size - 1));
-          const long long vrow = krow + (long long)n_kv * page_size;
-#pragma unroll
-          for (int hh = 0; hh < 2; hh++) {
-            tma_load_2d(sbase + hh * kPfHalf + r * 128, &kv_map, hh * 64, (int)krow, kv_full(stage), kEvictLast);
-            tma_load_2d(sbase + (2 + hh) * kPfHalf + r * 128, &kv_map, hh * 64, (int)vrow, kv_full(stage), kEvictLast);
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ===== MMA issuer (one thread) =====
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc<kPfTile>();              // M128 N64, A and B K-major
-      constexpr uint32_t idesc_o = umma_idesc<kPfD>() | (1u << 16);    // M128 N128, B (= V) MN-major
-      auto issue_s = [&](int j) {
-        const int stage = j % kPfStages;
-        mbar_wait(kv_full(stage), (uint32_t)(j / kPfStages) & 1u);
-        tc_fence_after();
-        const uint32_t kb = kv_base + stage * kPfStageBytes;
-#pragma unroll
-        for (int k = 0; k < kPfD / 16; k++) {
-          const uint32_t a = q_base + (k >> 2) * (128 * 128) + (k & 3) * 32;
-          const uint32_t b = kb + (k >> 2) * kPfHalf + (k & 3) * 32;
-          umma_bf16(tmem_base + (uint32_t)(j & 1) * kPfTile, umma_desc_sw128(a), umma_desc_sw128(b), idesc_s, k > 0 ? 1u : 0u);
-        }
-        umma_commit(s_full(j & 1));
-      };
-      auto issue_o = [&](int j) {
-        const int stage = j % kPfStages;
-        mbar_wait(p_full(j & 1), (uint32_t)(j >> 1) & 1u);
-        tc_fence_after();
-        const uint32_t vb = kv_base + stage * kPfStageBytes + 2 * kPfHalf;
-        const uint32_t pb = p_base + (j & 1) * kPfPBytes;
-#pragma unroll
-        for (int k = 0; k < kPfTile / 16; k++)
-          umma_bf16(tmem_base + 2 * kPfTile + (uint32_t)(j & 1) * kPfD, umma_desc_sw128(pb + k * 32),
-                    umma_desc_mn_sw128(vb + k * 2048, kPfHalf, 1024), idesc_o, k > 0 ? 1u : 0u);
-        umma_commit(o_full(j & 1));
-        umma_commit(kv_empty(stage));  // K_j was read by S_j, V_j by this product: the stage may be refilled
-      };
-      issue_s(0);
-      for (int j = 0; j < n_tiles; j++) {
-        if (j + 1 < n_tiles) issue_s(j + 1);
-        issue_o(j);
-      }
-    }
-  } else {
-    // ===== softmax + O accumulation: one thread per row =====
-    const int quarter = warp & 3;  // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
-    const int row = quarter * 32 + lane;
-    const int hl = row / QT, t = row % QT;
-    const int qp = pos0 + t;  // this row's query position
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const float scale_log2 = rsqrtf((float)kPfD) * 1.4426950408889634f;
-    float acc[kPfD];
-#pragma unroll
-    for (int i = 0; i < kPfD; i++) acc[i] = 0.f;
-    float m_run = -INFINITY, l_run = 0.f, corr_prev = 1.f;
-    auto fold_o = [&](int j, float corr) {  // acc = acc * corr + O_j
-      mbar_wait(o_full(j & 1), (uint32_t)(j >> 1) & 1u);
-      tc_fence_after();
-#pragma unroll
-      for (int c = 0; c < kPfD; c += 32) {
-        uint32_t v[32];
-        tmem_ld_32x32(lane_addr + 2 * kPfTile + (uint32_t)(j & 1) * kPfD + c, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; i++) acc[c + i] = fmaf(acc[c + i], corr, __uint_as_float(v[i]));
-      }
-    };
-    for (int j = 0; j < n_tiles; j++) {
-      mbar_wait(s_full(j & 1), (uint32_t)(j >> 1) & 1u);
-      tc_fence_after();
-      uint32_t s0[32], s1[32];
-      tmem_ld_32x32(lane_addr + (uint32_t)(j & 1) * kPfTile, s0);
-      tmem_ld_32x32(lane_addr + (uint32_t)(j & 1) * kPfTile + 32, s1);
-      tmem_ld_wait();
-      const int tile0 = j * kPfTile;
-      // One warp per scheduler runs this loop, so its length in instructions IS the kernel's time (ncu: 1060 warp
-      // instructions per 64-key tile before this diet, tensor pipe 21 % busy): the causal mask is applied only on the
-      // tiles that cross the diagonal, the scale is folded into the exponent's FMA, ex2.approx is issued directly.
-      float mx = -INFINITY;
-      if (tile0 + kPfTile - 1 > qp) {
-#pragma unroll
-        for (int i = 0; i < 32; i++) {
-          if (tile0 + i > qp) s0[i] = 0xff800000u;        // -inf
-          if (tile0 + 32 + i > qp) s1[i] = 0xff800000u;
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 32; i++) mx = fmaxf(mx, fmaxf(__uint_as_float(s0[i]), __uint_as_float(s1[i])));
-      const float m_new = fmaxf(m_run, mx * scale_log2);   // scale > 0: the max commutes with it; finite from tile 0 on
-      const float corr = ex2_approx(m_run - m_new);        // 0 at the first tile (m_run = -inf)
-      const float neg_m = -m_new;
-      float ps0 = 0.f, ps1 = 0.f;
-      uint8_t *prow = smem + (p_base - smem_base) + (j & 1) * kPfPBytes + (row >> 3) * 1024 + (row & 7) * 128;
-#pragma unroll
-      for (int c = 0; c < 8; c++) {  // 8 keys = one 16-byte chunk of the swizzled row
-        uint32_t pk[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int i = c * 8 + e * 2;
-          const float p0 = ex2_approx(fmaf(__uint_as_float(i < 32 ? s0[i] : s1[i - 32]), scale_log2, neg_m));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(i + 1 < 32 ? s0[i + 1] : s1[i + 1 - 32]), scale_log2, neg_m));
-          ps0 += p0; ps1 += p1;
-          pk[e] = float2_to_bf16x2(p0, p1);
-        }
-        *reinterpret_cast<uint4 *>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-      }
-      const float ps = ps0 + ps1;
-      l_run = l_run * corr + ps;
-      m_run = m_new;
-      fence_proxy_async();   // the PV MMA reads P through the async proxy
-      tc_fence_before();     // ... and this thread's TMEM reads of S_j are done before the issuer reuses the buffer
-      mbar_arrive(p_full(j & 1));
-      if (j > 0) fold_o(j - 1, corr_prev);
-      corr_prev = corr;
-    }
-    fold_o(n_tiles - 1, corr_prev);
-    if (t < len) {
-      const float inv = 1.0f / l_run;
-      uint4 *o = reinterpret_cast<uint4 *>(out + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * kPfD);
-#pragma unroll
-      for (int c = 0; c < 16; c++) {
-        uint4 v;
-        v.x = float2_to_bf16x2(acc[c * 8 + 0] * inv, acc[c * 8 + 1] * inv);
-        v.y = float2_to_bf16x2(acc[c * 8 + 2] * inv, acc[c * 8 + 3] * inv);
-        v.z = float2_to_bf16x2(acc[c * 8 + 4] * inv, acc[c * 8 + 5] * inv);
-        v.w = float2_to_bf16x2(acc[c * 8 + 6] * inv, acc[c * 8 + 7] * inv);
-        o[c] = v;
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc<kPfTmemCols>(tmem_base);
-}
-
 // ---------------------------------------------------------------------------------------- two CTAs per SM
-// ncu on the kernel above (profiles/r2_attn_prefill_tc_full.txt): tensor pipe 21 % busy, XU 22 %, one warp per scheduler
-// walking ~1000 dependent instructions per 64-key tile -- it is bound by the latency of its own instruction stream, and
-// 237 registers + 512 TMEM columns + 165 KB of shared memory allow one CTA per SM.  This variant is built to fit TWO:
-//   * O stays in TMEM and accumulates there over the tiles (tcgen05.mma accumulate), so the 128-register accumulator and
-//     the 128 FMAs + TMEM reads of the per-tile fold are gone.  The softmax reference m_ref is only raised when the running
+// Built to fit TWO CTAs per SM, one's MMAs under the other's softmax:
+//   warp 0      TMA producer: 64-key K/V tiles (128B-swizzled boxes out of the page pool)
+//   warp 1      one thread issues the MMAs:   S_j   = Q   K_j^T   M128 N64  K16 x 8   (A, B K-major)       -> TMEM S[j&1]
+//                                             O    += P_j V_j     M128 N128 K16 x 4   (B = V, MN-major)    -> TMEM O
+//   warps 2-5   one thread per row: S_j from TMEM, scale, causal mask, running max / sum (no shuffles: a thread
+//               owns a whole row), P_j = exp2(s - m) as bf16 into shared memory (the A operand of the PV MMA)
+//   * O stays in TMEM and accumulates there over the tiles (tcgen05.mma accumulate).  The softmax reference m_ref is only raised when the running
 //     maximum exceeds it by more than 8 (log2 domain): P = exp2(s - m_ref) <= 256 stays exact enough in bf16/fp32, the
 //     reference cancels in the final division by l, and the rescale of O (tcgen05.ld, scale, tcgen05.st, warp-uniformly
 //     decided) happens only on the few tiles where a row's maximum still grows;
@@ -524,63 +303,387 @@ attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
   if (warp == 1) tmem_dealloc<kPf2TmemCols>(tmem_base);
 }
 
-// Tokens per query block of the prefill attention for this head geometry: 128 / G on the tcgen05 kernel
-// (head_dim 128, GQA group 4 or 8), 16 on the mma.sync kernel.  DIS_ATTN_PREFILL=mma forces the latter (A/B runs).
-static int prefill_variant() {  // 0: mma.sync kernel, 1: tcgen05 with O folded in registers, 2: tcgen05, two CTAs per SM
+// ---------------------------------------------------------------------------------------- two softmax groups, P in TMEM
+constexpr int kPf3Threads = 320;
+constexpr int kPf3QHalf = 128 * 128;  // one [128 rows][64 dims] block of Q, 16 KB
+
+template <int D>
+constexpr int pf3_smem_bytes() { return (D / 64) * (kPf3QHalf + 4 * kPfHalf) + 3 * 128 * 4 + 256; }
+
+// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes x 16 bf16, two per column
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// Packed pairs: one issue slot for two lanes' worth of work
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+// producer-consumer barriers of a pair of warps: one arrives, the other waits
+__device__ __forceinline__ void named_sync_64(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void named_arrive_64(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+
+__device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// O's 32 columns from o_addr on, times f (a warp-collective read, scale and write back), eight at a time: it runs on few tiles, with the
+// scores of the tile live.
+__device__ __forceinline__ void rescale_32(uint32_t o_addr, float f) {
+#pragma unroll
+  for (int c = 0; c < 32; c += 8) {
+    uint32_t v[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(o_addr + c)
+                 : "memory");
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"r"(o_addr + c), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+  }
+}
+
+//   warp 0      TMA producer, as above
+//   warp 1      one thread issues S_j = Q K_j^T (M128 N64) and O += P_j V_j (M128 N=D, A = P from TMEM, B = V MN-major)
+//   warps 2-5   softmax of the even tiles, warps 6-9 of the odd ones, one thread per row; P_j = exp2(s - m) goes as packed bf16 back
+//               into S_j's own TMEM columns (no shared-memory write, proxy fence or second read of it)
+// TMEM per CTA: S0 | S1 64 columns each | O D columns; two CTAs per SM, so four softmax groups take turns on the exponentials (16 per
+// clock and SM, what bounds heads of 64: 1024 clocks per 128 rows x 128 keys against 512 of the tensor pipe).  The two groups share a
+// row's reference, handed from tile to tile through shared memory and raised lazily as above.
+// Heads of 64, six prompts of 276 to 1900 tokens, 32 / 4 heads (31.6 GFLOP): 164 us on the mma.sync kernel of k_attn_paged.cu, 89 us here.
+// Heads of 128 stay above: 382 us here against 367 us (six prompts of 437 to 3000 tokens, 32 / 8 heads, 258 GFLOP).
+template <int D, int G>
+__global__ void __launch_bounds__(kPf3Threads, 2)
+attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const uint16_t *__restrict__ q,
+                        const int *__restrict__ page_table, int max_pages, const int *__restrict__ qb_tok0,
+                        const int *__restrict__ qb_len, const int *__restrict__ qb_pos0, const int *__restrict__ qb_ptrow,
+                        uint16_t *__restrict__ out, int n_heads, int n_kv, int page_shift) {
+  constexpr int QT = 128 / G;
+  constexpr int kHalves = D / 64;
+  constexpr uint32_t kSlot = kHalves * kPfHalf;  // one K or V tile
+  extern __shared__ __align__(1024) uint8_t smem_al[];
+  const uint32_t smem_base = smem_u32(smem_al);
+  if (smem_base & 1023u) __trap();  // the 128B-swizzle atoms need 1024-byte alignment and there is no room for slack
+  uint8_t *smem = smem_al;
+  const uint32_t q_base = smem_base, k_base = q_base + kHalves * kPf3QHalf, v_base = k_base + 2 * kSlot;
+  const uint32_t bar_base = v_base + 2 * kSlot;
+  auto k_full = [&](int w) { return bar_base + 8u * w; };
+  auto k_empty = [&](int w) { return bar_base + 16u + 8u * w; };
+  auto v_full = [&](int w) { return bar_base + 32u + 8u * w; };
+  auto s_full = [&](int w) { return bar_base + 48u + 8u * w; };
+  auto p_full = [&](int w) { return bar_base + 64u + 8u * w; };
+  auto pv_done = [&](int w) { return bar_base + 80u + 8u * w; };
+  const uint32_t tmem_slot = bar_base + 96;
+  float *m_row = reinterpret_cast<float *>(smem + (bar_base - smem_base) + 256);  // [row]: the softmax reference, handed from tile to tile
+  float *l_row = m_row + 128;                                                     // [group][row]: at the end
+
+  // later query blocks of a sequence have more key tiles: launch them first, so that the longest CTAs do not form the tail
+  const int qb = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&kv_map);
+    for (int w = 0; w < 2; w++) {
+      mbar_init(k_full(w), 1); mbar_init(k_empty(w), 1); mbar_init(v_full(w), 1); mbar_init(s_full(w), 1); mbar_init(pv_done(w), 1);
+      mbar_init(p_full(w), 4);
+    }
+    fence_barrier_init();
+    fence_proxy_async();
+  }
+  if (warp == 1) tmem_alloc<kPf2TmemCols>(tmem_slot);
+  pdl_launch_dependents();
+  pdl_wait();  // q and this chunk's K/V rows come from the previous kernels
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem_base;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+  const uint32_t o_base = tmem_base + 2 * kPfTile;
+
+  const int tok0 = qb_tok0[qb], len = qb_len[qb], pos0 = qb_pos0[qb];
+  const int *pt = page_table + (size_t)qb_ptrow[qb] * max_pages;
+  const int page_size = 1 << page_shift;
+  const int box_rows = min(page_size, kPfTile);  // rows of the tensor map's box
+  const int end = pos0 + len;                    // keys [0, end)
+  const int n_tiles = (end + kPfTile - 1) / kPfTile;
+
+  if (warp >= 2) {  // Q tile: row = head * QT + token, K-major, 128B swizzle (rows of padding tokens are zero)
+    const int row = (warp & 3) * 32 + lane, grp = (warp - 2) >> 2;
+    const int hl = row / QT, t = row % QT;
+    const uint4 *src = reinterpret_cast<const uint4 *>(q + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * D);
+#pragma unroll
+    for (int cc = 0; cc < D / 16; cc++) {
+      const int c = grp * (D / 16) + cc;
+      const uint4 v = t < len ? src[c] : make_uint4(0u, 0u, 0u, 0u);
+      const uint32_t off = (uint32_t)(c >> 3) * kPf3QHalf + (uint32_t)(row >> 3) * 1024 + (uint32_t)(row & 7) * 128 +
+                           (uint32_t)(((c & 7) ^ (row & 7)) << 4);
+      *reinterpret_cast<uint4 *>(smem + off) = v;
+    }
+    fence_proxy_async();
+  }
+  __syncthreads();
+
+  if (warp == 0) {
+    // ===== TMA producer: K_t as soon as S_{t-2} has read its slot, V_t as soon as P_{t-2} V_{t-2} has =====
+    if (lane == 0) {
+      const int last_box = (end - 1) / box_rows * box_rows;
+      auto load = [&](int tile, bool is_v) {
+        const int w = tile & 1;
+        const uint32_t full = is_v ? v_full(w) : k_full(w);
+        if (tile >= 2) mbar_wait(is_v ? pv_done(w) : k_empty(w), (uint32_t)(tile / 2 - 1) & 1u);
+        const uint32_t sbase = (is_v ? v_base : k_base) + w * kSlot;
+        mbar_expect_tx(full, kSlot);
+        for (int r = 0; r < kPfTile; r += box_rows) {
+          // Boxes past the last key repeat the last one that holds a key: their scores are masked, and their values must be
+          // finite because they are multiplied by a weight of zero.
+          const int pos = min(tile * kPfTile + r, last_box);
+          const long long page = pt[pos >> page_shift];
+          const long long krow = row0 + ((page * 2 + (is_v ? 1 : 0)) * n_kv + kvh) * page_size + (pos & (page_size - 1));
+#pragma unroll
+          for (int hh = 0; hh < kHalves; hh++) tma_load_2d(sbase + hh * kPfHalf + r * 128, &kv_map, hh * 64, (int)krow, full, kEvictLast);
+        }
+      };
+      for (int t = 0; t <= n_tiles; t++) {
+        if (t < n_tiles) load(t, false);
+        if (t >= 1) load(t - 1, true);
+      }
+    }
+  } else if (warp == 1) {
+    // ===== MMA issuer (one thread) =====
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = umma_idesc<kPfTile>();
+      constexpr uint32_t idesc_o = umma_idesc<D>() | (1u << 16);  // B (= V) MN-major
+      auto issue_s = [&](int j) {
+        const int w = j & 1;
+        mbar_wait(k_full(w), (uint32_t)(j >> 1) & 1u);
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < D / 16; k++)
+          umma_bf16(tmem_base + w * kPfTile, umma_desc_sw128(q_base + (k >> 2) * kPf3QHalf + (k & 3) * 32),
+                    umma_desc_sw128(k_base + w * kSlot + (k >> 2) * kPfHalf + (k & 3) * 32), idesc_s, k > 0 ? 1u : 0u);
+        umma_commit(s_full(w));
+        umma_commit(k_empty(w));
+      };
+      issue_s(0);
+      if (n_tiles > 1) issue_s(1);
+      for (int j = 0; j < n_tiles; j++) {
+        const int w = j & 1;
+        mbar_wait(v_full(w), (uint32_t)(j >> 1) & 1u);
+        mbar_wait(p_full(w), (uint32_t)(j >> 1) & 1u);
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < kPfTile / 16; k++)
+          umma_bf16_ts(o_base, tmem_base + w * kPfTile + 8 * k, umma_desc_mn_sw128(v_base + w * kSlot + k * 2048, kPfHalf, 1024), idesc_o,
+                       (j > 0 || k > 0) ? 1u : 0u);
+        umma_commit(pv_done(w));
+        if (j + 2 < n_tiles) {
+          mbar_wait(pv_done(w), (uint32_t)(j >> 1) & 1u);  // S_{j+2} overwrites the columns that P_j V_j reads
+          issue_s(j + 2);
+        }
+      }
+    }
+  } else {
+    // ===== softmax: group 0 takes the even tiles, group 1 the odd ones; one thread per row; O lives in TMEM =====
+    const int quarter = warp & 3;  // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
+    const int grp = (warp - 2) >> 2;
+    const int row = quarter * 32 + lane;
+    const int hl = row / QT, t = row % QT;
+    const int qp = pos0 + t;
+    const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+    const uint32_t s_addr = tmem_base + lane_off + grp * kPfTile, o_addr = o_base + lane_off;
+    const int bar_in = 1 + 4 * grp + quarter, bar_out = 1 + 4 * (grp ^ 1) + quarter;  // hand-over of m_row to this group / to the other
+    const float scale_log2 = rsqrtf((float)D) * 1.4426950408889634f;
+    const float2 scale2 = make_float2(scale_log2, scale_log2);
+    float m_ref = -INFINITY, l_run = 0.f;
+    for (int j = grp; j < n_tiles; j += 2) {
+      mbar_wait(s_full(grp), (uint32_t)(j >> 1) & 1u);
+      tc_fence_after();
+      uint32_t s[2][32];
+      tmem_ld_32x32(s_addr, s[0]);
+      tmem_ld_32x32(s_addr + 32, s[1]);
+      tmem_ld_wait();
+      const int rest = qp - j * kPfTile;  // keys 0 .. rest of the tile are visible
+      if (rest < kPfTile - 1) {           // only the tiles that cross the diagonal need the causal mask
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+#pragma unroll
+          for (int i = 0; i < 32; i++)
+            if (32 * c + i > rest) s[c][i] = 0xff800000u;
+      }
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int i = 0; i < 32; i++) mx4[i & 3] = max3(mx4[i & 3], __uint_as_float(s[0][i]), __uint_as_float(s[1][i]));
+      const float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3])) * scale_log2;  // scale > 0: it commutes with the maximum
+      float m_now;
+      if (j == 0) {
+        m_now = mx;  // finite: key 0 is visible to every query; O is first written by P_0 V_0 (accumulate off)
+      } else {
+        named_sync_64(bar_in);
+        const float m_old = m_row[row];
+        const bool need = mx > m_old + kPf2Lazy;
+        m_now = need ? mx : m_old;
+        if (__any_sync(0xffffffffu, need)) {  // tcgen05.ld / st are warp-collective: decide per warp, scale per lane
+          // every P V so far must be in O; none follows before this tile's P is handed over
+          mbar_wait(pv_done(grp ^ 1), (uint32_t)((j - 1) >> 1) & 1u);
+          tc_fence_after();
+          const float f = need ? ex2_approx(m_old - mx) : 1.0f;
+#pragma unroll 1
+          for (int c = 0; c < D; c += 32) rescale_32(o_addr + c, f);
+          tmem_st_wait();
+        }
+      }
+      if (j + 1 < n_tiles) {
+        m_row[row] = m_now;
+        named_arrive_64(bar_out);
+      }
+      l_run *= ex2_approx(m_ref - m_now);  // what this group has summed so far, under the reference of now (0 at its first tile)
+      m_ref = m_now;
+      const float2 neg_m = make_float2(-m_ref, -m_ref);
+      float2 ps[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float2 p = fma2(make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), scale2, neg_m);
+          p.x = ex2_approx(p.x);
+          p.y = ex2_approx(p.y);
+          ps[(i >> 1) & 1] = add2(ps[(i >> 1) & 1], p);
+          pk[i >> 1] = float2_to_bf16x2(p.x, p.y);
+        }
+        tmem_st_32x16(s_addr + 16 * c, pk);
+      }
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full(grp));
+      l_run += (ps[0].x + ps[0].y) + (ps[1].x + ps[1].y);
+    }
+    // the group of the last tile publishes the final reference; then each brings its sum to it
+    if (grp == ((n_tiles - 1) & 1)) m_row[row] = m_ref;
+    asm volatile("bar.sync 9, 256;" ::: "memory");
+    l_row[grp * 128 + row] = l_run * ex2_approx(m_ref - m_row[row]);
+    asm volatile("bar.sync 9, 256;" ::: "memory");
+    const float inv = 1.0f / (l_row[row] + l_row[128 + row]);
+    mbar_wait(pv_done((n_tiles - 1) & 1), (uint32_t)((n_tiles - 1) >> 1) & 1u);
+    tc_fence_after();
+    uint4 *o = reinterpret_cast<uint4 *>(out + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * D);
+#pragma unroll
+    for (int cc = 0; cc < D / 2; cc += 32) {
+      const int c = grp * (D / 2) + cc;
+      uint32_t v[32];
+      tmem_ld_32x32(o_addr + c, v);
+      tmem_ld_wait();
+      if (t < len) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          uint4 w;
+          w.x = float2_to_bf16x2(__uint_as_float(v[i * 8 + 0]) * inv, __uint_as_float(v[i * 8 + 1]) * inv);
+          w.y = float2_to_bf16x2(__uint_as_float(v[i * 8 + 2]) * inv, __uint_as_float(v[i * 8 + 3]) * inv);
+          w.z = float2_to_bf16x2(__uint_as_float(v[i * 8 + 4]) * inv, __uint_as_float(v[i * 8 + 5]) * inv);
+          w.w = float2_to_bf16x2(__uint_as_float(v[i * 8 + 6]) * inv, __uint_as_float(v[i * 8 + 7]) * inv);
+          o[c / 8 + i] = w;
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc<kPf2TmemCols>(tmem_base);
+}
+
+// DIS_ATTN_PREFILL=mma sends every geometry to the mma.sync kernel of k_attn_paged.cu (A/B runs).
+static bool prefill_tc_enabled() {
   static int v = -1;
   if (v < 0) {
     const char *e = getenv("DIS_ATTN_PREFILL");
-    v = !e ? 2 : (!strcmp(e, "mma") ? 0 : (!strcmp(e, "tc1") ? 1 : 2));
+    v = e && !strcmp(e, "mma") ? 0 : 1;
   }
-  return v;
+  return v != 0;
 }
-static bool prefill_tc_enabled() { return prefill_variant() != 0; }
 
+// Head sizes 128 and 64 with groups of 4 or 8 query heads per kv head.  Smaller groups stay on the mma.sync kernel: its blocks
+// of 16 tokens would fill 16 or 32 of the 128 rows.
 bool attn_prefill_uses_tc(int n_heads, int n_kv, int d) {
   if (n_kv <= 0 || n_heads % n_kv != 0) return false;
   const int G = n_heads / n_kv;
-  return prefill_tc_enabled() && d == kPfD && (G == 4 || G == 8);
+  return prefill_tc_enabled() && (d == 128 || d == 64) && (G == 4 || G == 8);
 }
 
+// Most tokens a caller of the C ABI may put into one query block: 128 / G for heads of 128, 16 otherwise.
 int attn_prefill_block_tokens(int n_heads, int n_kv, int d) {
+  return d == 128 && attn_prefill_uses_tc(n_heads, n_kv, d) ? 128 / (n_heads / n_kv) : 16;
+}
+// The engine's own blocks: what the kernel takes.
+int attn_prefill_full_block(int n_heads, int n_kv, int d) {
   return attn_prefill_uses_tc(n_heads, n_kv, d) ? 128 / (n_heads / n_kv) : 16;
 }
 
-template <int G>
-static cudaError_t prefill_tc_launch(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,
-                                     int max_pages, const int *qb_tok0, const int *qb_len, const int *qb_pos0,
-                                     const int *qb_ptrow, uint16_t *out, int n_blocks, int n_heads, int n_kv,
-                                     int page_shift, cudaStream_t st) {
-  static DeviceOnce once;
+template <class K>
+static cudaError_t prefill_tc_launch(K kern, int threads, int smem, DeviceOnce &once, const TmaMap &kv_map, long long row0, const uint16_t *q,
+                                     const int *page_table, int max_pages, const int *qb_tok0, const int *qb_len, const int *qb_pos0,
+                                     const int *qb_ptrow, uint16_t *out, int n_blocks, int n_heads, int n_kv, int page_shift,
+                                     cudaStream_t st) {
   DIS_CUDA_TRY(once.run([&] {
-    cudaError_t e = cudaFuncSetAttribute(attn_prefill_tc_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPfSmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_prefill_tc2_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPf2SmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_prefill_tc2_kernel<G>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     return e;
   }));
-  if (prefill_variant() == 2)
-    return launch_k(attn_prefill_tc2_kernel<G>, dim3(n_blocks, n_kv), dim3(kPfThreads), (size_t)kPf2SmemBytes, st,
-                    *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0,
-                    qb_ptrow, out, n_heads, n_kv, page_shift);
-  return launch_k(attn_prefill_tc_kernel<G>, dim3(n_blocks, n_kv), dim3(kPfThreads), (size_t)kPfSmemBytes, st,
-                  *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0,
-                  qb_ptrow, out, n_heads, n_kv, page_shift);
+  return launch_k(kern, dim3(n_blocks, n_kv), dim3(threads), (size_t)smem, st, *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, q,
+                  page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_heads, n_kv, page_shift);
 }
 
-// Same contract as launch_attn_prefill (k_attn_paged.cu) with query blocks of up to attn_prefill_block_tokens() tokens.
+// Same contract as launch_attn_prefill (k_attn_paged.cu) with query blocks of up to 128 / G tokens.
 cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,
                                    int max_pages, const int *qb_tok0, const int *qb_len, const int *qb_pos0,
                                    const int *qb_ptrow, uint16_t *out, int n_blocks, int n_heads, int n_kv, int d,
                                    int page_size, cudaStream_t st) {
   if (n_blocks <= 0) return cudaSuccess;
-  if (n_kv <= 0 || n_heads % n_kv != 0 || n_kv > 65535 || d != kPfD) { set_last_error("attn_prefill_tc: bad head geometry"); return cudaErrorInvalidValue; }
+  if (n_kv <= 0 || n_heads % n_kv != 0 || n_kv > 65535) { set_last_error("attn_prefill_tc: bad head geometry"); return cudaErrorInvalidValue; }
   if (page_size < 8 || (page_size & (page_size - 1))) { set_last_error("attn_prefill_tc: page_size must be a power of two >= 8"); return cudaErrorInvalidValue; }
   int page_shift = 0;
   while ((1 << page_shift) < page_size) page_shift++;
   const int G = n_heads / n_kv;
-  if (G == 4) return prefill_tc_launch<4>(kv_map, row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_blocks, n_heads, n_kv, page_shift, st);
-  if (G == 8) return prefill_tc_launch<8>(kv_map, row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_blocks, n_heads, n_kv, page_shift, st);
-  set_last_error("attn_prefill_tc: the GQA group must be 4 or 8");
+#define DIS_PF_TC_CASE(DD, GG, KERN, THREADS, SMEM)                                                                              \
+  if (d == DD && G == GG) {                                                                                                      \
+    static DeviceOnce once;                                                                                                      \
+    return prefill_tc_launch(KERN, THREADS, SMEM, once, kv_map, row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, \
+                             out, n_blocks, n_heads, n_kv, page_shift, st);                                                      \
+  }
+  DIS_PF_TC_CASE(128, 4, attn_prefill_tc2_kernel<4>, kPfThreads, kPf2SmemBytes)
+  DIS_PF_TC_CASE(128, 8, attn_prefill_tc2_kernel<8>, kPfThreads, kPf2SmemBytes)
+  DIS_PF_TC_CASE(64, 4, (attn_prefill_tc3_kernel<64, 4>), kPf3Threads, pf3_smem_bytes<64>())
+  DIS_PF_TC_CASE(64, 8, (attn_prefill_tc3_kernel<64, 8>), kPf3Threads, pf3_smem_bytes<64>())
+#undef DIS_PF_TC_CASE
+  set_last_error("attn_prefill_tc: head_dim must be 64 or 128 and the GQA group 4 or 8");
   return cudaErrorInvalidValue;
 }
 

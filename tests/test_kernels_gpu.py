@@ -340,6 +340,51 @@ def test_attention_prefill_blocks(d, nh, nkv, page_size, short_blocks):
     assert np.abs(got - ref).max() <= 2 * BF16_ULP * np.abs(ref).max() + 1e-5, np.abs(got - ref).max()
 
 
+@pytest.mark.parametrize("nh,nkv,page_size", [(8, 1, 8), (8, 2, 64), (16, 2, 128)])
+@pytest.mark.parametrize("past", [0, 63, 200])
+def test_attention_prefill_heads_of_64(nh, nkv, page_size, past):
+    """The tcgen05 kernel for heads of 64 at the edges of its 64-key tiles: one tile (only one of its two softmax groups works), 64 and 65
+    keys, an odd number of tiles, portions behind keys already in the cache, and scores that grow along the keys so that the
+    softmax reference has to be raised after the first tile.  Against float64; two bf16 roundings (weights, result) of values up to
+    the largest |v|."""
+    g = torch.Generator(device=DEV); g.manual_seed(past + nh + page_size)
+    d, lens = 64, [1, 16, 64, 65, 129, 330]
+    BT = lib().dis_k_attn_prefill_block_tokens(nh, nkv, d)
+    total = [past + n for n in lens]
+    per = [(n + page_size - 1) // page_size for n in total]
+    n_pages = sum(per)
+    perm = np.random.default_rng(past).permutation(n_pages).astype(np.int32)
+    pt = np.zeros((len(lens), max(per)), np.int32)
+    at = 0
+    for s, p in enumerate(per):
+        pt[s, :p] = perm[at:at + p]; at += p
+    pool = torch.randn((n_pages, 2, nkv, page_size, d), device=DEV, generator=g)
+    for s, p in enumerate(per):  # keys grow with their position: later tiles hold the largest scores
+        pos = torch.arange(p * page_size, device=DEV).reshape(p, 1, page_size, 1)
+        pool[torch.as_tensor(pt[s, :p].astype(np.int64), device=DEV), 0] *= 0.2 + pos / 64.0
+    pool = pool.to(torch.bfloat16)
+    tok0, qlen, pos0, ptrow, t = [], [], [], [], 0
+    for s, n in enumerate(lens):
+        for p0 in range(0, n, BT):
+            tok0.append(t); qlen.append(min(BT, n - p0)); pos0.append(past + p0); ptrow.append(s); t += qlen[-1]
+    q = torch.randn((t, nh * d), device=DEV, generator=g).to(torch.bfloat16)
+    out = G.empty((t, nh * d), dtype=torch.bfloat16, device=DEV)
+    check(lib().dis_k_attn_prefill(ptr(q), ptr(pool), n_pages, ptr(dev_i32(pt)), pt.shape[1], ptr(dev_i32(tok0)), ptr(dev_i32(qlen)),
+                                   ptr(dev_i32(pos0)), ptr(dev_i32(ptrow)), ptr(out), len(tok0), nh, nkv, d, page_size, None))
+    sync()
+    row = 0
+    for s, n in enumerate(lens):
+        kv = pool[torch.as_tensor(pt[s, :per[s]].astype(np.int64), device=DEV)].double()
+        K, V = (kv[:, c].permute(1, 0, 2, 3).reshape(nkv, -1, d)[:, :total[s]] for c in (0, 1))
+        qs = q[row:row + n].double().reshape(n, nkv, nh // nkv, d).permute(1, 2, 0, 3)
+        sc = qs @ K.transpose(1, 2).unsqueeze(1) / d ** 0.5
+        sc = sc.masked_fill(torch.arange(total[s], device=DEV)[None] > torch.arange(past, total[s], device=DEV)[:, None], float("-inf"))
+        ref = (torch.softmax(sc, dim=-1) @ V.unsqueeze(1)).permute(2, 0, 1, 3).reshape(n, nh * d)
+        err = (out[row:row + n].double() - ref).abs().max().item()
+        assert err <= 2 * BF16_ULP * V.abs().max().item() + 1e-5, (s, n, err)
+        row += n
+
+
 def test_attention_prefill_full_size_against_torch():
     """Llama-3-8B geometry, a 3000-token prompt prefilled from position 0 and the last 1000 tokens of a 4000-token one
     (a later chunk of a chunked prefill), 64-token pages in shuffled order: causal attention against fp32 torch."""
