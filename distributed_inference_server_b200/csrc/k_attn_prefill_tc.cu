@@ -310,16 +310,6 @@ constexpr int kPf3QHalf = 128 * 128;  // one [128 rows][64 dims] block of Q, 16 
 template <int D>
 constexpr int pf3_smem_bytes() { return (D / 64) * (kPf3QHalf + 4 * kPfHalf) + 3 * 128 * 4 + 256; }
 
-// D[tmem] (+)= A[tmem] * B[smem]: A is 128 lanes x 16 bf16, two per column
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // Packed pairs: one issue slot for two lanes' worth of work
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   float2 d;
@@ -407,7 +397,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
 
   // later query blocks of a sequence have more key tiles: launch them first, so that the longest CTAs do not form the tail
   const int qb = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&kv_map);
@@ -477,37 +467,41 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
       }
     }
   } else if (warp == 1) {
-    // ===== MMA issuer (one thread) =====
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc<kPfTile>();
-      constexpr uint32_t idesc_o = umma_idesc<D>() | (1u << 16);  // B (= V) MN-major
-      auto issue_s = [&](int j) {
-        const int w = j & 1;
-        mbar_wait(k_full(w), (uint32_t)(j >> 1) & 1u);
-        tc_fence_after();
+    // ===== MMA issuer: the warp converged, one elected lane issues =====
+    constexpr uint32_t idesc_s = umma_idesc<kPfTile>();
+    constexpr uint32_t idesc_o = umma_idesc<D>() | (1u << 16);  // B (= V) MN-major
+    const uint32_t q_lo = umma_lo(q_base), k_lo = umma_lo(k_base), v_lo = umma_lo_mn(v_base, kPfHalf);
+    auto issue_s = [&](int j) {
+      const uint32_t w = (uint32_t)j & 1u;
+      mbar_wait(k_full(w), (uint32_t)(j >> 1) & 1u);
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t b = k_lo + w * (kSlot >> 4), d = tmem_base + w * kPfTile;
 #pragma unroll
-        for (int k = 0; k < D / 16; k++)
-          umma_bf16(tmem_base + w * kPfTile, umma_desc_sw128(q_base + (k >> 2) * kPf3QHalf + (k & 3) * 32),
-                    umma_desc_sw128(k_base + w * kSlot + (k >> 2) * kPfHalf + (k & 3) * 32), idesc_s, k > 0 ? 1u : 0u);
+        for (uint32_t k = 0; k < D / 16; k++)
+          umma_ss(d, q_lo + (k >> 2) * (kPf3QHalf >> 4) + (k & 3) * 2, b + (k >> 2) * (kPfHalf >> 4) + (k & 3) * 2, idesc_s, k > 0 ? 1u : 0u);
         umma_commit(s_full(w));
         umma_commit(k_empty(w));
-      };
-      issue_s(0);
-      if (n_tiles > 1) issue_s(1);
-      for (int j = 0; j < n_tiles; j++) {
-        const int w = j & 1;
-        mbar_wait(v_full(w), (uint32_t)(j >> 1) & 1u);
-        mbar_wait(p_full(w), (uint32_t)(j >> 1) & 1u);
-        tc_fence_after();
+      }
+      __syncwarp();
+    };
+    issue_s(0);
+    if (n_tiles > 1) issue_s(1);
+    for (int j = 0; j < n_tiles; j++) {
+      const uint32_t w = (uint32_t)j & 1u;
+      mbar_wait(v_full(w), (uint32_t)(j >> 1) & 1u);
+      mbar_wait(p_full(w), (uint32_t)(j >> 1) & 1u);
+      tc_fence_after();
+      if (elect_one()) {
+        const uint32_t b = v_lo + w * (kSlot >> 4), a = tmem_base + w * kPfTile;
 #pragma unroll
-        for (int k = 0; k < kPfTile / 16; k++)
-          umma_bf16_ts(o_base, tmem_base + w * kPfTile + 8 * k, umma_desc_mn_sw128(v_base + w * kSlot + k * 2048, kPfHalf, 1024), idesc_o,
-                       (j > 0 || k > 0) ? 1u : 0u);
+        for (uint32_t k = 0; k < kPfTile / 16; k++) umma_ts(o_base, a + 8 * k, b + k * 128, idesc_o, k > 0 ? 1u : (uint32_t)(j > 0));
         umma_commit(pv_done(w));
-        if (j + 2 < n_tiles) {
-          mbar_wait(pv_done(w), (uint32_t)(j >> 1) & 1u);  // S_{j+2} overwrites the columns that P_j V_j reads
-          issue_s(j + 2);
-        }
+      }
+      __syncwarp();
+      if (j + 2 < n_tiles) {
+        mbar_wait(pv_done(w), (uint32_t)(j >> 1) & 1u);  // S_{j+2} overwrites the columns that P_j V_j reads
+        issue_s(j + 2);
       }
     }
   } else {
@@ -576,8 +570,9 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
           float2 p = fma2(make_float2(__uint_as_float(s[c][i]), __uint_as_float(s[c][i + 1])), scale2, neg_m);
           p.x = ex2_approx(p.x);
           p.y = ex2_approx(p.y);
-          ps[(i >> 1) & 1] = add2(ps[(i >> 1) & 1], p);
           pk[i >> 1] = float2_to_bf16x2(p.x, p.y);
+          // the sum takes the weights as P V takes them, rounded: a row that one key dominates keeps that key's weight at 1
+          ps[(i >> 1) & 1] = add2(ps[(i >> 1) & 1], bf16x2_to_float2(pk[i >> 1]));
         }
         tmem_st_32x16(s_addr + 16 * c, pk);
       }
@@ -678,8 +673,8 @@ cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const u
     return prefill_tc_launch(KERN, THREADS, SMEM, once, kv_map, row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, \
                              out, n_blocks, n_heads, n_kv, page_shift, st);                                                      \
   }
-  DIS_PF_TC_CASE(128, 4, attn_prefill_tc2_kernel<4>, kPfThreads, kPf2SmemBytes)
-  DIS_PF_TC_CASE(128, 8, attn_prefill_tc2_kernel<8>, kPfThreads, kPf2SmemBytes)
+  DIS_PF_TC_CASE(128, 4, (attn_prefill_tc3_kernel<128, 4>), kPf3Threads, pf3_smem_bytes<128>())
+  DIS_PF_TC_CASE(128, 8, (attn_prefill_tc3_kernel<128, 8>), kPf3Threads, pf3_smem_bytes<128>())
   DIS_PF_TC_CASE(64, 4, (attn_prefill_tc3_kernel<64, 4>), kPf3Threads, pf3_smem_bytes<64>())
   DIS_PF_TC_CASE(64, 8, (attn_prefill_tc3_kernel<64, 8>), kPf3Threads, pf3_smem_bytes<64>())
 #undef DIS_PF_TC_CASE
