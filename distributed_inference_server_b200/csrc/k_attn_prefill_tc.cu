@@ -8,8 +8,21 @@
 // 128 query rows and the QK^T / PV products run at tcgen05 rate instead of through ldmatrix + mma.sync
 // (k_attn_paged.cu).  Tensor- and exponential-bound: 4 * rows * keys * d flop and rows * keys exponentials per (block, kv head).
 //
-// Heads of 128: attn_prefill_tc2_kernel, one softmax group per CTA, P through shared memory.  Heads of 64:
-// attn_prefill_tc3_kernel, two softmax groups per CTA on alternate key tiles, P in TMEM.
+//   warp 0      TMA producer: 64-key K and V tiles (128B-swizzled boxes out of the page pool), two slots each
+//   warp 1      the MMAs:  S_j = Q K_j^T   M128 N64 K16 x D/16  (A, B K-major, shared memory)
+//                          O  += P_j V_j   M128 N=D K16 x 4     (A = P from TMEM, B = V MN-major)
+//   warps 2-5   softmax of the even tiles, warps 6-9 of the odd ones, one thread per row: S_j from TMEM, causal mask, row maximum (no
+//               shuffles: a thread owns a whole row); P_j = exp2(s - m) goes as packed bf16 back into S_j's own TMEM columns (no
+//               shared-memory write, proxy fence or second read of it)
+// TMEM per CTA: S0 | S1 64 columns each | O D columns = 256; shared memory Q + 2 K + 2 V = 96 KB (D = 128): two CTAs per SM, so four
+// softmax groups take turns on the exponentials (16 per clock and SM: 1024 clocks per 128 rows x 128 keys, beside 512 or 1024 of the
+// tensor pipe).  O accumulates in TMEM; the two groups share a row's softmax reference m_ref, handed from tile to tile through shared
+// memory, and it is raised only when a row's maximum exceeds it by more than 8 in the log2 domain (P <= 256, the reference cancels in
+// the final division by l), so O is rescaled in TMEM on few tiles only (decided per warp, scaled per lane).
+//
+// Measured against what it replaced: heads of 64 (mma.sync), six prompts of 276 to 1900 tokens, 32 / 4 heads, 31.6 GFLOP: 164.6 -> 76.4
+// us; heads of 128 (one softmax group per CTA, P through shared memory), six prompts of 437 to 3000 tokens, 32 / 8 heads, 258 GFLOP:
+// 366.8 -> 349.1 us.  A key tile takes a CTA 1000 clocks (D = 64) or 1400 (D = 128), a CTA's start and end 8000 beside them.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -20,295 +33,24 @@
 
 namespace dis {
 
-constexpr int kPfThreads = 192;
-constexpr int kPfTile = 64;    // keys per stage
-constexpr int kPfD = 128;
-constexpr int kPfHalf = kPfTile * 128;                  // one [64 keys][64 dims] block, 8 KB
-constexpr int kPfQBytes = 2 * 128 * 128;                 // Q: two [128 rows][64 dims] halves, 32 KB
-constexpr int kPfPBytes = 128 * 128;                     // P: [128 rows][64 keys] bf16, 16 KB
+constexpr int kPfTile = 64;             // keys per tile
+constexpr int kPfHalf = kPfTile * 128;  // one [64 keys][64 dims] block of K or V, 8 KB
+constexpr int kPfTmemCols = 256;
+constexpr float kPfLazy = 8.0f;
 
-// shared-memory matrix descriptor, MN-major operand, 128B swizzle: element (mn, k) lives at
-//   (mn % 64) * 2 + (mn / 64) * LBO + (k % 8) * 128 + (k / 8) * SBO   -- the [keys][dims] V tile as TMA stores it
-__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | ((uint64_t)(lbo_bytes >> 4) << 16) | ((uint64_t)(sbo_bytes >> 4) << 32) |
-         (1ull << 46) | (2ull << 61);
-}
-
+// V's descriptor (umma_lo_mn) is MN-major, 128B swizzle: element (mn, k) lives at (mn % 64) * 2 + (mn / 64) * LBO + (k % 8) * 128 +
+// (k / 8) * SBO -- the [keys][dims] tile as TMA stores it, LBO the distance of its two 64-dim blocks.
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
-// ---------------------------------------------------------------------------------------- two CTAs per SM
-// Built to fit TWO CTAs per SM, one's MMAs under the other's softmax:
-//   warp 0      TMA producer: 64-key K/V tiles (128B-swizzled boxes out of the page pool)
-//   warp 1      one thread issues the MMAs:   S_j   = Q   K_j^T   M128 N64  K16 x 8   (A, B K-major)       -> TMEM S[j&1]
-//                                             O    += P_j V_j     M128 N128 K16 x 4   (B = V, MN-major)    -> TMEM O
-//   warps 2-5   one thread per row: S_j from TMEM, scale, causal mask, running max / sum (no shuffles: a thread
-//               owns a whole row), P_j = exp2(s - m) as bf16 into shared memory (the A operand of the PV MMA)
-//   * O stays in TMEM and accumulates there over the tiles (tcgen05.mma accumulate).  The softmax reference m_ref is only raised when the running
-//     maximum exceeds it by more than 8 (log2 domain): P = exp2(s - m_ref) <= 256 stays exact enough in bf16/fp32, the
-//     reference cancels in the final division by l, and the rescale of O (tcgen05.ld, scale, tcgen05.st, warp-uniformly
-//     decided) happens only on the few tiles where a row's maximum still grows;
-//   * TMEM: S0 | S1 | O = 256 columns; shared memory: Q 32 KB + two K and two V slots of 16 KB + one P tile = 112 KB;
-//     K and V have their own barriers, so K_{j+1} can be fetched as soon as S_{j-1} has read its slot, a whole tile
-//     before it is needed.
-constexpr int kPf2KSlot = 2 * kPfHalf;                   // one K (or V) tile: two [64 keys][64 dims] halves, 16 KB
-constexpr int kPf2SmemBytes = kPfQBytes + 4 * kPf2KSlot + kPfPBytes + 256;
-constexpr int kPf2TmemCols = 256;
-constexpr float kPf2Lazy = 8.0f;
-
-__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
-        "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]),
-        "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-template <int G>
-__global__ void __launch_bounds__(kPfThreads, 2)
-attn_prefill_tc2_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const uint16_t *__restrict__ q,
-                        const int *__restrict__ page_table, int max_pages, const int *__restrict__ qb_tok0,
-                        const int *__restrict__ qb_len, const int *__restrict__ qb_pos0, const int *__restrict__ qb_ptrow,
-                        uint16_t *__restrict__ out, int n_heads, int n_kv, int page_shift) {
-  constexpr int QT = 128 / G;
-  extern __shared__ __align__(1024) uint8_t smem_al[];
-  const uint32_t smem_base = smem_u32(smem_al);
-  if (smem_base & 1023u) __trap();  // the 128B-swizzle atoms need 1024-byte alignment and there is no room for slack
-  uint8_t *smem = smem_al;
-  const uint32_t q_base = smem_base;
-  const uint32_t k_base = q_base + kPfQBytes;            // K slots 0, 1
-  const uint32_t v_base = k_base + 2 * kPf2KSlot;        // V slots 0, 1
-  const uint32_t p_base = v_base + 2 * kPf2KSlot;
-  const uint32_t bar_base = p_base + kPfPBytes;
-  auto k_full = [&](int s) { return bar_base + 8u * s; };
-  auto k_empty = [&](int s) { return bar_base + 8u * (2 + s); };
-  auto v_full = [&](int s) { return bar_base + 8u * (4 + s); };
-  auto v_empty = [&](int s) { return bar_base + 8u * (6 + s); };
-  auto s_full = [&](int b) { return bar_base + 8u * (8 + b); };
-  const uint32_t p_full = bar_base + 8u * 10, o_full = bar_base + 8u * 11;
-  const uint32_t tmem_slot = bar_base + 8u * 12;
-
-  // later query blocks of a sequence have more key tiles: launch them first, so that the longest CTAs do not form the tail
-  const int qb = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&kv_map);
-    for (int s = 0; s < 2; s++) {
-      mbar_init(k_full(s), 1); mbar_init(k_empty(s), 1); mbar_init(v_full(s), 1); mbar_init(v_empty(s), 1); mbar_init(s_full(s), 1);
-    }
-    mbar_init(p_full, 128); mbar_init(o_full, 1);
-    fence_barrier_init();
-    fence_proxy_async();
-  }
-  if (warp == 1) tmem_alloc<kPf2TmemCols>(tmem_slot);
-  pdl_launch_dependents();
-  pdl_wait();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  uint32_t tmem_base;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
-
-  const int tok0 = qb_tok0[qb], len = qb_len[qb], pos0 = qb_pos0[qb];
-  const int *pt = page_table + (size_t)qb_ptrow[qb] * max_pages;
-  const int page_size = 1 << page_shift;
-  const int box_rows = min(page_size, kPfTile);
-  const int end = pos0 + len;
-  const int n_tiles = (end + kPfTile - 1) / kPfTile;
-
-  if (warp >= 2) {  // Q tile: row = head * QT + token, K-major, 128B swizzle (rows of padding tokens are zero)
-    const int row = (warp & 3) * 32 + lane;
-    const int hl = row / QT, t = row % QT;
-    const uint4 *src = reinterpret_cast<const uint4 *>(q + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * kPfD);
-#pragma unroll
-    for (int c = 0; c < 16; c++) {
-      const uint4 v = t < len ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-      const uint32_t off = (uint32_t)(c >> 3) * (128 * 128) + (uint32_t)(row >> 3) * 1024 + (uint32_t)(row & 7) * 128 +
-                           (uint32_t)(((c & 7) ^ (row & 7)) << 4);
-      *reinterpret_cast<uint4 *>(smem + off) = v;
-    }
-    fence_proxy_async();
-  }
-  __syncthreads();
-
-  if (warp == 0) {
-    // ===== TMA producer: K_t as soon as S_{t-2} has read its slot, V_{t-1} as soon as P_{t-3} V_{t-3} has =====
-    if (lane == 0) {
-      auto load = [&](int tile, bool is_v) {
-        const int slot = tile & 1;
-        const uint32_t full = is_v ? v_full(slot) : k_full(slot), empty = is_v ? v_empty(slot) : k_empty(slot);
-        if (tile >= 2) mbar_wait(empty, (uint32_t)(tile / 2 - 1) & 1u);
-        const uint32_t sbase = (is_v ? v_base : k_base) + slot * kPf2KSlot;
-        mbar_expect_tx(full, kPf2KSlot);
-        for (int r = 0; r < kPfTile; r += box_rows) {
-          const int pos = tile * kPfTile + r;
-          const long long page = pt[min(pos >> page_shift, max_pages - 1)];
-          const long long krow = row0 + ((page * 2 + (is_v ? 1 : 0)) * n_kv + kvh) * page_size + (pos & (page_size - 1));
-#pragma unroll
-          for (int hh = 0; hh < 2; hh++) tma_load_2d(sbase + hh * kPfHalf + r * 128, &kv_map, hh * 64, (int)krow, full, kEvictLast);
-        }
-      };
-      for (int t = 0; t <= n_tiles; t++) {
-        if (t < n_tiles) load(t, false);
-        if (t >= 1) load(t - 1, true);
-      }
-    }
-  } else if (warp == 1) {
-    // ===== MMA issuer (one thread) =====
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc<kPfTile>();
-      constexpr uint32_t idesc_o = umma_idesc<kPfD>() | (1u << 16);
-      auto issue_s = [&](int j) {
-        const int slot = j & 1;
-        mbar_wait(k_full(slot), (uint32_t)(j >> 1) & 1u);
-        tc_fence_after();
-        const uint32_t kb = k_base + slot * kPf2KSlot;
-#pragma unroll
-        for (int k = 0; k < kPfD / 16; k++) {
-          const uint32_t a = q_base + (k >> 2) * (128 * 128) + (k & 3) * 32;
-          const uint32_t b = kb + (k >> 2) * kPfHalf + (k & 3) * 32;
-          umma_bf16(tmem_base + (uint32_t)slot * kPfTile, umma_desc_sw128(a), umma_desc_sw128(b), idesc_s, k > 0 ? 1u : 0u);
-        }
-        umma_commit(s_full(slot));
-        umma_commit(k_empty(slot));
-      };
-      auto issue_o = [&](int j) {
-        const int slot = j & 1;
-        mbar_wait(p_full, (uint32_t)j & 1u);
-        mbar_wait(v_full(slot), (uint32_t)(j >> 1) & 1u);
-        tc_fence_after();
-        const uint32_t vb = v_base + slot * kPf2KSlot;
-#pragma unroll
-        for (int k = 0; k < kPfTile / 16; k++)
-          umma_bf16(tmem_base + 2 * kPfTile, umma_desc_sw128(p_base + k * 32), umma_desc_mn_sw128(vb + k * 2048, kPfHalf, 1024),
-                    idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-        umma_commit(o_full);
-        umma_commit(v_empty(slot));
-      };
-      issue_s(0);
-      for (int j = 0; j < n_tiles; j++) {
-        if (j + 1 < n_tiles) issue_s(j + 1);
-        issue_o(j);
-      }
-    }
-  } else {
-    // ===== softmax: one thread per row; O lives in TMEM =====
-    const int quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const int hl = row / QT, t = row % QT;
-    const int qp = pos0 + t;
-    const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16);
-    const uint32_t o_addr = lane_addr + 2 * kPfTile;
-    const float scale_log2 = rsqrtf((float)kPfD) * 1.4426950408889634f;
-    float m_ref = -INFINITY, l_run = 0.f;
-    for (int j = 0; j < n_tiles; j++) {
-      mbar_wait(s_full(j & 1), (uint32_t)(j >> 1) & 1u);
-      tc_fence_after();
-      uint32_t s0[32], s1[32];
-      tmem_ld_32x32(lane_addr + (uint32_t)(j & 1) * kPfTile, s0);
-      tmem_ld_32x32(lane_addr + (uint32_t)(j & 1) * kPfTile + 32, s1);
-      tmem_ld_wait();
-      const int tile0 = j * kPfTile;
-      if (tile0 + kPfTile - 1 > qp) {  // only the tiles that cross the diagonal need the causal mask
-#pragma unroll
-        for (int i = 0; i < 32; i++) {
-          if (tile0 + i > qp) s0[i] = 0xff800000u;
-          if (tile0 + 32 + i > qp) s1[i] = 0xff800000u;
-        }
-      }
-      // four independent chains each for the maximum and the row sum: two warps per scheduler do not hide the latency of
-      // one 32-deep dependent chain (ncu: "wait" and "long scoreboard" are the top two stall reasons)
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int i = 0; i < 32; i++) mx4[i & 3] = fmaxf(mx4[i & 3], fmaxf(__uint_as_float(s0[i]), __uint_as_float(s1[i])));
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      const float m_new = fmaxf(m_ref, mx * scale_log2);
-      if (j == 0) {
-        m_ref = m_new;  // finite: key 0 is visible to every query; O is first written by P_0 V_0 (accumulate off)
-      } else {
-        // P_{j-1} V_{j-1} must have finished before P's buffer is rewritten and before O may be rescaled
-        mbar_wait(o_full, (uint32_t)(j - 1) & 1u);
-        tc_fence_after();
-        const bool need = m_new > m_ref + kPf2Lazy;
-        if (__any_sync(0xffffffffu, need)) {  // tcgen05.ld / st are warp-collective: decide per warp, scale per lane
-          const float f = need ? ex2_approx(m_ref - m_new) : 1.0f;
-          if (need) m_ref = m_new;
-          l_run *= f;
-#pragma unroll
-          for (int c = 0; c < kPfD; c += 32) {
-            uint32_t v[32];
-            tmem_ld_32x32(o_addr + c, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
-            tmem_st_32x32(o_addr + c, v);
-          }
-          tmem_st_wait();
-        }
-      }
-      const float neg_m = -m_ref;
-      float ps4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint8_t *prow = smem + (p_base - smem_base) + (row >> 3) * 1024 + (row & 7) * 128;
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        uint32_t pk[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int i = c * 8 + e * 2;
-          const float p0 = ex2_approx(fmaf(__uint_as_float(i < 32 ? s0[i] : s1[i - 32]), scale_log2, neg_m));
-          const float p1 = ex2_approx(fmaf(__uint_as_float(i + 1 < 32 ? s0[i + 1] : s1[i + 1 - 32]), scale_log2, neg_m));
-          ps4[e] += p0 + p1;
-          pk[e] = float2_to_bf16x2(p0, p1);
-        }
-        *reinterpret_cast<uint4 *>(prow + ((c ^ (row & 7)) << 4)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-      }
-      l_run += (ps4[0] + ps4[1]) + (ps4[2] + ps4[3]);
-      fence_proxy_async();
-      tc_fence_before();
-      mbar_arrive(p_full);
-    }
-    mbar_wait(o_full, (uint32_t)(n_tiles - 1) & 1u);
-    tc_fence_after();
-    const float inv = 1.0f / l_run;
-    uint4 *o = reinterpret_cast<uint4 *>(out + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * kPfD);
-#pragma unroll
-    for (int c = 0; c < kPfD; c += 32) {
-      uint32_t v[32];
-      tmem_ld_32x32(o_addr + c, v);
-      tmem_ld_wait();
-      if (t < len) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          uint4 w;
-          w.x = float2_to_bf16x2(__uint_as_float(v[i * 8 + 0]) * inv, __uint_as_float(v[i * 8 + 1]) * inv);
-          w.y = float2_to_bf16x2(__uint_as_float(v[i * 8 + 2]) * inv, __uint_as_float(v[i * 8 + 3]) * inv);
-          w.z = float2_to_bf16x2(__uint_as_float(v[i * 8 + 4]) * inv, __uint_as_float(v[i * 8 + 5]) * inv);
-          w.w = float2_to_bf16x2(__uint_as_float(v[i * 8 + 6]) * inv, __uint_as_float(v[i * 8 + 7]) * inv);
-          o[c / 8 + i] = w;
-        }
-      }
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) tmem_dealloc<kPf2TmemCols>(tmem_base);
-}
-
-// ---------------------------------------------------------------------------------------- two softmax groups, P in TMEM
-constexpr int kPf3Threads = 320;
-constexpr int kPf3QHalf = 128 * 128;  // one [128 rows][64 dims] block of Q, 16 KB
+constexpr int kPfThreads = 320;
+constexpr int kPfQHalf = 128 * 128;  // one [128 rows][64 dims] block of Q, 16 KB
 
 template <int D>
-constexpr int pf3_smem_bytes() { return (D / 64) * (kPf3QHalf + 4 * kPfHalf) + 3 * 128 * 4 + 256; }
+constexpr int pf_smem_bytes() { return (D / 64) * (kPfQHalf + 4 * kPfHalf) + 3 * 128 * 4 + 256; }
 
 // Packed pairs: one issue slot for two lanes' worth of work
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -334,6 +76,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 __device__ __forceinline__ void named_sync_64(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
 __device__ __forceinline__ void named_arrive_64(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
 
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_32x16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -361,18 +104,9 @@ __device__ __forceinline__ void rescale_32(uint32_t o_addr, float f) {
   }
 }
 
-//   warp 0      TMA producer, as above
-//   warp 1      one thread issues S_j = Q K_j^T (M128 N64) and O += P_j V_j (M128 N=D, A = P from TMEM, B = V MN-major)
-//   warps 2-5   softmax of the even tiles, warps 6-9 of the odd ones, one thread per row; P_j = exp2(s - m) goes as packed bf16 back
-//               into S_j's own TMEM columns (no shared-memory write, proxy fence or second read of it)
-// TMEM per CTA: S0 | S1 64 columns each | O D columns; two CTAs per SM, so four softmax groups take turns on the exponentials (16 per
-// clock and SM, what bounds heads of 64: 1024 clocks per 128 rows x 128 keys against 512 of the tensor pipe).  The two groups share a
-// row's reference, handed from tile to tile through shared memory and raised lazily as above.
-// Heads of 64, six prompts of 276 to 1900 tokens, 32 / 4 heads (31.6 GFLOP): 164 us on the mma.sync kernel of k_attn_paged.cu, 89 us here.
-// Heads of 128 stay above: 382 us here against 367 us (six prompts of 437 to 3000 tokens, 32 / 8 heads, 258 GFLOP).
 template <int D, int G>
-__global__ void __launch_bounds__(kPf3Threads, 2)
-attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const uint16_t *__restrict__ q,
+__global__ void __launch_bounds__(kPfThreads, 2)
+attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const uint16_t *__restrict__ q,
                         const int *__restrict__ page_table, int max_pages, const int *__restrict__ qb_tok0,
                         const int *__restrict__ qb_len, const int *__restrict__ qb_pos0, const int *__restrict__ qb_ptrow,
                         uint16_t *__restrict__ out, int n_heads, int n_kv, int page_shift) {
@@ -383,7 +117,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
   const uint32_t smem_base = smem_u32(smem_al);
   if (smem_base & 1023u) __trap();  // the 128B-swizzle atoms need 1024-byte alignment and there is no room for slack
   uint8_t *smem = smem_al;
-  const uint32_t q_base = smem_base, k_base = q_base + kHalves * kPf3QHalf, v_base = k_base + 2 * kSlot;
+  const uint32_t q_base = smem_base, k_base = q_base + kHalves * kPfQHalf, v_base = k_base + 2 * kSlot;
   const uint32_t bar_base = v_base + 2 * kSlot;
   auto k_full = [&](int w) { return bar_base + 8u * w; };
   auto k_empty = [&](int w) { return bar_base + 16u + 8u * w; };
@@ -408,7 +142,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
     fence_barrier_init();
     fence_proxy_async();
   }
-  if (warp == 1) tmem_alloc<kPf2TmemCols>(tmem_slot);
+  if (warp == 1) tmem_alloc<kPfTmemCols>(tmem_slot);
   pdl_launch_dependents();
   pdl_wait();  // q and this chunk's K/V rows come from the previous kernels
   tc_fence_before();
@@ -433,7 +167,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
     for (int cc = 0; cc < D / 16; cc++) {
       const int c = grp * (D / 16) + cc;
       const uint4 v = t < len ? src[c] : make_uint4(0u, 0u, 0u, 0u);
-      const uint32_t off = (uint32_t)(c >> 3) * kPf3QHalf + (uint32_t)(row >> 3) * 1024 + (uint32_t)(row & 7) * 128 +
+      const uint32_t off = (uint32_t)(c >> 3) * kPfQHalf + (uint32_t)(row >> 3) * 1024 + (uint32_t)(row & 7) * 128 +
                            (uint32_t)(((c & 7) ^ (row & 7)) << 4);
       *reinterpret_cast<uint4 *>(smem + off) = v;
     }
@@ -479,7 +213,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
         const uint32_t b = k_lo + w * (kSlot >> 4), d = tmem_base + w * kPfTile;
 #pragma unroll
         for (uint32_t k = 0; k < D / 16; k++)
-          umma_ss(d, q_lo + (k >> 2) * (kPf3QHalf >> 4) + (k & 3) * 2, b + (k >> 2) * (kPfHalf >> 4) + (k & 3) * 2, idesc_s, k > 0 ? 1u : 0u);
+          umma_ss(d, q_lo + (k >> 2) * (kPfQHalf >> 4) + (k & 3) * 2, b + (k >> 2) * (kPfHalf >> 4) + (k & 3) * 2, idesc_s, k > 0 ? 1u : 0u);
         umma_commit(s_full(w));
         umma_commit(k_empty(w));
       }
@@ -542,7 +276,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
       } else {
         named_sync_64(bar_in);
         const float m_old = m_row[row];
-        const bool need = mx > m_old + kPf2Lazy;
+        const bool need = mx > m_old + kPfLazy;
         m_now = need ? mx : m_old;
         if (__any_sync(0xffffffffu, need)) {  // tcgen05.ld / st are warp-collective: decide per warp, scale per lane
           // every P V so far must be in O; none follows before this tile's P is handed over
@@ -612,7 +346,7 @@ attn_prefill_tc3_kernel(const __grid_constant__ CUtensorMap kv_map, long long ro
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) tmem_dealloc<kPf2TmemCols>(tmem_base);
+  if (warp == 1) tmem_dealloc<kPfTmemCols>(tmem_base);
 }
 
 // DIS_ATTN_PREFILL=mma sends every geometry to the mma.sync kernel of k_attn_paged.cu (A/B runs).
@@ -673,10 +407,10 @@ cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const u
     return prefill_tc_launch(KERN, THREADS, SMEM, once, kv_map, row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, \
                              out, n_blocks, n_heads, n_kv, page_shift, st);                                                      \
   }
-  DIS_PF_TC_CASE(128, 4, (attn_prefill_tc3_kernel<128, 4>), kPf3Threads, pf3_smem_bytes<128>())
-  DIS_PF_TC_CASE(128, 8, (attn_prefill_tc3_kernel<128, 8>), kPf3Threads, pf3_smem_bytes<128>())
-  DIS_PF_TC_CASE(64, 4, (attn_prefill_tc3_kernel<64, 4>), kPf3Threads, pf3_smem_bytes<64>())
-  DIS_PF_TC_CASE(64, 8, (attn_prefill_tc3_kernel<64, 8>), kPf3Threads, pf3_smem_bytes<64>())
+  DIS_PF_TC_CASE(128, 4, (attn_prefill_tc_kernel<128, 4>), kPfThreads, pf_smem_bytes<128>())
+  DIS_PF_TC_CASE(128, 8, (attn_prefill_tc_kernel<128, 8>), kPfThreads, pf_smem_bytes<128>())
+  DIS_PF_TC_CASE(64, 4, (attn_prefill_tc_kernel<64, 4>), kPfThreads, pf_smem_bytes<64>())
+  DIS_PF_TC_CASE(64, 8, (attn_prefill_tc_kernel<64, 8>), kPfThreads, pf_smem_bytes<64>())
 #undef DIS_PF_TC_CASE
   set_last_error("attn_prefill_tc: head_dim must be 64 or 128 and the GQA group 4 or 8");
   return cudaErrorInvalidValue;

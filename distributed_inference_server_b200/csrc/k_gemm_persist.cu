@@ -51,7 +51,7 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   auto a2_tile = [&](int s) { return a_tile(s) + Cfg::kABytes; };
   auto b_tile = [&](int s) { return a_tile(s) + (kDual ? 2 : 1) * Cfg::kABytes; };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int num_kb = (K + kBK - 1) / kBK;
   const int n_tiles = tiles_n * tiles_t;
   // tile -> (weight tile, token tile).  The ~148 tiles in flight together should cover ALL tiles of the smaller
@@ -97,32 +97,36 @@ gemm_persist_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // ===== MMA issuer (one thread): accumulator buffers alternate per tile =====
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc<BN>();
-      int s = 0, buf = 0;
-      uint32_t phase = 0, aphase[2] = {0u, 0u};
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        mbar_wait(acc_empty(buf), aphase[buf] ^ 1u);  // the epilogue has drained this buffer (passes on first use)
+    // ===== MMA issuer (the warp converged, one elected lane issues): accumulator buffers alternate per tile =====
+    constexpr uint32_t idesc = umma_idesc<BN>();
+    const uint32_t lo0 = umma_lo(smem_base);
+    constexpr uint32_t a2_off = Cfg::kABytes >> 4, b_off = ((kDual ? 2 : 1) * Cfg::kABytes) >> 4;
+    uint32_t lo = lo0;
+    int s = 0;
+    uint32_t phase = 0, buf = 0, aphase = 0;  // aphase: the phase of both accumulator barriers, flipped after buffer 1
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      mbar_wait(acc_empty(buf), aphase ^ 1u);  // the epilogue has drained this buffer (passes on first use)
+      tc_fence_after();
+      const uint32_t acc_addr = tmem_base + buf * Cfg::kAccCols;
+      for (int kb = 0; kb < num_kb; kb++) {
+        mbar_wait(full_bar(s), phase);
         tc_fence_after();
-        const uint32_t acc_addr = tmem_base + (uint32_t)(buf * Cfg::kAccCols);
-        for (int kb = 0; kb < num_kb; kb++) {
-          mbar_wait(full_bar(s), phase);
-          tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; k++) {
-            const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-            const uint64_t bd = umma_desc_sw128(b_tile(s) + k * 32);
-            umma_bf16(acc_addr, umma_desc_sw128(a_tile(s) + k * 32), bd, idesc, acc);
-            if (kDual) umma_bf16(acc_addr + BN, umma_desc_sw128(a2_tile(s) + k * 32), bd, idesc, acc);
+          for (uint32_t k = 0; k < kBK / 16; k++) {
+            const uint32_t acc = k > 0 ? 1u : (uint32_t)(kb > 0);
+            umma_ss(acc_addr, lo + 2 * k, lo + b_off + 2 * k, idesc, acc);
+            if (kDual) umma_ss(acc_addr + BN, lo + a2_off + 2 * k, lo + b_off + 2 * k, idesc, acc);
           }
-          umma_commit(empty_bar(s));  // slot reusable once these MMAs have read it
-          if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
+          umma_commit(empty_bar(s));                       // slot reusable once these MMAs have read it
+          if (kb == num_kb - 1) umma_commit(acc_full(buf));  // this tile's accumulator is complete
         }
-        umma_commit(acc_full(buf));  // this tile's accumulator is complete
-        aphase[buf] ^= 1u;
-        buf ^= 1;
+        __syncwarp();
+        lo += Cfg::kStageBytes >> 4;
+        if (++s == Cfg::kStages) { s = 0; phase ^= 1u; lo = lo0; }
       }
+      aphase ^= buf;
+      buf ^= 1u;
     }
   } else {
     // ===== epilogue warps: TMEM -> registers -> global, one tile behind the MMA warp =====
@@ -222,7 +226,7 @@ gemm_persist_pair_kernel(const __grid_constant__ CUtensorMap w_map64, const __gr
   auto a_tile = [&](int s) { return smem_base + s * Cfg::kStageBytes; };
   auto b_tile = [&](int s) { return a_tile(s) + Cfg::kABytes; };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   const int num_kb = (K + kBK - 1) / kBK;
   const int n_tiles = tiles_n * tiles_t;
   auto tile_n0 = [&](int tile) { return (t_fast ? tile / tiles_t : tile % tiles_n) * kHalf; };
@@ -263,28 +267,31 @@ gemm_persist_pair_kernel(const __grid_constant__ CUtensorMap w_map64, const __gr
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc<BN>();
-      int s = 0, buf = 0;
-      uint32_t phase = 0, aphase[2] = {0u, 0u};
-      for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        mbar_wait(acc_empty(buf), aphase[buf] ^ 1u);
+    constexpr uint32_t idesc = umma_idesc<BN>();
+    const uint32_t lo0 = umma_lo(smem_base);
+    uint32_t lo = lo0;
+    int s = 0;
+    uint32_t phase = 0, buf = 0, aphase = 0;
+    for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+      mbar_wait(acc_empty(buf), aphase ^ 1u);
+      tc_fence_after();
+      const uint32_t acc_addr = tmem_base + buf * BN;
+      for (int kb = 0; kb < num_kb; kb++) {
+        mbar_wait(full_bar(s), phase);
         tc_fence_after();
-        const uint32_t acc_addr = tmem_base + (uint32_t)(buf * BN);
-        for (int kb = 0; kb < num_kb; kb++) {
-          mbar_wait(full_bar(s), phase);
-          tc_fence_after();
+        if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kBK / 16; k++)
-            umma_bf16(acc_addr, umma_desc_sw128(a_tile(s) + k * 32), umma_desc_sw128(b_tile(s) + k * 32), idesc,
-                      (kb > 0 || k > 0) ? 1u : 0u);
+          for (uint32_t k = 0; k < kBK / 16; k++)
+            umma_ss(acc_addr, lo + 2 * k, lo + (Cfg::kABytes >> 4) + 2 * k, idesc, k > 0 ? 1u : (uint32_t)(kb > 0));
           umma_commit(empty_bar(s));
-          if (++s == Cfg::kStages) { s = 0; phase ^= 1u; }
+          if (kb == num_kb - 1) umma_commit(acc_full(buf));
         }
-        umma_commit(acc_full(buf));
-        aphase[buf] ^= 1u;
-        buf ^= 1;
+        __syncwarp();
+        lo += Cfg::kStageBytes >> 4;
+        if (++s == Cfg::kStages) { s = 0; phase ^= 1u; lo = lo0; }
       }
+      aphase ^= buf;
+      buf ^= 1u;
     }
   } else {
     const int quarter = warp & 3;

@@ -70,7 +70,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
   auto a2_tile = [&](int s) { return a_tile(s) + a_bytes; };
   auto b_tile = [&](int s) { return a_tile(s) + (kDual ? 2u : 1u) * a_bytes; };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp(), lane = threadIdx.x & 31;
   // tile_rows (<= 128, the weight map's box height) output features per CTA: a 128-row MMA runs on a
   // partly filled A tile; lanes >= tile_rows compute on stale shared memory and are never stored.
   const int n0 = blockIdx.x * tile_rows;
@@ -128,26 +128,30 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    // ===== MMA issuer (one thread) =====
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc<BN>();
-      int s = 0;
-      uint32_t phase = 0;
-      for (int kb = kb0; kb < kb1; kb++) {
-        mbar_wait(full_bar(s), phase);
-        tc_fence_after();
+    // ===== MMA issuer: the warp converged, one elected lane issues (ptx.cuh: the issue path) =====
+    constexpr uint32_t idesc = umma_idesc<BN>();
+    int s = 0;
+    uint32_t phase = 0;
+    const uint32_t lo0 = umma_lo(smem_base), lo_step = stage_bytes >> 4, a2_off = a_bytes >> 4, b_off = ((kDual ? 2u : 1u) * a_bytes) >> 4;
+    uint32_t lo = lo0;
+    for (int kb = kb0; kb < kb1; kb++) {
+      mbar_wait(full_bar(s), phase);
+      tc_fence_after();
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < kBK / 16; k++) {
-          const uint32_t acc = (kb > kb0 || k > 0) ? 1u : 0u;
-          const uint64_t bd = umma_desc_sw128(b_tile(s) + k * 32);
-          umma_bf16(tmem_base, umma_desc_sw128(a_tile(s) + k * 32), bd, idesc, acc);
-          if (kDual) umma_bf16(tmem_base + BN, umma_desc_sw128(a2_tile(s) + k * 32), bd, idesc, acc);
+        for (uint32_t k = 0; k < kBK / 16; k++) {
+          const uint32_t acc = k > 0 ? 1u : (uint32_t)(kb > kb0);
+          umma_ss(tmem_base, lo + 2 * k, lo + b_off + 2 * k, idesc, acc);
+          if (kDual) umma_ss(tmem_base + BN, lo + a2_off + 2 * k, lo + b_off + 2 * k, idesc, acc);
         }
         umma_commit(empty_bar(s));  // slot reusable once these MMAs have read it
-        if (++s == n_stages) { s = 0; phase ^= 1u; }
       }
-      umma_commit(tmem_full_bar);  // accumulator complete
+      __syncwarp();
+      lo += lo_step;
+      if (++s == n_stages) { s = 0; phase ^= 1u; lo = lo0; }
     }
+    if (elect_one()) umma_commit(tmem_full_bar);  // accumulator complete
+    __syncwarp();
   } else {
     // ===== epilogue: TMEM -> registers -> global =====
     mbar_wait(tmem_full_bar, 0);

@@ -66,24 +66,17 @@ template <int kCols>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "n"(kCols) : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem]^T, bf16 x bf16 -> fp32
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // The issue path.  A batch of MMAs costs its issuing thread some twenty dependent instructions each when every descriptor is built
 // from an address in front of it (measured with clock stamps: 140 clocks per MMA on a busy SM, against 32 to 64 that the MMA takes), so
 // the descriptors' upper halves are a constant (SBO = 1024 bytes, version 1, 128B swizzle), the lower halves are built once and
 // stepped by an add, and the issuing warp runs its loop converged, with one elected lane for the MMAs, so that these values stay in
 // uniform registers.
+// Shared-memory matrix descriptor, canonical 128B-swizzle layout (rows of 64 bf16 = 128 B, 8-row groups 1024 B apart):
+// start >> 4 | LBO << 16 | SBO << 32 | version 1 << 46 | SW128 << 61.
 constexpr uint32_t kUmmaDescHi = 64u | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t umma_lo(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16); }  // K-major
 __device__ __forceinline__ uint32_t umma_lo_mn(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr >> 4) & 0x3FFFu) | ((lbo_bytes >> 4) << 16); }
+// D[tmem] (+)= A[smem] * B[smem]^T, bf16 x bf16 -> fp32
 __device__ __forceinline__ void umma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
@@ -129,11 +122,6 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// Shared-memory matrix descriptor, K-major operand in the canonical 128B-swizzle layout
-// (rows of 64 bf16 = 128 B, 8-row groups 1024 B apart): start>>4 | LBO=1 | SBO=64 | version=1 | SW128.
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
-  return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
 // Instruction descriptor: D=f32, A=B=bf16, both K-major, M=128, N=kN.
 template <int kN>
 __host__ __device__ constexpr uint32_t umma_idesc() {
