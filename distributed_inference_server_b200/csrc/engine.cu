@@ -766,6 +766,8 @@ cudaError_t Engine::enqueue_layers(int T, int n_splits) {
 // final norm on the rows that need logits, lm_head, sampling
 cudaError_t Engine::enqueue_head(int R, bool all_greedy) {
   const int H = m.hidden;
+  struct PdlOff { ~PdlOff() { pdl_enabled() = false; } } pdl_off;
+  pdl_enabled() = use_pdl && !profiling && tp_size == 1;  // the norm, the head's product and the sampler follow kernels on this stream
   prof_mark(P_HEAD_NORM);
   RET_CUDA(consume_pending(final_norm, rowmap_identity ? nullptr : cur_meta->d<int>(cur_meta->o_rowmap), R, last_T));
   const bool gemv = (cfg.flags & DIS_FLAG_FORCE_GEMV) || R <= gemv_max_t;

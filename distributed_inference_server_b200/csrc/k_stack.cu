@@ -3,6 +3,7 @@
 // per-slot tail, the two recurrences, latent attention over paged latents, the clamped gated unit and the expert router.
 // Everything the family defines as 32-bit -- norms, decays, recurrent state, scores and softmax, routers, the residual --
 // is fp32 here whatever the element type of the matrices.
+#include "ptx.cuh"
 #include "stack_dev.cuh"
 
 namespace dis {
@@ -15,6 +16,8 @@ constexpr int GB = kStackGemmTile, GK = 16;
 
 template <bool AF32, bool WF32>
 __global__ void __launch_bounds__(256) stack_gemm_kernel(StackGemm g) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float As[GK][GB + 4], Ws[GK][GB + 4];
   int row0, rows, grp = 0;
   if (g.tiles) {
@@ -122,6 +125,8 @@ __device__ __forceinline__ void unpack8(const FewRaw<WF32> &r, float (&w)[8]) {
 }
 template <bool AF32, bool WF32>
 __global__ void __launch_bounds__(256) stack_gemm_few_kernel(StackGemm g) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ __align__(16) float as[kFewRows][kFewK];
   int row0, rows, grp = 0;
   if (g.tiles) {
@@ -215,23 +220,25 @@ cudaError_t launch_stack_gemm(const StackGemm &g, cudaStream_t st) {
   if (few) {
     dim3 grid(g.tiles ? g.max_tiles : (g.M + kStackGemmTile - 1) / kStackGemmTile, (g.N + kFewCols - 1) / kFewCols, g.batch);
     if (grid.x == 0) return cudaSuccess;
-    if (g.a_f32 && g.w_f32) stack_gemm_few_kernel<true, true><<<grid, 256, 0, st>>>(g);
-    else if (g.a_f32) stack_gemm_few_kernel<true, false><<<grid, 256, 0, st>>>(g);
-    else if (g.w_f32) stack_gemm_few_kernel<false, true><<<grid, 256, 0, st>>>(g);
-    else stack_gemm_few_kernel<false, false><<<grid, 256, 0, st>>>(g);
+    if (g.a_f32 && g.w_f32) launch_k(stack_gemm_few_kernel<true, true>, dim3(grid), dim3(256), 0, st, g);
+    else if (g.a_f32) launch_k(stack_gemm_few_kernel<true, false>, dim3(grid), dim3(256), 0, st, g);
+    else if (g.w_f32) launch_k(stack_gemm_few_kernel<false, true>, dim3(grid), dim3(256), 0, st, g);
+    else launch_k(stack_gemm_few_kernel<false, false>, dim3(grid), dim3(256), 0, st, g);
     return cudaGetLastError();
   }
   dim3 grid(g.tiles ? g.max_tiles : (g.M + GB - 1) / GB, (g.N + GB - 1) / GB, g.batch);
   if (grid.x == 0) return cudaSuccess;
-  if (g.a_f32 && g.w_f32) stack_gemm_kernel<true, true><<<grid, 256, 0, st>>>(g);
-  else if (g.a_f32) stack_gemm_kernel<true, false><<<grid, 256, 0, st>>>(g);
-  else if (g.w_f32) stack_gemm_kernel<false, true><<<grid, 256, 0, st>>>(g);
-  else stack_gemm_kernel<false, false><<<grid, 256, 0, st>>>(g);
+  if (g.a_f32 && g.w_f32) launch_k(stack_gemm_kernel<true, true>, dim3(grid), dim3(256), 0, st, g);
+  else if (g.a_f32) launch_k(stack_gemm_kernel<true, false>, dim3(grid), dim3(256), 0, st, g);
+  else if (g.w_f32) launch_k(stack_gemm_kernel<false, true>, dim3(grid), dim3(256), 0, st, g);
+  else launch_k(stack_gemm_kernel<false, false>, dim3(grid), dim3(256), 0, st, g);
   return cudaGetLastError();
 }
 
 __global__ void stack_sum_bias_kernel(const float *part, int n_part, long long stride, const float *bias, float *out, long long n,
                                       int N) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s = bias ? bias[i % N] : 0.f;
     for (int k = 0; k < n_part; k++) s += part[(long long)k * stride + i];
@@ -242,7 +249,7 @@ cudaError_t launch_stack_sum_bias(const float *part, int n_part, long long strid
                                   cudaStream_t st) {
   const long long n = (long long)M * N;
   if (n <= 0) return cudaSuccess;
-  stack_sum_bias_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(part, n_part, stride, bias, out, n, N);
+  launch_k(stack_sum_bias_kernel, dim3((int)std::min<long long>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, part, n_part, stride, bias, out, n, N);
   return cudaGetLastError();
 }
 
@@ -253,6 +260,8 @@ cudaError_t launch_stack_sum_bias(const float *part, int n_part, long long strid
 template <bool F32>
 __global__ void stack_embed_kernel(const void *embed, const uint32_t *tokens, const int *pos, const double *pos_freq, float *x, float *x0,
                                    float scale, int W, int S) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long t = blockIdx.x;
   const long long row = tokens[t];
   const int p = pos_freq ? pos[t] : 0;
@@ -270,13 +279,15 @@ __global__ void stack_embed_kernel(const void *embed, const uint32_t *tokens, co
 cudaError_t launch_stack_embed(const void *embed, bool f32, const uint32_t *tokens, const int *pos, const double *pos_freq, float *x,
                                float *x0, float scale, int T, int W, int streams, cudaStream_t st) {
   if (streams < 1) streams = 1;
-  if (f32) stack_embed_kernel<true><<<T, 128, 0, st>>>(embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
-  else stack_embed_kernel<false><<<T, 128, 0, st>>>(embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
+  if (f32) launch_k(stack_embed_kernel<true>, dim3(T), dim3(128), 0, st, embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
+  else launch_k(stack_embed_kernel<false>, dim3(T), dim3(128), 0, st, embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
   return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(256) stack_resid_norm_kernel(float *x, const float *y, const float *post, const float *pre,
                                                                float *hn, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sh[32];
   const long long t = blockIdx.x;
   float *xr = x + t * W;
@@ -297,12 +308,14 @@ __global__ void __launch_bounds__(256) stack_resid_norm_kernel(float *x, const f
 }
 cudaError_t launch_stack_resid_norm(float *x, const float *y, const float *post, const float *pre, float *hn, int T, int W,
                                     float eps, cudaStream_t st) {
-  stack_resid_norm_kernel<<<T, 256, 0, st>>>(x, y, post, pre, hn, W, eps);
+  launch_k(stack_resid_norm_kernel, dim3(T), dim3(256), 0, st, x, y, post, pre, hn, W, eps);
   return cudaGetLastError();
 }
 
 template <bool F32>
 __global__ void stack_final_norm_kernel(const float *x, const int *row_map, const float *g, void *out, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sh[32];
   const long long r = blockIdx.x;
   const float *xr = x + (long long)(row_map ? row_map[r] : r) * W;
@@ -314,8 +327,8 @@ __global__ void stack_final_norm_kernel(const float *x, const int *row_map, cons
 }
 cudaError_t launch_stack_final_norm(const float *x, const int *row_map, const float *g, void *out, bool f32, int R, int W, float eps,
                                     cudaStream_t st) {
-  if (f32) stack_final_norm_kernel<true><<<R, 256, 0, st>>>(x, row_map, g, out, W, eps);
-  else stack_final_norm_kernel<false><<<R, 256, 0, st>>>(x, row_map, g, out, W, eps);
+  if (f32) launch_k(stack_final_norm_kernel<true>, dim3(R), dim3(256), 0, st, x, row_map, g, out, W, eps);
+  else launch_k(stack_final_norm_kernel<false>, dim3(R), dim3(256), 0, st, x, row_map, g, out, W, eps);
   return cudaGetLastError();
 }
 
@@ -330,6 +343,8 @@ __global__ void __launch_bounds__(256) stack_boundary_ln_kernel(float *x, const 
                                                                 const float *post_w, const float *post_b, const float *pre_w,
                                                                 const float *pre_b, float *hn, void *hc, const float *x0, void *cat,
                                                                 int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float row[];  // [W]
   __shared__ float sh[32];
   const long long t = blockIdx.x;
@@ -473,7 +488,7 @@ cudaError_t launch_stack_boundary_ln(float *x, const float *y, int n_part, long 
   }));
   const size_t shb = (size_t)W * 4;
 #define DIS_BOUNDARY(F, R) \
-  stack_boundary_ln_kernel<F, R><<<T, 256, shb, st>>>(x, y, n_part, stride, bias, post_w, post_b, pre_w, pre_b, hn, hc, x0, cat, W, eps)
+  launch_k(stack_boundary_ln_kernel<F, R>, dim3(T), dim3(256), (size_t)(shb), st, x, y, n_part, stride, bias, post_w, post_b, pre_w, pre_b, hn, hc, x0, cat, W, eps)
   if (f32 && rms) DIS_BOUNDARY(true, true);
   else if (f32) DIS_BOUNDARY(true, false);
   else if (rms) DIS_BOUNDARY(false, true);
@@ -486,6 +501,8 @@ cudaError_t launch_stack_boundary_ln(float *x, const float *y, int n_part, long 
 template <bool F32>
 __global__ void stack_final_ln_kernel(const float *x, const int *row_map, const float *w, const float *b, void *out, int W, float eps,
                                       float scale, int S) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float frow[];  // [W] when S > 1
   __shared__ float sh[32];
   const long long r = blockIdx.x;
@@ -519,8 +536,8 @@ cudaError_t launch_stack_final_ln(const float *x, const int *row_map, const floa
     cudaError_t e = cudaFuncSetAttribute(stack_final_ln_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
     return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_final_ln_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
   }));
-  if (f32) stack_final_ln_kernel<true><<<R, 256, shb, st>>>(x, row_map, w, b, out, W, eps, scale, streams);
-  else stack_final_ln_kernel<false><<<R, 256, shb, st>>>(x, row_map, w, b, out, W, eps, scale, streams);
+  if (f32) launch_k(stack_final_ln_kernel<true>, dim3(R), dim3(256), (size_t)(shb), st, x, row_map, w, b, out, W, eps, scale, streams);
+  else launch_k(stack_final_ln_kernel<false>, dim3(R), dim3(256), (size_t)(shb), st, x, row_map, w, b, out, W, eps, scale, streams);
   return cudaGetLastError();
 }
 
@@ -537,6 +554,8 @@ template <bool F32, int SS, bool VEC>
 __global__ void __launch_bounds__(256) stack_boundary_hc_kernel(float *xs, int S_rt, const float *__restrict__ y, int n_part, long long stride,
                                                                 const float *__restrict__ bias, const float *prev, const float *next,
                                                                 const float *__restrict__ pre_w, void *hc, int W, float eps, float mult) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float row[];  // [W]: u
   __shared__ float sh[32];
   __shared__ float cf[2 * kHcMaxStreams + kHcMaxStreams * kHcMaxStreams];  // out[S] | mix[S][S] of prev, then in[S] of next
@@ -641,7 +660,7 @@ static cudaError_t boundary_hc_go(float *xs, int streams, const float *y, int n_
                                   const float *next, const float *pre_w, void *hc, int T, int W, float eps, float mult, cudaStream_t st) {
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_boundary_hc_kernel<F32, SS, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); }));
-  stack_boundary_hc_kernel<F32, SS, VEC><<<T, 256, (size_t)W * 4, st>>>(xs, streams, y, n_part, stride, bias, prev, next, pre_w, hc, W, eps, mult);
+  launch_k(stack_boundary_hc_kernel<F32, SS, VEC>, dim3(T), dim3(256), (size_t)((size_t)W * 4), st, xs, streams, y, n_part, stride, bias, prev, next, pre_w, hc, W, eps, mult);
   return cudaGetLastError();
 }
 cudaError_t launch_stack_boundary_hc(float *xs, int streams, const float *y, int n_part, long long stride, const float *bias,
@@ -665,6 +684,8 @@ cudaError_t launch_stack_boundary_hc(float *xs, int streams, const float *y, int
 template <bool F32, bool VEC>
 __global__ void __launch_bounds__(256) stack_boundary_par_kernel(float *x, StackParBoundary b, float mult, const float *__restrict__ w1, void *h1,
                                                                  const float *__restrict__ w2, void *h2, int W, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float row[];  // [W]
   __shared__ float sh[32], wts[32];
   __shared__ long long at[32];  // offsets of the experts' rows
@@ -773,7 +794,7 @@ cudaError_t launch_stack_boundary_par(float *x, const StackParBoundary &b, float
   do {                                                                                                                                                  \
     static DeviceOnce once;                                                                                                                             \
     DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_boundary_par_kernel<F, VV>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); })); \
-    stack_boundary_par_kernel<F, VV><<<T, 256, (size_t)W * 4, st>>>(x, b, mult, w1, h1, w2, h2, W, eps);                                               \
+    launch_k(stack_boundary_par_kernel<F, VV>, dim3(T), dim3(256), (size_t)((size_t)W * 4), st, x, b, mult, w1, h1, w2, h2, W, eps);                                               \
   } while (0)
   if (f32 && vec) DIS_PAR(true, true);
   else if (f32) DIS_PAR(true, false);
@@ -784,21 +805,25 @@ cudaError_t launch_stack_boundary_par(float *x, const StackParBoundary &b, float
 }
 
 __global__ void stack_scale_kernel(float *v, long long n, float s) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) v[i] *= s;
 }
 cudaError_t launch_stack_scale(float *v, long long n, float s, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  stack_scale_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(v, n, s);
+  launch_k(stack_scale_kernel, dim3((int)std::min<long long>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, v, n, s);
   return cudaGetLastError();
 }
 
 __global__ void stack_softcap_kernel(float *v, long long n, float cap, float inv) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     v[i] = cap * tanhf(v[i] * inv);
 }
 cudaError_t launch_stack_softcap(float *v, long long n, float cap, cudaStream_t st) {
   if (n <= 0 || !(cap > 0.f)) return cudaSuccess;
-  stack_softcap_kernel<<<(int)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(v, n, cap, 1.f / cap);
+  launch_k(stack_softcap_kernel, dim3((int)std::min<long long>((n + 255) / 256, 148 * 8)), dim3(256), 0, st, v, n, cap, 1.f / cap);
   return cudaGetLastError();
 }
 
@@ -810,6 +835,8 @@ constexpr int kCanonMaxTaps = 16;
 
 template <bool F32>
 __global__ void stack_canon_kernel(const float *hn, const float *w, const float *state, StackSpans sp, void *hc, int W, int taps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x;
   const int s = sp.span[t], tok0 = sp.sp_tok0[s], pos0 = sp.sp_pos0[s], slot = sp.sp_slot[s];
   const int back_in_span = t - tok0;  // tokens of the span in front of t
@@ -832,6 +859,8 @@ __global__ void stack_canon_kernel(const float *hn, const float *w, const float 
 }
 
 __global__ void stack_canon_state_kernel(const float *hn, float *state, StackSpans sp, int W, int taps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x;
   const int tok0 = sp.sp_tok0[s], len = sp.sp_len[s], pos0 = sp.sp_pos0[s], slot = sp.sp_slot[s];
   float *tail = state + (long long)slot * (taps - 1) * W;
@@ -850,9 +879,9 @@ __global__ void stack_canon_state_kernel(const float *hn, float *state, StackSpa
 cudaError_t launch_stack_canon(const float *hn, const float *w, float *state, const StackSpans &sp, void *hc, bool f32, int W,
                                int taps, cudaStream_t st) {
   if (taps < 1 || taps > kCanonMaxTaps) return cudaErrorInvalidValue;
-  if (f32) stack_canon_kernel<true><<<sp.T, 256, 0, st>>>(hn, w, state, sp, hc, W, taps);
-  else stack_canon_kernel<false><<<sp.T, 256, 0, st>>>(hn, w, state, sp, hc, W, taps);
-  if (taps > 1) stack_canon_state_kernel<<<sp.n_spans, 256, 0, st>>>(hn, state, sp, W, taps);
+  if (f32) launch_k(stack_canon_kernel<true>, dim3(sp.T), dim3(256), 0, st, hn, w, state, sp, hc, W, taps);
+  else launch_k(stack_canon_kernel<false>, dim3(sp.T), dim3(256), 0, st, hn, w, state, sp, hc, W, taps);
+  if (taps > 1) launch_k(stack_canon_state_kernel, dim3(sp.n_spans), dim3(256), 0, st, hn, state, sp, W, taps);
   return cudaGetLastError();
 }
 
@@ -864,6 +893,8 @@ template <bool F32>
 __global__ void __launch_bounds__(256) stack_boundary_single_kernel(float *x, const float *y, int n_part, long long stride, const float *bias,
                                                                     const float *post, const float *pre, const float *cw, float *cstate,
                                                                     StackSpans sp, void *hc, int W, int taps, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float row[];  // [W]
   __shared__ float sh[32];
   const long long t = blockIdx.x;
@@ -913,20 +944,22 @@ cudaError_t launch_stack_boundary_single(float *x, const float *y, int n_part, l
     return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_boundary_single_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
   }));
   const size_t shb = (size_t)W * 4;
-  if (f32) stack_boundary_single_kernel<true><<<sp.T, 256, shb, st>>>(x, y, n_part, stride, bias, post, pre, cw, cstate, sp, hc, W, taps, eps);
-  else stack_boundary_single_kernel<false><<<sp.T, 256, shb, st>>>(x, y, n_part, stride, bias, post, pre, cw, cstate, sp, hc, W, taps, eps);
+  if (f32) launch_k(stack_boundary_single_kernel<true>, dim3(sp.T), dim3(256), (size_t)(shb), st, x, y, n_part, stride, bias, post, pre, cw, cstate, sp, hc, W, taps, eps);
+  else launch_k(stack_boundary_single_kernel<false>, dim3(sp.T), dim3(256), (size_t)(shb), st, x, y, n_part, stride, bias, post, pre, cw, cstate, sp, hc, W, taps, eps);
   return cudaGetLastError();
 }
 
 template <bool F32>
 __global__ void stack_copy_act_kernel(const float *hn, void *hc, long long n) {
+  pdl_launch_dependents();
+  pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
     st_el<F32>(hc, i, hn[i]);
 }
 cudaError_t launch_stack_copy_act(const float *hn, void *hc, bool f32, long long n, cudaStream_t st) {
   const int grid = (int)std::min<long long>((n + 255) / 256, 148 * 8);
-  if (f32) stack_copy_act_kernel<true><<<grid, 256, 0, st>>>(hn, hc, n);
-  else stack_copy_act_kernel<false><<<grid, 256, 0, st>>>(hn, hc, n);
+  if (f32) launch_k(stack_copy_act_kernel<true>, dim3(grid), dim3(256), 0, st, hn, hc, n);
+  else launch_k(stack_copy_act_kernel<false>, dim3(grid), dim3(256), 0, st, hn, hc, n);
   return cudaGetLastError();
 }
 
@@ -945,6 +978,8 @@ __device__ __forceinline__ float glu_unit(float g, float u, float limit) {
 template <bool F32, int ACT, bool VEC>
 __global__ void stack_glu_kernel(const float *__restrict__ gu, int n_part, long long stride, const float *__restrict__ bias,
                                  void *__restrict__ act, const int *rows_ptr, int M, int ff, float limit, long long ld_gu, long long ld_act) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int rows = rows_ptr ? min(M, rows_ptr[0]) : M;
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     constexpr bool GATED = ACT != DIS_ACT_RELU2;
@@ -991,7 +1026,7 @@ cudaError_t launch_stack_glu(const float *gu, int n_part, long long stride, cons
   const int per = vec ? 4 : 1;
   // few rows: the columns are spread over grid.y as well
   const dim3 grid(std::min(M, 148 * 16), M >= 512 ? 1 : std::min((ff + 256 * per - 1) / (256 * per), 16));
-#define DIS_GLU(F, A, V) stack_glu_kernel<F, A, V><<<grid, 256, 0, st>>>(gu, n_part, stride, bias, act, rows_ptr, M, ff, limit, ld_gu, ld_act)
+#define DIS_GLU(F, A, V) launch_k(stack_glu_kernel<F, A, V>, dim3(grid), dim3(256), 0, st, gu, n_part, stride, bias, act, rows_ptr, M, ff, limit, ld_gu, ld_act)
 #define DIS_GLU_ACT(A)                     \
   do {                                     \
     if (f32 && vec) DIS_GLU(true, A, true); \
@@ -1036,6 +1071,8 @@ __global__ void __launch_bounds__(kRouteWarps * 32) stack_route_kernel(const voi
                                                                        int top, int kind, const float *__restrict__ correction, int groups,
                                                                        int keep, const float *__restrict__ extra, float *extra_out,
                                                                        int *idx, float *wt) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float zs[];  // per token: [E] logits (sigmoid scores), [E] choice scores, [groups] run scores, [groups] kept flags;
                                  // then [E] correction, [warps][TB] partial sums of the extra row
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -1251,7 +1288,7 @@ cudaError_t launch_stack_route(const void *hc, bool f32, const float *router, in
   const size_t sh = (size_t)(tb * per_tok + E + tb * kRouteWarps) * sizeof(float);
   const int grid = (T + tb - 1) / tb, th = kRouteWarps * 32;
 #define DIS_ROUTE(F, B) \
-  stack_route_kernel<F, B><<<grid, th, sh, st>>>(hc, router, T, W, E, top, kind, correction, groups, keep, extra, extra_out, idx, wt)
+  launch_k(stack_route_kernel<F, B>, dim3(grid), dim3(th), (size_t)(sh), st, hc, router, T, W, E, top, kind, correction, groups, keep, extra, extra_out, idx, wt)
   if (f32 && tb == 8) DIS_ROUTE(true, 8);
   else if (f32) DIS_ROUTE(true, 1);
   else if (tb == 8) DIS_ROUTE(false, 8);
@@ -1265,6 +1302,8 @@ cudaError_t launch_stack_route(const void *hc, bool f32, const float *router, in
 // threads arrive; a row's result does not depend on where in the range it lies, so the values are the same run to run.
 __global__ void stack_moe_plan_kernel(const int *idx, int n, int top, int E, int tile_rows, int *counts, int *perm_tok, int *where,
                                       int *tiles, int max_tiles) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ int sh[];  // [E] counts, [E] cursors
   int *cnt = sh, *cur = sh + E;
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
@@ -1293,20 +1332,22 @@ __global__ void stack_moe_plan_kernel(const int *idx, int n, int top, int E, int
 }
 cudaError_t launch_stack_moe_plan(const int *idx, int T, int top, int E, int tile_rows, int *counts, int *perm_tok, int *where,
                                   int *tiles, int max_tiles, cudaStream_t st) {
-  stack_moe_plan_kernel<<<1, 1024, (size_t)2 * E * sizeof(int), st>>>(idx, T * top, top, E, tile_rows, counts, perm_tok, where, tiles,
+  launch_k(stack_moe_plan_kernel, dim3(1), dim3(1024), (size_t)((size_t)2 * E * sizeof(int)), st, idx, T * top, top, E, tile_rows, counts, perm_tok, where, tiles,
                                                                       max_tiles);
   return cudaGetLastError();
 }
 
 // rows of the expert row space, in bf16: row o = activation row perm_tok[o]
 __global__ void stack_moe_gather_kernel(const uint16_t *hc, const int *perm_tok, uint16_t *xs, int W) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long o = blockIdx.x;
   const uint16_t *src = hc + (long long)perm_tok[o] * W;
   for (int i = threadIdx.x; i < W; i += blockDim.x) xs[o * W + i] = src[i];
 }
 cudaError_t launch_stack_moe_gather(const void *hc, const int *perm_tok, void *xs, int rows, int W, cudaStream_t st) {
   if (rows <= 0) return cudaSuccess;
-  stack_moe_gather_kernel<<<rows, 128, 0, st>>>(reinterpret_cast<const uint16_t *>(hc), perm_tok, reinterpret_cast<uint16_t *>(xs), W);
+  launch_k(stack_moe_gather_kernel, dim3(rows), dim3(128), 0, st, reinterpret_cast<const uint16_t *>(hc), perm_tok, reinterpret_cast<uint16_t *>(xs), W);
   return cudaGetLastError();
 }
 
@@ -1314,6 +1355,8 @@ cudaError_t launch_stack_moe_gather(const void *hc, const int *perm_tok, void *x
 // joins here behind its per-token gate
 __global__ void stack_moe_combine_kernel(const float *rows, const int *where, const float *wt, const float *shared, int n_part,
                                          long long stride, const float *shared_gate, float *y, int W, int top) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long t = blockIdx.x;
   const float sg = shared ? (shared_gate ? sigmoid_precise(shared_gate[t]) : 1.f) : 0.f;  // no gate: the shared unit joins as it is
   if (((W | (int)(stride & 3)) & 3) == 0) {  // four columns per thread and step, 16-byte accesses
@@ -1350,7 +1393,7 @@ __global__ void stack_moe_combine_kernel(const float *rows, const int *where, co
 }
 cudaError_t launch_stack_moe_combine(const float *rows, const int *where, const float *wt, const float *shared, int n_part,
                                      long long stride, const float *shared_gate, float *y, int T, int W, int top, cudaStream_t st) {
-  stack_moe_combine_kernel<<<T, 256, 0, st>>>(rows, where, wt, shared, n_part < 1 ? 1 : n_part, stride, shared_gate, y, W, top);
+  launch_k(stack_moe_combine_kernel, dim3(T), dim3(256), 0, st, rows, where, wt, shared, n_part < 1 ? 1 : n_part, stride, shared_gate, y, W, top);
   return cudaGetLastError();
 }
 

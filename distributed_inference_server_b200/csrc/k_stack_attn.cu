@@ -5,6 +5,7 @@
 // softmax (optionally with a per-head sink logit in the denominator) or per-head sigmoid weights, under a causal mask that may
 // be cut into chunks of positions, over the whole visible history or a slice of it, with an optional per-head sigmoid gate on
 // the output.  Scores, weights, norms and angles are fp32 (angles are formed in double) whatever the cache's element type.
+#include "ptx.cuh"
 #include "stack_dev.cuh"
 
 namespace dis {
@@ -24,6 +25,8 @@ __global__ void __launch_bounds__(512) stack_attn_prep_kernel(const float *proj,
                                                               const double *vfreq, StackAttn c, StackSpans sp, float *qf, void *kpool,
                                                               void *vpool, float *vrot, const int *page_table, int max_pages,
                                                               int page_size, StackVMix mix) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float tab[];  // cos [half], sin [half], value cos [dv/2], value sin [dv/2], per-head factors [H + G], summed row
   const int HM = c.H * c.maps, GM = c.G * c.maps;  // heads of queries and keys, each map a head of its own here
   const int srow_off = (c.rot_dims + c.dv + HM + GM + 3) & ~3;  // the summed row starts on a 16-byte boundary
@@ -143,8 +146,8 @@ cudaError_t launch_stack_attn_prep(const float *proj, long long ld, int n_part, 
     return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_attn_prep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   }));
   const int th = sp.T <= 148 ? 512 : 128;  // few tokens: a block per token leaves the GPU empty, so the blocks are large
-  if (f32) stack_attn_prep_kernel<true><<<sp.T, th, sh, st>>>(proj, ld, n_part, stride, n_cols, gate_off, gate_out, ld_gate, q_off, k_off, v_off, bias, qn, kn, freq, vfreq, c, sp, qf, kpool, vpool, vrot, page_table, max_pages, page_size, mix);
-  else stack_attn_prep_kernel<false><<<sp.T, th, sh, st>>>(proj, ld, n_part, stride, n_cols, gate_off, gate_out, ld_gate, q_off, k_off, v_off, bias, qn, kn, freq, vfreq, c, sp, qf, kpool, vpool, vrot, page_table, max_pages, page_size, mix);
+  if (f32) launch_k(stack_attn_prep_kernel<true>, dim3(sp.T), dim3(th), (size_t)(sh), st, proj, ld, n_part, stride, n_cols, gate_off, gate_out, ld_gate, q_off, k_off, v_off, bias, qn, kn, freq, vfreq, c, sp, qf, kpool, vpool, vrot, page_table, max_pages, page_size, mix);
+  else launch_k(stack_attn_prep_kernel<false>, dim3(sp.T), dim3(th), (size_t)(sh), st, proj, ld, n_part, stride, n_cols, gate_off, gate_out, ld_gate, q_off, k_off, v_off, bias, qn, kn, freq, vfreq, c, sp, qf, kpool, vpool, vrot, page_table, max_pages, page_size, mix);
   return cudaGetLastError();
 }
 
@@ -211,6 +214,8 @@ __global__ void __launch_bounds__(kAtWarps * 32) stack_attn_kernel(const float *
                                                                    const float *pb, const float *sink, StackAttn c, StackSpans sp, const int *qb_tok0,
                                                                    const int *qb_len, const int *page_table, int max_pages,
                                                                    int page_size, AttnOut o, int keys_per_split, float *part) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float shm[];
   // with two maps a head counts twice: pair p = ((token * heads of the group) + head) * maps + map, a key row holds both maps
   const int maps = c.maps, d = c.d, dk = d * maps, dv = c.dv, DP = dk + 1, VP = dv + 1, R = c.H / c.G * maps, g = blockIdx.y;
@@ -335,6 +340,8 @@ __global__ void __launch_bounds__(kAtWarps * 32) stack_attn_kernel(const float *
 // Slices that lie wholly behind the token (nothing visible) wrote m = -inf, l = 0 and zeros.
 template <bool F32, bool SIG>
 __global__ void stack_attn_merge_kernel(const float *part, int n_split, int T, int H, int dv, AttnOut o) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float msh[];  // [dv] merged sums, [n_split] factors
   float *a = msh, *ws = msh + dv;
   __shared__ float inv_den;
@@ -377,6 +384,8 @@ __global__ void stack_attn_merge_kernel(const float *part, int n_split, int T, i
 template <bool F32>
 __global__ void __launch_bounds__(128) stack_attn_merge_maps_kernel(const float *part, int n_split, int T, int H, int dv, AttnOut o, float lambda,
                                                                     float diff_out, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float msh[];  // [dv] joined sums, [2][n_split] factors
   float *a = msh, *ws = msh + dv;
   __shared__ float sh[32];
@@ -533,6 +542,8 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
                                                                        const float *pb, const float *sink, StackAttn c, StackSpans sp, const int *qb_tok0,
                                                                        const int *qb_len, const int *page_table, int max_pages,
                                                                        int page_size, AttnOut o, int keys_per_split, float *part) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int KP = DQ * (DIFF ? 2 : 1) + 8, VP = DV + 8;  // elements per shared row: 16-byte rows land in distinct bank groups
   extern __shared__ __align__(16) uint16_t smem[];
   uint16_t *Ks = smem;                               // [2][64][KP]
@@ -850,7 +861,7 @@ static cudaError_t attn_mma_go(const float *qf, long long ldq, const AttnKV &kv,
     const int dqm = c.d <= 64 ? 64 : 128, dvm = small ? 64 : 128;
     const size_t shd = std::max((size_t)2 * kMmKeys * (2 * dqm + dvm + 16) * sizeof(uint16_t), (size_t)kMmRows * (dvm + 4) * sizeof(float));
 #define DIS_ATTN_DIFF_MMA(Q, V) \
-  stack_attn_mma_kernel<Q, V, false, false, true><<<grid, kMmWarps * 64, shd, st>>>(qf, ldq, kv, temp, pb, nullptr, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
+  launch_k(stack_attn_mma_kernel<Q, V, false, false, true>, dim3(grid), dim3(kMmWarps * 64), (size_t)(shd), st, qf, ldq, kv, temp, pb, nullptr, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
     if (dqm == 64 && dvm == 64) DIS_ATTN_DIFF_MMA(64, 64);
     else if (dqm == 64) DIS_ATTN_DIFF_MMA(64, 128);
     else DIS_ATTN_DIFF_MMA(128, 128);
@@ -860,7 +871,7 @@ static cudaError_t attn_mma_go(const float *qf, long long ldq, const AttnKV &kv,
   if (c.d > dq || c.dv > dvp || (dq == 192 && (sig || dist))) return cudaErrorInvalidValue;
   const size_t shm = (size_t)2 * kMmKeys * (dq + dvp + 16) * sizeof(uint16_t);
 #define DIS_ATTN_MMA(Q, V, S, B) \
-  stack_attn_mma_kernel<Q, V, S, B><<<grid, kMmWarps * 32, shm, st>>>(qf, ldq, kv, temp, pb, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
+  launch_k(stack_attn_mma_kernel<Q, V, S, B>, dim3(grid), dim3(kMmWarps * 32), (size_t)(shm), st, qf, ldq, kv, temp, pb, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
   if (dq == 192) DIS_ATTN_MMA(192, 128, false, false);
   else if (small && sig) DIS_ATTN_MMA(64, 64, true, false);
   else if (small && dist) DIS_ATTN_MMA(64, 64, false, true);
@@ -924,15 +935,15 @@ cudaError_t launch_stack_attn(const float *qf, const void *kpool, const void *vp
     if (part) {
       const size_t msh = (size_t)(c.dv + n_split) * sizeof(float);
       if (c.maps > 1)
-        stack_attn_merge_maps_kernel<false><<<sp.T * c.H, 128, msh + n_split * sizeof(float), st>>>(part, n_split, sp.T, c.H, c.dv, o, c.diff_lambda, c.diff_out, c.eps);
-      else if (sig) stack_attn_merge_kernel<false, true><<<sp.T * c.H, 128, msh, st>>>(part, n_split, sp.T, c.H, c.dv, o);
-      else stack_attn_merge_kernel<false, false><<<sp.T * c.H, 128, msh, st>>>(part, n_split, sp.T, c.H, c.dv, o);
+        launch_k(stack_attn_merge_maps_kernel<false>, dim3(sp.T * c.H), dim3(128), (size_t)(msh + n_split * sizeof(float)), st, part, n_split, sp.T, c.H, c.dv, o, c.diff_lambda, c.diff_out, c.eps);
+      else if (sig) launch_k(stack_attn_merge_kernel<false, true>, dim3(sp.T * c.H), dim3(128), (size_t)(msh), st, part, n_split, sp.T, c.H, c.dv, o);
+      else launch_k(stack_attn_merge_kernel<false, false>, dim3(sp.T * c.H), dim3(128), (size_t)(msh), st, part, n_split, sp.T, c.H, c.dv, o);
     }
     return cudaGetLastError();
   }
   const int th = kAtWarps * 32;
 #define DIS_ATTN_LAUNCH(F, S) \
-  stack_attn_kernel<F, S><<<grid, th, sh, st>>>(qf, kpool, vpool, temp, pb, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
+  launch_k(stack_attn_kernel<F, S>, dim3(grid), dim3(th), (size_t)(sh), st, qf, kpool, vpool, temp, pb, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
   if (f32 && sig) DIS_ATTN_LAUNCH(true, true);
   else if (f32) DIS_ATTN_LAUNCH(true, false);
   else if (sig) DIS_ATTN_LAUNCH(false, true);
@@ -942,12 +953,12 @@ cudaError_t launch_stack_attn(const float *qf, const void *kpool, const void *vp
     const size_t msh = (size_t)(c.dv + n_split) * sizeof(float);
     const int rows = sp.T * c.H;
     if (c.maps > 1) {
-      if (f32) stack_attn_merge_maps_kernel<true><<<rows, 128, msh + n_split * sizeof(float), st>>>(part, n_split, sp.T, c.H, c.dv, o, c.diff_lambda, c.diff_out, c.eps);
-      else stack_attn_merge_maps_kernel<false><<<rows, 128, msh + n_split * sizeof(float), st>>>(part, n_split, sp.T, c.H, c.dv, o, c.diff_lambda, c.diff_out, c.eps);
-    } else if (f32 && sig) stack_attn_merge_kernel<true, true><<<rows, 64, msh, st>>>(part, n_split, sp.T, c.H, c.dv, o);
-    else if (f32) stack_attn_merge_kernel<true, false><<<rows, 64, msh, st>>>(part, n_split, sp.T, c.H, c.dv, o);
-    else if (sig) stack_attn_merge_kernel<false, true><<<rows, 64, msh, st>>>(part, n_split, sp.T, c.H, c.dv, o);
-    else stack_attn_merge_kernel<false, false><<<rows, 64, msh, st>>>(part, n_split, sp.T, c.H, c.dv, o);
+      if (f32) launch_k(stack_attn_merge_maps_kernel<true>, dim3(rows), dim3(128), (size_t)(msh + n_split * sizeof(float)), st, part, n_split, sp.T, c.H, c.dv, o, c.diff_lambda, c.diff_out, c.eps);
+      else launch_k(stack_attn_merge_maps_kernel<false>, dim3(rows), dim3(128), (size_t)(msh + n_split * sizeof(float)), st, part, n_split, sp.T, c.H, c.dv, o, c.diff_lambda, c.diff_out, c.eps);
+    } else if (f32 && sig) launch_k(stack_attn_merge_kernel<true, true>, dim3(rows), dim3(64), (size_t)(msh), st, part, n_split, sp.T, c.H, c.dv, o);
+    else if (f32) launch_k(stack_attn_merge_kernel<true, false>, dim3(rows), dim3(64), (size_t)(msh), st, part, n_split, sp.T, c.H, c.dv, o);
+    else if (sig) launch_k(stack_attn_merge_kernel<false, true>, dim3(rows), dim3(64), (size_t)(msh), st, part, n_split, sp.T, c.H, c.dv, o);
+    else launch_k(stack_attn_merge_kernel<false, false>, dim3(rows), dim3(64), (size_t)(msh), st, part, n_split, sp.T, c.H, c.dv, o);
   }
   return cudaGetLastError();
 }

@@ -2,6 +2,7 @@
 // decays and step sizes of the pass's tokens, and the recurrence itself over a per-slot state.  Everything that enters the
 // recurrence is fp32, and so is the state.
 #include <algorithm>
+#include "ptx.cuh"
 #include "stack_dev.cuh"
 
 namespace dis {
@@ -48,6 +49,8 @@ __device__ __forceinline__ float delta_row_dot(const void *w, long long row, con
 // is one token, and its thread moves the tail on itself.
 template <int TAPS, bool WF32>
 __global__ void __launch_bounds__(kDeltaTh) stack_delta_prep_kernel(StackDelta c, StackDeltaPrep a, StackSpans sp, int tile, int nvb, int ndb, int single) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float sh[];
   const int t0 = blockIdx.x * tile, t1 = min(sp.T, t0 + tile);
   const int taps = TAPS ? TAPS : c.taps, C = c.C;
@@ -178,6 +181,8 @@ __global__ void __launch_bounds__(kDeltaTh) stack_delta_prep_kernel(StackDelta c
 constexpr int kDeltaWarpTok = 8, kDeltaVecTile = kDeltaWarpTok * kDeltaTh / 32;
 template <int TAPS>
 __global__ void __launch_bounds__(kDeltaTh, 4) stack_delta_prep_vec_kernel(StackDelta c, StackDeltaPrep a, StackSpans sp, int nvb) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, C = c.C;
   const int t0 = blockIdx.x * kDeltaVecTile + w * kDeltaWarpTok, nt = min(kDeltaWarpTok, sp.T - t0);
   if (nt <= 0) return;
@@ -292,10 +297,10 @@ cudaError_t launch_stack_delta_prep(const StackDelta &c, const StackDeltaPrep &a
       al(a.z) && al(a.cstate)) {
     const dim3 vgrid((sp.T + kDeltaVecTile - 1) / kDeltaVecTile, c.G + nvb + ndb);
     switch (c.taps) {
-      case 1: stack_delta_prep_vec_kernel<1><<<vgrid, kDeltaTh, 0, st>>>(c, a, sp, nvb); break;
-      case 2: stack_delta_prep_vec_kernel<2><<<vgrid, kDeltaTh, 0, st>>>(c, a, sp, nvb); break;
-      case 3: stack_delta_prep_vec_kernel<3><<<vgrid, kDeltaTh, 0, st>>>(c, a, sp, nvb); break;
-      default: stack_delta_prep_vec_kernel<4><<<vgrid, kDeltaTh, 0, st>>>(c, a, sp, nvb);
+      case 1: launch_k(stack_delta_prep_vec_kernel<1>, dim3(vgrid), dim3(kDeltaTh), 0, st, c, a, sp, nvb); break;
+      case 2: launch_k(stack_delta_prep_vec_kernel<2>, dim3(vgrid), dim3(kDeltaTh), 0, st, c, a, sp, nvb); break;
+      case 3: launch_k(stack_delta_prep_vec_kernel<3>, dim3(vgrid), dim3(kDeltaTh), 0, st, c, a, sp, nvb); break;
+      default: launch_k(stack_delta_prep_vec_kernel<4>, dim3(vgrid), dim3(kDeltaTh), 0, st, c, a, sp, nvb);
     }
     DIS_CUDA_TRY(cudaGetLastError());
     return c.taps > 1 ? launch_stack_conv_tail(a.proj, a.ld, a.n_part, a.stride, 0, a.cstate, sp, c.C, c.taps, st) : cudaSuccess;
@@ -308,7 +313,7 @@ cudaError_t launch_stack_delta_prep(const StackDelta &c, const StackDeltaPrep &a
   do {                                                                                                                                                  \
     static DeviceOnce once;                                                                                                                             \
     DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_delta_prep_kernel<TP, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); })); \
-    stack_delta_prep_kernel<TP, F><<<grid, kDeltaTh, shb, st>>>(c, a, sp, tile, nvb, ndb, single);                                                      \
+    launch_k(stack_delta_prep_kernel<TP, F>, dim3(grid), dim3(kDeltaTh), (size_t)(shb), st, c, a, sp, tile, nvb, ndb, single);                                                      \
   } while (0)
 #define DIS_DELTA_PREP_T(F)                                                                                                                              \
   do {                                                                                                                                                  \
@@ -333,6 +338,8 @@ cudaError_t launch_stack_delta_prep(const StackDelta &c, const StackDeltaPrep &a
 template <bool F32>
 __global__ void stack_delta_pack_kernel(const float *proj, long long ld, int n_part, long long stride, int a_off, int ra, int g_off, int rg,
                                         void *ua, void *ug) {
+  pdl_launch_dependents();
+  pdl_wait();
   const long long t = blockIdx.x;
   for (int i = threadIdx.x; i < ra + rg; i += blockDim.x) {
     const float *p = proj + t * ld + (i < ra ? a_off + i : g_off + i - ra);
@@ -344,8 +351,8 @@ __global__ void stack_delta_pack_kernel(const float *proj, long long ld, int n_p
 }
 cudaError_t launch_stack_delta_pack(const StackDelta &c, const StackDeltaPrep &a, bool f32, int T, void *ua, void *ug, cudaStream_t st) {
   if (T <= 0) return cudaSuccess;
-  if (f32) stack_delta_pack_kernel<true><<<T, 128, 0, st>>>(a.proj, a.ld, a.n_part, a.stride, c.a_off, c.ra, c.g_off, c.rg, ua, ug);
-  else stack_delta_pack_kernel<false><<<T, 128, 0, st>>>(a.proj, a.ld, a.n_part, a.stride, c.a_off, c.ra, c.g_off, c.rg, ua, ug);
+  if (f32) launch_k(stack_delta_pack_kernel<true>, dim3(T), dim3(128), 0, st, a.proj, a.ld, a.n_part, a.stride, c.a_off, c.ra, c.g_off, c.rg, ua, ug);
+  else launch_k(stack_delta_pack_kernel<false>, dim3(T), dim3(128), 0, st, a.proj, a.ld, a.n_part, a.stride, c.a_off, c.ra, c.g_off, c.rg, ua, ug);
   return cudaGetLastError();
 }
 
@@ -398,6 +405,8 @@ constexpr int kDeltaCols = 2;  // columns of a group of eight lanes
 template <int RL, int MW>
 __global__ void __launch_bounds__(MW * 32, 1) stack_delta_kernel(StackDelta c, const float *__restrict__ buf, int ld_b, float *state, StackSpans sp,
                                                                  float *__restrict__ o, int ncb, int vec, DeltaFin fin) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float sh[];
   constexpr int DP = 8 * RL, NM = RL / 4, NP = RL / 2, CL = kDeltaCols, CW = 4 * CL, CT = kDeltaTok;
   const int H = c.H, d = c.d, dv = c.dv;
@@ -657,7 +666,7 @@ static cudaError_t delta_go(const StackDelta &c, const float *buf, long long ld_
   const size_t shb = (size_t)delta_smem_floats<RL>(nw, VC) * sizeof(float);
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_delta_kernel<RL, MW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024); }));
-  stack_delta_kernel<RL, MW><<<(unsigned)((long long)sp.n_spans * c.H * ncb), nw * 32, shb, st>>>(c, buf, (int)ld_b, state, sp, o, ncb, vec, fin);
+  launch_k(stack_delta_kernel<RL, MW>, dim3((unsigned)((long long)sp.n_spans * c.H * ncb)), dim3(nw * 32), (size_t)(shb), st, c, buf, (int)ld_b, state, sp, o, ncb, vec, fin);
   DIS_CUDA_TRY(cudaGetLastError());
   *launches += fin.act ? 1 : 2;
   return fin.act ? cudaSuccess : launch_stack_headnorm_silu(o, norm, gate, (long long)c.H * c.dv, act, ld_act, 0, 1.f, f32, sp.T, c.H, c.dv, c.eps, st, true);

@@ -2,6 +2,7 @@
 // gated recurrence, the state-space mixer, and latent attention (query absorption happens in a batched matrix product in stack.cu; here: rotary + cache write, and the
 // attention itself over the paged latents).  States and scores are fp32.
 #include <cstdlib>
+#include "ptx.cuh"
 #include "stack_dev.cuh"
 
 namespace dis {
@@ -22,6 +23,8 @@ template <int GATE>
 __global__ void __launch_bounds__(256) stack_lightning_kernel(const float *proj, long long ld, LightCols col, const float *decay,
                                                               const float *dec, float qscale, float *state, StackSpans sp, float *o, int H,
                                                               int d, int dv) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float shm[];
   const int s = blockIdx.x, h = blockIdx.y;
   const int tok0 = sp.sp_tok0[s], len = sp.sp_len[s], pos0 = sp.sp_pos0[s], slot = sp.sp_slot[s];
@@ -104,6 +107,8 @@ __global__ void __launch_bounds__(256, 2) stack_lightning_reg_kernel(const float
                                                                      const float *decay, const float *__restrict__ dec, float qscale,
                                                                      float *state, StackSpans sp, float *__restrict__ o, int H, int d,
                                                                      int dv, float *seg, float *seg_a, int max_seg, LightFin fin) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float shm[];
   constexpr int DP = RI * 8, DVP = RJ * 32;
   constexpr bool DEC = GATE == 1 || GATE == 2;  // decays come per token
@@ -280,6 +285,8 @@ __global__ void __launch_bounds__(256, 2) stack_lightning_reg_kernel(const float
 // product of each segment's decays per key channel; otherwise the head's decay to the power of the segment's length.
 __global__ void stack_lightning_carry_kernel(const float *decay, const float *seg_a, float *state, StackSpans sp, float *seg, int H,
                                              int d, int dv) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int n_el = d * dv;
   const int nz = (n_el + blockDim.x - 1) / blockDim.x;
   const int z = blockIdx.x % nz, h = (blockIdx.x / nz) % H, s = blockIdx.x / (nz * H);
@@ -363,13 +370,13 @@ static cudaError_t lightning_reg(const float *proj, long long ld, LightCols col,
     return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_lightning_reg_kernel<RI, RJ, 2, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
   }));
   if (!seg || (DEC && !seg_a) || max_len <= kLightSeg) {
-    stack_lightning_reg_kernel<RI, RJ, 0, GATE><<<sp.n_spans * H, 256, sh, st>>>(proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, nullptr, nullptr, 1, fin);
+    launch_k(stack_lightning_reg_kernel<RI, RJ, 0, GATE>, dim3(sp.n_spans * H), dim3(256), (size_t)(sh), st, proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, nullptr, nullptr, 1, fin);
     return cudaGetLastError();
   }
   const int max_seg = (max_len + kLightSeg - 1) / kLightSeg;
-  stack_lightning_reg_kernel<RI, RJ, 1, GATE><<<sp.n_spans * max_seg * H, 256, sh, st>>>(proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_seg, fin);
-  stack_lightning_carry_kernel<<<sp.n_spans * H * ((d * dv + 255) / 256), 256, 0, st>>>(decay, DEC ? seg_a : nullptr, state, sp, seg, H, d, dv);
-  stack_lightning_reg_kernel<RI, RJ, 2, GATE><<<sp.n_spans * max_seg * H, 256, sh, st>>>(proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_seg, fin);
+  launch_k(stack_lightning_reg_kernel<RI, RJ, 1, GATE>, dim3(sp.n_spans * max_seg * H), dim3(256), (size_t)(sh), st, proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_seg, fin);
+  launch_k(stack_lightning_carry_kernel, dim3(sp.n_spans * H * ((d * dv + 255) / 256)), dim3(256), 0, st, decay, DEC ? seg_a : nullptr, state, sp, seg, H, d, dv);
+  launch_k(stack_lightning_reg_kernel<RI, RJ, 2, GATE>, dim3(sp.n_spans * max_seg * H), dim3(256), (size_t)(sh), st, proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_seg, fin);
   return cudaGetLastError();
 }
 
@@ -383,7 +390,7 @@ cudaError_t launch_stack_lightning(const float *proj, long long ld, const float 
   if (sh > 220 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_lightning_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); }));
-  stack_lightning_kernel<0><<<dim3(sp.n_spans, H), threads, sh, st>>>(proj, ld, col, decay, nullptr, 1.f, state, sp, o, H, d, dv);
+  launch_k(stack_lightning_kernel<0>, dim3(sp.n_spans, H), dim3(threads), (size_t)(sh), st, proj, ld, col, decay, nullptr, 1.f, state, sp, o, H, d, dv);
   return cudaGetLastError();
 }
 
@@ -395,6 +402,8 @@ __global__ void __launch_bounds__(512) stack_retention_prep_kernel(const float *
                                                                    int n_cols, float *dst, long long ld_dst, int q_off, int k_off, int H,
                                                                    int d, const double *__restrict__ freq, int rot_dims, float kscale,
                                                                    const int *__restrict__ pos) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float rsh[];  // cos [half], sin [half], then (n_part > 1) the summed row
   const int t = blockIdx.x, half = rot_dims >> 1;
   float *cs = rsh, *sn = rsh + half;
@@ -449,7 +458,7 @@ cudaError_t launch_stack_retention_prep(const float *src, long long ld_src, int 
   if (sh > 200 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_retention_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); }));
-  stack_retention_prep_kernel<<<sp.T, sp.T <= 148 ? 512 : 256, sh, st>>>(src, ld_src, n_part, stride, n_cols, dst, ld_dst, q_off, k_off, H, d, freq, rot_dims, kscale, sp.pos);
+  launch_k(stack_retention_prep_kernel, dim3(sp.T), dim3(sp.T <= 148 ? 512 : 256), (size_t)(sh), st, src, ld_src, n_part, stride, n_cols, dst, ld_dst, q_off, k_off, H, d, freq, rot_dims, kscale, sp.pos);
   return cudaGetLastError();
 }
 
@@ -488,7 +497,7 @@ cudaError_t launch_stack_retention(const float *proj, long long ld, int q_off, i
   if (sh > 220 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_lightning_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); }));
-  stack_lightning_kernel<3><<<dim3(sp.n_spans, H), threads, sh, st>>>(proj, ld, col, decay, nullptr, 1.f, state, sp, o, H, d, dv);
+  launch_k(stack_lightning_kernel<3>, dim3(sp.n_spans, H), dim3(threads), (size_t)(sh), st, proj, ld, col, decay, nullptr, 1.f, state, sp, o, H, d, dv);
   DIS_CUDA_TRY(cudaGetLastError());
   return launch_stack_headnorm_silu(o, nullptr, gate, ldg, act, ld_act, 0, 1.f, f32, sp.T, H0, dv0, eps, st);
 }
@@ -501,6 +510,8 @@ constexpr int kDecTok = 16;
 template <bool WF32>
 __global__ void __launch_bounds__(128) stack_gla_decay_kernel(const float *proj, long long ld, int a_off, const void *a2, const float *b,
                                                               int T, int n, int rank, float inv_tau, float *dec) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float u[];  // [kDecTok][rank]
   const int t0 = blockIdx.x * kDecTok, nt = min(kDecTok, T - t0);
   for (int i = threadIdx.x; i < kDecTok * rank; i += blockDim.x) {
@@ -533,8 +544,8 @@ cudaError_t launch_stack_gla_decay(const float *proj, long long ld, int a_off, c
   const dim3 grid((T + kDecTok - 1) / kDecTok, (n + 127) / 128);
   const size_t sh = (size_t)kDecTok * rank * sizeof(float);
   if (sh > 48 * 1024) return cudaErrorInvalidValue;
-  if (w_f32) stack_gla_decay_kernel<true><<<grid, 128, sh, st>>>(proj, ld, a_off, a2, b, T, n, rank, 1.f / tau, dec);
-  else stack_gla_decay_kernel<false><<<grid, 128, sh, st>>>(proj, ld, a_off, a2, b, T, n, rank, 1.f / tau, dec);
+  if (w_f32) launch_k(stack_gla_decay_kernel<true>, dim3(grid), dim3(128), (size_t)(sh), st, proj, ld, a_off, a2, b, T, n, rank, 1.f / tau, dec);
+  else launch_k(stack_gla_decay_kernel<false>, dim3(grid), dim3(128), (size_t)(sh), st, proj, ld, a_off, a2, b, T, n, rank, 1.f / tau, dec);
   return cudaGetLastError();
 }
 
@@ -555,7 +566,7 @@ cudaError_t launch_stack_gla(const float *proj, long long ld, int q_off, int k_o
   if (sh > 220 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_lightning_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); }));
-  stack_lightning_kernel<1><<<dim3(sp.n_spans, H), threads, sh, st>>>(proj, ld, col, nullptr, dec, qscale, state, sp, o, H, d, dv);
+  launch_k(stack_lightning_kernel<1>, dim3(sp.n_spans, H), dim3(threads), (size_t)(sh), st, proj, ld, col, nullptr, dec, qscale, state, sp, o, H, d, dv);
   return cudaGetLastError();
 }
 
@@ -580,7 +591,7 @@ cudaError_t launch_stack_ssd(const float *buf, long long ld_b, int c_off, int b_
   if (sh > 220 * 1024) return cudaErrorInvalidValue;
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_lightning_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); }));
-  stack_lightning_kernel<1><<<dim3(sp.n_spans, H), threads, sh, st>>>(buf, ld_b, col, nullptr, dec, 1.f, state, sp, o, H, d, dv);
+  launch_k(stack_lightning_kernel<1>, dim3(sp.n_spans, H), dim3(threads), (size_t)(sh), st, buf, ld_b, col, nullptr, dec, 1.f, state, sp, o, H, d, dv);
   return cudaGetLastError();
 }
 
@@ -597,6 +608,8 @@ __global__ void __launch_bounds__(256) stack_ssm_conv_kernel(const float *__rest
                                                              const float *__restrict__ vec, float *cstate, StackSpans sp,
                                                              float *__restrict__ buf, long long ld_b, float *__restrict__ dec,
                                                              float *__restrict__ dtv) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int V = VEC ? 4 : 1;
   const int t = blockIdx.x;
   const int s = sp.span[t], tok0 = sp.sp_tok0[s], pos0 = sp.sp_pos0[s], slot = sp.sp_slot[s];
@@ -646,6 +659,8 @@ __global__ void __launch_bounds__(256) stack_ssm_conv_tile_kernel(const float *_
                                                                   const float *__restrict__ vec, const float *__restrict__ cstate,
                                                                   StackSpans sp, float *__restrict__ buf, long long ld_b,
                                                                   float *__restrict__ dec, float *__restrict__ dtv) {
+  pdl_launch_dependents();
+  pdl_wait();
   constexpr int V = VEC ? 4 : 1;
   const int t0 = blockIdx.x * kConvTile, t1 = min(sp.T, t0 + kConvTile);
   if (blockIdx.y == 0)
@@ -710,6 +725,8 @@ __global__ void __launch_bounds__(256) stack_ssm_conv_tile_kernel(const float *_
 // The tail moves on to the span's last taps - 1 inputs (a span shorter than that keeps the end of the old tail in front).
 __global__ void stack_ssm_tail_kernel(const float *__restrict__ proj, long long ld, int n_part, long long stride, int x_off, float *cstate,
                                       StackSpans sp, int C, int taps) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x;
   const int tok0 = sp.sp_tok0[s], len = sp.sp_len[s], pos0 = sp.sp_pos0[s], slot = sp.sp_slot[s];
   float *tail = cstate + (long long)slot * (taps - 1) * C;
@@ -731,7 +748,7 @@ cudaError_t launch_stack_conv_tail(const float *proj, long long ld, int n_part, 
                                    int C, int taps, cudaStream_t st) {
   if (taps < 1 || taps > kConvMaxTaps) return cudaErrorInvalidValue;
   if (taps == 1) return cudaSuccess;
-  stack_ssm_tail_kernel<<<dim3(sp.n_spans, (C + 1023) / 1024), 256, 0, st>>>(proj, ld, n_part, stride, x_off, cstate, sp, C, taps);
+  launch_k(stack_ssm_tail_kernel, dim3(sp.n_spans, (C + 1023) / 1024), dim3(256), 0, st, proj, ld, n_part, stride, x_off, cstate, sp, C, taps);
   return cudaGetLastError();
 }
 cudaError_t launch_stack_ssm_conv(const float *proj, long long ld, int x_off, int dt_off, int C, int H, int taps, const float *cw,
@@ -744,8 +761,8 @@ cudaError_t launch_stack_ssm_conv(const float *proj, long long ld, int x_off, in
   const bool single = sp.T == sp.n_spans;  // every span one token long
   const int per = v4 ? 4 : 1;
   const dim3 grid(sp.T, (C + 256 * per - 1) / (256 * per));
-#define DIS_CONV(V, S) stack_ssm_conv_kernel<V, S><<<grid, 256, 0, st>>>(proj, ld, x_off, dt_off, C, H, taps, cw, cb, vec, cstate, sp, buf, ld_b, dec, dtv)
-#define DIS_CONV_TILE(TP, V) stack_ssm_conv_tile_kernel<TP, V><<<tgrid, 256, 0, st>>>(proj, ld, x_off, dt_off, C, H, cw, cb, vec, cstate, sp, buf, ld_b, dec, dtv)
+#define DIS_CONV(V, S) launch_k(stack_ssm_conv_kernel<V, S>, dim3(grid), dim3(256), 0, st, proj, ld, x_off, dt_off, C, H, taps, cw, cb, vec, cstate, sp, buf, ld_b, dec, dtv)
+#define DIS_CONV_TILE(TP, V) launch_k(stack_ssm_conv_tile_kernel<TP, V>, dim3(tgrid), dim3(256), 0, st, proj, ld, x_off, dt_off, C, H, cw, cb, vec, cstate, sp, buf, ld_b, dec, dtv)
   const dim3 tgrid((sp.T + kConvTile - 1) / kConvTile, grid.y);
   if (single && taps > 1) { if (v4) DIS_CONV(true, true); else DIS_CONV(false, true); }
   else if (!single && taps == 2) { if (v4) DIS_CONV_TILE(2, true); else DIS_CONV_TILE(2, false); }
@@ -766,6 +783,8 @@ __global__ void __launch_bounds__(256) stack_ssm_out_kernel(const float *__restr
                                                             const float *__restrict__ z, long long ld, const float *__restrict__ D,
                                                             const float *__restrict__ w, int parts, void *__restrict__ out, int H, int P,
                                                             float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float yrow[];  // [H*P]
   __shared__ float sh[32];
   constexpr int V = VEC ? 4 : 1;
@@ -831,7 +850,7 @@ static cudaError_t ssm_out_go(const float *o, const float *buf, long long ld_b, 
                               int parts, void *out, int T, int H, int P, float eps, cudaStream_t st) {
   static DeviceOnce once;
   DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(stack_ssm_out_kernel<F32, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); }));
-  stack_ssm_out_kernel<F32, VEC><<<T, 256, (size_t)H * P * 4, st>>>(o, buf, ld_b, z, ld, D, w, parts, out, H, P, eps);
+  launch_k(stack_ssm_out_kernel<F32, VEC>, dim3(T), dim3(256), (size_t)((size_t)H * P * 4), st, o, buf, ld_b, z, ld, D, w, parts, out, H, P, eps);
   return cudaGetLastError();
 }
 cudaError_t launch_stack_ssm_out(const float *o, const float *buf, long long ld_b, const float *z, long long ld, const float *D,
@@ -852,6 +871,8 @@ cudaError_t launch_stack_ssm_out(const float *o, const float *buf, long long ld_
 template <bool F32>
 __global__ void __launch_bounds__(256) stack_headnorm_silu_kernel(const float *o, const float *w, const float *gate, long long ldg, void *out,
                                                                   long long ldo, int off, float scale, int rows, int H, int dv, float eps, int sig) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), l = threadIdx.x & 31;
   if (row >= rows) return;
   const int t = row / H, h = row - t * H;
@@ -869,14 +890,16 @@ cudaError_t launch_stack_headnorm_silu(const float *o, const float *w, const flo
                                        int off, float scale, bool f32, int T, int H, int dv, float eps, cudaStream_t st, bool sig) {
   const int rows = T * H;
   if (rows <= 0) return cudaSuccess;
-  if (f32) stack_headnorm_silu_kernel<true><<<(rows + 7) / 8, 256, 0, st>>>(o, w, gate, ldg, out, ldo, off, scale, rows, H, dv, eps, sig ? 1 : 0);
-  else stack_headnorm_silu_kernel<false><<<(rows + 7) / 8, 256, 0, st>>>(o, w, gate, ldg, out, ldo, off, scale, rows, H, dv, eps, sig ? 1 : 0);
+  if (f32) launch_k(stack_headnorm_silu_kernel<true>, dim3((rows + 7) / 8), dim3(256), 0, st, o, w, gate, ldg, out, ldo, off, scale, rows, H, dv, eps, sig ? 1 : 0);
+  else launch_k(stack_headnorm_silu_kernel<false>, dim3((rows + 7) / 8), dim3(256), 0, st, o, w, gate, ldg, out, ldo, off, scale, rows, H, dv, eps, sig ? 1 : 0);
   return cudaGetLastError();
 }
 
 template <bool F32>
 __global__ void __launch_bounds__(256) stack_norm_gate_kernel(const float *o, const float *w, const float *gate, long long ldg,
                                                               void *out, int n, float eps) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sh[32];
   const long long t = blockIdx.x;
   const float *r = o + t * n;
@@ -889,8 +912,8 @@ __global__ void __launch_bounds__(256) stack_norm_gate_kernel(const float *o, co
 }
 cudaError_t launch_stack_norm_gate(const float *o, const float *w, const float *gate, long long ldg, void *out, bool f32, int T,
                                    int n, float eps, cudaStream_t st) {
-  if (f32) stack_norm_gate_kernel<true><<<T, 256, 0, st>>>(o, w, gate, ldg, out, n, eps);
-  else stack_norm_gate_kernel<false><<<T, 256, 0, st>>>(o, w, gate, ldg, out, n, eps);
+  if (f32) launch_k(stack_norm_gate_kernel<true>, dim3(T), dim3(256), 0, st, o, w, gate, ldg, out, n, eps);
+  else launch_k(stack_norm_gate_kernel<false>, dim3(T), dim3(256), 0, st, o, w, gate, ldg, out, n, eps);
   return cudaGetLastError();
 }
 
@@ -898,6 +921,8 @@ cudaError_t launch_stack_norm_gate(const float *o, const float *w, const float *
 template <bool F32>
 __global__ void stack_gate_kernel(const float *__restrict__ o, const float *__restrict__ gate, long long ldg, void *__restrict__ out, int T,
                                   int n, int heads, long long ldo) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int hw = heads > 0 ? n / heads : n;
   for (int t = blockIdx.x; t < T; t += gridDim.x) {
     for (int c = threadIdx.x; c < n; c += blockDim.x) {
@@ -911,8 +936,8 @@ cudaError_t launch_stack_gate(const float *o, const float *gate, long long ldg, 
   if (T <= 0) return cudaSuccess;
   if (ldo <= 0) ldo = n;
   const int grid = std::min(T, 148 * 16);
-  if (f32) stack_gate_kernel<true><<<grid, 256, 0, st>>>(o, gate, ldg, out, T, n, heads, ldo);
-  else stack_gate_kernel<false><<<grid, 256, 0, st>>>(o, gate, ldg, out, T, n, heads, ldo);
+  if (f32) launch_k(stack_gate_kernel<true>, dim3(grid), dim3(256), 0, st, o, gate, ldg, out, T, n, heads, ldo);
+  else launch_k(stack_gate_kernel<false>, dim3(grid), dim3(256), 0, st, o, gate, ldg, out, T, n, heads, ldo);
   return cudaGetLastError();
 }
 
@@ -920,6 +945,8 @@ cudaError_t launch_stack_gate(const float *o, const float *gate, long long ldg, 
 // `wd` of them -> dst bf16 [H][T][wd]; and back: src fp32 [H][T][wd] -> dst fp32 [T][ld] at columns off + h * hs.
 __global__ void stack_heads_pack_kernel(const float *__restrict__ src, long long ld, int off, int hs, int wd, int T, int H,
                                         uint16_t *__restrict__ dst) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x / H, h = blockIdx.x - t * H;  // one (token, head) row per block
   const float *sr = src + (long long)t * ld + off + (long long)h * hs;
   uint16_t *dr = dst + ((long long)h * T + t) * wd;
@@ -927,6 +954,8 @@ __global__ void stack_heads_pack_kernel(const float *__restrict__ src, long long
 }
 __global__ void stack_heads_unpack_kernel(const float *__restrict__ src, int wd, int T, int H, float *__restrict__ dst, long long ld,
                                           int off, int hs) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int t = blockIdx.x / H, h = blockIdx.x - t * H;
   const float *sr = src + ((long long)h * T + t) * wd;
   float *dr = dst + (long long)t * ld + off + (long long)h * hs;
@@ -934,12 +963,12 @@ __global__ void stack_heads_unpack_kernel(const float *__restrict__ src, int wd,
 }
 cudaError_t launch_stack_heads_pack(const float *src, long long ld, int off, int hs, int wd, int T, int H, uint16_t *dst, cudaStream_t st) {
   if ((long long)T * H <= 0 || wd <= 0) return cudaSuccess;
-  stack_heads_pack_kernel<<<T * H, 128, 0, st>>>(src, ld, off, hs, wd, T, H, dst);
+  launch_k(stack_heads_pack_kernel, dim3(T * H), dim3(128), 0, st, src, ld, off, hs, wd, T, H, dst);
   return cudaGetLastError();
 }
 cudaError_t launch_stack_heads_unpack(const float *src, int wd, int T, int H, float *dst, long long ld, int off, int hs, cudaStream_t st) {
   if ((long long)T * H <= 0 || wd <= 0) return cudaSuccess;
-  stack_heads_unpack_kernel<<<T * H, 128, 0, st>>>(src, wd, T, H, dst, ld, off, hs);
+  launch_k(stack_heads_unpack_kernel, dim3(T * H), dim3(128), 0, st, src, wd, T, H, dst, ld, off, hs);
   return cudaGetLastError();
 }
 
@@ -948,6 +977,8 @@ cudaError_t launch_stack_heads_unpack(const float *src, int wd, int T, int H, fl
 template <bool F32>
 __global__ void stack_mingru_kernel(const float *__restrict__ proj, long long ld, const float *bias, float *state, StackSpans sp,
                                     void *__restrict__ out, int n) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -982,6 +1013,8 @@ template <bool F32>
 __global__ void __launch_bounds__(kGruSlices * 32) stack_mingru_sliced_kernel(const float *__restrict__ proj, long long ld,
                                                                               const float *bias, float *state, StackSpans sp,
                                                                               void *__restrict__ out, int n, int n_cb) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float As[kGruSlices][32], Bs[kGruSlices][32];
   const int s = blockIdx.x / n_cb, cb = blockIdx.x - s * n_cb;
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -1038,13 +1071,13 @@ cudaError_t launch_stack_mingru(const float *proj, long long ld, const float *bi
                                 bool f32, int n, int max_len, cudaStream_t st) {
   if (max_len >= 4 * kGruSlices) {
     const int n_cb = (n + 31) / 32;
-    if (f32) stack_mingru_sliced_kernel<true><<<sp.n_spans * n_cb, kGruSlices * 32, 0, st>>>(proj, ld, bias, state, sp, out, n, n_cb);
-    else stack_mingru_sliced_kernel<false><<<sp.n_spans * n_cb, kGruSlices * 32, 0, st>>>(proj, ld, bias, state, sp, out, n, n_cb);
+    if (f32) launch_k(stack_mingru_sliced_kernel<true>, dim3(sp.n_spans * n_cb), dim3(kGruSlices * 32), 0, st, proj, ld, bias, state, sp, out, n, n_cb);
+    else launch_k(stack_mingru_sliced_kernel<false>, dim3(sp.n_spans * n_cb), dim3(kGruSlices * 32), 0, st, proj, ld, bias, state, sp, out, n, n_cb);
     return cudaGetLastError();
   }
   dim3 grid(sp.n_spans, (n + 127) / 128);
-  if (f32) stack_mingru_kernel<true><<<grid, 128, 0, st>>>(proj, ld, bias, state, sp, out, n);
-  else stack_mingru_kernel<false><<<grid, 128, 0, st>>>(proj, ld, bias, state, sp, out, n);
+  if (f32) launch_k(stack_mingru_kernel<true>, dim3(grid), dim3(128), 0, st, proj, ld, bias, state, sp, out, n);
+  else launch_k(stack_mingru_kernel<false>, dim3(grid), dim3(128), 0, st, proj, ld, bias, state, sp, out, n);
   return cudaGetLastError();
 }
 
@@ -1073,6 +1106,8 @@ __global__ void __launch_bounds__(512) stack_latent_prep_kernel(const float *pro
                                                                 int keep_off, int keep_n, const double *__restrict__ freq,
                                                                 StackLatent c, StackSpans sp, float *qf, float *qx, long long ld_qx, void *pool,
                                                                 const int *page_table, int max_pages, int page_size) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) float lsh[];  // cos [half], sin [half], then (n_part > 1) the summed row
   __shared__ float sh[32];
   const int t = blockIdx.x;
@@ -1151,7 +1186,7 @@ cudaError_t launch_stack_latent_prep(const StackLatentPrep &a, const StackLatent
     return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_latent_prep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
   }));
 #define DIS_LAT_PREP(F)                                                                                                                      \
-  stack_latent_prep_kernel<F><<<sp.T, sp.T <= 148 ? 512 : 256, sh, st>>>(a.proj, a.ld, n_part, a.stride, a.n_cols, a.q_off, a.dkv_off, a.dkv_norm, a.dq_off, a.dq_norm, \
+  launch_k(stack_latent_prep_kernel<F>, dim3(sp.T), dim3(sp.T <= 148 ? 512 : 256), (size_t)(sh), st, a.proj, a.ld, n_part, a.stride, a.n_cols, a.q_off, a.dkv_off, a.dkv_norm, a.dq_off, a.dq_norm, \
                                                      a.cq, a.keep, a.ld_keep, a.keep_off, a.keep_n, a.freq, c, sp, a.qf, a.qx, a.ld_qx, a.pool, page_table, max_pages, page_size)
   if (f32) DIS_LAT_PREP(true);
   else DIS_LAT_PREP(false);
@@ -1179,6 +1214,8 @@ __global__ void __launch_bounds__(kLatWarps * 32) stack_latent_attn_kernel(const
                                                                            StackLatent c, StackSpans sp, const int *qb_tok0,
                                                                            const int *qb_len, const int *page_table, int max_pages,
                                                                            int page_size, float *ol, int keys_per_split, float *part) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ float shm[];
   const int D = c.r + c.dr, DP = D + 1, r = c.r;
   const int tok0 = qb_tok0[blockIdx.x], nq = qb_len[blockIdx.x];
@@ -1301,6 +1338,8 @@ __global__ void __launch_bounds__(256) stack_latent_attn_mma_kernel(const float 
                                                                     StackSpans sp, const int *qb_tok0, const int *qb_len,
                                                                     const int *page_table, int max_pages, int page_size, float *ol,
                                                                     int keys_per_split, float *part) {
+  pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = c.r + c.dr, r = c.r, DS = D + 8;
   uint16_t *qs = reinterpret_cast<uint16_t *>(smraw);                  // [16][DS]
@@ -1462,6 +1501,8 @@ __global__ void __launch_bounds__(256) stack_latent_attn_mma_kernel(const float 
 
 // Merge of the slices: out = sum_s acc_s e^(m_s - M) / (e^(sink - M) + sum_s l_s e^(m_s - M)), M = max(sink, max_s m_s).
 __global__ void stack_latent_merge_kernel(const float *part, const float *sink, int n_split, int pairs_total, int H, int r, float *ol) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float ws[kLatMaxSplit];  // per slice e^(m_s - M), 0 for an empty slice
   __shared__ float inv_den;
   const int p = blockIdx.x;
@@ -1503,6 +1544,8 @@ __global__ void __launch_bounds__(256) stack_latent_rows_kernel(const uint16_t *
                                                                 const int *__restrict__ ls, const int *__restrict__ lin,
                                                                 const int *__restrict__ page_table, int max_pages, int page_size,
                                                                 uint16_t *__restrict__ cg, uint16_t *__restrict__ krot) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int s = ls[blockIdx.y], pos0 = sp.sp_pos0[s], slot = sp.sp_slot[s], D = c.r + c.dr, l = threadIdx.x & 31;
   const int key = stack_latent_row_lo(c, pos0) + blockIdx.x * 8 + (threadIdx.x >> 5);
   if (key >= pos0 + sp.sp_len[s]) return;
@@ -1520,7 +1563,7 @@ cudaError_t launch_stack_latent_rows(const void *pool, const StackLatent &c, con
                                      cudaStream_t st) {
   if (n_ls <= 0 || max_keys <= 0) return cudaSuccess;
   if (c.r % 8 || c.dr % 8) return cudaErrorInvalidValue;
-  stack_latent_rows_kernel<<<dim3((max_keys + 7) / 8, n_ls), 256, 0, st>>>(reinterpret_cast<const uint16_t *>(pool), c, sp, ls, lin, page_table,
+  launch_k(stack_latent_rows_kernel, dim3((max_keys + 7) / 8, n_ls), dim3(256), 0, st, reinterpret_cast<const uint16_t *>(pool), c, sp, ls, lin, page_table,
                                                                           max_pages, page_size, cg, krot);
   return cudaGetLastError();
 }
@@ -1530,6 +1573,8 @@ cudaError_t launch_stack_latent_rows(const void *pool, const StackLatent &c, con
 // tensor-core product, and the kernel between them turns a block of score rows into softmax weights (fp32, causal, sink).
 __global__ void stack_latent_gather_kernel(const uint16_t *pool, const int *pt, int page_size, int D, int r, int ctx, int ctx8,
                                            uint16_t *cg, uint16_t *cgt, int first) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int kp = blockIdx.x, key = first + kp;  // row kp holds the latent of position first + kp
   const long long prow = kp < ctx ? (long long)pt[key / page_size] * page_size + key % page_size : 0;
   for (int c = threadIdx.x; c < D; c += blockDim.x) {
@@ -1540,7 +1585,7 @@ __global__ void stack_latent_gather_kernel(const uint16_t *pool, const int *pt, 
 }
 cudaError_t launch_stack_latent_gather(const void *pool, const int *pt_row, int page_size, int D, int r, int ctx, int ctx8,
                                        uint16_t *cg, uint16_t *cgt, int first, cudaStream_t st) {
-  stack_latent_gather_kernel<<<ctx8, 128, 0, st>>>(reinterpret_cast<const uint16_t *>(pool), pt_row, page_size, D, r, ctx, ctx8, cg, cgt, first);
+  launch_k(stack_latent_gather_kernel, dim3(ctx8), dim3(128), 0, st, reinterpret_cast<const uint16_t *>(pool), pt_row, page_size, D, r, ctx, ctx8, cg, cgt, first);
   return cudaGetLastError();
 }
 
@@ -1548,6 +1593,8 @@ cudaError_t launch_stack_latent_gather(const void *pool, const int *pt_row, int 
 // from the first gathered key; window > 0: only the last `window` keys up to the query's own are seen).
 __global__ void __launch_bounds__(256) stack_latent_softmax_kernel(const float *S, int ld, const float *sink, int H, int pos_first,
                                                                    float scale, uint16_t *P, int window) {
+  pdl_launch_dependents();
+  pdl_wait();
   __shared__ float sh[32];
   const long long row = blockIdx.x;
   const int h = (int)(row % H), qpos = pos_first + (int)(row / H);
@@ -1572,7 +1619,7 @@ __global__ void __launch_bounds__(256) stack_latent_softmax_kernel(const float *
 cudaError_t launch_stack_latent_softmax(const float *S, int rows, int ld, const float *sink, int H, int pos_first, float scale,
                                         uint16_t *P, int window, cudaStream_t st) {
   if (rows <= 0) return cudaSuccess;
-  stack_latent_softmax_kernel<<<rows, 256, 0, st>>>(S, ld, sink, H, pos_first, scale, P, window);
+  launch_k(stack_latent_softmax_kernel, dim3(rows), dim3(256), 0, st, S, ld, sink, H, pos_first, scale, P, window);
   return cudaGetLastError();
 }
 
@@ -1596,9 +1643,9 @@ cudaError_t launch_stack_latent_attn(const float *qf, const void *pool, bool f32
     if (shm > 220 * 1024) return cudaErrorInvalidValue;
     const dim3 grid(n_qb, n_split, (c.H + kMmaRows - 1) / kMmaRows);
     const uint16_t *pl = reinterpret_cast<const uint16_t *>(pool);
-    if (c.r <= 512) stack_latent_attn_mma_kernel<8><<<grid, 256, shm, st>>>(qf, pl, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
-    else stack_latent_attn_mma_kernel<16><<<grid, 256, shm, st>>>(qf, pl, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
-    if (part) stack_latent_merge_kernel<<<sp.T * c.H, c.r > 256 ? 512 : 128, 0, st>>>(part, sink, n_split, sp.T * c.H, c.H, c.r, ol);
+    if (c.r <= 512) launch_k(stack_latent_attn_mma_kernel<8>, dim3(grid), dim3(256), (size_t)(shm), st, qf, pl, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
+    else launch_k(stack_latent_attn_mma_kernel<16>, dim3(grid), dim3(256), (size_t)(shm), st, qf, pl, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
+    if (part) launch_k(stack_latent_merge_kernel, dim3(sp.T * c.H), dim3(c.r > 256 ? 512 : 128), 0, st, part, sink, n_split, sp.T * c.H, c.H, c.r, ol);
     return cudaGetLastError();
   }
   const int D = c.r + c.dr, bq = stack_latent_block_tokens(c);
@@ -1610,9 +1657,9 @@ cudaError_t launch_stack_latent_attn(const float *qf, const void *pool, bool f32
     return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_latent_attn_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
   }));
   const dim3 grid(n_qb, n_split);
-  if (f32) stack_latent_attn_kernel<true><<<grid, kLatWarps * 32, sh, st>>>(qf, pool, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
-  else stack_latent_attn_kernel<false><<<grid, kLatWarps * 32, sh, st>>>(qf, pool, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
-  if (part) stack_latent_merge_kernel<<<sp.T * c.H, c.r > 256 ? 512 : 128, 0, st>>>(part, sink, n_split, sp.T * c.H, c.H, c.r, ol);
+  if (f32) launch_k(stack_latent_attn_kernel<true>, dim3(grid), dim3(kLatWarps * 32), (size_t)(sh), st, qf, pool, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
+  else launch_k(stack_latent_attn_kernel<false>, dim3(grid), dim3(kLatWarps * 32), (size_t)(sh), st, qf, pool, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, ol, keys_per_split, part);
+  if (part) launch_k(stack_latent_merge_kernel, dim3(sp.T * c.H), dim3(c.r > 256 ? 512 : 128), 0, st, part, sink, n_split, sp.T * c.H, c.H, c.r, ol);
   return cudaGetLastError();
 }
 

@@ -951,6 +951,8 @@ int Engine::init_stack(const dis_engine_config *c, const dis_stack_config *sc) {
   ENG_CUDA(alloc(reinterpret_cast<void **>(&M.d_out), (size_t)2 * M.max_rows * 4));
   ENG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&M.h_out), (size_t)2 * M.max_rows * 4));
   ENG_CUDA(stack_meta(meta_pre, cap_tokens, M.max_rows));
+  ENG_CUDA(stack_meta(meta_dec, max_batch, M.max_rows));
+  use_pdl = !(c->flags & DIS_FLAG_NO_PDL);
   cur_meta = &meta_pre;
   // ---- pages: one pool per latent layer that owns a cache (rows of kv_rank + rot_dim elements), a key and a value pool per
   // attention layer that owns one; a page id is valid in all
@@ -1121,7 +1123,12 @@ int Engine::stack_step(int n, const int *slots, int max_prefill_tokens, uint32_t
   if (idx.empty()) { last_rows = 0; return DIS_OK; }
   std::vector<int> take(idx.size());
   plan_mixed_step((int)idx.size(), rem.data(), max_prefill_tokens > 0 ? max_prefill_tokens : cap_tokens, cap_tokens, take.data());
-  StepMeta &mt = meta_pre;
+  // The block of step metadata is copied whole: passes of few tokens (decode passes always) use a small one.  With room for 8192 tokens
+  // the copy was 0.5 MB, 12 us in front of every decode pass.
+  long long planned = 0;
+  for (int t : take) planned += std::max(t, 0);
+  cur_meta = planned <= max_batch ? &meta_dec : &meta_pre;
+  StepMeta &mt = *cur_meta;
   int T = 0, R = 0, SP = 0, QB = 0, KB = 0, LB = 0, LS = 0;
   stack_max_ctx = 0;
   stack_spans_h.clear();
@@ -1345,7 +1352,7 @@ int Engine::stack_step(int n, const int *slots, int max_prefill_tokens, uint32_t
 
 cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_greedy) {
   StackModel &M = *stack;
-  StepMeta &mt = meta_pre;
+  StepMeta &mt = *cur_meta;
   const int W = M.c.width, taps = M.c.canon_taps;
   const float res_mult = M.c.residual_mult;
   const float *vfirst = nullptr;  // values of the pass's first value-mixing layer, once it has run
@@ -1357,7 +1364,11 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   int pend_parts = 1;  // the product whose result the next boundary consumes: slices left unsummed, their stride, its bias
   long long pend_stride = 0;
   const float *pend_bias = nullptr, *pend_src = nullptr;
-  pdl_enabled() = false;  // this family's kernels are plain launches: every kernel starts after the one before it has ended
+  // Programmatic dependent launch: a kernel's CTAs are placed while the one before it drains and wait for its results in their
+  // first instruction (products fill their ring with weights before that).  The pass's first kernel follows a copy and stays plain.
+  struct PdlOff { ~PdlOff() { pdl_enabled() = false; } } pdl_off;
+  pdl_enabled() = false;
+  auto plain = [](auto launch) { const bool on = pdl_enabled(); pdl_enabled() = false; const cudaError_t e = launch(); pdl_enabled() = on; return e; };
   // Dense projection out[Mrows][N] = A[Mrows][K] W[N][K]^T (+ bias).  bf16 operands go to the tcgen05 product the Llama path
   // uses (fp32 accumulation in TMEM; split-K slices summed, with the bias, by one more kernel); float operands, and shapes a
   // TMA map cannot describe (K not a multiple of 8), to the fp32-FMA product.  a_rows: rows the buffer behind A holds.
@@ -1415,6 +1426,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   StackParBoundary pend_par;                      // parallel layers with two norms: what the next boundary joins
   const int n_streams = std::max(1, M.c.streams);
   RET_CUDA(launch_stack_embed(M.embed.ptr, f32, sp.tokens, sp.pos, M.pos_freq, M.x, M.x0, M.c.embed_scale, T, W, n_streams, stream)); kl++;
+  pdl_enabled() = use_pdl;
   const float *pend_y = nullptr, *pend_post = nullptr, *pend_post_b = nullptr;
   const float *pend_hc = nullptr, *next_hc = nullptr;  // stream coefficients of the sublayer whose product is pending / of the coming one
   const bool ln = M.c.norm_kind == DIS_NORM_LAYER || M.c.norm_kind == DIS_NORM_RMS;  // norms with vectors: one boundary kernel
@@ -1893,12 +1905,13 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
             TmaMap qm, cm, pm, ctm;
             RET_CUDA(make_tma_map_2d(&qm, M.lat_qb + (size_t)(sh.tok0 + j) * H * D, (uint64_t)rows, (uint64_t)D, (uint32_t)gemm_token_tile(rows)));
             RET_CUDA(make_tma_map_2d(&cm, M.lat_cg, (uint64_t)nkeys, (uint64_t)D, 128));
-            RET_CUDA(launch_gemm_partial(cm, qm, M.lat_s, rows, nkeys, D, 0, 1, stream));
+            // (plain: a product fetches its second operand before it waits, and here that one is made by the kernels before)
+            RET_CUDA(plain([&] { return launch_gemm_partial(cm, qm, M.lat_s, rows, nkeys, D, 0, 1, stream); }));
             RET_CUDA(launch_stack_latent_softmax(M.lat_s, rows, nkeys, reinterpret_cast<const float *>(L.sink.ptr), H, pos0 + j, sl.scale,
                                                  M.lat_p, sl.window, stream));
             RET_CUDA(make_tma_map_2d(&pm, M.lat_p, (uint64_t)rows, (uint64_t)nkeys, (uint32_t)gemm_token_tile(rows)));
             RET_CUDA(make_tma_map_2d(&ctm, M.lat_cgt, (uint64_t)r, (uint64_t)ctx8, 128));
-            RET_CUDA(launch_gemm_partial(ctm, pm, M.mix + (size_t)(sh.tok0 + j) * H * r, rows, r, nkeys, 0, 1, stream));
+            RET_CUDA(plain([&] { return launch_gemm_partial(ctm, pm, M.mix + (size_t)(sh.tok0 + j) * H * r, rows, r, nkeys, 0, 1, stream); }));
             kl += 3;
           }
         }
