@@ -83,7 +83,7 @@ __device__ __forceinline__ float4 attn_sum_slices(const float *p, int n, long lo
 }
 
 template <int D, int G>
-__global__ void __launch_bounds__(kAttnThreads, 2)
+__global__ void __launch_bounds__(kAttnThreads + 32, 2)
 attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const AttnRope rope, const uint16_t *__restrict__ q,
                   const int *__restrict__ page_table, int max_pages, const int *__restrict__ pt_row,
                   const int *__restrict__ ctx_len, uint16_t *__restrict__ out, float *__restrict__ scratch,
@@ -97,6 +97,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + n_stages * Cfg::kStageBytes;
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 32u + 8u * s; };
 
   const int t = blockIdx.z;
   const int kvh = blockIdx.y;
@@ -107,7 +108,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&kv_map);
-    for (int s = 0; s < n_stages; s++) mbar_init(full_bar(s), 1);
+    for (int s = 0; s < n_stages; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 4); }
     fence_barrier_init();
     fence_proxy_async();
   }
@@ -146,13 +147,23 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     }
   };
 
-  // One stage is kept back for the refill at the top of iteration 0.  Filling the whole ring up front (nothing consumes a
-  // tile before the RoPE prologue is over) was measured: 3.491 / 3.495 against 3.531 / 3.479 ms per step at
-  // batch 32, 4.269 against 4.253 at batch 64 -- no gain, not kept.
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < n_stages - 1; s++)
-      if (s < n_tiles) load_tile(s, s);
+  // Warp 4 loads and does nothing else, the four computing warps free a stage each for themselves: no barrier of the whole block per
+  // tile.  A batch of ragged histories is as slow as its longest one, which a single CTA walks: with the loads issued by a computing
+  // thread behind a block barrier that took 1.04 us per tile.  Batch 32, histories of 500 to 6000 keys, 32 / 8 heads of 128, 318 MB:
+  // 100.5 -> 78.4 us; 64 equal histories of 1600: 65.2 -> 63.4 us; 32 x 512: 14.5 us on both.
+  if (warp == 4) {
+    if (lane == 0)
+      for (int tile = 0; tile < n_tiles; tile++) {
+        const int stage = tile % n_stages;
+        if (tile >= n_stages) mbar_wait(empty_bar(stage), (uint32_t)(tile / n_stages - 1) & 1u);
+        load_tile(tile, stage);
+      }
+    __syncwarp();
+    __syncthreads();  // (the two barriers around the merge below)
+    __syncthreads();
+    return;
   }
+  auto sync_compute = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };  // the four computing warps
 
   const int new_pos = ctx - 1;                               // the position this decode step appends
   const bool owner = fused && new_pos >= begin && new_pos < end;  // the split that holds it
@@ -188,7 +199,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
         *reinterpret_cast<uint2 *>(s_kvnew[1] + i) = o;
       }
     }
-    __syncthreads();
+    sync_compute();
     if (owner && threadIdx.x < 2 * (D / 8)) {  // the new row goes to the page pool for the steps to come
       const int kv = threadIdx.x / (D / 8), c = threadIdx.x % (D / 8);
       const long long page = pt[new_pos >> page_shift];
@@ -217,28 +228,24 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
 
   const int wtok = warp * 16;  // this warp's token slice inside a tile
   for (int tile = 0; tile < n_tiles; tile++) {
-    __syncthreads();  // everyone is done with the stage consumed last iteration
-    if (threadIdx.x == 0) {
-      const int nt = tile + n_stages - 1;
-      if (nt < n_tiles) load_tile(nt, nt % n_stages);
-    }
     const int stage = tile % n_stages;
     mbar_wait(full_bar(stage), (uint32_t)(tile / n_stages) & 1u);
     const uint32_t ks_addr = smem_base + stage * Cfg::kStageBytes;
     const uint32_t vs_addr = ks_addr + Cfg::kHalves * Cfg::kHalfBytes;
     const int tile_len = min(kAttnTile, end - (begin + tile * kAttnTile));
-    if (owner && tile == n_tiles - 1) {
-      // the tile TMA fetched predates this step's K/V row: patch it in (same 128B swizzle as the TMA boxes)
-      const int r = new_pos - (begin + tile * kAttnTile);
-      if (threadIdx.x < 2 * (D / 8)) {
-        const int kv = threadIdx.x / (D / 8), c = threadIdx.x % (D / 8);
+    const int new_row = new_pos - (begin + tile * kAttnTile);
+    if (owner && tile == n_tiles - 1 && (new_row >> 4) == warp) {
+      // the tile TMA fetched predates this step's K/V row: the warp that reads the row patches it in (same 128B swizzle as the TMA boxes)
+      const int r = new_row;
+      if (lane < 2 * (D / 8)) {
+        const int kv = lane / (D / 8), c = lane % (D / 8);
         const uint32_t dst = (kv ? vs_addr : ks_addr) + (c >> 3) * Cfg::kHalfBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4);
         const uint4 v = *reinterpret_cast<const uint4 *>(s_kvnew[kv] + c * 8);
         asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
       }
-      __syncthreads();
+      __syncwarp();
     }
-    if (wtok >= tile_len) continue;  // warp-uniform: nothing of this tile belongs to this warp
+    if (wtok >= tile_len) continue;  // warp-uniform: nothing of this tile belongs to this warp (only a split's last tile is short)
 
     // ---- S = Q K^T for this warp's 16 tokens (two n-tiles of 8)
     float sacc[2][4];
@@ -296,8 +303,10 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
         mma_bf16_16816(oacc[n + 1], pa[0], 0u, pa[1], 0u, b2, b3);
       }
     }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty_bar(stage));
   }
-  __syncthreads();  // all TMA loads issued were waited for above: the stage memory is free
+  __syncthreads();  // every warp waited for every load: the stage memory is free
 
   // ---- merge the four warps' (m, l, O) through the stage memory
   float *s_o = reinterpret_cast<float *>(smem);        // [4 warps][G][D]
@@ -559,7 +568,7 @@ static cudaError_t attn_launch(const TmaMap &kv_map, long long row0, const AttnR
     stages = stages < 2 ? 2 : (stages > AttnCfg<D>::kStages ? AttnCfg<D>::kStages : stages);
   }
   const int smem = stages * AttnCfg<D>::kStageBytes + 1024 + 64;
-  DIS_CUDA_TRY(launch_k(attn_paged_kernel<D, G>, grid, dim3(kAttnThreads), (size_t)smem, st,
+  DIS_CUDA_TRY(launch_k(attn_paged_kernel<D, G>, grid, dim3(kAttnThreads + 32), (size_t)smem, st,
                         *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
                         scratch, n_splits, T, n_heads, n_kv, page_shift, stages));
   if (n_splits > 1)
