@@ -115,21 +115,21 @@ cudaError_t launch_gemm_partial(const TmaMap &w_map, const TmaMap &x_map, float 
                                 int w_row0, int split_k, cudaStream_t st);
 // out[T][N] = the same product in one slice, rounded to bf16
 cudaError_t launch_gemm_bf16(const TmaMap &w_map, const TmaMap &x_map, uint16_t *out, int T, int N, int K, int w_row0, cudaStream_t st);
-cudaError_t launch_gemm_persist_bf16(const TmaMap &w_map128, const TmaMap &x_map256, uint16_t *out, int T, int N, int K, int w_row0,
+cudaError_t launch_gemm_persist_bf16(const TmaMap &w_map128, const TmaMap &x_map128, uint16_t *out, int T, int N, int K, int w_row0,
                                      cudaStream_t st);
 // act[T][I] = bf16(silu(gate) * up); gate rows at w_row0, up rows at w_row0 + I.  w_map's box height must be
 // tile_rows = gemm_pick_tile_rows(I).
 int gemm_pick_tile_rows(int N);
-// k_gemm_persist.cu : persistent, TMEM-double-buffered variant for prefill-sized T (no split-K)
-bool gemm_use_persist(int T, int N, bool dual);
-cudaError_t launch_gemm_persist_partial(const TmaMap &w_map128, const TmaMap &x_map256, float *out, int T, int N, int K,
-                                        int w_row0, cudaStream_t st);
+// k_gemm_persist.cu : persistent pairs of CTAs for prompt-sized T; 128-row boxes of both operands
+bool gemm_use_persist(int T, int N, int split, bool dual);
+cudaError_t launch_gemm_persist_partial(const TmaMap &w_map128, const TmaMap &x_map128, float *out, int T, int N, int K,
+                                        int w_row0, int split, cudaStream_t st);
 // the same product, its epilogue writing bf16(relu(sum)^2) (an ungated unit's activation) instead of the fp32 sums
-cudaError_t launch_gemm_persist_relu2(const TmaMap &w_map128, const TmaMap &x_map256, uint16_t *act, int T, int N, int K, int w_row0,
+cudaError_t launch_gemm_persist_relu2(const TmaMap &w_map128, const TmaMap &x_map128, uint16_t *act, int T, int N, int K, int w_row0,
                                       cudaStream_t st);
-cudaError_t launch_gemm_persist_silu(const TmaMap &w_map64, const TmaMap &x_map256, uint16_t *act, int T, int I, int K,
+cudaError_t launch_gemm_persist_silu(const TmaMap &w_map128, const TmaMap &x_map128, uint16_t *act, int T, int I, int K,
                                      int w_row0, cudaStream_t st);
-cudaError_t launch_gemm_persist_glu(const TmaMap &w_map64, const TmaMap &x_map256, uint16_t *act, int T, int I, int K,
+cudaError_t launch_gemm_persist_glu(const TmaMap &w_map128, const TmaMap &x_map128, uint16_t *act, int T, int I, int K,
                                     int w_row0, int act_kind, cudaStream_t st, int ld_act = 0);  // ld_act: row stride of act (0: I)
 cudaError_t launch_gemm_silu(const TmaMap &w_map, const TmaMap &x_map, uint16_t *act, int T, int I, int K,
                              int w_row0, int tile_rows, cudaStream_t st);

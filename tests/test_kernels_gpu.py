@@ -121,6 +121,36 @@ def test_gemm_full_size_against_torch(T, N, K, silu):
         assert err <= 2e-4 * ref.abs().max().item(), err
 
 
+# Sizes at the edges of the pair kernel's tiles (256 tokens x 256, 224 or 192 columns, a K block of 64), rows that are and are not pieces
+# of 32 bytes, K slices, several rounds of its 74 pairs (the last three, whose tile widths differ).
+@pytest.mark.parametrize("T,N,K,split", [(1030, 131, 72, 1), (1281, 256, 64, 1), (1024, 1000, 200, 2), (1300, 264, 136, 3), (129, 4096, 256, 4),
+                                         (1100, 4100, 64, 1), (1300, 8192, 128, 2), (3000, 2504, 64, 1), (2600, 5000, 72, 1)])
+def test_gemm_pairs(T, N, K, split):
+    """Pairs of CTAs against float64 of the same bf16 operands: the sums are fp32, at most K terms of |x w|."""
+    g = torch.Generator(device=DEV); g.manual_seed(T + N + K)
+    X, W = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((T, K), (N, K)))
+    out = G.empty((split, T, N), dtype=torch.float32, device=DEV)
+    check(lib().dis_k_gemm(ptr(X), ptr(W), ptr(out), T, N, K, split, None))
+    sync()
+    ref = X.double() @ W.double().T
+    bound = K * 2.0 ** -24 * (X.double().abs() @ W.double().abs().T).max().item()
+    assert (out.double().sum(0) - ref).abs().max().item() <= bound
+
+
+@pytest.mark.parametrize("T,I,K", [(129, 40, 72), (256, 128, 64), (257, 131, 136), (700, 1000, 64), (1000, 4104, 64), (1300, 5632, 72), (3000, 2504, 64)])
+def test_gemm_silu_pairs(T, I, K):
+    """The gate-up product of the same kernel: silu(gate) * up against float64, one bf16 rounding plus the fast exponential and division."""
+    g = torch.Generator(device=DEV); g.manual_seed(T + I + K)
+    X, W = torch.randn((T, K), device=DEV, generator=g).to(torch.bfloat16), (torch.randn((2 * I, K), device=DEV, generator=g) * K ** -0.5).to(torch.bfloat16)
+    act = G.empty((T, I), dtype=torch.bfloat16, device=DEV)
+    check(lib().dis_k_gemm_silu(ptr(X), ptr(W), ptr(act), T, I, K, None))
+    sync()
+    gate, up = X.double() @ W[:I].double().T, X.double() @ W[I:].double().T
+    ref = gate * torch.sigmoid(gate) * up
+    # rounding to bf16's 8 significant bits is off by at most 2^-8 of the value; the fast functions add a few 1e-6 of it, the sums 1e-6 K
+    assert ((act.double() - ref).abs() <= BF16_ULP * ref.abs() * 1.01 + 1e-5).all()
+
+
 def test_gemm_rejects_empty_split():
     X, W = dev_bf16(np.zeros((8, 576), np.float32)), dev_bf16(np.zeros((128, 576), np.float32))
     out = G.zeros((4, 8, 128), dtype=torch.float32, device=DEV)
