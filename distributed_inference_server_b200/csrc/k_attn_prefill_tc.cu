@@ -20,9 +20,10 @@
 // memory, and it is raised only when a row's maximum exceeds it by more than 8 in the log2 domain (P <= 256, the reference cancels in
 // the final division by l), so O is rescaled in TMEM on few tiles only (decided per warp, scaled per lane).
 //
-// Measured against what it replaced: heads of 64 (mma.sync), six prompts of 276 to 1900 tokens, 32 / 4 heads, 31.6 GFLOP: 164.6 -> 76.4
+// Measured against what it replaced: heads of 64 (mma.sync), six prompts of 276 to 1900 tokens, 32 / 4 heads, 31.6 GFLOP: 164.6 -> 73.7
 // us; heads of 128 (one softmax group per CTA, P through shared memory), six prompts of 437 to 3000 tokens, 32 / 8 heads, 258 GFLOP:
-// 366.8 -> 349.1 us.  A key tile takes a CTA 1000 clocks (D = 64) or 1400 (D = 128), a CTA's start and end 8000 beside them.
+// 366.8 -> 345.2 us.  With two CTAs on an SM a key tile takes each 1230 clocks (D = 64: 620 per tile and SM, 512 of them exponentials) or
+// 1800 (D = 128: 900, 768 of them shared memory -- Q and K for S, V, and the tiles' arrival); a CTA's start and end take 5000 and 10000.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -125,7 +126,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
   auto s_full = [&](int w) { return bar_base + 48u + 8u * w; };
   auto p_full = [&](int w) { return bar_base + 64u + 8u * w; };
   auto pv_done = [&](int w) { return bar_base + 80u + 8u * w; };
-  const uint32_t tmem_slot = bar_base + 96;
+  const uint32_t q_full = bar_base + 96, tmem_slot = bar_base + 104;
   float *m_row = reinterpret_cast<float *>(smem + (bar_base - smem_base) + 256);  // [row]: the softmax reference, handed from tile to tile
   float *l_row = m_row + 128;                                                     // [group][row]: at the end
 
@@ -139,12 +140,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
       mbar_init(k_full(w), 1); mbar_init(k_empty(w), 1); mbar_init(v_full(w), 1); mbar_init(s_full(w), 1); mbar_init(pv_done(w), 1);
       mbar_init(p_full(w), 4);
     }
+    mbar_init(q_full, 8);
     fence_barrier_init();
     fence_proxy_async();
   }
   if (warp == 1) tmem_alloc<kPfTmemCols>(tmem_slot);
   pdl_launch_dependents();
   pdl_wait();  // q and this chunk's K/V rows come from the previous kernels
+  const int tok0 = qb_tok0[qb], len = qb_len[qb], pos0 = qb_pos0[qb];
+  const int *pt = page_table + (size_t)qb_ptrow[qb] * max_pages;
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -152,13 +156,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   const uint32_t o_base = tmem_base + 2 * kPfTile;
 
-  const int tok0 = qb_tok0[qb], len = qb_len[qb], pos0 = qb_pos0[qb];
-  const int *pt = page_table + (size_t)qb_ptrow[qb] * max_pages;
   const int page_size = 1 << page_shift;
   const int box_rows = min(page_size, kPfTile);  // rows of the tensor map's box
   const int end = pos0 + len;                    // keys [0, end)
   const int n_tiles = (end + kPfTile - 1) / kPfTile;
 
+  // Q is handed to the MMA warp by a barrier of its own: the key tiles are under way meanwhile
   if (warp >= 2) {  // Q tile: row = head * QT + token, K-major, 128B swizzle (rows of padding tokens are zero)
     const int row = (warp & 3) * 32 + lane, grp = (warp - 2) >> 2;
     const int hl = row / QT, t = row % QT;
@@ -172,8 +175,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
       *reinterpret_cast<uint4 *>(smem + off) = v;
     }
     fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(q_full);
   }
-  __syncthreads();
 
   if (warp == 0) {
     // ===== TMA producer: K_t as soon as S_{t-2} has read its slot, V_t as soon as P_{t-2} V_{t-2} has =====
@@ -219,6 +223,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
       }
       __syncwarp();
     };
+    mbar_wait(q_full, 0);
     issue_s(0);
     if (n_tiles > 1) issue_s(1);
     for (int j = 0; j < n_tiles; j++) {
