@@ -329,12 +329,264 @@ __global__ void stack_lightning_carry_kernel(const float *decay, const float *se
   st[e] = S;
 }
 
+// ---- the segments of a long span in block form, where the decay is one number per token and head (GATE 0, 2, 3)
+// Token by token, a segment's contribution and outputs cost 2 + 3 operations per state element and token, every one behind a dependent
+// update of the state, and the register kernel above reaches 26 and 31 % of the fp32 issue peak with them.  Over a segment of 64
+// tokens the same sums are matrix products, fp32 like everything here:
+//   contribution  sum_t w_t k_t v_t^T          w_t = prod_{u > t} a_u                              d dv per token
+//   outputs       o_i = sum_{j <= i} D_ij (q_i k_j) v_j + c_i q_i S_in    D_ij = prod_{j < u <= i} a_u, c_i = prod_{u <= i} a_u
+//                                                                                                  64 (d + dv/2) + d dv per token
+// with both operands of an outer product in registers (8 x 8 or 4 x 8 results per thread).  The decays' products are formed by
+// multiplication, never as quotients or exponentials, so a decay of zero needs no care.
+// Retention, 8 heads of 128 x 128, 6554 tokens of eight spans: contributions 161 -> 55 us, outputs 213 -> 160 us.
+constexpr int kLbLd = kLightSeg + 4;  // tokens of a transposed row, padded: float4 rows that start on different banks
+
+struct LightSpanSeg { int first, n; size_t at; };
+// false: this CTA's segment does not exist
+__device__ __forceinline__ bool light_segment(const StackSpans &sp, int max_seg, int H, int &h, LightSpanSeg &g) {
+  h = blockIdx.x % H;
+  const int sc = blockIdx.x / H, s = sc / max_seg, c = sc - s * max_seg;
+  const int tok0 = sp.sp_tok0[s], len = sp.sp_len[s];
+  if (c * kLightSeg >= len) return false;
+  g.first = tok0 + c * kLightSeg;
+  g.n = min(kLightSeg, len - c * kLightSeg);
+  g.at = (size_t)(tok0 / kLightSeg + s + c) * H + h;
+  return true;
+}
+template <int GATE>
+__device__ __forceinline__ float4 light_in(float4 v, float f) {
+  if (GATE == 0) return make_float4(silu_(v.x), silu_(v.y), silu_(v.z), silu_(v.w));
+  return make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+}
+
+template <int DT, int DVT, int GATE>
+__global__ void __launch_bounds__(256, 2) stack_light_contrib_kernel(const float *__restrict__ proj, long long ld, LightCols col, const float *decay,
+                                                                     const float *__restrict__ dec, StackSpans sp, int H, int d, int dv,
+                                                                     float *__restrict__ seg, float *__restrict__ seg_a, int max_seg) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float shm[];
+  float *ks = shm, *vs = ks + kLightSeg * DT, *wt = vs + kLightSeg * DVT;  // [tok][DT], [tok][DVT], [tok]
+  int h;
+  LightSpanSeg g;
+  if (!light_segment(sp, max_seg, H, h, g)) return;
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {  // w_t: products over the tokens behind t, lane l owning tokens 2 l and 2 l + 1
+    auto a_of = [&](int t) { return t < g.n ? (GATE == 2 ? dec[(long long)(g.first + t) * H + h] : decay[h]) : 1.f; };
+    const float a0 = a_of(2 * lane), a1 = a_of(2 * lane + 1);
+    float p = a0 * a1;  // -> product over this and all later lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float m = __shfl_down_sync(0xffffffffu, p, o);
+      if (lane + o < 32) p *= m;
+    }
+    float after = __shfl_down_sync(0xffffffffu, p, 1);
+    if (lane == 31) after = 1.f;
+    auto f_of = [&](int t) { return GATE == 2 && t < g.n ? col.vscale[(long long)(g.first + t) * H + h] : 1.f; };
+    wt[2 * lane] = a1 * after * f_of(2 * lane);
+    wt[2 * lane + 1] = after * f_of(2 * lane + 1);
+    const float all = __shfl_sync(0xffffffffu, p, 0);
+    if (GATE == 2)
+      for (int i = lane; i < d; i += 32) seg_a[g.at * d + i] = all;
+  }
+  __syncthreads();
+  const float *kp = proj + col.k + (long long)(h / col.hpg) * d, *vp = proj + col.v + (long long)h * dv;
+  const int d4 = d >> 2, dv4 = dv >> 2;
+  for (int e = threadIdx.x; e < g.n * d4; e += 256) {
+    const int t = e / d4, c = (e - t * d4) * 4;
+    *reinterpret_cast<float4 *>(ks + t * DT + c) = light_in<GATE>(*reinterpret_cast<const float4 *>(kp + (long long)(g.first + t) * ld + c), 1.f);
+  }
+  for (int e = threadIdx.x; e < g.n * dv4; e += 256) {
+    const int t = e / dv4, c = (e - t * dv4) * 4;
+    float4 v = light_in<GATE>(*reinterpret_cast<const float4 *>(vp + (long long)(g.first + t) * ld + c), 1.f);
+    const float f = wt[t];
+    *reinterpret_cast<float4 *>(vs + t * DVT + c) = make_float4(v.x * f, v.y * f, v.z * f, v.w * f);
+  }
+  __syncthreads();
+  constexpr int RI = DT / 16, RJ = DVT / 16;
+  const int ti = (threadIdx.x >> 4) * 4, tj = (threadIdx.x & 15) * 4;
+  float acc[RI][RJ];
+#pragma unroll
+  for (int i = 0; i < RI; i++)
+#pragma unroll
+    for (int j = 0; j < RJ; j++) acc[i][j] = 0.f;
+#pragma unroll 2
+  for (int t = 0; t < g.n; t++) {
+    float k[RI], v[RJ];
+#pragma unroll
+    for (int i = 0; i < RI; i += 4) *reinterpret_cast<float4 *>(k + i) = *reinterpret_cast<const float4 *>(ks + t * DT + ti + i * 16);
+#pragma unroll
+    for (int j = 0; j < RJ; j += 4) *reinterpret_cast<float4 *>(v + j) = *reinterpret_cast<const float4 *>(vs + t * DVT + tj + j * 16);
+#pragma unroll
+    for (int i = 0; i < RI; i++)
+#pragma unroll
+      for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(k[i], v[j], acc[i][j]);
+  }
+  float *sg = seg + g.at * d * dv;
+#pragma unroll
+  for (int i = 0; i < RI; i++) {
+    const int r = ti + (i >> 2) * 64 + (i & 3);
+#pragma unroll
+    for (int j = 0; j < RJ; j += 4) {
+      const int c = tj + j * 16;
+      if (r < d && c < dv) *reinterpret_cast<float4 *>(sg + (size_t)r * dv + c) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+    }
+  }
+}
+
+template <int DT, int DVT, int GATE>
+__global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float *__restrict__ proj, long long ld, LightCols col, const float *decay,
+                                                                    const float *__restrict__ dec, float qscale, StackSpans sp,
+                                                                    float *__restrict__ o, int H, int d, int dv, const float *__restrict__ seg,
+                                                                    int max_seg) {
+  pdl_launch_dependents();
+  pdl_wait();
+  extern __shared__ __align__(16) float shm[];
+  constexpr int kKv = DT * kLbLd > kLightSeg * DVT ? DT * kLbLd : kLightSeg * DVT;
+  float *qt = shm, *kv = qt + DT * kLbLd, *at = kv + kKv, *as = at + kLightSeg * kLbLd, *ci = as + kLightSeg;  // [c][tok], [c][tok] then [tok][DVT], [j][i], [tok], [tok]
+  int h;
+  LightSpanSeg g;
+  if (!light_segment(sp, max_seg, H, h, g)) return;
+  const int tid = threadIdx.x, dv4 = dv >> 2;
+  if (tid < kLightSeg) as[tid] = tid < g.n ? (GATE == 2 ? dec[(long long)(g.first + tid) * H + h] : decay[h]) : 1.f;
+  const float *qp = proj + col.q + (long long)(h / col.hpg) * d, *kp = proj + col.k + (long long)(h / col.hpg) * d, *vp = proj + col.v + (long long)h * dv;
+  {
+    const int t = tid & (kLightSeg - 1);
+    const long long row = (long long)(g.first + t) * ld;
+    for (int c = (tid >> 6) * 4; c < d; c += 16) {  // lanes are tokens: the transposed writes hit different banks
+      float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
+      if (t < g.n) {
+        q = light_in<GATE>(*reinterpret_cast<const float4 *>(qp + row + c), qscale);
+        k = light_in<GATE>(*reinterpret_cast<const float4 *>(kp + row + c), 1.f);
+      }
+      qt[(c + 0) * kLbLd + t] = q.x; qt[(c + 1) * kLbLd + t] = q.y; qt[(c + 2) * kLbLd + t] = q.z; qt[(c + 3) * kLbLd + t] = q.w;
+      kv[(c + 0) * kLbLd + t] = k.x; kv[(c + 1) * kLbLd + t] = k.y; kv[(c + 2) * kLbLd + t] = k.z; kv[(c + 3) * kLbLd + t] = k.w;
+    }
+  }
+  __syncthreads();
+  if (tid < kLightSeg) {  // thread j: D_ij times the factor on value j, zero above the diagonal
+    const float f = GATE == 2 && tid < g.n ? col.vscale[(long long)(g.first + tid) * H + h] : 1.f;
+    float p = 1.f;
+    for (int i = 0; i < kLightSeg; i++) {
+      if (i > tid) p *= as[i];
+      at[tid * kLbLd + i] = i < tid || tid >= g.n ? 0.f : p * f;
+    }
+  } else if (tid == kLightSeg) {
+    float p = 1.f;
+    for (int i = 0; i < kLightSeg; i++) { p *= as[i]; ci[i] = p; }
+  }
+  const int i0 = (tid >> 4) * 4, tj = (tid & 15) * 4;
+  float a[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) a[i][j] = 0.f;
+  if (tj <= i0 + 3) {  // (above the diagonal nothing is wanted)
+#pragma unroll 4
+    for (int c = 0; c < d; c++) {
+      const float4 q = *reinterpret_cast<const float4 *>(qt + c * kLbLd + i0), k = *reinterpret_cast<const float4 *>(kv + c * kLbLd + tj);
+      const float qv[4] = {q.x, q.y, q.z, q.w}, kw[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) a[i][j] = fmaf(qv[i], kw[j], a[i][j]);
+    }
+  }
+  __syncthreads();  // D is complete and the keys are no longer needed
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    float4 *p = reinterpret_cast<float4 *>(at + (tj + j) * kLbLd + i0);
+    const float4 f = *p;
+    *p = make_float4(f.x * a[0][j], f.y * a[1][j], f.z * a[2][j], f.w * a[3][j]);
+  }
+  for (int e = tid; e < g.n * dv4; e += 256) {
+    const int t = e / dv4, c = (e - t * dv4) * 4;
+    *reinterpret_cast<float4 *>(kv + t * DVT + c) = light_in<GATE>(*reinterpret_cast<const float4 *>(vp + (long long)(g.first + t) * ld + c), 1.f);
+  }
+  constexpr int RJ = DVT / 16;
+  float acc[4][RJ];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < RJ; j++) acc[i][j] = 0.f;
+  const float *sg = seg + g.at * d * dv;
+  bool in[RJ / 4];
+#pragma unroll
+  for (int j = 0; j < RJ / 4; j++) in[j] = tj + j * 64 < dv;
+#pragma unroll 4
+  for (int c = 0; c < d; c++) {
+    const float4 q = *reinterpret_cast<const float4 *>(qt + c * kLbLd + i0);
+    const float qv[4] = {q.x, q.y, q.z, q.w};
+    float s[RJ];
+#pragma unroll
+    for (int j = 0; j < RJ; j += 4)
+      *reinterpret_cast<float4 *>(s + j) = in[j / 4] ? *reinterpret_cast<const float4 *>(sg + (size_t)c * dv + tj + j * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(qv[i], s[j], acc[i][j]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float f = ci[i0 + i];
+#pragma unroll
+    for (int j = 0; j < RJ; j++) acc[i][j] *= f;
+  }
+  __syncthreads();
+  const int last = min(i0 + 4, g.n);
+#pragma unroll 2
+  for (int t = 0; t < last; t++) {
+    const float4 w = *reinterpret_cast<const float4 *>(at + t * kLbLd + i0);
+    const float wv[4] = {w.x, w.y, w.z, w.w};
+    float v[RJ];
+#pragma unroll
+    for (int j = 0; j < RJ; j += 4) *reinterpret_cast<float4 *>(v + j) = *reinterpret_cast<const float4 *>(kv + t * DVT + tj + j * 16);
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(wv[i], v[j], acc[i][j]);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    if (i0 + i >= g.n) continue;
+    float *op = o + (long long)(g.first + i0 + i) * H * dv + (long long)h * dv;
+#pragma unroll
+    for (int j = 0; j < RJ; j += 4)
+      if (in[j / 4]) *reinterpret_cast<float4 *>(op + tj + j * 16) = make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
+  }
+}
+
+// The block form reads rows as float4: heads, offsets and strides in fours, rows that start on 16 bytes.
+static bool light_block_ok(const float *proj, long long ld, const LightCols &col, const float *o, const float *seg, int d, int dv) {
+  auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  return stack_lightning_block(d, dv) && ld % 4 == 0 && col.q % 4 == 0 && col.k % 4 == 0 && col.v % 4 == 0 && al(proj) && al(o) && al(seg);
+}
+template <int DT, int DVT, int GATE>
+static cudaError_t light_block(const float *proj, long long ld, const LightCols &col, const float *decay, const float *dec, float qscale, float *state,
+                               const StackSpans &sp, float *o, int H, int d, int dv, float *seg, float *seg_a, int max_len, cudaStream_t st) {
+  const size_t sh_a = (size_t)kLightSeg * (DT + DVT + 1) * sizeof(float);
+  const size_t sh_b = (size_t)(DT * kLbLd + (DT * kLbLd > kLightSeg * DVT ? DT * kLbLd : kLightSeg * DVT) + kLightSeg * kLbLd + 2 * kLightSeg) * sizeof(float);
+  static DeviceOnce once;
+  DIS_CUDA_TRY(once.run([&] {
+    const cudaError_t e = cudaFuncSetAttribute(stack_light_contrib_kernel<DT, DVT, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh_a);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(stack_light_output_kernel<DT, DVT, GATE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh_b);
+  }));
+  const int max_seg = (max_len + kLightSeg - 1) / kLightSeg;
+  launch_k(stack_light_contrib_kernel<DT, DVT, GATE>, dim3(sp.n_spans * max_seg * H), dim3(256), sh_a, st, proj, ld, col, decay, dec, sp, H, d, dv, seg, seg_a, max_seg);
+  launch_k(stack_lightning_carry_kernel, dim3(sp.n_spans * H * ((d * dv + 255) / 256)), dim3(256), 0, st, decay, GATE == 2 ? seg_a : nullptr, state, sp, seg, H, d, dv);
+  launch_k(stack_light_output_kernel<DT, DVT, GATE>, dim3(sp.n_spans * max_seg * H), dim3(256), sh_b, st, proj, ld, col, decay, dec, qscale, sp, o, H, d, dv, seg, max_seg);
+  return cudaGetLastError();
+}
+
 int stack_lightning_seg_tokens() { return kLightSeg; }
+bool stack_lightning_block(int d, int dv) { return d <= 128 && dv <= 128 && d % 4 == 0 && dv % 4 == 0; }
 // Whether a pass should cut its long spans into segments.  Walking a span in one piece costs its length times three
 // operations per state element, once per wave of (span, head) CTAs (two fit an SM); the segments cost five operations per
 // element (contributions, then outputs) over all segment CTAs in waves, plus the carry.  Many sequences with many heads fill
-// the GPU without segments and then pay less; a single long prompt needs them.
-bool stack_lightning_segmented(int n_spans, int T, int H, int max_len) {
+// the GPU without segments and then pay less; a single long prompt needs them.  block: the segments run in block form, whose
+// contributions and outputs together take about what two operations per element take here (a state-space pass of 256 (sequence, head)
+// pairs, 8 x 1024 tokens, 32 heads of 128 x 64 in four layers: 5.1 ms cut, 5.6 whole).
+bool stack_lightning_segmented(int n_spans, int T, int H, int max_len, bool block) {
   if (max_len <= kLightSeg) return false;
   const char *force = getenv("DIS_STACK_LIGHT_SEGMENTS");  // 2: always cut (tests)
   if (force && atoi(force) == 2) return true;
@@ -347,7 +599,7 @@ bool stack_lightning_segmented(int n_spans, int T, int H, int max_len) {
   const long long pairs = (long long)n_spans * H;
   const long long whole = (long long)max_len * ((pairs + slots - 1) / slots) * 3;
   const long long seg_ctas = ((long long)T / kLightSeg + n_spans) * H;
-  const long long cut = ((seg_ctas + slots - 1) / slots) * kLightSeg * 5 + kLightSeg;
+  const long long cut = ((seg_ctas + slots - 1) / slots) * kLightSeg * (block ? 2 : 5) + kLightSeg;
   return cut < whole;
 }
 size_t stack_lightning_seg_floats(int cap_tokens, int max_spans, int H, int d, int dv) {
@@ -372,6 +624,12 @@ static cudaError_t lightning_reg(const float *proj, long long ld, LightCols col,
   if (!seg || (DEC && !seg_a) || max_len <= kLightSeg) {
     launch_k(stack_lightning_reg_kernel<RI, RJ, 0, GATE>, dim3(sp.n_spans * H), dim3(256), (size_t)(sh), st, proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, nullptr, nullptr, 1, fin);
     return cudaGetLastError();
+  }
+  if constexpr (GATE != 1) {
+    if (light_block_ok(proj, ld, col, o, seg, d, dv)) {
+      auto f = d <= 64 ? (dv <= 64 ? light_block<64, 64, GATE> : light_block<64, 128, GATE>) : (dv <= 64 ? light_block<128, 64, GATE> : light_block<128, 128, GATE>);
+      return f(proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_len, st);
+    }
   }
   const int max_seg = (max_len + kLightSeg - 1) / kLightSeg;
   launch_k(stack_lightning_reg_kernel<RI, RJ, 1, GATE>, dim3(sp.n_spans * max_seg * H), dim3(256), (size_t)(sh), st, proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_seg, fin);

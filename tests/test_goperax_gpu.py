@@ -239,6 +239,24 @@ def test_many_heads_and_sequences_walk_long_spans_whole(monkeypatch, force):
     e.close()
 
 
+@pytest.mark.parametrize("state,vdim,heads,groups", [(128, 64, 4, 2), (20, 36, 6, 3), (68, 128, 2, 1)])
+def test_segments_in_block_form(monkeypatch, state, vdim, heads, groups):
+    """State-space spans cut into segments of 64 tokens that run as matrix products, with one decay and step size per token and head:
+    a segment exactly full, one token more, a single token, and second portions from a state that is not zero.  Against the oracle."""
+    monkeypatch.setenv("DIS_STACK_LIGHT_SEGMENTS", "2")
+    cfg = U.config([(U.ssm(heads=heads, vdim=vdim, state=state, groups=groups, conv=3, norm_groups=2), None)], width=40, streams=0)
+    W = U.weights(cfg, seed=state + vdim)
+    seqs = {k: toks(195, seed=70 + k) for k in range(3)}
+    e = U.engine(cfg, W, pool_tokens=3 * 208, page_size=16, max_batch=3, max_step_tokens=512)
+    f = U.Feeder(e)
+    f.step([(0, seqs[0], 64), (1, seqs[1], 65), (2, seqs[2], 1)])
+    f.step([(0, seqs[0], 131), (1, seqs[1], 67), (2, seqs[2], 131)])
+    for k in seqs:
+        got = f.end(k)
+        assert U.rel_err(got, U.oracle_logits(cfg, W, seqs[k])[:len(got)]) < 5e-5
+    e.close()
+
+
 def test_large_passes_take_the_tensor_core_expert_products(monkeypatch):
     """A pass of 1280 prompt tokens in bfloat16: per-expert tensor-core products over rows sorted by expert and the shared unit
     on the tensor cores.  Against the oracle, and against the same pass on the tiled fp32-FMA products (DIS_STACK_TC=0), which

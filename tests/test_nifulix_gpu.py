@@ -222,6 +222,25 @@ def test_many_heads_and_sequences_walk_long_spans_whole(monkeypatch, force):
     e.close()
 
 
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (64, 64), (36, 68), (100, 64), (68, 128)])
+def test_segments_in_block_form(monkeypatch, dim, vdim):
+    """Spans cut into segments of 64 tokens that run as matrix products (heads in fours up to 128): one token beside a long span, a
+    segment exactly full, one token more, a last segment of three, a second portion from a state that is not zero, a decay of
+    almost zero and one of almost one.  Float32, against the oracle token by token."""
+    monkeypatch.setenv("DIS_STACK_LIGHT_SEGMENTS", "2")
+    cfg = U.config([(U.retention(heads=3, dim=dim, vdim=vdim, rot=min(dim, 32), decay=[1e-3, 0.9, 0.9999]), None)], width=48)
+    W = U.weights(cfg, seed=dim + vdim)
+    seqs = {k: toks(131 + 64, seed=60 + k) for k in range(3)}
+    e = U.engine(cfg, W, pool_tokens=3 * 208, page_size=16, max_batch=3, max_step_tokens=512)
+    f = U.Feeder(e)
+    f.step([(0, seqs[0], 64), (1, seqs[1], 65), (2, seqs[2], 1)])
+    f.step([(0, seqs[0], 131), (1, seqs[1], 67), (2, seqs[2], 131)])
+    for k in seqs:
+        got = f.end(k)
+        assert U.rel_err(got, U.oracle_logits(cfg, W, seqs[k])[:len(got)]) < 5e-5
+    e.close()
+
+
 def test_large_prompt_passes_on_the_persistent_products(monkeypatch):
     """2048 prompt tokens in bfloat16 through parallel layers wide enough for the persistent tensor-core products, whose gated-unit
     epilogue writes into the columns behind the mixer's.  Against the oracle at a few positions, and against the same pass with
