@@ -241,7 +241,7 @@ __global__ void stack_sum_bias_kernel(const float *part, int n_part, long long s
   pdl_wait();
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float s = bias ? bias[i % N] : 0.f;
-    for (int k = 0; k < n_part; k++) s += part[(long long)k * stride + i];
+    each_slice<8>(0, n_part, [&](int k) { return part[(long long)k * stride + i]; }, [&](float p) { s += p; });
     out[i] = s;
   }
 }
@@ -279,8 +279,9 @@ __global__ void stack_embed_kernel(const void *embed, const uint32_t *tokens, co
 cudaError_t launch_stack_embed(const void *embed, bool f32, const uint32_t *tokens, const int *pos, const double *pos_freq, float *x,
                                float *x0, float scale, int T, int W, int streams, cudaStream_t st) {
   if (streams < 1) streams = 1;
-  if (f32) launch_k(stack_embed_kernel<true>, dim3(T), dim3(128), 0, st, embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
-  else launch_k(stack_embed_kernel<false>, dim3(T), dim3(128), 0, st, embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
+  const int th = T <= 148 ? 512 : 128;  // few tokens: an angle or two per thread
+  if (f32) launch_k(stack_embed_kernel<true>, dim3(T), dim3(th), 0, st, embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
+  else launch_k(stack_embed_kernel<false>, dim3(T), dim3(th), 0, st, embed, tokens, pos, pos_freq, x, x0, scale, W, streams);
   return cudaGetLastError();
 }
 
@@ -555,7 +556,6 @@ __global__ void __launch_bounds__(256) stack_boundary_hc_kernel(float *xs, int S
                                                                 const float *__restrict__ bias, const float *prev, const float *next,
                                                                 const float *__restrict__ pre_w, void *hc, int W, float eps, float mult) {
   pdl_launch_dependents();
-  pdl_wait();
   extern __shared__ __align__(16) float row[];  // [W]: u
   __shared__ float sh[32];
   __shared__ float cf[2 * kHcMaxStreams + kHcMaxStreams * kHcMaxStreams];  // out[S] | mix[S][S] of prev, then in[S] of next
@@ -569,6 +569,7 @@ __global__ void __launch_bounds__(256) stack_boundary_hc_kernel(float *xs, int S
     c_in[threadIdx.x] = next ? next[threadIdx.x] : (threadIdx.x == 0 ? 1.f : 0.f);
   }
   if (threadIdx.x < S * S) c_mix[threadIdx.x] = prev ? prev[2 * S + threadIdx.x] : (threadIdx.x % (S + 1) == 0 ? 1.f : 0.f);
+  pdl_wait();  // the coefficients are weights; everything below comes from the kernels before
   __syncthreads();
   auto ld = [](const float *p, float (&o)[V]) {
     if (VEC) { const float4 v = *reinterpret_cast<const float4 *>(p); o[0] = v.x; o[V > 1 ? 1 : 0] = v.y; o[V > 2 ? 2 : 0] = v.z; o[V > 3 ? 3 : 0] = v.w; }
@@ -599,12 +600,11 @@ __global__ void __launch_bounds__(256) stack_boundary_hc_kernel(float *xs, int S
 #pragma unroll
         for (int e = 0; e < V; e++) v[e] = 0.f;
       }
-      for (int k = 0; k < n_part; k++) {
-        float p[V];
-        ld(y + (long long)k * stride + t * W + i, p);
+      struct Piece { float p[V]; };
+      each_slice<8>(0, n_part, [&](int k) { Piece q; ld(y + (long long)k * stride + t * W + i, q.p); return q; }, [&](const Piece &q) {
 #pragma unroll
-        for (int e = 0; e < V; e++) v[e] += p[e];
-      }
+        for (int e = 0; e < V; e++) v[e] += q.p[e];
+      });
 #pragma unroll
       for (int e = 0; e < V; e++) v[e] *= mult;
 #pragma unroll
@@ -992,11 +992,13 @@ __global__ void stack_glu_kernel(const float *__restrict__ gu, int n_part, long 
           const float4 bg = *reinterpret_cast<const float4 *>(bias + c), bu = GATED ? *reinterpret_cast<const float4 *>(bias + ff + c) : zero4;
           g.x += bg.x; g.y += bg.y; g.z += bg.z; g.w += bg.w; u.x += bu.x; u.y += bu.y; u.z += bu.z; u.w += bu.w;
         }
-        for (int k = 1; k < n_part; k++) {
-          const float4 pg = *reinterpret_cast<const float4 *>(gr + (long long)k * stride + c);
-          const float4 pu = GATED ? *reinterpret_cast<const float4 *>(gr + (long long)k * stride + ff + c) : zero4;
-          g.x += pg.x; g.y += pg.y; g.z += pg.z; g.w += pg.w; u.x += pu.x; u.y += pu.y; u.z += pu.z; u.w += pu.w;
-        }
+        struct Two { float4 g, u; };
+        each_slice<4>(1, n_part, [&](int k) {
+          const float *p = gr + (long long)k * stride + c;
+          return Two{*reinterpret_cast<const float4 *>(p), GATED ? *reinterpret_cast<const float4 *>(p + ff) : zero4};
+        }, [&](const Two &p) {
+          g.x += p.g.x; g.y += p.g.y; g.z += p.g.z; g.w += p.g.w; u.x += p.u.x; u.y += p.u.y; u.z += p.u.z; u.w += p.u.w;
+        });
         const float v0 = glu_unit<ACT>(g.x, u.x, limit), v1 = glu_unit<ACT>(g.y, u.y, limit), v2 = glu_unit<ACT>(g.z, u.z, limit),
                     v3 = glu_unit<ACT>(g.w, u.w, limit);
         if (F32) *reinterpret_cast<float4 *>(reinterpret_cast<float *>(act) + (long long)r * ld_act + c) = make_float4(v0, v1, v2, v3);

@@ -4,6 +4,22 @@
 
 namespace dis {
 
+// K slices first .. n - 1 of a product, added in order with B of them on their way at a time: read one by one, sixteen slices of a decode
+// pass's down projection cost a boundary kernel sixteen L2 latencies.
+template <int B, class Load, class Add>
+__device__ __forceinline__ void each_slice(int first, int n, Load load, Add add) {
+  if (n == first + 1) { add(load(first)); return; }  // prompt passes: one slice
+  for (int k0 = first; k0 < n; k0 += B) {
+    decltype(load(0)) p[B];
+#pragma unroll
+    for (int j = 0; j < B; j++)
+      if (k0 + j < n) p[j] = load(k0 + j);
+#pragma unroll
+    for (int j = 0; j < B; j++)
+      if (k0 + j < n) add(p[j]);
+  }
+}
+
 template <bool F32>
 __device__ __forceinline__ float ld_el(const void *p, long long i) {
   if (F32) return reinterpret_cast<const float *>(p)[i];
