@@ -145,13 +145,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
     fence_proxy_async();
   }
   if (warp == 1) tmem_alloc<kPfTmemCols>(tmem_slot);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  // Only now, with the allocation done: a CTA of the next kernel that took its columns first would wait for this grid, and this CTA for
+  // those columns.
   pdl_launch_dependents();
   pdl_wait();  // q and this chunk's K/V rows come from the previous kernels
   const int tok0 = qb_tok0[qb], len = qb_len[qb], pos0 = qb_pos0[qb];
   const int *pt = page_table + (size_t)qb_ptrow[qb] * max_pages;
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
   uint32_t tmem_base;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
   const uint32_t o_base = tmem_base + 2 * kPfTile;

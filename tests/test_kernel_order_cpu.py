@@ -1,0 +1,43 @@
+"""Order of the steps in a kernel's start, read from the sources.
+
+A kernel that allocates tensor memory may let the next kernel's CTAs onto its SM (programmatic dependent launch) only when the whole CTA
+knows that the allocation is done: the trigger of any one thread counts for its CTA, and two kernels that each hold a part of an SM's 512
+columns and wait for the rest would never end."""
+import glob
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "distributed_inference_server_b200", "csrc")
+
+
+def kernels():
+    for path in sorted(glob.glob(os.path.join(CSRC, "*.cu"))):
+        s = re.sub(r"//[^\n]*", "", open(path).read())
+        for m in re.finditer(r"__global__", s):
+            name = re.search(r"(\w*kernel\w*)\s*\(", s[m.start():])
+            at = m.start() + name.end()
+            depth = 1
+            while depth:  # the end of the parameter list
+                depth += {"(": 1, ")": -1}.get(s[at], 0)
+                at += 1
+            start = at = s.index("{", at)
+            depth = 0
+            while True:
+                depth += {"{": 1, "}": -1}.get(s[at], 0)
+                at += 1
+                if depth == 0:
+                    break
+            yield name.group(1), s[start:at]
+
+
+def test_tensor_memory_is_allocated_before_the_next_kernel_may_start():
+    seen = 0
+    for name, body in kernels():
+        alloc = re.search(r"tmem_alloc|tcgen05\.alloc", body)
+        trigger = body.find("pdl_launch_dependents")
+        if alloc is None or trigger < 0:
+            continue
+        seen += 1
+        barrier = body.find("__syncthreads()", alloc.end())
+        assert 0 <= barrier < trigger, f"{name}: the trigger stands in front of the barrier that follows the allocation"
+    assert seen >= 3
