@@ -14,18 +14,25 @@
 //   warps 2-5   softmax of the even tiles, warps 6-9 of the odd ones, one thread per row: S_j from TMEM, causal mask, row maximum (no
 //               shuffles: a thread owns a whole row); P_j = exp2(s - m) goes as packed bf16 back into S_j's own TMEM columns (no
 //               shared-memory write, proxy fence or second read of it)
-// TMEM per CTA: S0 | S1 64 columns each | O D columns = 256; shared memory Q + 2 K + 2 V = 96 KB (D = 128): two CTAs per SM, so four
-// softmax groups take turns on the exponentials (16 per clock and SM: 1024 clocks per 128 rows x 128 keys, beside 512 or 1024 of the
-// tensor pipe).  O accumulates in TMEM; the two groups share a row's softmax reference m_ref, handed from tile to tile through shared
-// memory, and it is raised only when a row's maximum exceeds it by more than 8 in the log2 domain (P <= 256, the reference cancels in
-// the final division by l), so O is rescaled in TMEM on few tiles only (decided per warp, scaled per lane).
+// TMEM per CTA: S0 | S1 64 columns each | O (D = 128: 128 columns; D = 64: one of 64 for each group) = 256; shared memory Q + 2 K + 2 V =
+// 96 KB (D = 128): two CTAs per SM, so four softmax groups take turns on the exponentials (16 per clock and SM: 1024 clocks per 128 rows x
+// 128 keys, beside 512 or 1024 of the tensor pipe).  O accumulates in TMEM.
+//   D = 64   each group has an O and a reference of its own, the running maximum of its tiles: a row's largest weight is exactly 1 when it
+//            is rounded to bf16, and O is rescaled behind the group's own P V, which the next S waits for anyway.  The two are joined at
+//            the end.  With the lazy reference below the results were 3.5 % further from 64 bits than weights rounded under the row's own
+//            maximum are, as the mma.sync kernel rounds them; so they are no further.
+//   D = 128  no columns are left for a second O: the two groups share a row's reference m_ref, handed from tile to tile through shared
+//            memory and raised only when a row's maximum exceeds it by more than 8 in the log2 domain (P <= 256, the reference cancels
+//            in the final division by l), so O is rescaled on few tiles only (decided per warp, scaled per lane).
 //
-// Measured against what it replaced: heads of 64 (mma.sync), six prompts of 276 to 1900 tokens, 32 / 4 heads, 31.6 GFLOP: 164.6 -> 73.7
-// us; heads of 128 (one softmax group per CTA, P through shared memory), six prompts of 437 to 3000 tokens, 32 / 8 heads, 258 GFLOP:
-// 366.8 -> 345.2 us.  With two CTAs on an SM a key tile takes each 1230 clocks (D = 64: 620 per tile and SM, 512 of them exponentials) or
-// 1800 (D = 128: 900, 768 of them shared memory -- Q and K for S, V, and the tiles' arrival); a CTA's start and end take 5000 and 10000.
+// Measured against what it replaced: heads of 64 (mma.sync), six prompts of 276 to 1900 tokens, 32 / 4 heads, 31.6 GFLOP: 165.1 -> 78.8
+// us (with the lazy reference 74.0); heads of 128 (one softmax group per CTA, P through shared memory), six prompts of 437 to 3000
+// tokens, 32 / 8 heads, 258 GFLOP: 362.4 -> 340.5 us.  With two CTAs on an SM a key tile takes each 1230 clocks (D = 64, lazy: 620 per
+// tile and SM, 512 of them exponentials) or 1800 (D = 128: 900, 768 of them shared memory -- Q and K for S, V, and the tiles' arrival);
+// a CTA's start and end take 5000 and 10000.
 #include <cuda.h>
 
+#include <cfloat>
 #include <cstdlib>
 #include <cstring>
 
@@ -51,7 +58,7 @@ constexpr int kPfThreads = 320;
 constexpr int kPfQHalf = 128 * 128;  // one [128 rows][64 dims] block of Q, 16 KB
 
 template <int D>
-constexpr int pf_smem_bytes() { return (D / 64) * (kPfQHalf + 4 * kPfHalf) + 3 * 128 * 4 + 256; }
+constexpr int pf_smem_bytes() { return (D / 64) * (kPfQHalf + 4 * kPfHalf) + 4 * 128 * 4 + 256; }
 
 // Packed pairs: one issue slot for two lanes' worth of work
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
@@ -113,6 +120,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
                         uint16_t *__restrict__ out, int n_heads, int n_kv, int page_shift) {
   constexpr int QT = 128 / G;
   constexpr int kHalves = D / 64;
+  constexpr bool kOwn = 2 * kPfTile + 2 * D <= kPfTmemCols;  // an O and a softmax reference of each group's own
   constexpr uint32_t kSlot = kHalves * kPfHalf;  // one K or V tile
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t smem_base = smem_u32(smem_al);
@@ -127,8 +135,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
   auto p_full = [&](int w) { return bar_base + 64u + 8u * w; };
   auto pv_done = [&](int w) { return bar_base + 80u + 8u * w; };
   const uint32_t q_full = bar_base + 96, tmem_slot = bar_base + 104;
-  float *m_row = reinterpret_cast<float *>(smem + (bar_base - smem_base) + 256);  // [row]: the softmax reference, handed from tile to tile
-  float *l_row = m_row + 128;                                                     // [group][row]: at the end
+  float *l_row = reinterpret_cast<float *>(smem + (bar_base - smem_base) + 256);  // [group][row]: at the end
+  float *m_row = l_row + 256;  // one O: [row], the softmax reference, handed from tile to tile; two: [group][row], at the end
 
   // later query blocks of a sequence have more key tiles: launch them first, so that the longest CTAs do not form the tail
   const int qb = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y;
@@ -236,7 +244,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
       if (elect_one()) {
         const uint32_t b = v_lo + w * (kSlot >> 4), a = tmem_base + w * kPfTile;
 #pragma unroll
-        for (uint32_t k = 0; k < kPfTile / 16; k++) umma_ts(o_base, a + 8 * k, b + k * 128, idesc_o, k > 0 ? 1u : (uint32_t)(j > 0));
+        for (uint32_t k = 0; k < kPfTile / 16; k++)
+          umma_ts(o_base + (kOwn ? w * D : 0), a + 8 * k, b + k * 128, idesc_o, k > 0 ? 1u : (uint32_t)(j > (kOwn ? 1 : 0)));
         umma_commit(pv_done(w));
       }
       __syncwarp();
@@ -253,11 +262,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
     const int hl = row / QT, t = row % QT;
     const int qp = pos0 + t;
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-    const uint32_t s_addr = tmem_base + lane_off + grp * kPfTile, o_addr = o_base + lane_off;
+    const uint32_t s_addr = tmem_base + lane_off + grp * kPfTile, o_addr = o_base + lane_off + (kOwn ? grp * D : 0);
     const int bar_in = 1 + 4 * grp + quarter, bar_out = 1 + 4 * (grp ^ 1) + quarter;  // hand-over of m_row to this group / to the other
     const float scale_log2 = rsqrtf((float)D) * 1.4426950408889634f;
     const float2 scale2 = make_float2(scale_log2, scale_log2);
-    float m_ref = -INFINITY, l_run = 0.f;
+    float m_ref = kOwn ? -FLT_MAX : -INFINITY, l_run = 0.f;  // (finite where a group's first tile may hide every key of a row)
     for (int j = grp; j < n_tiles; j += 2) {
       mbar_wait(s_full(grp), (uint32_t)(j >> 1) & 1u);
       tc_fence_after();
@@ -277,8 +286,14 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
 #pragma unroll
       for (int i = 0; i < 32; i++) mx4[i & 3] = max3(mx4[i & 3], __uint_as_float(s[0][i]), __uint_as_float(s[1][i]));
       const float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3])) * scale_log2;  // scale > 0: it commutes with the maximum
-      float m_now;
-      if (j == 0) {
+      float m_now, f = 1.0f;
+      bool rescale = false;
+      if (kOwn) {
+        // S_j was issued behind P_{j-2} V_{j-2}: this group's O is complete, and nobody else touches it
+        m_now = fmaxf(m_ref, mx);
+        rescale = j >= 2 && __any_sync(0xffffffffu, mx > m_ref);
+        f = ex2_approx(m_ref - m_now);
+      } else if (j == 0) {
         m_now = mx;  // finite: key 0 is visible to every query; O is first written by P_0 V_0 (accumulate off)
       } else {
         named_sync_64(bar_in);
@@ -289,13 +304,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
           // every P V so far must be in O; none follows before this tile's P is handed over
           mbar_wait(pv_done(grp ^ 1), (uint32_t)((j - 1) >> 1) & 1u);
           tc_fence_after();
-          const float f = need ? ex2_approx(m_old - mx) : 1.0f;
+          f = need ? ex2_approx(m_old - mx) : 1.0f;
 #pragma unroll 1
           for (int c = 0; c < D; c += 32) rescale_32(o_addr + c, f);
           tmem_st_wait();
         }
       }
-      if (j + 1 < n_tiles) {
+      if (!kOwn && j + 1 < n_tiles) {
         m_row[row] = m_now;
         named_arrive_64(bar_out);
       }
@@ -317,18 +332,35 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
         }
         tmem_st_32x16(s_addr + 16 * c, pk);
       }
+      if (kOwn && rescale) {
+#pragma unroll
+        for (int c = 0; c < D; c += 32) rescale_32(o_addr + c, f);
+      }
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full(grp));
       l_run += (ps[0].x + ps[0].y) + (ps[1].x + ps[1].y);
     }
-    // the group of the last tile publishes the final reference; then each brings its sum to it
-    if (grp == ((n_tiles - 1) & 1)) m_row[row] = m_ref;
-    asm volatile("bar.sync 9, 256;" ::: "memory");
-    l_row[grp * 128 + row] = l_run * ex2_approx(m_ref - m_row[row]);
-    asm volatile("bar.sync 9, 256;" ::: "memory");
-    const float inv = 1.0f / (l_row[row] + l_row[128 + row]);
+    float inv, f0 = 1.f, f1 = 1.f;  // what the two groups' O are weighted with
+    if (kOwn) {
+      m_row[grp * 128 + row] = m_ref;
+      l_row[grp * 128 + row] = l_run;
+      asm volatile("bar.sync 9, 256;" ::: "memory");
+      const float m0 = m_row[row], m1 = m_row[128 + row], m = fmaxf(m0, m1);
+      f0 = ex2_approx(m0 - m);
+      f1 = ex2_approx(m1 - m);
+      inv = 1.0f / (l_row[row] * f0 + l_row[128 + row] * f1);
+      f0 *= inv;
+      f1 *= inv;
+    } else {
+      // the group of the last tile publishes the final reference; then each brings its sum to it
+      if (grp == ((n_tiles - 1) & 1)) m_row[row] = m_ref;
+      asm volatile("bar.sync 9, 256;" ::: "memory");
+      l_row[grp * 128 + row] = l_run * ex2_approx(m_ref - m_row[row]);
+      asm volatile("bar.sync 9, 256;" ::: "memory");
+      inv = 1.0f / (l_row[row] + l_row[128 + row]);
+    }
     mbar_wait(pv_done((n_tiles - 1) & 1), (uint32_t)((n_tiles - 1) >> 1) & 1u);
     tc_fence_after();
     uint4 *o = reinterpret_cast<uint4 *>(out + ((size_t)(tok0 + t) * n_heads + kvh * G + hl) * D);
@@ -336,8 +368,20 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
     for (int cc = 0; cc < D / 2; cc += 32) {
       const int c = grp * (D / 2) + cc;
       uint32_t v[32];
-      tmem_ld_32x32(o_addr + c, v);
+      tmem_ld_32x32(o_base + lane_off + c, v);
       tmem_ld_wait();
+      if (kOwn) {
+#pragma unroll
+        for (int i = 0; i < 32; i++) v[i] = __float_as_uint(__uint_as_float(v[i]) * f0);
+        if (n_tiles > 1) {
+          uint32_t u[32];
+          tmem_ld_32x32(o_base + lane_off + D + c, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; i++) v[i] = __float_as_uint(fmaf(__uint_as_float(u[i]), f1, __uint_as_float(v[i])));
+        }
+        inv = 1.f;
+      }
       if (t < len) {
 #pragma unroll
         for (int i = 0; i < 4; i++) {
