@@ -351,6 +351,7 @@ sample_kernel(const float *__restrict__ logits, long long ld, int V, const float
     }
     tau = lo;
   }
+  tau = max(tau, 1u);  // a weight of zero is never kept: the draw's last-token fallback may not return it
   kept = mass_at_least(row, V, inv_t, m, inv_z, tau, red);
 
   // ---- draw: first kept token, in index order, whose running mass exceeds u * kept

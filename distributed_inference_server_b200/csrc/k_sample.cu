@@ -210,6 +210,7 @@ sample_cluster_kernel(const float *__restrict__ logits, long long ld, int V, con
       tau += (uint32_t)j << sh;
     }
   }
+  tau = max(tau, 1u);  // a weight of zero (a masked logit, an underflow) is never kept: no draw may return it
   // ---- draw: first kept token in index order whose running mass exceeds u * kept
   float local = 0.f;
 #pragma unroll
@@ -270,11 +271,14 @@ sample_cluster_kernel(const float *__restrict__ logits, long long ld, int V, con
           const float n = __shfl_up_sync(0xffffffffu, incl, o);
           if (lane >= o) incl += n;
         }
-        float x2 = at + (incl - mine);
+        // a lane starts at the very number the lane before it ends with: were the two rounded apart, a token at the edge could gain
+        // mass that is not its own
+        const float before = __shfl_up_sync(0xffffffffu, incl, 1);
+        float x2 = lane == 0 ? at : at + before;
         int first = 0x7fffffff, end = -1;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          x2 += kp[j];
+          x2 = j < 3 ? x2 + kp[j] : at + incl;
           if (in[j]) { end = base + k * 128 + j; if (x2 > target && first == 0x7fffffff) first = end; }
         }
         first = __reduce_min_sync(0xffffffffu, first);

@@ -219,7 +219,7 @@ tp_sample_kernel(TpSampPeers sp, const float *__restrict__ logits, long long ld,
     }
     round++;
   } while (cut && hi - lo > 1u && round <= kSearchRounds);
-  const uint32_t tau = lo;
+  const uint32_t tau = max(lo, 1u);  // a weight of zero is never kept: the draw's last-token fallback may not return it
 
   // ---- which rank's slice holds the draw
   float kept = 0.f;
