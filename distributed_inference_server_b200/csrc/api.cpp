@@ -261,7 +261,10 @@ int dis_k_attn_prefill(const uint16_t *q, const uint16_t *kv_pool, int64_t n_pag
   dis::TmaMap map;
   cudaError_t e = dis::make_kv_map(&map, kv_pool, (long long)n_pages * 2 * n_kv * page_size, d, page_size);
   if (e != cudaSuccess) return k_ret(e);
-  auto fn = dis::attn_prefill_uses_tc(n_heads, n_kv, d) ? dis::launch_attn_prefill_tc : dis::launch_attn_prefill;
+  // Heads of 64 off a 16-byte boundary: the mma.sync kernel moves q and out in words of 4 bytes and takes the 16-token blocks that this
+  // entry point promises for them.  (Blocks of heads of 128 are longer: those are refused.)
+  const bool tc = dis::attn_prefill_uses_tc(n_heads, n_kv, d) && (d != 64 || dis::attn_prefill_tc_aligned(q, out));
+  auto fn = tc ? dis::launch_attn_prefill_tc : dis::launch_attn_prefill;
   return k_ret(fn(map, 0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_blocks, n_heads, n_kv, d, page_size,
                   (cudaStream_t)stream));
 }

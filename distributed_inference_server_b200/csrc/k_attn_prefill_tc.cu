@@ -418,6 +418,11 @@ bool attn_prefill_uses_tc(int n_heads, int n_kv, int d) {
   return prefill_tc_enabled() && (d == 128 || d == 64) && (G == 4 || G == 8);
 }
 
+// q is read and out written 16 bytes at a time; rows of 64 or 128 bf16 keep the alignment of the first.
+bool attn_prefill_tc_aligned(const uint16_t *q, const uint16_t *out) {
+  return ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
+}
+
 // Most tokens a caller of the C ABI may put into one query block: 128 / G for heads of 128, 16 otherwise.
 int attn_prefill_block_tokens(int n_heads, int n_kv, int d) {
   return d == 128 && attn_prefill_uses_tc(n_heads, n_kv, d) ? 128 / (n_heads / n_kv) : 16;
@@ -448,6 +453,7 @@ cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const u
                                    int page_size, cudaStream_t st) {
   if (n_blocks <= 0) return cudaSuccess;
   if (n_kv <= 0 || n_heads % n_kv != 0 || n_kv > 65535) { set_last_error("attn_prefill_tc: bad head geometry"); return cudaErrorInvalidValue; }
+  if (!attn_prefill_tc_aligned(q, out)) { set_last_error("attn_prefill_tc: q and out must start on 16 bytes"); return cudaErrorInvalidValue; }
   if (page_size < 8 || (page_size & (page_size - 1))) { set_last_error("attn_prefill_tc: page_size must be a power of two >= 8"); return cudaErrorInvalidValue; }
   int page_shift = 0;
   while ((1 << page_shift) < page_size) page_shift++;

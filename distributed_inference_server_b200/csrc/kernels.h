@@ -100,6 +100,7 @@ cudaError_t launch_attn_prefill(const TmaMap &kv_map, long long row0, const uint
 // k_attn_prefill_tc.cu : the same contract on tcgen05 / TMEM for heads of 128 or 64 and GQA groups of 4 or 8; the kernels take query
 // blocks of attn_prefill_full_block() tokens (128 / G), the C ABI promises attn_prefill_block_tokens()
 bool attn_prefill_uses_tc(int n_heads, int n_kv, int d);
+bool attn_prefill_tc_aligned(const uint16_t *q, const uint16_t *out);
 int attn_prefill_block_tokens(int n_heads, int n_kv, int d);
 int attn_prefill_full_block(int n_heads, int n_kv, int d);
 cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,

@@ -386,7 +386,9 @@ DIS_API int dis_k_attn_paged_static(const uint16_t *q, const uint16_t *kv_pool, 
  * The block's own K/V must already be in the pages.  q / out are [tokens][nh*d] bf16.
  * qb_len[b] <= dis_k_attn_prefill_block_tokens(n_heads, n_kv, d): 128 / (n_heads / n_kv) for heads of 128 with 4 or 8 query
  * heads per kv head (the tcgen05 / TMEM kernel of k_attn_prefill_tc.cu: S = Q K^T and P V over 128 query rows), else 16 (heads of 64
- * with such groups run on the same kernel, other groups on the mma.sync kernel). */
+ * with such groups run on the same kernel, other groups on the mma.sync kernel).
+ * q and out start on 4 bytes; on 16 bytes for heads of 128 with 4 or 8 query heads per kv head, else the call is refused.  (Heads of 64
+ * with such groups off a 16-byte boundary run on the mma.sync kernel.) */
 DIS_API int dis_k_attn_prefill_block_tokens(int32_t n_heads, int32_t n_kv, int32_t d);
 DIS_API int dis_k_attn_prefill(const uint16_t *q, const uint16_t *kv_pool, int64_t n_pages, const int32_t *page_table,
                                int32_t max_pages, const int32_t *qb_tok0, const int32_t *qb_len,

@@ -415,6 +415,42 @@ def test_attention_prefill_heads_of_64(nh, nkv, page_size, past):
         row += n
 
 
+def _prefill_call(nh, nkv, d, off_q, off_out, n=50, ps=64):
+    """One prompt of n tokens, q and out starting off_* bf16 elements behind a 16-byte boundary -> (return code, q, pool, out)."""
+    g = torch.Generator(device=DEV); g.manual_seed(nh)
+    BT = lib().dis_k_attn_prefill_block_tokens(nh, nkv, d)
+    pool = torch.randn((1, 2, nkv, ps, d), device=DEV, generator=g).to(torch.bfloat16)
+    q = torch.randn(n * nh * d + 8, device=DEV, generator=g).to(torch.bfloat16)[off_q:][:n * nh * d]
+    out = G.zeros(n * nh * d + 8, dtype=torch.bfloat16, device=DEV)[off_out:][:n * nh * d]
+    t0 = list(range(0, n, BT))
+    ln = [min(BT, n - t) for t in t0]
+    rc = lib().dis_k_attn_prefill(ptr(q), ptr(pool), 1, ptr(dev_i32([[0]])), 1, ptr(dev_i32(t0)), ptr(dev_i32(ln)), ptr(dev_i32(t0)),
+                                  ptr(dev_i32([0] * len(t0))), ptr(out), len(t0), nh, nkv, d, ps, None)
+    sync()
+    return rc, q.view(n, nh * d), pool, out.view(n, nh * d)
+
+
+@pytest.mark.parametrize("off_q,off_out", [(2, 0), (0, 2), (6, 4), (0, 0)])
+@pytest.mark.parametrize("nh,nkv", [(8, 1), (8, 2)])
+def test_attention_prefill_heads_of_64_off_a_16_byte_boundary(nh, nkv, off_q, off_out):
+    """q or out on 4 or 8 bytes only: against float64, as test_attention_prefill_heads_of_64."""
+    rc, q, pool, out = _prefill_call(nh, nkv, 64, off_q, off_out)
+    check(rc)
+    n, kv = q.shape[0], pool[0].double()
+    K, V = kv[0][:, :n], kv[1][:, :n]
+    sc = q.double().reshape(n, nkv, nh // nkv, 64).permute(1, 2, 0, 3) @ K.transpose(1, 2).unsqueeze(1) / 8.0
+    sc = sc.masked_fill(torch.ones(n, n, device=DEV).triu(1).bool(), float("-inf"))
+    ref = (torch.softmax(sc, dim=-1) @ V.unsqueeze(1)).permute(2, 0, 1, 3).reshape(n, nh * 64)
+    assert (out.double() - ref).abs().max().item() <= 2 * BF16_ULP * V.abs().max().item() + 1e-5
+
+
+@pytest.mark.parametrize("off_q,off_out", [(2, 0), (0, 4)])
+def test_attention_prefill_heads_of_128_off_a_16_byte_boundary_are_refused(off_q, off_out):
+    rc, _, _, out = _prefill_call(8, 2, 128, off_q, off_out)
+    assert rc != 0 and b"16 bytes" in lib().dis_last_error()
+    assert not out.any()
+
+
 @pytest.mark.parametrize("nh,nkv", [(32, 4), (16, 4)])
 def test_attention_prefill_heads_of_64_rounds_no_more_than_a_running_maximum(nh, nkv):
     """The 2-norm error against float64 is no larger than that of softmax weights rounded to bf16 under the row's own maximum (whose
