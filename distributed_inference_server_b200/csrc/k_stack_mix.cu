@@ -493,11 +493,14 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
     }
   }
   __syncthreads();  // D is complete and the keys are no longer needed
+  // Above the diagonal nothing is multiplied, here and with the values below: zero times a key or value that is not finite would carry a
+  // later token into an earlier one's output.
 #pragma unroll
   for (int j = 0; j < 4; j++) {
     float4 *p = reinterpret_cast<float4 *>(at + (tj + j) * kLbLd + i0);
     const float4 f = *p;
-    *p = make_float4(f.x * a[0][j], f.y * a[1][j], f.z * a[2][j], f.w * a[3][j]);
+    const int rest = tj + j - i0;  // rows below this one of the four see nothing of token tj + j
+    *p = make_float4(rest > 0 ? 0.f : f.x * a[0][j], rest > 1 ? 0.f : f.y * a[1][j], rest > 2 ? 0.f : f.z * a[2][j], rest > 3 ? 0.f : f.w * a[3][j]);
   }
   for (int e = tid; e < g.n * dv4; e += 256) {
     const int t = e / dv4, c = (e - t * dv4) * 4;
@@ -533,9 +536,7 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
     for (int j = 0; j < RJ; j++) acc[i][j] *= f;
   }
   __syncthreads();
-  const int last = min(i0 + 4, g.n);
-#pragma unroll 2
-  for (int t = 0; t < last; t++) {
+  auto add_token = [&](int t, int first) {  // rows first .. 3 see token t
     const float4 w = *reinterpret_cast<const float4 *>(at + t * kLbLd + i0);
     const float wv[4] = {w.x, w.y, w.z, w.w};
     float v[RJ];
@@ -543,9 +544,16 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
     for (int j = 0; j < RJ; j += 4) *reinterpret_cast<float4 *>(v + j) = *reinterpret_cast<const float4 *>(kv + t * DVT + tj + j * 16);
 #pragma unroll
     for (int i = 0; i < 4; i++)
+      if (i >= first)
 #pragma unroll
-      for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(wv[i], v[j], acc[i][j]);
-  }
+        for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(wv[i], v[j], acc[i][j]);
+  };
+  const int below = min(i0 + 1, g.n);
+#pragma unroll 2
+  for (int t = 0; t < below; t++) add_token(t, 0);
+#pragma unroll
+  for (int u = 1; u < 4; u++)
+    if (i0 + u < g.n) add_token(i0 + u, u);
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     if (i0 + i >= g.n) continue;

@@ -257,6 +257,32 @@ def test_segments_in_block_form(monkeypatch, state, vdim, heads, groups):
     e.close()
 
 
+@pytest.mark.parametrize("state,vdim", [(32, 32), (128, 64)])
+@pytest.mark.parametrize("at", [64, 89, 90, 91, 129])
+def test_a_token_that_is_not_finite_leaves_earlier_outputs_alone(monkeypatch, state, vdim, at):
+    """State-space spans in block form with one token whose keys and values are not finite, at every place of a group of four rows and at the
+    start of a segment: the logits of every token in front of it are the oracle's."""
+    monkeypatch.setenv("DIS_STACK_LIGHT_SEGMENTS", "2")
+    cfg = U.config([(U.ssm(heads=4, vdim=vdim, state=state, groups=2, conv=3, norm_groups=2), None)], width=40, streams=0)
+    W = U.weights(cfg, seed=state)
+    t = toks(150, seed=at)
+    bad = int(W["embed"].shape[0]) - 1
+    t = [x if x != bad else 0 for x in t]
+    t[at] = bad
+    want = U.oracle_logits(cfg, W, t[:at])
+    W["embed"][bad] = np.inf
+    e = U.engine(cfg, W, pool_tokens=208, page_size=16, max_batch=1, max_step_tokens=256)
+    slot = e.seq_add(t, InferenceParams(max_tokens=1 << 30, temperature=0.0))
+    e.seq_probe(slot, list(range(len(t))))
+    e.step([slot])
+    cols = np.arange(W["embed"].shape[0]) != bad  # (a head that shares the embedding reads that row as well)
+    got = e.last_logits(e.last_logit_rows())[:len(t), cols]
+    e.seq_remove(slot)
+    assert np.isfinite(got[:at]).all() and not np.isfinite(got[at:]).any()
+    assert U.rel_err(got[:at], want[:, cols]) < 5e-5
+    e.close()
+
+
 def test_large_passes_take_the_tensor_core_expert_products(monkeypatch):
     """A pass of 1280 prompt tokens in bfloat16: per-expert tensor-core products over rows sorted by expert and the shared unit
     on the tensor cores.  Against the oracle, and against the same pass on the tiled fp32-FMA products (DIS_STACK_TC=0), which
