@@ -565,9 +565,9 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
 }
 
 // The block form reads rows as float4: heads, offsets and strides in fours, rows that start on 16 bytes.
-static bool light_block_ok(const float *proj, long long ld, const LightCols &col, const float *o, const float *seg, int d, int dv) {
+bool stack_lightning_block(const float *proj, long long ld, int q, int k, int v, const float *o, const float *seg, int d, int dv) {
   auto al = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-  return stack_lightning_block(d, dv) && ld % 4 == 0 && col.q % 4 == 0 && col.k % 4 == 0 && col.v % 4 == 0 && al(proj) && al(o) && al(seg);
+  return d <= 128 && dv <= 128 && d % 4 == 0 && dv % 4 == 0 && ld % 4 == 0 && q % 4 == 0 && k % 4 == 0 && v % 4 == 0 && al(proj) && al(o) && al(seg);
 }
 template <int DT, int DVT, int GATE>
 static cudaError_t light_block(const float *proj, long long ld, const LightCols &col, const float *decay, const float *dec, float qscale, float *state,
@@ -587,11 +587,11 @@ static cudaError_t light_block(const float *proj, long long ld, const LightCols 
 }
 
 int stack_lightning_seg_tokens() { return kLightSeg; }
-bool stack_lightning_block(int d, int dv) { return d <= 128 && dv <= 128 && d % 4 == 0 && dv % 4 == 0; }
 // Whether a pass should cut its long spans into segments.  Walking a span in one piece costs its length times three
 // operations per state element, once per wave of (span, head) CTAs (two fit an SM); the segments cost five operations per
 // element (contributions, then outputs) over all segment CTAs in waves, plus the carry.  Many sequences with many heads fill
-// the GPU without segments and then pay less; a single long prompt needs them.  block: the segments run in block form, whose
+// the GPU without segments and then pay less; a single long prompt needs them.  block: the segments run in block form (what
+// stack_lightning_block says of the very pointers and strides of the launch), whose
 // contributions and outputs together take about what two operations per element take here (a state-space pass of 256 (sequence, head)
 // pairs, 8 x 1024 tokens, 32 heads of 128 x 64 in four layers: 5.1 ms cut, 5.6 whole).
 bool stack_lightning_segmented(int n_spans, int T, int H, int max_len, bool block) {
@@ -634,7 +634,7 @@ static cudaError_t lightning_reg(const float *proj, long long ld, LightCols col,
     return cudaGetLastError();
   }
   if constexpr (GATE != 1) {
-    if (light_block_ok(proj, ld, col, o, seg, d, dv)) {
+    if (stack_lightning_block(proj, ld, col.q, col.k, col.v, o, seg, d, dv)) {
       auto f = d <= 64 ? (dv <= 64 ? light_block<64, 64, GATE> : light_block<64, 128, GATE>) : (dv <= 64 ? light_block<128, 64, GATE> : light_block<128, 128, GATE>);
       return f(proj, ld, col, decay, dec, qscale, state, sp, o, H, d, dv, seg, seg_a, max_len, st);
     }

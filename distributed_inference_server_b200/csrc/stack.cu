@@ -1692,7 +1692,8 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
       const int H = lc.heads, d = lc.dim, dv = lc.vdim;
       int max_len = 0;
       for (auto &sh : stack_spans_h) max_len = std::max(max_len, sh.len);
-      const bool segments = M.light_seg && stack_lightning_segmented(sp.n_spans, T, H, max_len, stack_lightning_block(d, dv)) && d <= 128 && dv <= 128;
+      const bool segments = M.light_seg && d <= 128 && dv <= 128 &&
+                            stack_lightning_segmented(sp.n_spans, T, H, max_len, stack_lightning_block(M.proj, N, 0, H * d, 2 * H * d, M.mix, M.light_seg, d, dv));
       RET_CUDA(launch_stack_lightning(M.proj, N, reinterpret_cast<const float *>(L.decay_d.ptr), Rn.state, sp, M.mix, H, d, dv,
                                       segments ? M.light_seg : nullptr, max_len, stream));
       if (segments) kl += 2;
@@ -1703,7 +1704,9 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
       const int H = lc.heads, d = lc.dim, dv = lc.vdim, nb = stack_retention_blocks(d, dv);
       RET_CUDA(launch_stack_retention_prep(in_src, N, in_parts, in_stride, L.n_in, M.proj, N, 0, L.k_off, H, d, L.freq, lc.rot_dims,
                                            1.f / std::sqrt((float)d), sp, stream));
-      const bool segments = M.light_seg && d <= 128 && stack_lightning_segmented(sp.n_spans, T, H * nb, max_span, stack_lightning_block(d, dv / nb));
+      const bool segments = M.light_seg && d <= 128 &&
+                            stack_lightning_segmented(sp.n_spans, T, H * nb, max_span,
+                                                      stack_lightning_block(M.proj, N, 0, L.k_off, L.v_off, M.mix, M.light_seg, d, dv / nb));
       RET_CUDA(launch_stack_retention(M.proj, N, 0, L.k_off, L.v_off, reinterpret_cast<const float *>(L.decay_d.ptr), Rn.state, sp, M.mix, H, d, dv,
                                       segments ? M.light_seg : nullptr, max_span, M.proj + L.g_off, N, M.act, L.ld_act, f32, eps, stream));
       kl += segments ? 5 : nb > 1 || d > 128 || dv > 128 ? 3 : 2;
@@ -1739,7 +1742,9 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
       RET_CUDA(launch_stack_ssm_conv(M.proj, N, L.x_off, L.dt_off, C, H, lc.conv_taps, reinterpret_cast<const float *>(L.conv_w.ptr),
                                      reinterpret_cast<const float *>(L.conv_b.ptr), vec, Rn.conv_state, sp, M.ssm, ld_b, M.dec, dtv, stream));
       kl += lc.conv_taps > 1 && T != sp.n_spans ? 2 : 1;
-      const bool segments = M.light_seg && M.light_seg_a && stack_lightning_segmented(sp.n_spans, T, H, max_span, stack_lightning_block(Ns, P)) && Ns <= 128 && P <= 128;
+      const bool segments = M.light_seg && M.light_seg_a && Ns <= 128 && P <= 128 &&
+                            stack_lightning_segmented(sp.n_spans, T, H, max_span,
+                                                      stack_lightning_block(M.ssm, ld_b, inner + G * Ns, inner, 0, M.mix, M.light_seg, Ns, P));
       RET_CUDA(launch_stack_ssd(M.ssm, ld_b, inner + G * Ns, inner, 0, H / G, M.dec, dtv, Rn.state, sp, M.mix, H, Ns, P, segments ? M.light_seg : nullptr,
                                 segments ? M.light_seg_a : nullptr, max_span, stream));
       kl += segments ? 3 : 1;

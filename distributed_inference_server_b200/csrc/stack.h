@@ -93,7 +93,8 @@ size_t stack_lightning_seg_floats(int cap_tokens, int max_spans, int H, int d, i
 int stack_lightning_seg_tokens();
 // whether a pass of n_spans spans (T tokens, the longest max_len) over H heads is faster cut into segments than span by span
 bool stack_lightning_segmented(int n_spans, int T, int H, int max_len, bool block);
-bool stack_lightning_block(int d, int dv);  // whether segments of such heads run in block form (one decay per token and head)
+// whether segments run in block form (one decay per token and head): q, k, v the columns of the first head in proj
+bool stack_lightning_block(const float *proj, long long ld, int q, int k, int v, const float *o, const float *seg, int d, int dv);
 cudaError_t launch_stack_lightning(const float *proj, long long ld, const float *decay, float *state, const StackSpans &sp,
                                    float *o, int H, int d, int dv, float *seg, int max_len, cudaStream_t st);
 // Gated linear attention (per-channel decay): S = diag(a_t) S + k_t v_t^T, o_t = S^T (q_t / sqrt(d)).

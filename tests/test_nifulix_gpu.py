@@ -669,3 +669,25 @@ def test_random_configurations_and_schedules(seed, dtype):
             assert U.rel_err(got[k], want[k]) < 5e-5, (seed, k)
         else:
             assert U.row_errs(got[k], want[k]).max() < 6e-2, (seed, k)
+
+
+@pytest.mark.parametrize("ff,cut", [(33, False), (34, True)])
+def test_spans_are_cut_at_the_cost_of_the_kernel_that_walks_them(monkeypatch, ff, cut):
+    """Two prompts of 256 tokens over 128 heads: in block form (rows of the fused projection in fours: an even ff) cutting them into
+    segments costs less than walking them whole, with the register kernel (an odd ff) it costs more.  Three more launches show a cut;
+    DIS_STACK_LIGHT_SEGMENTS=0 never cuts.  Both against the oracle."""
+    cfg = U.config([(U.retention(heads=128, dim=4, vdim=4, rot=4, decay=[0.5 + 0.4 * h / 128 for h in range(128)]), U.dense(ff))])
+    W = U.weights(cfg, seed=ff)
+    seqs = {k: [int(x) for x in np.random.default_rng(ff + k).integers(0, 50, 256)] for k in range(2)}
+    counts = []
+    for force in ("0", "1"):
+        monkeypatch.setenv("DIS_STACK_LIGHT_SEGMENTS", force)
+        e = U.engine(cfg, W, pool_tokens=544, page_size=16, max_batch=2, max_step_tokens=512)
+        f = U.Feeder(e)
+        before = e.status().kernel_launches
+        f.step([(k, seqs[k], 256) for k in seqs])
+        counts.append(e.status().kernel_launches - before)
+        for k in seqs:
+            assert U.rel_err(f.end(k), U.oracle_logits(cfg, W, seqs[k])) < 1e-4
+        e.close()
+    assert counts[1] - counts[0] == (3 if cut else 0), counts
