@@ -779,7 +779,7 @@ cudaError_t Engine::enqueue_head(int R, bool all_greedy) {
   float *d_logprob = reinterpret_cast<float *>(d_out_tokens + max_batch);  // TokenEvent.logprob, models.rs:276
   if (tp_size == 1) {
     kernel_launches++;
-    return launch_sample(logits, vocab_l, R, vocab_l, temp, topp, seed, step, d_out_tokens, 0, nullptr, nullptr, d_logprob, stream);
+    return launch_sample_rows(logits, vocab_l, R, all_greedy, temp, topp, seed, step, d_out_tokens, d_logprob, stream);
   }
   if (all_greedy && tp_custom) {
     // vocab-parallel argmax: local (value, id, sum-exp), exchanged and merged over peer memory in one kernel

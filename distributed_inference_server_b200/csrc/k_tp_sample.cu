@@ -328,4 +328,17 @@ cudaError_t launch_tp_sample(const TpSampPeers &sp, const float *logits, long lo
                   seeds, steps, step_ptr, step_imm, out_tokens, out_logprob);
 }
 
+// The rows of an engine on one GPU.  A row that a cluster's registers hold goes to k_sample.cu; of longer ones the greedy go to
+// sample_kernel (two walks over the row) and the sampled come here as a single rank: 8 walks over the row where sample_kernel's
+// bisection takes 31.
+cudaError_t launch_sample_rows(const float *logits, int V, int T, bool all_greedy, const float *temperature, const float *top_p,
+                               const unsigned long long *seeds, const unsigned long long *steps, uint32_t *out_tokens, float *out_logprob,
+                               cudaStream_t st) {
+  if (all_greedy || V <= kSampleClusterMaxV)
+    return launch_sample(logits, V, T, V, temperature, top_p, seeds, steps, out_tokens, 0, nullptr, nullptr, out_logprob, st);
+  TpSampPeers solo{};
+  solo.rank = 0; solo.tp = 1; solo.cap_rows = T;
+  return launch_tp_sample(solo, logits, V, T, V, temperature, top_p, seeds, steps, nullptr, 0, out_tokens, out_logprob, st);
+}
+
 }  // namespace dis

@@ -71,6 +71,9 @@ cudaError_t launch_tp_sample(const TpSampPeers &sp, const float *logits, long lo
                              const float *temperature, const float *top_p, const unsigned long long *seeds,
                              const unsigned long long *steps, const uint32_t *step_ptr, uint32_t step_imm,
                              uint32_t *out_tokens, float *out_logprob, cudaStream_t st);
+cudaError_t launch_sample_rows(const float *logits, int V, int T, bool all_greedy, const float *temperature, const float *top_p,
+                               const unsigned long long *seeds, const unsigned long long *steps, uint32_t *out_tokens, float *out_logprob,
+                               cudaStream_t st);
 
 // k_gemv.cu : out[t][n] = sum_k X[t][k] W[n][k]  (T <= kGemvMaxT per launch; launcher loops)
 constexpr int kGemvMaxT = 4;

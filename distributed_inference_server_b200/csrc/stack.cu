@@ -2011,7 +2011,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   const unsigned long long *seed = mt.d<unsigned long long>(mt.o_seed), *step = mt.d<unsigned long long>(mt.o_step);
   float *d_logprob = reinterpret_cast<float *>(M.d_out + M.max_rows);
   kl++;
-  return launch_sample(M.logits, M.c.vocab, R, M.c.vocab, temp, topp, seed, step, M.d_out, 0, nullptr, nullptr, d_logprob, stream);
+  return launch_sample_rows(M.logits, M.c.vocab, R, all_greedy, temp, topp, seed, step, M.d_out, d_logprob, stream);
 }
 
 }  // namespace dis

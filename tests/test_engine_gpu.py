@@ -429,3 +429,40 @@ def test_decode_batch_padded_to_graph_bucket_changes_nothing():
     mimic = O.Oracle(shape, act_round=True); mimic.fill_synthetic(77, True)
     got = [[step[b] for step in outs[0][0][:7]] for b in range(13)]
     assert_greedy_matches(got, mimic, prompts, 7, "bucket-padded")
+
+
+def test_sampled_rows_of_a_vocabulary_longer_than_the_cluster_sampler_takes():
+    """262208 logits (k_sample.cu holds 262144): the engine draws what the oracle draws from its logits, and a whole decode step takes
+    less time than the bisecting kernel alone takes for the row."""
+    import torch
+    V = 262208
+    shape = O.ModelShape(V, 64, 1, 4, 1, 64, 64, 128, 10000.0, 1e-5)
+    e = make_engine(shape, seed=3, max_batch=1, kv_pages=16)
+    slot = e.seq_add([3, 1, 4], InferenceParams(max_tokens=64, temperature=0.8, top_p=0.9, seed=77))
+    toks, _ = e.prefill([slot])
+    ms = []
+    for i in range(12):
+        z = e.last_logits(1)[0].astype(np.float64) / 0.8
+        want, tau, _ = O.sample(e.last_logits(1)[0], 0.8, 0.9, 77, i)
+        p = np.exp(z - z.max())
+        p /= p.sum()
+        got = int(toks[0])
+        assert p[got] >= tau * (1 - 1e-5)
+        between = p[min(got, want):max(got, want)]  # flat rows: fp32 sums of 262208 terms may land a few tokens away
+        assert between[between >= tau].sum() <= 1e-4, (i, got, want)
+        toks, _ = e.decode([slot])
+        ms.append(e.status().last_step_ms)
+    e.close()
+    lg = torch.randn(1, V, device="cuda")
+    t, p = torch.full((1,), 0.8, device="cuda"), torch.full((1,), 0.9, device="cuda")
+    s, n, out = (torch.zeros(1, dtype=d, device="cuda") for d in (torch.int64, torch.int64, torch.int32))
+    lib, alone = B.load(), []
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        rc = lib.dis_k_sample(*(x.data_ptr() if hasattr(x, "data_ptr") else x for x in (lg, V, 1, V, t, p, s, n, out)), None,
+                              torch.cuda.current_stream().cuda_stream)
+        b.record(); b.synchronize()
+        assert rc == B.OK
+        alone.append(a.elapsed_time(b))
+    assert min(ms) < min(alone), (min(ms), min(alone))
