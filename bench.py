@@ -292,7 +292,7 @@ def workload_config(n_gpus, batch, prompt_len, model="8b"):
 
 def roofline_traffic(kernel_key):
     """dram__bytes_read.sum + dram__bytes_write.sum per launch of the dominant kernel, from the committed summary of the
-    ncu --set full capture (profiles/roofline_traffic.json, written by scripts/summarize_profile.py) -- a profiler is
+    ncu --set full capture (profiles/roofline_traffic.json) -- a profiler is
     never run inside the bench.  None when there is no capture for this kernel/shape."""
     p = os.path.join(ROOT, "profiles", "roofline_traffic.json")
     try:
