@@ -370,16 +370,17 @@ def test_attention_prefill_blocks(d, nh, nkv, page_size, short_blocks):
     assert np.abs(got - ref).max() <= 2 * BF16_ULP * np.abs(ref).max() + 1e-5, np.abs(got - ref).max()
 
 
-@pytest.mark.parametrize("nh,nkv,page_size", [(8, 1, 8), (8, 2, 64), (16, 2, 128)])
+@pytest.mark.parametrize("nh,nkv,page_size,BT", [(8, 1, 8, 16), (8, 2, 64, 16), (8, 2, 64, 32), (16, 2, 128, 16), (16, 4, 16, 32)])
 @pytest.mark.parametrize("past", [0, 63, 200])
-def test_attention_prefill_heads_of_64(nh, nkv, page_size, past):
+def test_attention_prefill_heads_of_64(nh, nkv, page_size, past, BT):
     """The tcgen05 kernel for heads of 64 at the edges of its 64-key tiles: one tile (only one of its two softmax groups works), 64 and 65
     keys, an odd number of tiles, portions behind keys already in the cache, and scores that grow along the keys so that the
-    softmax reference has to be raised after the first tile.  Against float64; two bf16 roundings (weights, result) of values up to
+    softmax reference has to be raised after the first tile.  Blocks of 16 tokens, as the C ABI promises, and of 32 for groups of 4, as
+    the engine makes them (all 128 query rows), full and ragged.  Against float64; two bf16 roundings (weights, result) of values up to
     the largest |v|."""
     g = torch.Generator(device=DEV); g.manual_seed(past + nh + page_size)
-    d, lens = 64, [1, 16, 64, 65, 129, 330]
-    BT = lib().dis_k_attn_prefill_block_tokens(nh, nkv, d)
+    d, lens = 64, [1, 16, 17, 31, 32, 33, 64, 65, 129, 330]
+    assert lib().dis_k_attn_prefill_block_tokens(nh, nkv, d) == 16
     total = [past + n for n in lens]
     per = [(n + page_size - 1) // page_size for n in total]
     n_pages = sum(per)
