@@ -204,6 +204,8 @@ int dis_k_add_rmsnorm(float *x, const uint32_t *tokens, const uint16_t *embed, c
 static int gemm_common(const uint16_t *X, const uint16_t *W, float *out, uint16_t *act, int T, int N, int K, int split,
                        bool silu, cudaStream_t st) {
   if (int rc = need_gpu()) return rc;
+  // A slice count below 1 has always meant one slice where the tiles of 128 x 256 fill the GPU twice, and is refused elsewhere.
+  if (split < 1 && T >= 512 && (long long)((N + 127) / 128) * ((T + 255) / 256) >= 2 * dis::kNumSMs) split = 1;
   dis::TmaMap wm, xm;
   const bool persist = dis::gemm_use_persist(T, N, split, silu);  // the engine's choice for this shape
   const int bn = persist ? 128 : dis::gemm_token_tile(T);

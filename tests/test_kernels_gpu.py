@@ -370,6 +370,23 @@ def test_attention_prefill_blocks(d, nh, nkv, page_size, short_blocks):
     assert np.abs(got - ref).max() <= 2 * BF16_ULP * np.abs(ref).max() + 1e-5, np.abs(got - ref).max()
 
 
+@pytest.mark.parametrize("T,N,ok", [(1024, 9472, True), (600, 12672, True), (1024, 9344, False), (500, 18944, False), (32, 256, False)])
+def test_gemm_slice_count_of_zero(T, N, ok):
+    """Zero slices: the plain product where 128 x 256 tiles fill the GPU twice from 512 tokens on, an error elsewhere, as ever."""
+    g = torch.Generator(device=DEV); g.manual_seed(T)
+    X, W = (torch.randn(s, device=DEV, generator=g).to(torch.bfloat16) for s in ((T, 64), (N, 64)))
+    a, b = (G.zeros((T, N)) for _ in range(2))
+    rc = lib().dis_k_gemm(ptr(X), ptr(W), ptr(a), T, N, 64, 0, None)
+    sync()
+    assert (rc == 0) == ok
+    if ok:
+        check(lib().dis_k_gemm(ptr(X), ptr(W), ptr(b), T, N, 64, 1, None))
+        sync()
+        assert torch.equal(a, b)
+    else:
+        assert not a.any()
+
+
 @pytest.mark.parametrize("nh,nkv,page_size,BT", [(8, 1, 8, 16), (8, 2, 64, 16), (8, 2, 64, 32), (16, 2, 128, 16), (16, 4, 16, 32)])
 @pytest.mark.parametrize("past", [0, 63, 200])
 def test_attention_prefill_heads_of_64(nh, nkv, page_size, past, BT):
