@@ -567,7 +567,11 @@ int Engine::seq_remove(int slot) {
   return DIS_OK;
 }
 
-void Engine::finish_check(Sequence &s, uint32_t tok) {
+// Takes a row's sampled token into the sequence; returns it, or 0 where there is none.
+uint32_t Engine::finish_check(Sequence &s, uint32_t tok) {
+  // A row of logits without a number in it (NaN or -inf throughout) has no token: the sampler writes one past every vocabulary, which as
+  // the next pass's input would be read outside of the embedding.  The sequence fails alone.
+  if (tok >= (uint32_t)m.vocab) { s.finish = DIS_FINISH_FAILED; return 0; }
   s.generated++;
   tokens_generated++;
   s.last_token = tok;
@@ -577,11 +581,12 @@ void Engine::finish_check(Sequence &s, uint32_t tok) {
   for (auto &st : s.stop) longest = std::max(longest, st.size());
   if (s.tail.size() > longest && longest > 0) s.tail.erase(s.tail.begin(), s.tail.end() - (long)longest);
   if (longest == 0) s.tail.clear();
-  if (cfg.eos_token >= 0 && tok == (uint32_t)cfg.eos_token) { s.finish = DIS_FINISH_STOP; return; }
+  if (cfg.eos_token >= 0 && tok == (uint32_t)cfg.eos_token) { s.finish = DIS_FINISH_STOP; return tok; }
   for (auto &st : s.stop)
-    if (st.size() <= s.tail.size() && std::equal(st.begin(), st.end(), s.tail.end() - (long)st.size())) { s.finish = DIS_FINISH_STOP_SEQUENCE; return; }
-  if (s.generated >= s.max_tokens) { s.finish = DIS_FINISH_LENGTH; return; }
-  if (s.len + 1 >= m.max_ctx) { s.finish = DIS_FINISH_LENGTH; return; }
+    if (st.size() <= s.tail.size() && std::equal(st.begin(), st.end(), s.tail.end() - (long)st.size())) { s.finish = DIS_FINISH_STOP_SEQUENCE; return tok; }
+  if (s.generated >= s.max_tokens) { s.finish = DIS_FINISH_LENGTH; return tok; }
+  if (s.len + 1 >= m.max_ctx) { s.finish = DIS_FINISH_LENGTH; return tok; }
+  return tok;
 }
 
 // ------------------------------------------------------------------------------------ step plumbing
@@ -938,7 +943,7 @@ int Engine::prefill(int n, const int *slots, uint32_t *out_tokens, int *out_fini
     s.prefill_pos = s.len;
     s.prefilled = true;
     pages_ix.commit(s.prompt.data(), s.len / page_size, s.pages);  // full prompt pages become reusable (no-op when off)
-    finish_check(s, out_tokens[i]);
+    out_tokens[i] = finish_check(s, out_tokens[i]);
     out_finish[i] = s.finish;
   }
   return DIS_OK;
@@ -1075,11 +1080,10 @@ int Engine::step_mixed(int n, const int *slots, int max_prefill_tokens, uint32_t
       s.prefilled = true;
       pages_ix.commit(s.prompt.data(), s.len / page_size, s.pages);
     }
-    out_tokens[i] = h_out_tokens[r];
+    out_tokens[i] = finish_check(s, h_out_tokens[r]);
     s.last_logprob = reinterpret_cast<const float *>(h_out_tokens + max_batch)[r];
-    finish_check(s, h_out_tokens[r]);
     out_finish[i] = s.finish;
-    out_produced[i] = 1;
+    out_produced[i] = s.finish != DIS_FINISH_FAILED ? 1 : 0;
     r++;
   }
   return DIS_OK;
@@ -1199,9 +1203,8 @@ int Engine::decode(int n, const int *slots, uint32_t *out_tokens, int *out_finis
     const int i = live[(size_t)r];
     Sequence &s = seqs[(size_t)slots[i]];
     s.len += 1;  // the consumed token is now in the cache
-    out_tokens[i] = h_out_tokens[r];
+    out_tokens[i] = finish_check(s, h_out_tokens[r]);
     s.last_logprob = reinterpret_cast<const float *>(h_out_tokens + max_batch)[r];
-    finish_check(s, h_out_tokens[r]);
     out_finish[i] = s.finish;
   }
   return DIS_OK;

@@ -227,7 +227,7 @@ struct Engine {
   cudaError_t allreduce_partials(int split, int T);
   cudaError_t gather_full_logits(int R);
   int pick_attn_splits(int T, int max_ctx_in_batch) const;
-  void finish_check(Sequence &s, uint32_t tok);
+  uint32_t finish_check(Sequence &s, uint32_t tok);
   struct TensorSlot { void *ptr; size_t rows, cols, ld, row0, col0, full_rows, full_cols; bool f32; };
   bool tensor_slot(int kind, int layer, TensorSlot *out);
 };

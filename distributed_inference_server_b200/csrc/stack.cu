@@ -1340,11 +1340,10 @@ int Engine::stack_step(int n, const int *slots, int max_prefill_tokens, uint32_t
     s.probes.resize(keep);
     if (s.len < (int)s.prompt.size()) continue;  // more chunks to come
     s.prefilled = true;
-    out_tokens[i] = M.h_out[r];
+    out_tokens[i] = finish_check(s, M.h_out[r]);
     s.last_logprob = reinterpret_cast<const float *>(M.h_out + M.max_rows)[r];
-    finish_check(s, M.h_out[r]);
     out_finish[i] = s.finish;
-    out_produced[i] = 1;
+    out_produced[i] = s.finish != DIS_FINISH_FAILED ? 1 : 0;
     r++;
   }
   return DIS_OK;

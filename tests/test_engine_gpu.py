@@ -466,3 +466,29 @@ def test_sampled_rows_of_a_vocabulary_longer_than_the_cluster_sampler_takes():
         assert rc == B.OK
         alone.append(a.elapsed_time(b))
     assert min(ms) < min(alone), (min(ms), min(alone))
+
+
+def test_a_row_of_logits_without_a_number_fails_its_sequence_alone():
+    """A token whose embedding is infinite leaves NaN logits: its sequence ends as failed without a token and takes part in no later pass,
+    greedy or sampled; the one beside it goes on as if alone."""
+    shape = O.ModelShape(512, 64, 1, 4, 1, 64, 64, 128, 10000.0, 1e-5)
+    oracle = O.Oracle(shape); oracle.fill_synthetic(8, True)
+    e = Engine(WorkerConfig(to_engine_shape(shape), max_batch=3, kv_pages=24, page_size=16, max_step_tokens=64))
+    for n, (kind, layer, arr) in enumerate(oracle.tensors()):
+        arr = np.array(arr)
+        if n == 0:
+            assert arr.size == 512 * 64
+            arr.reshape(512, 64)[7] = np.inf
+        e.load_tensor(kind, layer, arr)
+    e.finalize()
+    P = InferenceParams(max_tokens=16, temperature=0.0)
+    alone = greedy(e, [[1, 2, 3]], 6)[0][0]
+    if 7 in alone[:5]:
+        pytest.skip("the healthy sequence draws the broken token itself")
+    slots = [e.seq_add([5, 7], P), e.seq_add([1, 2, 3], P), e.seq_add([5, 7], InferenceParams(max_tokens=16, temperature=0.9, top_p=0.9, seed=3))]
+    toks, fin = e.prefill(slots)
+    assert [int(f) == B.FINISH_FAILED for f in fin] == [True, False, True] and [int(t) for t in toks] == [0, alone[0], 0]
+    for i in range(1, 6):
+        toks, fin = e.decode(slots)
+        assert [int(f) == B.FINISH_FAILED for f in fin] == [True, False, True] and int(toks[1]) == alone[i]
+    e.close()
