@@ -15,7 +15,7 @@ steps; `e2e` is the same loop on the host clock through the C-ABI decode call, w
 Other lines (diagnostics and the remaining BASELINE configs, never the default):
   --batch 1 / --model 70b            configs[1] batch 1, configs[3] Llama-3-70B TP = 8 batch 32
   --workload serving                 configs[4]: 256 requests, prompts 128-8192, through dis_serving_*
-  --workload prefix                  TTFT with prefix KV reuse (SURVEY.md §8 row f2)
+  --workload prefix                  TTFT with prefix KV reuse
   --shard-of N                       one rank's shard of a TP = N run on one GPU, no exchange
   --tp-exchange / --nccl-allreduce   A/B of the exchange kernels (k_tp.cu) against each other and NCCL
 Extra keys: roofline (dominant kernel, from an eager step timed per kernel class), step_roofline (whole step),
@@ -69,7 +69,7 @@ def tensor_peak():
 
 # --------------------------------------------------------------------------------------- byte model
 def model_bytes(shape, tp):
-    """Algorithmic bytes per decode step per GPU (SURVEY.md §8d): every streamed weight once + KV."""
+    """Algorithmic bytes per decode step per GPU: every streamed weight once + KV."""
     H, d, L = shape.hidden, shape.head_dim, shape.layers
     qd, kd = shape.n_heads * d, shape.n_kv_heads * d
     per_layer = H * qd + 2 * H * kd + qd * H + 3 * H * shape.inter + 2 * H

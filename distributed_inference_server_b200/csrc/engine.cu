@@ -1,7 +1,7 @@
 // engine.cu -- decoder engine: weights, paged KV cache, prefill / decode steps, CUDA-graph replay of
 // the decode step, Megatron tensor parallelism.  This is the body of the spec'd InferenceWorker
 // (.kiro/specs/distributed-inference-server/design.md:334-342); the reference's own worker file is
-// empty (crates/inference/src/worker.rs:1), so the step structure follows SURVEY.md §3.3.
+// empty (crates/inference/src/worker.rs:1), so the step structure is this engine's own.
 #include "engine.h"
 
 #include <algorithm>
@@ -950,8 +950,8 @@ int Engine::prefill(int n, const int *slots, uint32_t *out_tokens, int *out_fini
 }
 
 // ------------------------------------------------------------------------------------ mixed step
-// How one forward pass is shared between running sequences and prompts that are still being read (chunked prefill,
-// SURVEY.md §8 row f1): every decode row gets its one token; the remaining room -- at most `budget` prompt tokens and
+// How one forward pass is shared between running sequences and prompts that are still being read (chunked prefill):
+// every decode row gets its one token; the remaining room -- at most `budget` prompt tokens and
 // never more than `cap` tokens in the pass -- goes to the unfinished prompts IN LIST ORDER: the caller's list is the
 // schedule (the batcher lists them by priority class, then shortest prompt first with aging, serving.cpp).  Pure function:
 // exported as dis_serving_plan_step so that the rule is property-tested without a GPU.

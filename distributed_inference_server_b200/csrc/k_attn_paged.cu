@@ -1,4 +1,4 @@
-// k_attn_paged.cu -- attention of single query tokens over a paged bf16 KV cache (SURVEY.md §2.2 K3).
+// k_attn_paged.cu -- attention of single query tokens over a paged bf16 KV cache.
 //
 // One CTA handles one (query token, kv head, split of the history) for all query heads of the GQA
 // group, so K and V are read from HBM once per group.  64-token K/V tiles are staged by TMA into
@@ -348,7 +348,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
 }
 
 // ---------------------------------------------------------------------------------------- prefill
-// Attention of a BLOCK of up to 16 consecutive query tokens of one sequence (SURVEY.md §2.2 K4).
+// Attention of a BLOCK of up to 16 consecutive query tokens of one sequence.
 // One CTA = (query block, kv head); warp w owns query head h0 + w: a 16-row MMA tile whose rows are the
 // block's tokens.  All warps walk the same 64-token K/V tiles (TMA ring shared by the GQA group, so K/V
 // are read once per 16 tokens x G heads), causal mask by position, online softmax per row, P in bf16.

@@ -1,4 +1,4 @@
-// k_attn_prefill_tc.cu -- causal prefill attention on the 5th-generation tensor cores (SURVEY.md §2.2 K4):
+// k_attn_prefill_tc.cu -- causal prefill attention on the 5th-generation tensor cores:
 // tcgen05.mma with S = Q K^T and the per-tile P V product accumulated in TMEM, K/V tiles staged by TMA.
 // No reference counterpart (the reference has no tensor code at all).
 //

@@ -4,7 +4,7 @@
 //   reduce_partials  split-K reduce alone (feeds the tensor-parallel all-reduce)
 //   sample           argmax / temperature + nucleus sampler (warp-shuffle reductions)
 //   synth_bf16       counter-hash synthetic weights
-// None of these has a reference counterpart; they implement §3.3's decoder step.
+// None of these has a reference counterpart; they implement the decoder step.
 #include "kernels.h"
 #include "ptx.cuh"
 

@@ -1,4 +1,4 @@
-// k_gemm_persist.cu -- the projection GEMM for PROMPT-sized token counts (SURVEY.md §2.2 K2), sm_100a: pairs of CTAs, one
+// k_gemm_persist.cu -- the projection GEMM for PROMPT-sized token counts, sm_100a: pairs of CTAs, one
 // 256 x 256 tile per pair (tcgen05.mma cta_group::2).
 //
 // What bounds it: with one CTA per tile of 128 x 256 every k-block brings 48 KB into an SM for 512 clocks of tensor work, 96 bytes a

@@ -1,4 +1,4 @@
-// k_gemm_tcgen05.cu -- the projection GEMM of the decoder (SURVEY.md §2.2 K2), written for sm_100a:
+// k_gemm_tcgen05.cu -- the projection GEMM of the decoder, written for sm_100a:
 // TMA (cp.async.bulk.tensor) stages bf16 tiles into 128B-swizzled shared memory, one elected thread
 // issues tcgen05.mma with the fp32 accumulator in TMEM, four epilogue warps read it back with
 // tcgen05.ld.  No reference counterpart (the reference has no tensor code at all).

@@ -1,4 +1,4 @@
-// k_gemv.cu -- bandwidth-bound GEMV for batch-1 (and very small batch) decode (SURVEY.md §2.2 K1).
+// k_gemv.cu -- bandwidth-bound GEMV for batch-1 (and very small batch) decode.
 // y[t][n] = sum_k X[t][k] * W[n][k], bf16 weights streamed once with 16-byte no-allocate loads,
 // fp32 accumulate, four weight rows per CTA with K split over its warps, warp-shuffle + shared-memory reduction.
 // Algorithmic bytes per launch: 2*N*K (weights) + 2*T*K (activations, L1/L2 resident) + 4*T*N.

@@ -1,4 +1,4 @@
-// prefix_index.hpp -- KV page allocator with prefix reuse (SURVEY.md §8 row f2), host side, header only.
+// prefix_index.hpp -- KV page allocator with prefix reuse, host side, header only.
 //
 // The reference specifies a KVCacheManager whose get_prefix(tokens) returns cached K/V for the longest cached
 // prefix of a request (.kiro/specs/distributed-inference-server/design.md:363-413; Property 9 `:734-738`,

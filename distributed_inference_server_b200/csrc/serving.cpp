@@ -1,4 +1,4 @@
-// serving.cpp -- the callers either side of the hot path (SURVEY.md §8 row f1/f3), host side, above the C ABI:
+// serving.cpp -- the callers either side of the hot path, host side, above the C ABI:
 //
 //   RequestQueue       three FIFO lanes drained High -> Normal -> Low, admission refused while the queue is over
 //                      capacity or in back-pressure, hysteresis between a high and a low watermark, expiry of

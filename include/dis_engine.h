@@ -2,7 +2,7 @@
  * dis_engine.h -- C ABI of the B200-native decoder forward path for
  * its-me-ojas/distributed-inference-server.
  *
- * The reference has no FFI boundary today (no extern "C", no build.rs; SURVEY.md §8b).  Its only seam
+ * The reference has no FFI boundary today (no extern "C", no build.rs).  Its only seam
  * for this path is the spec'd `InferenceWorker` trait (.kiro/specs/distributed-inference-server/
  * design.md:334-342), whose implementing file is empty (crates/inference/src/worker.rs:1).  Every
  * entry point below is what a Rust `impl InferenceWorker` in crates/inference would bind through a
@@ -161,8 +161,8 @@ DIS_API int dis_engine_prefill(dis_engine *e, int32_t n, const int32_t *slots, u
 /* One decode step: each listed sequence consumes its last sampled token and yields the next. */
 DIS_API int dis_engine_decode(dis_engine *e, int32_t n, const int32_t *slots, uint32_t *out_tokens,
                               int32_t *out_finish);
-/* One forward pass shared by running sequences and prompts that are still being read (chunked prefill; SURVEY.md §8
- * row f1; the reference's batcher is a 50 ms window batcher in its spec only, design.md:227-267).  A listed sequence
+/* One forward pass shared by running sequences and prompts that are still being read (chunked prefill;
+ * the reference's batcher is a 50 ms window batcher in its spec only, design.md:227-267).  A listed sequence
  * that has been prefilled decodes one token exactly as in dis_engine_decode; one that has not advances through its
  * prompt by a chunk -- all unfinished prompts together get at most max_prefill_tokens tokens (0 = the engine's
  * max_step_tokens), handed out in list order -- and samples its first token in the pass that reaches the prompt's
@@ -227,7 +227,7 @@ DIS_API int dis_worker_infer(dis_engine *e, int32_t n, const uint32_t *input_ids
                              int32_t *out_finish, dis_batch_result *result, dis_token_callback on_token,
                              void *user);
 
-/* ---- admission queue + continuous batching (SURVEY.md §8 row f1/f3) ------------------------------- *
+/* ---- admission queue + continuous batching ------------------------------- *
  * Host-side callers of the step-wise entry points above.  The queue restates the behaviour of the reference's
  * PriorityQueueManager (crates/core/src/queue.rs:75-250): three FIFO lanes served High -> Normal -> Low
  * (Priority, types.rs:17-28), enqueue refused (DIS_ERR_QUEUE_FULL) at max_queue_size or while back-pressure
@@ -287,7 +287,7 @@ DIS_API int dis_serving_order_prompts(int32_t n, const int32_t *priority, const 
 DIS_API int dis_serving_plan_step(int32_t n, const int32_t *remaining_prompt, int32_t budget, int32_t cap, int32_t *take);
 DIS_API int dis_serving_debug_pop(dis_serving *s, int32_t max, uint8_t *ids /* [max][16] */, int32_t *n);
 
-/* ---- prefix KV reuse (SURVEY.md §8 row f2) -------------------------------------------------------- *
+/* ---- prefix KV reuse -------------------------------------------------------- *
  * The spec's KVCacheManager (design.md:363-413) caches K/V per token sequence as host Vec<f32> and hands the
  * longest cached prefix back through get_prefix (Property 9, design.md:734-738), evicting least-recently-used
  * entries under memory pressure (Property 10).  Here the cache is the device page pool itself: with
@@ -324,7 +324,7 @@ DIS_API int dis_prefix_index_stats(dis_prefix_index *ix, dis_prefix_stats *out);
 /* ---- kernel-level entry points ------------------------------------------------------------------ *
  * One per hand-written kernel, taking DEVICE pointers and a cudaStream_t (NULL = default stream).
  * They exist so that parity tests can drive each kernel through the C ABI; the reference has no
- * counterpart for any of them ("None").  bf16 buffers are uint16_t bit patterns. */
+ * counterpart for any of them.  bf16 buffers are uint16_t bit patterns. */
 
 /* x[T][H] fp32 residual.  If tokens != NULL: v = embed[tokens[r]] (bf16 table); else
  * v = x[r] + sum_s partial[s*partial_stride + r*H ...] (n_partial may be 0), with r = row_map ? row_map[t] : t.

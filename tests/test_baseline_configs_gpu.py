@@ -9,7 +9,7 @@ configs[1]  Llama-3-8B (32 layers, H=4096, 32/8 heads, d=128, I=14336, V=128256)
             transformers' LlamaForCausalLM in fp32 (eager attention, TF32 off) holding the same synthetic tensors.
             torch/transformers are the checker here, never the product path.
 
-Random-init logits are nearly flat (SURVEY.md §7 hard part 2): a greedy id may legitimately differ from the fp32
+Random-init logits are nearly flat: a greedy id may legitimately differ from the fp32
 reference where the reference's own top-1/top-2 margin is below bf16 noise.  Two checks separate the two effects:
   * teacher-forced: the reference is run on the ENGINE's token history, so all 64 steps are judged even after a
     flip; at each step the engine's token must be the reference argmax, or the reference's margin between its

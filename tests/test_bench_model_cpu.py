@@ -1,4 +1,4 @@
-"""bench.py's byte model against the figures SURVEY.md §8(d) derives for BASELINE.json's configs: the roofline fractions
+"""bench.py's byte model against the figures derived for the workloads it names: the roofline fractions
 the bench line reports are only as good as these denominators, so they are pinned here (no GPU needed)."""
 import importlib.util
 import os
@@ -20,7 +20,7 @@ def step_bytes(shape, tp, batch, ctx):
 
 def test_streamed_parameters_and_kv_bytes_per_token():
     w8, kv8 = bench.model_bytes(LLAMA3_8B, 1)
-    assert w8 / 2 == pytest.approx(7.5049e9, rel=1e-4)            # P_stream, SURVEY.md §8(d)
+    assert w8 / 2 == pytest.approx(7.5049e9, rel=1e-4)            # P_stream: parameters read per step
     assert kv8 == 128 * 1024                                      # 128 KiB of bf16 K/V per token of context
     w70, kv70 = bench.model_bytes(LLAMA3_70B, 1)
     assert w70 / 2 == pytest.approx(69.503e9, rel=1e-4) and kv70 == 320 * 1024

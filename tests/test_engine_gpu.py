@@ -58,8 +58,8 @@ def rel_err(a, b):
 def assert_greedy_matches(got, oracle, prompts, n_new, label, max_flipped=None):
     """Greedy ids equal the oracle's wherever the oracle's own top-1/top-2 logit margin is above the
     noise left by a different fp32 summation order (and bf16 P in attention) once it has flipped a bf16
-    rounding somewhere upstream: 5e-3 of max|logit|.  Random-init logits are nearly flat (SURVEY.md §7
-    hard part 2); a sequence that diverges at a sub-noise margin is reported, not hidden."""
+    rounding somewhere upstream: 5e-3 of max|logit|.  Random-init logits are nearly flat;
+    a sequence that diverges at a sub-noise margin is reported, not hidden."""
     want = oracle.generate(prompts, n_new, n_logit_steps=n_new)
     flipped = 0
     for b in range(len(prompts)):
@@ -214,7 +214,7 @@ def test_llama3_8b_full_size_properties():
     e.close()
 
 
-# ---- the worker interface: structural contracts of the spec (SURVEY.md §4) -----------------------
+# ---- the worker interface: structural contracts of the spec -----------------------
 
 def small_worker(**kw):
     shape = ModelShape(1024, 256, 2, 4, 1, 128, 512, 128)

@@ -1,6 +1,6 @@
 """The oracle against an independent implementation (transformers LlamaForCausalLM, fp32 CPU).
 
-The reference has no golden vectors for the forward path (SURVEY.md §8c), so tests/golden/*.npz,
+The reference has no golden vectors for the forward path, so tests/golden/*.npz,
 produced by oracle/make_golden.py, are what pins oracle/llama_oracle.c.
 """
 import glob

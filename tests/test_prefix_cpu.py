@@ -1,4 +1,4 @@
-"""Prefix KV reuse, host logic (SURVEY.md §8 row f2), property-tested without a GPU through dis_prefix_index_*.
+"""Prefix KV reuse, host logic, property-tested without a GPU through dis_prefix_index_*.
 
 The reference specifies (.kiro/specs/distributed-inference-server/design.md:734-744)
   Property 9  -- a request whose tokens start with a cached request's tokens reuses the cached K/V for the shared

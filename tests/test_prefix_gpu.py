@@ -1,4 +1,4 @@
-"""Prefix KV reuse on the device page pool (SURVEY.md §8 row f2; spec Property 9 / 10,
+"""Prefix KV reuse on the device page pool (spec Property 9 / 10,
 .kiro/specs/distributed-inference-server/design.md:734-744), through the C ABI.
 
 A request that starts with the tokens of an earlier one must (a) really reuse the pages -- the prefix counters say
