@@ -207,7 +207,7 @@ static int gemm_common(const uint16_t *X, const uint16_t *W, float *out, uint16_
   // A slice count below 1 has always meant one slice where the tiles of 128 x 256 fill the GPU twice, and is refused elsewhere.
   if (split < 1 && T >= 512 && (long long)((N + 127) / 128) * ((T + 255) / 256) >= 2 * dis::kNumSMs) split = 1;
   dis::TmaMap wm, xm;
-  const bool persist = dis::gemm_use_persist(T, N, split, silu);  // the engine's choice for this shape
+  const bool persist = dis::gemm_use_persist(T, N, K, split, silu);  // the engine's choice for this shape
   const int bn = persist ? 128 : dis::gemm_token_tile(T);
   const int rows = silu && !persist ? dis::gemm_pick_tile_rows(N) : 128;
   cudaError_t e = dis::make_tma_map_2d(&wm, W, (uint64_t)(silu ? 2 * N : N), (uint64_t)K, (uint32_t)rows);
@@ -222,6 +222,7 @@ int dis_k_gemm(const uint16_t *X, const uint16_t *W, float *out, int32_t T, int3
                void *stream) {
   return gemm_common(X, W, out, nullptr, T, N, K, split_k, false, (cudaStream_t)stream);
 }
+int dis_k_gemm_in_pairs(int32_t T, int32_t N, int32_t K, int32_t split_k) { return dis::gemm_use_persist(T, N, K, split_k, false) ? 1 : 0; }
 int dis_k_gemm_pick_split(int32_t T, int32_t N, int32_t K) { return dis::gemm_pick_split_k(T, N, K); }
 int dis_k_gemm_silu(const uint16_t *X, const uint16_t *Wgu, uint16_t *act, int32_t T, int32_t I, int32_t K, void *stream) {
   return gemm_common(X, Wgu, nullptr, act, T, I, K, 1, true, (cudaStream_t)stream);

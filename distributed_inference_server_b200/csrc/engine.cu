@@ -634,7 +634,7 @@ cudaError_t Engine::linear_partial(const TmaMap *xmaps, const uint16_t *xptr, co
   if ((size_t)s * T * N > partial_elems) s = 1;
   *split_out = s;
   kernel_launches++;
-  if (use_persist && gemm_use_persist(T, N, s, false)) return launch_gemm_persist_partial(wmap, xmaps[2], partial, T, N, K, w_row0, s, stream);
+  if (use_persist && gemm_use_persist(T, N, K, s, false)) return launch_gemm_persist_partial(wmap, xmaps[2], partial, T, N, K, w_row0, s, stream);
   return launch_gemm_partial(wmap, xmaps[tile_index(T)], partial, T, N, K, w_row0, s, stream);
 }
 
@@ -739,7 +739,7 @@ cudaError_t Engine::enqueue_layers(int T, int n_splits) {
     if (gemv) {
       RET_CUDA(launch_gemv_silu(xn, wgu + (size_t)l * 2 * inter_l * H, act, T, inter_l, H, stream));
       kernel_launches += (uint64_t)((T + kGemvMaxT - 1) / kGemvMaxT);
-    } else if (use_persist && gemm_use_persist(T, inter_l, 1, true)) {
+    } else if (use_persist && gemm_use_persist(T, inter_l, H, 1, true)) {
       RET_CUDA(launch_gemm_persist_silu(wgu_map128, xn_map[2], act, T, inter_l, H, l * 2 * inter_l, stream));
       kernel_launches++;
     } else if (gemm_token_tile(T) >= 128) {

@@ -321,14 +321,20 @@ cudaError_t pair_launch(const TmaMap &w_map, const TmaMap &x_map, float *out, ui
 
 // Which passes run in pairs.  Gate-up products (dual) from 129 tokens: the kernel for fewer (k_gemm_tcgen05.cu) walks its one tile per
 // CTA at half the rate (14336 x 4096, 200 tokens: 78.2 us against 50.8; 4096 x 1024, 1000 tokens: 124 against 27).  Plain products from
-// 1024 tokens always (4096 x 4096, 1300 tokens: 69.9 us against 41.3); below that where their tiles fill the pairs in fewer rounds than
-// the 128 x 128 tiles of that kernel fill the SMs (4096 x 4096 in 3 K slices, 320 tokens: two rounds of either, 24.9 us in pairs of 256
-// columns and 20.8 there; 400 tokens in 2 slices: one round against two, 21.2 against 24.5).
-bool gemm_use_persist(int T, int N, int split, bool dual) {
+// 1024 tokens always (4096 x 4096, 1300 tokens: 64.8 us there, 39.8 here; 512 x 512, 1024 tokens: 12.6 and 8.2).  Below that by what the
+// two take behind their launch, in hundredths of a microsecond, fitted to 21 shapes from 512 x 512 to 8192 x 28672 at ten token counts
+// each, weights from HBM: there 100 + 20 per k-block for every 148 CTAs of 128 x 128, here 320 + 33 per k-block for every round of 256
+// columns, less 40.  The faster is taken within 2 % at 207 of the 210 points and within 8 % at the rest; counting rounds alone took the slower at
+// 39 (us there / here: 2048 x 2048 in 8 slices, 200 tokens 9.9 / 11.0; 1024 x 5120 in 16, 200 tokens 10.4 / 11.4; while 3072 x 1024 in
+// 4, 200 tokens 9.6 / 8.9; 4096 x 4096 in 2, 400 tokens 21.8 / 20.7; 4096 x 14336 in 4, 200 tokens 36.6 / 31.5).
+bool gemm_use_persist(int T, int N, int K, int split, bool dual) {
   if (T <= 128) return false;
   if (dual || T >= 1024) return true;
-  const long long tiles = (long long)((N + kBM - 1) / kBM) * ((T + 127) / 128) * split;
-  return pair_rounds(T, N, split, false, pair_columns(T, N, split, false)) < (tiles + kNumSMs - 1) / kNumSMs;
+  if (split < 1) return false;
+  const long long kb = ((K + kBK - 1) / kBK + split - 1) / split;
+  const long long ctas = (long long)((N + kBM - 1) / kBM) * ((T + 127) / 128) * split;
+  const int bn = pair_columns(T, N, split, false);
+  return (pair_rounds(T, N, split, false, bn) * bn * (320 + 33 * kb)) / 256 - 40 < (ctas + kNumSMs - 1) / kNumSMs * (100 + 20 * kb);
 }
 
 // w_map, x_map: 128-row boxes.  out[s][t][n] fp32, s the K slice.

@@ -125,7 +125,7 @@ cudaError_t launch_gemm_persist_bf16(const TmaMap &w_map128, const TmaMap &x_map
 // tile_rows = gemm_pick_tile_rows(I).
 int gemm_pick_tile_rows(int N);
 // k_gemm_persist.cu : persistent pairs of CTAs for prompt-sized T; 128-row boxes of both operands
-bool gemm_use_persist(int T, int N, int split, bool dual);
+bool gemm_use_persist(int T, int N, int K, int split, bool dual);
 cudaError_t launch_gemm_persist_partial(const TmaMap &w_map128, const TmaMap &x_map128, float *out, int T, int N, int K,
                                         int w_row0, int split, cudaStream_t st);
 // the same product, its epilogue writing bf16(relu(sum)^2) (an ungated unit's activation) instead of the fp32 sums

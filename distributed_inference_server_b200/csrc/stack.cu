@@ -1387,7 +1387,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
     if (stack_tc && !f32 && !a_f32 && !Wt.f32 && a_rows > 0 && K % 8 == 0 && lda == K && (w_off * 2) % 16 == 0) {
       int s = gemm_pick_split_k(Mrows, N, K);
       if ((size_t)s * Mrows * N > cur_scratch_elems) s = 1;
-      const bool pairs = stack_persist && gemm_use_persist(Mrows, N, s, false);  // prompt-sized products: persistent pairs of CTAs
+      const bool pairs = stack_persist && gemm_use_persist(Mrows, N, K, s, false);  // prompt-sized products: persistent pairs of CTAs
       const TmaMap *xm = stack_map(A, (uint64_t)a_rows, (uint64_t)K, pairs ? 128u : (uint32_t)gemm_token_tile(Mrows));
       const TmaMap *wm = stack_map(reinterpret_cast<const uint16_t *>(Wt.ptr) + w_off, (uint64_t)N, (uint64_t)K, 128);
       if (!xm || !wm) return cudaErrorInvalidValue;
@@ -1491,7 +1491,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   auto glu_product = [&](const StackTensor &w_gu, int ff, int act_kind, void *act, int ld_act) -> cudaError_t {
     const int tc_act = act_kind == DIS_ACT_GELU_TANH ? 1 : 0;
     kl++;
-    if (stack_persist && gemm_use_persist(T, ff, 1, true)) {  // gate and up tiles side by side on the persistent kernel
+    if (stack_persist && gemm_use_persist(T, ff, W, 1, true)) {  // gate and up tiles side by side on the persistent kernel
       const TmaMap *xm = stack_map(ff_in, (uint64_t)cap_tokens, (uint64_t)W, 128);
       const TmaMap *wm = stack_map(w_gu.ptr, (uint64_t)2 * ff, (uint64_t)W, 128);
       if (!xm || !wm) return cudaErrorInvalidValue;
@@ -1513,7 +1513,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
       return gemm(cur_act, f32, ff, w_down, 0, nullptr, out, T, W, ff, cap_tokens, nullptr, later_ok);
     }
     // an ungated unit in prompt-sized bf16 passes: the persistent product's epilogue squares the relu and writes bf16
-    if (stack_tc && stack_persist && !f32 && act_kind == DIS_ACT_RELU2 && !b_gu.ptr && W % 8 == 0 && !w_gu.f32 && gemm_use_persist(T, ff, 1, false)) {
+    if (stack_tc && stack_persist && !f32 && act_kind == DIS_ACT_RELU2 && !b_gu.ptr && W % 8 == 0 && !w_gu.f32 && gemm_use_persist(T, ff, W, 1, false)) {
       const TmaMap *xm = stack_map(ff_in, (uint64_t)cap_tokens, (uint64_t)W, 128);
       const TmaMap *wm = stack_map(w_gu.ptr, (uint64_t)ff, (uint64_t)W, 128);
       if (!xm || !wm) return cudaErrorInvalidValue;
@@ -1949,7 +1949,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
         const int nkv = H * (d + dv);
         RET_CUDA(launch_stack_latent_rows(KV.pool, sl, sp, mt.d<int>(mt.o_ls) + g.ls0, g.n, g.max_keys, lin, d_page_table, max_pages, page_size,
                                           M.lat_rc, M.lat_rk, stream));
-        const bool persist = stack_persist && gemm_use_persist(g.rows, nkv, 1, false);
+        const bool persist = stack_persist && gemm_use_persist(g.rows, nkv, r, 1, false);
         const TmaMap *xm = stack_map(M.lat_rc, (uint64_t)M.lat_rows, (uint64_t)r, persist ? 128u : (uint32_t)gemm_token_tile(g.rows));
         const TmaMap *wm = stack_map(L.ukv.ptr, (uint64_t)nkv, (uint64_t)r, 128);
         if (!xm || !wm) return cudaErrorInvalidValue;

@@ -339,6 +339,8 @@ DIS_API int dis_k_gemm(const uint16_t *X, const uint16_t *W, float *out, int32_t
                        int32_t split_k, void *stream);
 /* The split-K factor the engine uses for a [T][K] x [N][K]^T projection (never leaves a slice empty). */
 DIS_API int dis_k_gemm_pick_split(int32_t T, int32_t N, int32_t K);
+/* Whether that product runs in pairs of CTAs (k_gemm_persist.cu) or in one CTA per tile (k_gemm_tcgen05.cu).  Needs no GPU. */
+DIS_API int dis_k_gemm_in_pairs(int32_t T, int32_t N, int32_t K, int32_t split_k);
 /* act[T][I] = bf16(silu(X*Wg^T) * (X*Wu^T)); Wgu is [2I][K]: gate rows then up rows. */
 DIS_API int dis_k_gemm_silu(const uint16_t *X, const uint16_t *Wgu, uint16_t *act, int32_t T, int32_t I,
                             int32_t K, void *stream);
