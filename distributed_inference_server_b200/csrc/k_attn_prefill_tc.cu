@@ -214,7 +214,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
         if (t >= 1) load(t - 1, true);
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 && n_tiles > 0) {  // (an empty block at position 0 has no tile to wait for)
     // ===== MMA issuer: the warp converged, one elected lane issues =====
     constexpr uint32_t idesc_s = umma_idesc<kPfTile>();
     constexpr uint32_t idesc_o = umma_idesc<D>() | (1u << 16);  // B (= V) MN-major
@@ -254,7 +254,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
         issue_s(j + 2);
       }
     }
-  } else {
+  } else if (warp >= 2 && n_tiles > 0) {
     // ===== softmax: group 0 takes the even tiles, group 1 the odd ones; one thread per row; O lives in TMEM =====
     const int quarter = warp & 3;  // a warp may only touch TMEM lanes [32 * (warp % 4), +32)
     const int grp = (warp - 2) >> 2;

@@ -433,6 +433,25 @@ def test_attention_prefill_heads_of_64(nh, nkv, page_size, past, BT):
         row += n
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(8, 1, 64), (8, 2, 64), (8, 2, 128), (4, 4, 64)])
+def test_attention_prefill_with_empty_blocks(nh, nkv, d):
+    """Blocks of no tokens, at position 0 (no key either) and behind keys, beside a block of seven: they write nothing, and the block beside
+    them is what it is alone."""
+    g = torch.Generator(device=DEV); g.manual_seed(d + nh)
+    ps, T = 16, 7
+    pool = torch.randn((1, 2, nkv, ps, d), device=DEV, generator=g).to(torch.bfloat16)
+    q = torch.randn((T, nh * d), device=DEV, generator=g).to(torch.bfloat16)
+    outs = []
+    for tok0, ln, pos0 in (([0], [T], [0]), ([0, 0, 7, 0], [0, T, 0, 0], [0, 0, 0, 9])):
+        out = G.zeros((T, nh * d), dtype=torch.bfloat16, device=DEV)
+        check(lib().dis_k_attn_prefill(ptr(q), ptr(pool), 1, ptr(dev_i32([[0]])), 1, ptr(dev_i32(tok0)), ptr(dev_i32(ln)), ptr(dev_i32(pos0)),
+                                       ptr(dev_i32([0] * len(ln))), ptr(out), len(ln), nh, nkv, d, ps, None))
+        sync()
+        outs.append(out)
+    assert torch.isfinite(outs[0]).all() and outs[0].any()
+    assert torch.equal(outs[0], outs[1])
+
+
 def _prefill_call(nh, nkv, d, off_q, off_out, n=50, ps=64):
     """One prompt of n tokens, q and out starting off_* bf16 elements behind a 16-byte boundary -> (return code, q, pool, out)."""
     g = torch.Generator(device=DEV); g.manual_seed(nh)
