@@ -193,10 +193,27 @@ static int need_gpu() {
   return DIS_OK;
 }
 
+// The kernels of these calls start while the kernel in front of them on the stream still runs (programmatic dependent launch) and wait
+// for it before they read or write: the launch and the prologue no longer lie between two calls.  Not under capture, where the edge
+// would have to come from a kernel node.  Back to back, weights from HBM: down projection of 32 tokens, 4096 x 14336, and its norm 29.7 ->
+// 25.0 us; the same of 1000 tokens, 4096 x 4096, 46.4 -> 44.1; gate-up of 32 tokens, 14336 x 4096, 42.7 -> 40.4; decode attention of 32
+// ragged histories 78.3 -> 74.7; a row's norm alone stays at its caller's pace (11.4).
+struct CallOverlap {
+  explicit CallOverlap(void *stream) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing((cudaStream_t)stream, &cs);
+    if (e != cudaSuccess) (void)cudaGetLastError();  // (another thread captures what the legacy stream would have to wait for: the launch says so)
+    dis::pdl_enabled() = e == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+    dis::pdl_weights_settled() = false;
+  }
+  ~CallOverlap() { dis::pdl_enabled() = false; dis::pdl_weights_settled() = true; }
+};
+
 int dis_k_add_rmsnorm(float *x, const uint32_t *tokens, const uint16_t *embed, const float *partial, int32_t n_partial,
                       int64_t partial_stride, const float *gain, uint16_t *xn, const int32_t *row_map, int32_t T,
                       int32_t H, float eps, void *stream) {
   if (int rc = need_gpu()) return rc;
+  CallOverlap overlap(stream);
   return k_ret(dis::launch_add_rmsnorm(x, tokens, embed, partial, n_partial, partial_stride, gain, xn, row_map, T, H, eps,
                                        (cudaStream_t)stream));
 }
@@ -204,6 +221,7 @@ int dis_k_add_rmsnorm(float *x, const uint32_t *tokens, const uint16_t *embed, c
 static int gemm_common(const uint16_t *X, const uint16_t *W, float *out, uint16_t *act, int T, int N, int K, int split,
                        bool silu, cudaStream_t st) {
   if (int rc = need_gpu()) return rc;
+  CallOverlap overlap(st);
   // A slice count below 1 has always meant one slice where the tiles of 128 x 256 fill the GPU twice, and is refused elsewhere.
   if (split < 1 && T >= 512 && (long long)((N + 127) / 128) * ((T + 255) / 256) >= 2 * dis::kNumSMs) split = 1;
   dis::TmaMap wm, xm;
@@ -240,6 +258,7 @@ int dis_k_rope_kv_write(const float *qkv, int32_t n_partial, int64_t partial_str
                         const float *rope_cos, const float *rope_sin, int32_t T, int32_t n_heads, int32_t n_kv, int32_t d,
                         int32_t page_size, void *stream) {
   if (int rc = need_gpu()) return rc;
+  CallOverlap overlap(stream);
   return k_ret(dis::launch_rope_kv_write(qkv, n_partial, partial_stride, q, kv_pool, page_table, max_pages, pt_row, pos,
                                          rope_cos, rope_sin, T, n_heads, n_kv, d, page_size, (cudaStream_t)stream));
 }
@@ -250,6 +269,7 @@ int dis_k_attn_paged(const uint16_t *q, const uint16_t *kv_pool, int64_t n_pages
                      int32_t max_pages, const int32_t *pt_row, const int32_t *ctx, uint16_t *out, float *scratch,
                      int32_t n_splits, int32_t T, int32_t n_heads, int32_t n_kv, int32_t d, int32_t page_size, void *stream) {
   if (int rc = need_gpu()) return rc;
+  CallOverlap overlap(stream);
   dis::TmaMap map;
   cudaError_t e = dis::make_kv_map(&map, kv_pool, (long long)n_pages * 2 * n_kv * page_size, d, page_size);
   if (e != cudaSuccess) return k_ret(e);
@@ -261,6 +281,7 @@ int dis_k_attn_prefill(const uint16_t *q, const uint16_t *kv_pool, int64_t n_pag
                        const int32_t *qb_ptrow, uint16_t *out, int32_t n_blocks, int32_t n_heads, int32_t n_kv, int32_t d,
                        int32_t page_size, void *stream) {
   if (int rc = need_gpu()) return rc;
+  CallOverlap overlap(stream);
   dis::TmaMap map;
   cudaError_t e = dis::make_kv_map(&map, kv_pool, (long long)n_pages * 2 * n_kv * page_size, d, page_size);
   if (e != cudaSuccess) return k_ret(e);
@@ -277,6 +298,7 @@ int dis_k_attn_prefill_block_tokens(int32_t n_heads, int32_t n_kv, int32_t d) {
 int dis_k_sample(const float *logits, int64_t ld, int32_t T, int32_t V, const float *temperature, const float *top_p,
                  const uint64_t *seeds, const uint64_t *steps, uint32_t *out_tokens, float *out_logprob, void *stream) {
   if (int rc = need_gpu()) return rc;
+  CallOverlap overlap(stream);
   return k_ret(dis::launch_sample(logits, ld, T, V, temperature, top_p, reinterpret_cast<const unsigned long long *>(seeds),
                                   reinterpret_cast<const unsigned long long *>(steps), out_tokens, 0, nullptr, nullptr,
                                   out_logprob, (cudaStream_t)stream));

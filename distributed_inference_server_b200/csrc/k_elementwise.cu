@@ -14,6 +14,10 @@ bool &pdl_enabled() {
   static thread_local bool on = false;
   return on;
 }
+bool &pdl_weights_settled() {
+  static thread_local bool on = true;
+  return on;
+}
 
 // ------------------------------------------------------------------------------ block reductions
 // kThreads = 0: use blockDim.x (a multiple of 32)

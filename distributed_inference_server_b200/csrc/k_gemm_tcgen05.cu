@@ -36,6 +36,9 @@ namespace dis {
 // streaming GEMM advances one k-block per (memory latency / stages), whatever the stage holds.
 constexpr int kMaxStages = 12;
 constexpr int kMaxDynSmem = 227 * 1024;
+// When a CTA's first weight tiles are fetched: by the thread that initialises the barriers, behind the CTA's barrier, or behind
+// pdl_wait() where the weight is not settled (pdl_weights_settled())
+enum { kWeightsAfterBarrier = 0, kWeightsFirst = 1, kWeightsAfterWait = 2 };
 
 template <int BN, bool kDual>
 struct GemmCfg {
@@ -54,7 +57,7 @@ template <int BN, bool kDual>
 __global__ void __launch_bounds__(kGemmThreads)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
                     float *__restrict__ out_partial, uint16_t *__restrict__ out_act, int T, int N, int K,
-                    int w_row0, int up_row_off, int kb_per_split, int tile_rows, int n_stages, int early_tma, int act_kind, int ld_act) {
+                    int w_row0, int up_row_off, int kb_per_split, int tile_rows, int n_stages, int w_order, int act_kind, int ld_act) {
   using Cfg = GemmCfg<BN, kDual>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -98,7 +101,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     // Weights depend neither on the previous kernel nor on this CTA's TMEM allocation: the thread that has just
     // initialised the barriers can fill the ring with weight tiles at once, before the CTA-wide barrier below
     // (DIS_GEMM_EARLY_TMA=0 keeps the earlier order for A/B runs)
-    if (early_tma) issue_weights();
+    if (w_order == kWeightsFirst) issue_weights();
+    // A weight that the kernel ahead may be writing: its first tiles are brought as far as L2
+    if (w_order == kWeightsAfterWait)
+      for (int i = 0; i < pre; i++) {
+        tma_prefetch_2d(&w_map, (kb0 + i) * kBK, w_row0 + n0);
+        if (kDual) tma_prefetch_2d(&w_map, (kb0 + i) * kBK, w_row0 + up_row_off + n0);
+      }
   }
   if (warp == 1) tmem_alloc<Cfg::kTmemCols>(tmem_slot);
   tc_fence_before();
@@ -113,8 +122,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     if (lane == 0) {
       // Weights do not depend on the previous kernel: fill the ring with weight tiles first, and only
       // then wait for the producer of the activations (programmatic dependent launch).
-      if (!early_tma) issue_weights();
+      if (w_order == kWeightsAfterBarrier) issue_weights();
       pdl_wait();
+      if (w_order == kWeightsAfterWait) issue_weights();
       for (int i = 0; i < pre; i++) tma_load_2d(b_tile(i), &x_map, (kb0 + i) * kBK, t0, full_bar(i), kEvictLast);
       int s = pre == n_stages ? 0 : pre;
       uint32_t phase = pre == n_stages ? 1u : 0u;
@@ -289,9 +299,10 @@ static cudaError_t gemm_launch(const TmaMap &w_map, const TmaMap &x_map, float *
   const int smem = Cfg::smem_bytes(stages, tile_rows);
   if (smem > kMaxDynSmem) { set_last_error("gemm: tile does not fit shared memory"); return cudaErrorInvalidValue; }
   static int early = -1;
-  if (early < 0) { const char *e = getenv("DIS_GEMM_EARLY_TMA"); early = (e && atoi(e) == 0) ? 0 : 1; }
+  if (early < 0) { const char *e = getenv("DIS_GEMM_EARLY_TMA"); early = (e && atoi(e) == 0) ? kWeightsAfterBarrier : kWeightsFirst; }
+  const int w_order = pdl_enabled() && !pdl_weights_settled() ? (int)kWeightsAfterWait : early;
   return launch_k(kern, grid, dim3(kGemmThreads), (size_t)smem, st, *reinterpret_cast<const CUtensorMap *>(&w_map),
-                  *reinterpret_cast<const CUtensorMap *>(&x_map), out, act, T, N, K, w_row0, up_off, per, tile_rows, stages, early, act_kind, ld_act > 0 ? ld_act : N);
+                  *reinterpret_cast<const CUtensorMap *>(&x_map), out, act, T, N, K, w_row0, up_off, per, tile_rows, stages, w_order, act_kind, ld_act > 0 ? ld_act : N);
 }
 
 cudaError_t launch_gemm_partial(const TmaMap &w_map, const TmaMap &x_map, float *out, int T, int N, int K,

@@ -48,6 +48,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void *map, int c
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "l"(policy)
       : "memory");
 }
+// The same tile into L2 only.  L2 is where writes of running kernels meet reads, so what a kernel ahead still writes arrives there too.
+__device__ __forceinline__ void tma_prefetch_2d(const void *map, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(c0), "r"(c1) : "memory");
+}
 constexpr uint64_t kEvictFirst = 0x12F0000000000000ull;  // stream-once data (weights)
 constexpr uint64_t kEvictLast = 0x14F0000000000000ull;   // data every CTA re-reads (activations)
 
@@ -143,6 +147,9 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 
 // Host: whether launches made through launch_k() on this thread carry the PDL attribute.
 bool &pdl_enabled();
+// Host: whether the weights of the products launched on this thread may be read before pdl_wait().  True for an engine, whose weights
+// are written once; false for a call of the C ABI, whose weight may be what the kernel in front of it writes.
+bool &pdl_weights_settled();
 
 template <class... KArgs, class... Args>
 cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {

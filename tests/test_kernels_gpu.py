@@ -151,6 +151,56 @@ def test_gemm_silu_pairs(T, I, K):
     assert ((act.double() - ref).abs() <= BF16_ULP * ref.abs() * 1.01 + 1e-5).all()
 
 
+@pytest.mark.parametrize("T,H,I", [(5, 512, 1024), (32, 2048, 5632), (200, 1024, 4096), (1100, 1024, 1024)])
+def test_calls_in_a_row_take_what_the_one_before_wrote(T, H, I):
+    """A kernel of the C ABI starts while the one in front of it still runs: activations and even a weight that the call before wrote
+    have to be seen whole, in plain stream order, on a stream of its own and from a captured graph."""
+    g = torch.Generator(device=DEV); g.manual_seed(T + H + I)
+    W = (torch.randn((2 * I, H), device=DEV, generator=g) * H ** -0.5).to(torch.bfloat16)
+    W2 = (torch.randn((H, I), device=DEV, generator=g) * I ** -0.5).to(torch.bfloat16)
+    x0, gain = torch.randn((T, H), device=DEV, generator=g), torch.ones(H, device=DEV)
+    S = lib().dis_k_gemm_pick_split(T, H, I)
+    St = lib().dis_k_gemm_pick_split(T, T, H)
+    act, part = torch.empty((T, I), dtype=torch.bfloat16, device=DEV), torch.empty((S, T, H), device=DEV)
+    xn, x, gram = torch.empty((T, H), dtype=torch.bfloat16, device=DEV), torch.empty_like(x0), torch.empty((St, T, T), device=DEV)
+
+    def chain(after=lambda: None):
+        s = torch.cuda.current_stream().cuda_stream
+        x.copy_(x0)
+        part.zero_()
+        check(lib().dis_k_add_rmsnorm(ptr(x), None, None, ptr(part), S, T * H, ptr(gain), ptr(xn), None, T, H, 1e-5, s))
+        for _ in range(3):
+            after()
+            check(lib().dis_k_gemm_silu(ptr(xn), ptr(W), ptr(act), T, I, H, s))
+            after()
+            check(lib().dis_k_gemm(ptr(act), ptr(W2), ptr(part), T, H, I, S, s))
+            after()
+            check(lib().dis_k_add_rmsnorm(ptr(x), None, None, ptr(part), S, T * H, ptr(gain), ptr(xn), None, T, H, 1e-5, s))
+            after()
+            check(lib().dis_k_gemm(ptr(xn), ptr(xn), ptr(gram), T, T, H, St, s))  # xn is the weight as well
+        return [t.clone() for t in (x, xn, act, gram)]
+
+    want = chain(sync)
+    sync()
+    side = torch.cuda.Stream()
+    for k in range(6):
+        for t in (act, part, xn, gram):
+            t.fill_(float("nan"))
+        sync()
+        with torch.cuda.stream(side if k % 2 else torch.cuda.current_stream()):
+            got = chain()
+        sync()
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), k
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = chain()
+    for t in (act, part, xn, gram):
+        t.fill_(float("nan"))
+    graph.replay()
+    sync()
+    assert all(torch.equal(a, b) for a, b in zip(out, want))
+
+
 def test_gemm_rejects_empty_split():
     X, W = dev_bf16(np.zeros((8, 576), np.float32)), dev_bf16(np.zeros((128, 576), np.float32))
     out = G.zeros((4, 8, 128), dtype=torch.float32, device=DEV)
