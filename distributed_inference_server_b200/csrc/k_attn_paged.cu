@@ -13,6 +13,7 @@
 //
 // With n_splits > 1 every split writes (m, l, unnormalised o) to scratch and a combine pass merges
 // them (flash-decoding); that keeps all 148 SMs busy at batch 1.
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 
@@ -22,8 +23,9 @@
 
 namespace dis {
 
-constexpr int kAttnThreads = 128;
-constexpr int kAttnTile = 64;  // tokens per pipeline stage: 16 per warp
+constexpr int kAttnThreads = 256;  // computing threads: two groups of four warps
+constexpr int kAttnWarps = kAttnThreads / 32;
+constexpr int kAttnTile = 64;  // tokens per pipeline stage: 16 per warp of a group
 
 template <int D>
 struct AttnCfg {
@@ -31,7 +33,8 @@ struct AttnCfg {
   static constexpr int kHalfBytes = kAttnTile * 128;                      // one [64 tokens][64 dims] block
   static constexpr int kStageBytes = 2 * kHalves * kHalfBytes;            // K tile + V tile, bf16
   static constexpr int kStages = D == 128 ? 3 : 4;                        // 96 KB / 64 KB -> two CTAs per SM
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 64;    // + alignment slack + barriers
+  static constexpr int kExtraBytes = 1024 + 128;                          // alignment slack + barriers
+  static constexpr int kSmemBytes = kStages * kStageBytes + kExtraBytes;
 };
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t &r0, uint32_t &r1, uint32_t &r2, uint32_t &r3) {
@@ -42,6 +45,12 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t &r0, u
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
+// an 8x8 matrix of bf16 pairs transposed across the warp
+__device__ __forceinline__ uint32_t movmatrix(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
 // D(16x8, f32) += A(16x16, bf16, row) * B(16x8, bf16, col)
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                                uint32_t b0, uint32_t b1) {
@@ -50,12 +59,23 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// One CTA = one (query token, kv head, split).  The GQA group's query heads (<= 8) are rows 0..G-1 of a
-// 16-row MMA tile; rows G..15 are zero padding (the kernel is HBM-bound, the wasted MMA rows are free).
-// K/V tiles of 64 tokens arrive by TMA (one elected thread, 128B-swizzled boxes of min(page,64) rows,
-// mbarrier completion) into a 3-4 stage ring.  Each of the 4 warps owns 16 of a tile's 64 tokens and
-// keeps its own online-softmax state (m, l, O[16 x D] in mma accumulator fragments); the four states
-// are merged once at the end.  P is rounded to bf16 for the P.V MMA (the usual flash-attention choice).
+// One CTA = one (query token, kv head, split).  K/V tiles of 64 tokens arrive by TMA (a warp of its own, 128B-swizzled boxes of
+// min(page,64) rows, mbarrier completion) into a 3-4 stage ring.  Two groups of four warps take the tiles in turn, each warp 16 of a
+// tile's 64 tokens, with an online-softmax state (m, l, O) of its own; the eight states are merged once at the end.
+//
+// What bounds it is HBM where the histories are alike; in a ragged batch the longest one, which a single CTA walks: the time of a tile
+// in a warp is a chain of latencies (barrier, ldmatrix, MMAs, shuffles, exponential, MMAs), so what counts is how short the chain is
+// and how many run side by side.  Tokens are therefore the MMAs' rows and the group's query heads (<= 8) their eight columns: S^T = K Q^T and
+// O^T = V^T P^T fill the m16n8k16 shape, half the MMAs and half the accumulators (D / 2 registers) of heads as 16 padded rows, and eight
+// warps fit the registers of two CTAs per SM where four did.  P^T is turned from accumulator to operand by movmatrix.  Batch 32, histories of
+// 500 to 6000 keys, 32 / 8 heads of 128, 318 MB: 74.7 us before, 56 now (5.7 TB/s).
+//
+// A ragged batch in one wave is as slow as its longest history if every history has a CTA of its own (the eight warps alone moved those 74.7 us
+// to 74: the long CTAs get their share of HBM only when the short ones are done).  So the CTAs of a cluster lay the histories of up to
+// eight tokens end to end and take equal shares; pieces of one history meet in the shared memory of the CTA that has its first.  Clusters of four
+// level less (70 us).  Equal histories pay for it: 32 x 6000 115 -> 117 us, heads of 64, 64 x 2000 24.4 -> 26.
+//
+// P is rounded to bf16 for the P.V MMA (the usual flash-attention choice).
 // Rows past the context inside a box hold stale (finite) cache contents and get probability 0; the
 // engine zero-fills the pool once so that they can never be NaN.
 // Decode steps fuse the RoPE + KV-write stage into this kernel (rope.qkv != nullptr): the CTA sums the split-K
@@ -82,268 +102,375 @@ __device__ __forceinline__ float4 attn_sum_slices(const float *p, int n, long lo
   return a;
 }
 
-template <int D, int G>
+__device__ __forceinline__ float ld_cluster(const float *p, uint32_t rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void attn_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+constexpr int kAttnMaxCluster = 8;  // the portable size
+
+// kShared: a cluster's CTAs share the histories of per_cluster tokens; otherwise a CTA has one slice of one history
+template <int D, int G, bool kShared>
 __global__ void __launch_bounds__(kAttnThreads + 32, 2)
 attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const AttnRope rope, const uint16_t *__restrict__ q,
                   const int *__restrict__ page_table, int max_pages, const int *__restrict__ pt_row,
                   const int *__restrict__ ctx_len, uint16_t *__restrict__ out, float *__restrict__ scratch,
-                  int n_splits, int T, int n_heads, int n_kv, int page_shift, int n_stages) {
+                  int n_splits, int T, int n_heads, int n_kv, int page_shift, int n_stages, int per_cluster) {
   using Cfg = AttnCfg<D>;
-  constexpr int KS = D / 16;  // k-steps of the QK^T MMA
-  constexpr int NT = D / 8;   // n-tiles of the P.V MMA
+  constexpr int KS = D / 16;  // k-steps of the K Q^T MMA, m-tiles of the V^T P^T MMA
+  static_assert(kAttnWarps * G * D * 4 <= Cfg::kStageBytes, "the warps' states are merged in one stage");
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // 128B swizzle atoms are 1024-byte aligned
   uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + n_stages * Cfg::kStageBytes;
-  auto full_bar = [&](int s) { return bar_base + 8u * s; };
-  auto empty_bar = [&](int s) { return bar_base + 32u + 8u * s; };
+  // A stage has a full barrier for each of the two groups: tile i completes number i % (2 n_stages), whose phases then all belong to the
+  // group that waits for it.  (With one per stage and three stages, a group that runs ahead would take the other group's phase for its own.)
+  auto full_bar = [&](int tile) { return bar_base + 8u * (uint32_t)(tile % (2 * n_stages)); };
+  auto empty_bar = [&](int s) { return bar_base + 64u + 8u * s; };
 
-  const int t = blockIdx.z;
+  const int t0 = kShared ? (int)blockIdx.z * per_cluster : (int)blockIdx.z;
+  const int count = kShared ? min(per_cluster, T - t0) : 1;
   const int kvh = blockIdx.y;
-  const int split = blockIdx.x;
+  const int rank = blockIdx.x, ranks = gridDim.x;
   const int h0 = kvh * G;  // first query head of this CTA (G = n_heads / n_kv)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;  // mma fragment coordinates
 
+  __shared__ __align__(16) uint16_t s_q[G][D];
+  __shared__ __align__(16) uint16_t s_kvnew[2][D];
+  __shared__ float s_m[kAttnWarps][G], s_l[kAttnWarps][G];
+  __shared__ float p_o[kShared ? 2 : 1][G][kShared ? D : 1], p_m[2][G], p_l[2][G];  // pieces of a history: one begun by a CTA before, one that goes on in the next
+  __shared__ int s_ctx[kAttnMaxCluster], s_row[kAttnMaxCluster];
+
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&kv_map);
-    for (int s = 0; s < n_stages; s++) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 4); }
+    for (int s = 0; s < 2 * n_stages; s++) mbar_init(full_bar(s), 1);
+    for (int s = 0; s < n_stages; s++) mbar_init(empty_bar(s), 4);
     fence_barrier_init();
     fence_proxy_async();
   }
   pdl_launch_dependents();
   const bool fused = rope.qkv != nullptr;
-  __shared__ __align__(16) uint16_t s_q[G][D];
-  __shared__ __align__(16) uint16_t s_kvnew[2][D];
   if (!fused) pdl_wait();  // q and this step's K/V rows come from the previous kernels
+  int ctx_0 = 0, row_0 = 0;
+  if (!kShared) {
+    ctx_0 = ctx_len[t0];
+    row_0 = pt_row[t0];
+  } else if (threadIdx.x < (unsigned)count) {
+    s_ctx[threadIdx.x] = ctx_len[t0 + threadIdx.x];
+    s_row[threadIdx.x] = pt_row[t0 + threadIdx.x];
+  }
   __syncthreads();
 
   const int page_size = 1 << page_shift;
   const int box_rows = min(page_size, kAttnTile);
-  const int ctx = ctx_len[t];
-  int chunk = (ctx + n_splits - 1) / n_splits;
-  chunk = (chunk + kAttnTile - 1) / kAttnTile * kAttnTile;
-  const int begin = split * chunk;
-  const int end = min(ctx, begin + chunk);
-  const int n_tiles = end > begin ? (end - begin + kAttnTile - 1) / kAttnTile : 0;
-  const int *pt = page_table + (size_t)pt_row[t] * max_pages;
-
-  // pool rows: [page][2 (K,V)][n_kv][page_size] of d elements each
-  auto load_tile = [&](int tile, int stage) {  // one thread
-    const int tile0 = begin + tile * kAttnTile;
-    const uint32_t sbase = smem_base + stage * Cfg::kStageBytes;
-    mbar_expect_tx(full_bar(stage), Cfg::kStageBytes);
-    for (int r = 0; r < kAttnTile; r += box_rows) {
-      const int pos = tile0 + r;
-      const long long page = pt[min(pos >> page_shift, max_pages - 1)];
-      const long long krow = row0 + ((page * 2 + 0) * n_kv + kvh) * page_size + (pos & (page_size - 1));
-      const long long vrow = krow + (long long)n_kv * page_size;
-#pragma unroll
-      for (int h = 0; h < Cfg::kHalves; h++) {
-        tma_load_2d(sbase + h * Cfg::kHalfBytes + r * 128, &kv_map, h * 64, (int)krow, full_bar(stage), kEvictFirst);
-        tma_load_2d(sbase + (Cfg::kHalves + h) * Cfg::kHalfBytes + r * 128, &kv_map, h * 64, (int)vrow, full_bar(stage), kEvictFirst);
+  // ---- which tiles are this CTA's: [bound(rank), bound(rank + 1)) of the histories laid end to end
+  auto tiles_of = [&](int i) { return max(1, ((kShared ? s_ctx[i] : ctx_0) + kAttnTile - 1) / kAttnTile); };
+  int total = 0, most = 0;
+  for (int i = 0; i < count; i++) {
+    const int n = tiles_of(i);
+    total += n;
+    if (kShared) most = max(most, n);
+  }
+  // A history of its own for every n_splits CTAs, or equal shares of all where that is shorter by more than a piece's start and end cost
+  const int share = kShared ? (total + ranks - 1) / ranks : 0;
+  const bool level = kShared && most > (share + 2) * n_splits;
+  const bool pieces = kShared && (level || n_splits > 1);  // (the same in every CTA of the cluster)
+  auto bound = [&](int r) {
+    if (!kShared) return min(total, r * ((total + n_splits - 1) / n_splits));
+    if (level) return min(total, r * share);
+    const int item = r / n_splits;
+    int at = 0;
+    for (int i = 0; i < min(item, count); i++) at += tiles_of(i);
+    if (item >= count) return at;
+    const int n = tiles_of(item);
+    return at + min(n, (r % n_splits) * ((n + n_splits - 1) / n_splits));
+  };
+  const int lo = bound(rank), hi = bound(rank + 1);
+  // f(history, first tile, end tile, tiles of the history) for every piece in [lo, hi)
+  auto for_pieces = [&](auto f) {
+    if constexpr (!kShared) {
+      f(0, lo, hi, total);  // (an empty slice writes an empty state)
+    } else {
+      for (int i = 0, at = 0; i < count && at < hi; i++) {
+        const int n = tiles_of(i);
+        if (at + n > lo && hi > lo) f(i, max(lo - at, 0), min(hi - at, n), n);
+        at += n;
       }
     }
   };
 
-  // Warp 4 loads and does nothing else, the four computing warps free a stage each for themselves: no barrier of the whole block per
-  // tile.  A batch of ragged histories is as slow as its longest one, which a single CTA walks: with the loads issued by a computing
-  // thread behind a block barrier that took 1.04 us per tile.  Batch 32, histories of 500 to 6000 keys, 32 / 8 heads of 128, 318 MB:
-  // 100.5 -> 78.4 us; 64 equal histories of 1600: 65.2 -> 63.4 us; 32 x 512: 14.5 us on both.
-  if (warp == 4) {
-    if (lane == 0)
-      for (int tile = 0; tile < n_tiles; tile++) {
-        const int stage = tile % n_stages;
-        if (tile >= n_stages) mbar_wait(empty_bar(stage), (uint32_t)(tile / n_stages - 1) & 1u);
-        load_tile(tile, stage);
-      }
+  // The last warp loads and does nothing else, the computing warps free a stage each for themselves: no barrier of the whole block per
+  // tile (with one, the longest history of a ragged batch took 1.04 us per tile, without it and four computing warps 0.83).
+  if (warp == kAttnWarps) {
+    if (lane == 0) {
+      int k = 0;  // stages handed out so far
+      auto next_stage = [&] {
+        const int stage = k % n_stages;
+        if (k >= n_stages) mbar_wait(empty_bar(stage), (uint32_t)(k / n_stages - 1) & 1u);
+        return stage;
+      };
+      for_pieces([&](int i, int a, int b, int n) {
+        const int *pt = page_table + (size_t)(kShared ? s_row[i] : row_0) * max_pages;
+        for (int tile = a; tile < b; tile++, k++) {
+          // pool rows: [page][2 (K,V)][n_kv][page_size] of d elements each
+          const uint32_t sbase = smem_base + next_stage() * Cfg::kStageBytes, bar = full_bar(k);
+          mbar_expect_tx(bar, Cfg::kStageBytes);
+          for (int r = 0; r < kAttnTile; r += box_rows) {
+            const int pos = tile * kAttnTile + r;
+            const long long page = pt[min(pos >> page_shift, max_pages - 1)];
+            const long long krow = row0 + ((page * 2 + 0) * n_kv + kvh) * page_size + (pos & (page_size - 1));
+            const long long vrow = krow + (long long)n_kv * page_size;
+#pragma unroll
+            for (int h = 0; h < Cfg::kHalves; h++) {
+              tma_load_2d(sbase + h * Cfg::kHalfBytes + r * 128, &kv_map, h * 64, (int)krow, bar, kEvictFirst);
+              tma_load_2d(sbase + (Cfg::kHalves + h) * Cfg::kHalfBytes + r * 128, &kv_map, h * 64, (int)vrow, bar, kEvictFirst);
+            }
+          }
+        }
+        next_stage();  // one more, empty: the warps merge their states in it while the next piece's tiles are under way
+        mbar_arrive(full_bar(k));
+        k++;
+      });
+    }
     __syncwarp();
-    __syncthreads();  // (the two barriers around the merge below)
-    __syncthreads();
+    if (pieces) attn_cluster_sync();
+    if (kShared) attn_cluster_sync();
     return;
   }
-  auto sync_compute = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };  // the four computing warps
+  auto sync_compute = [] { asm volatile("bar.sync 1, %0;" ::"n"(kAttnThreads) : "memory"); };  // the computing warps
 
-  const int new_pos = ctx - 1;                               // the position this decode step appends
-  const bool owner = fused && new_pos >= begin && new_pos < end;  // the split that holds it
-  if (fused) {
-    pdl_wait();  // the QKV projection's slices
-    constexpr int HQ = D / 8;  // float4 rotate-half items per head
-    const int nq = n_heads * D, nk = n_kv * D;
-    const float *base = rope.qkv + (size_t)t * (nq + 2 * nk);
-    const float *cs = rope.cos_t + (size_t)new_pos * (D / 2), *sn = rope.sin_t + (size_t)new_pos * (D / 2);
-    for (int item = threadIdx.x; item < (G + 1) * HQ + D / 4; item += kAttnThreads) {
-      if (item < (G + 1) * HQ) {
-        const bool is_q = item < G * HQ;
-        if (!is_q && !owner) continue;
-        const int hh = is_q ? item / HQ : 0, i = (item % HQ) * 4;
-        const int col = is_q ? (h0 + hh) * D + i : nq + kvh * D + i;
-        const float4 a = attn_sum_slices(base + col, rope.n_partial, rope.stride);
-        const float4 b = attn_sum_slices(base + col + D / 2, rope.n_partial, rope.stride);
-        const float4 c = *reinterpret_cast<const float4 *>(cs + i), sv = *reinterpret_cast<const float4 *>(sn + i);
-        uint2 lo, hi;
-        lo.x = float2_to_bf16x2(a.x * c.x - b.x * sv.x, a.y * c.y - b.y * sv.y);
-        lo.y = float2_to_bf16x2(a.z * c.z - b.z * sv.z, a.w * c.w - b.w * sv.w);
-        hi.x = float2_to_bf16x2(b.x * c.x + a.x * sv.x, b.y * c.y + a.y * sv.y);
-        hi.y = float2_to_bf16x2(b.z * c.z + a.z * sv.z, b.w * c.w + a.w * sv.w);
-        uint16_t *dst = is_q ? s_q[hh] : s_kvnew[0];
-        *reinterpret_cast<uint2 *>(dst + i) = lo;
-        *reinterpret_cast<uint2 *>(dst + D / 2 + i) = hi;
-      } else if (owner) {
-        const int i = (item - (G + 1) * HQ) * 4;
-        const float4 a = attn_sum_slices(base + nq + nk + kvh * D + i, rope.n_partial, rope.stride);
-        uint2 o;
-        o.x = float2_to_bf16x2(a.x, a.y);
-        o.y = float2_to_bf16x2(a.z, a.w);
-        *reinterpret_cast<uint2 *>(s_kvnew[1] + i) = o;
+  const float scale_log2 = rsqrtf((float)D) * 1.4426950408889634f;  // scores are kept in the log2 domain
+  const int grp = warp >> 2, wtok = (warp & 3) * 16;                // this warp's token slice inside a tile
+  const int mi = lane >> 3, mr = lane & 7;
+  const int k_tok = wtok + (mi & 1) * 8 + mr, v_tok = wtok + (mi >> 1) * 8 + mr;  // the row whose address this lane gives ldmatrix
+  if (fused) pdl_wait();  // the QKV projection's slices
+  int k0 = 0, open = -1;  // stages consumed so far; the history whose first piece is here and goes on elsewhere
+  for_pieces([&](int item, int a, int b, int n) {
+    const int t = t0 + item, ctx = kShared ? s_ctx[item] : ctx_0;
+    const int new_pos = ctx - 1;             // the position this decode step appends
+    const bool owner = fused && b == n && b > a;  // the piece that holds it
+    if (fused) {
+      constexpr int HQ = D / 8;  // float4 rotate-half items per head
+      const int nq = n_heads * D, nk = n_kv * D;
+      const float *base = rope.qkv + (size_t)t * (nq + 2 * nk);
+      const float *cs = rope.cos_t + (size_t)new_pos * (D / 2), *sn = rope.sin_t + (size_t)new_pos * (D / 2);
+      for (int it = threadIdx.x; it < (G + 1) * HQ + D / 4; it += kAttnThreads) {
+        if (it < (G + 1) * HQ) {
+          const bool is_q = it < G * HQ;
+          if (!is_q && !owner) continue;
+          const int hh = is_q ? it / HQ : 0, i = (it % HQ) * 4;
+          const int col = is_q ? (h0 + hh) * D + i : nq + kvh * D + i;
+          const float4 va = attn_sum_slices(base + col, rope.n_partial, rope.stride);
+          const float4 vb = attn_sum_slices(base + col + D / 2, rope.n_partial, rope.stride);
+          const float4 c = *reinterpret_cast<const float4 *>(cs + i), sv = *reinterpret_cast<const float4 *>(sn + i);
+          uint2 w0, w1;
+          w0.x = float2_to_bf16x2(va.x * c.x - vb.x * sv.x, va.y * c.y - vb.y * sv.y);
+          w0.y = float2_to_bf16x2(va.z * c.z - vb.z * sv.z, va.w * c.w - vb.w * sv.w);
+          w1.x = float2_to_bf16x2(vb.x * c.x + va.x * sv.x, vb.y * c.y + va.y * sv.y);
+          w1.y = float2_to_bf16x2(vb.z * c.z + va.z * sv.z, vb.w * c.w + va.w * sv.w);
+          uint16_t *dst = is_q ? s_q[hh] : s_kvnew[0];
+          *reinterpret_cast<uint2 *>(dst + i) = w0;
+          *reinterpret_cast<uint2 *>(dst + D / 2 + i) = w1;
+        } else if (owner) {
+          const int i = (it - (G + 1) * HQ) * 4;
+          const float4 v = attn_sum_slices(base + nq + nk + kvh * D + i, rope.n_partial, rope.stride);
+          uint2 o;
+          o.x = float2_to_bf16x2(v.x, v.y);
+          o.y = float2_to_bf16x2(v.z, v.w);
+          *reinterpret_cast<uint2 *>(s_kvnew[1] + i) = o;
+        }
+      }
+      sync_compute();
+      if (owner && threadIdx.x < 2 * (D / 8)) {  // the new row goes to the page pool for the steps to come
+        const int kv = threadIdx.x / (D / 8), c = threadIdx.x % (D / 8);
+        const long long page = page_table[(size_t)(kShared ? s_row[item] : row_0) * max_pages + (new_pos >> page_shift)];
+        uint16_t *dst = rope.kv_base + ((((size_t)page * 2 + kv) * n_kv + kvh) * page_size + (new_pos & (page_size - 1))) * D + c * 8;
+        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(s_kvnew[kv] + c * 8);
+      }
+    }
+
+    // ---- Q^T as the B operand: column g = head g (g < G), everything else zero
+    uint32_t qb[KS][2];
+#pragma unroll
+    for (int ks = 0; ks < KS; ks++) {
+      qb[ks][0] = 0u; qb[ks][1] = 0u;
+      if (g < G) {
+        const uint16_t *qp = fused ? s_q[g] + ks * 16 + tq * 2 : q + ((size_t)t * n_heads + h0 + g) * D + ks * 16 + tq * 2;
+        qb[ks][0] = *reinterpret_cast<const uint32_t *>(qp);
+        qb[ks][1] = *reinterpret_cast<const uint32_t *>(qp + 8);
+      }
+    }
+
+    float oacc[KS][4];  // O^T: dims 16 n + g (+ 8) of heads 2 tq (+ 1)
+#pragma unroll
+    for (int m = 0; m < KS; m++) { oacc[m][0] = 0.f; oacc[m][1] = 0.f; oacc[m][2] = 0.f; oacc[m][3] = 0.f; }
+    float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};  // heads 2 tq (+ 1); l_run: this thread's tokens (summed at the end)
+
+    for (int tile = a + ((k0 ^ grp) & 1); tile < b; tile += 2) {  // stage number k0 + tile - a: even ones are group 0's
+      const int k = k0 + tile - a, stage = k % n_stages;
+      mbar_wait(full_bar(k), (uint32_t)(k / (2 * n_stages)) & 1u);
+      const uint32_t ks_addr = smem_base + stage * Cfg::kStageBytes;
+      const uint32_t vs_addr = ks_addr + Cfg::kHalves * Cfg::kHalfBytes;
+      const int tile_len = min(kAttnTile, ctx - tile * kAttnTile);
+      if (owner && tile == n - 1 && ((new_pos - tile * kAttnTile) >> 4) == (warp & 3)) {
+        // the tile TMA fetched predates this step's K/V row: the warp that reads the row patches it in (same 128B swizzle as the TMA boxes)
+        const int r = new_pos - tile * kAttnTile;
+        if (lane < 2 * (D / 8)) {
+          const int kv = lane / (D / 8), c = lane % (D / 8);
+          const uint32_t dst = (kv ? vs_addr : ks_addr) + (c >> 3) * Cfg::kHalfBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+          const uint4 v = *reinterpret_cast<const uint4 *>(s_kvnew[kv] + c * 8);
+          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+          fence_proxy_async();  // (a later tile may land in this stage)
+        }
+        __syncwarp();
+      }
+      if (wtok < tile_len) {  // warp-uniform (only a history's last tile is short)
+        // ---- S^T = K Q^T for this warp's 16 tokens: tokens wtok + g (+ 8), heads 2 tq (+ 1); two accumulators halve the chain
+        float sacc[2][4];
+#pragma unroll
+        for (int e = 0; e < 2; e++) { sacc[e][0] = 0.f; sacc[e][1] = 0.f; sacc[e][2] = 0.f; sacc[e][3] = 0.f; }
+#pragma unroll
+        for (int ks = 0; ks < KS; ks++) {
+          const int c = ks * 2 + (mi >> 1);  // 16-byte chunk of the row
+          uint32_t a0, a1, a2, a3;
+          ldmatrix_x4(ks_addr + (c >> 3) * Cfg::kHalfBytes + k_tok * 128 + (((c & 7) ^ (k_tok & 7)) << 4), a0, a1, a2, a3);
+          mma_bf16_16816(sacc[0], a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
+        }
+        // ---- online softmax of the two heads
+        const bool in0 = wtok + g < tile_len, in1 = wtok + g + 8 < tile_len;
+        float p[4], corr[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          p[e] = in0 ? sacc[0][e] + sacc[1][e] : -INFINITY;
+          p[2 + e] = in1 ? sacc[0][2 + e] + sacc[1][2 + e] : -INFINITY;
+          float mx = fmaxf(p[e], p[2 + e]);
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+          mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+          const float m_new = fmaxf(m_run[e], mx * scale_log2);  // finite: token wtok is valid
+          corr[e] = exp2f(m_run[e] - m_new);        // 0 on the first tile
+          m_run[e] = m_new;
+          p[e] = exp2f(fmaf(p[e], scale_log2, -m_new));
+          p[2 + e] = exp2f(fmaf(p[2 + e], scale_log2, -m_new));
+        }
+        // the sums take the weights as P V takes them, rounded: the weights of a row then add up to one
+        const uint32_t p01 = float2_to_bf16x2(p[0], p[1]), p23 = float2_to_bf16x2(p[2], p[3]);
+        const float2 r01 = bf16x2_to_float2(p01), r23 = bf16x2_to_float2(p23);
+        l_run[0] = l_run[0] * corr[0] + (r01.x + r23.x);
+        l_run[1] = l_run[1] * corr[1] + (r01.y + r23.y);
+        const uint32_t pb0 = movmatrix(p01), pb1 = movmatrix(p23);
+#pragma unroll
+        for (int m = 0; m < KS; m++) { oacc[m][0] *= corr[0]; oacc[m][1] *= corr[1]; oacc[m][2] *= corr[0]; oacc[m][3] *= corr[1]; }
+        // ---- O^T += V^T P^T : A = V^T by ldmatrix.trans of the [tokens][dims] tile
+#pragma unroll
+        for (int m = 0; m < KS; m++) {
+          const int c = m * 2 + (mi & 1);
+          uint32_t a0, a1, a2, a3;
+          ldmatrix_x4_trans(vs_addr + (c >> 3) * Cfg::kHalfBytes + v_tok * 128 + (((c & 7) ^ (v_tok & 7)) << 4), a0, a1, a2, a3);
+          mma_bf16_16816(oacc[m], a0, a1, a2, a3, pb0, pb1);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(empty_bar(stage));
+    }
+    k0 += b - a;
+
+    // ---- merge the warps' (m, l, O) in the stage that was handed out empty: [warps][G][D], a pair of heads 8 dims from the next (no bank twice)
+    const int stage = k0 % n_stages;
+    const bool mine = (k0 & 1) == grp;
+    if (mine) mbar_wait(full_bar(k0), (uint32_t)(k0 / (2 * n_stages)) & 1u);
+    k0++;
+    sync_compute();
+    float *s_o = reinterpret_cast<float *>(smem + stage * Cfg::kStageBytes);
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 4);
+      l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 8);
+      l_run[e] += __shfl_xor_sync(0xffffffffu, l_run[e], 16);
+      const int hh = tq * 2 + e;
+      if (hh < G) {
+        float *o = s_o + (warp * G + hh) * D;
+#pragma unroll
+        for (int m = 0; m < KS; m++) { o[(m * 16 + g) ^ (tq * 8)] = oacc[m][e]; o[(m * 16 + 8 + g) ^ (tq * 8)] = oacc[m][2 + e]; }
+        if (g == 0) { s_m[warp][hh] = m_run[e]; s_l[warp][hh] = l_run[e]; }
       }
     }
     sync_compute();
-    if (owner && threadIdx.x < 2 * (D / 8)) {  // the new row goes to the page pool for the steps to come
-      const int kv = threadIdx.x / (D / 8), c = threadIdx.x % (D / 8);
-      const long long page = pt[new_pos >> page_shift];
-      uint16_t *dst = rope.kv_base + ((((size_t)page * 2 + kv) * n_kv + kvh) * page_size + (new_pos & (page_size - 1))) * D + c * 8;
-      *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(s_kvnew[kv] + c * 8);
-    }
-  }
-
-  // ---- Q as the A operand: row g = head g (g < G), everything else zero
-  uint32_t qa[KS][2];
+    const bool whole = kShared ? a == 0 && b == n : n_splits == 1;
+    const int slot = a > 0 ? 0 : 1;
+    if (kShared && !whole && slot == 1) open = item;
+    for (int e = threadIdx.x; e < G * D; e += kAttnThreads) {
+      const int hh = e / D, dd = e - hh * D;
+      float M = -INFINITY;
 #pragma unroll
-  for (int ks = 0; ks < KS; ks++) {
-    qa[ks][0] = 0u; qa[ks][1] = 0u;
-    if (g < G) {
-      const uint16_t *qp = fused ? s_q[g] + ks * 16 + tq * 2 : q + ((size_t)t * n_heads + h0 + g) * D + ks * 16 + tq * 2;
-      qa[ks][0] = *reinterpret_cast<const uint32_t *>(qp);
-      qa[ks][1] = *reinterpret_cast<const uint32_t *>(qp + 8);
-    }
-  }
-  const float scale_log2 = rsqrtf((float)D) * 1.4426950408889634f;  // scores are kept in the log2 domain
-
-  float oacc[NT][4];
+      for (int w = 0; w < kAttnWarps; w++) M = fmaxf(M, s_m[w][hh]);
+      float L = 0.f, o = 0.f;
 #pragma unroll
-  for (int n = 0; n < NT; n++) { oacc[n][0] = 0.f; oacc[n][1] = 0.f; oacc[n][2] = 0.f; oacc[n][3] = 0.f; }
-  float m_run = -INFINITY, l_run = 0.f;  // row g; l_run is this thread's partial sum (quad-reduced at the end)
-
-  const int wtok = warp * 16;  // this warp's token slice inside a tile
-  for (int tile = 0; tile < n_tiles; tile++) {
-    const int stage = tile % n_stages;
-    mbar_wait(full_bar(stage), (uint32_t)(tile / n_stages) & 1u);
-    const uint32_t ks_addr = smem_base + stage * Cfg::kStageBytes;
-    const uint32_t vs_addr = ks_addr + Cfg::kHalves * Cfg::kHalfBytes;
-    const int tile_len = min(kAttnTile, end - (begin + tile * kAttnTile));
-    const int new_row = new_pos - (begin + tile * kAttnTile);
-    if (owner && tile == n_tiles - 1 && (new_row >> 4) == warp) {
-      // the tile TMA fetched predates this step's K/V row: the warp that reads the row patches it in (same 128B swizzle as the TMA boxes)
-      const int r = new_row;
-      if (lane < 2 * (D / 8)) {
-        const int kv = lane / (D / 8), c = lane % (D / 8);
-        const uint32_t dst = (kv ? vs_addr : ks_addr) + (c >> 3) * Cfg::kHalfBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4);
-        const uint4 v = *reinterpret_cast<const uint4 *>(s_kvnew[kv] + c * 8);
-        asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+      for (int w = 0; w < kAttnWarps; w++) {
+        const float mw = s_m[w][hh];
+        const float wgt = mw == -INFINITY ? 0.f : exp2f(mw - M);
+        L += s_l[w][hh] * wgt;
+        o += s_o[(w * G + hh) * D + (dd ^ ((hh >> 1) * 8))] * wgt;
       }
-      __syncwarp();
-    }
-    if (wtok >= tile_len) continue;  // warp-uniform: nothing of this tile belongs to this warp (only a split's last tile is short)
-
-    // ---- S = Q K^T for this warp's 16 tokens (two n-tiles of 8)
-    float sacc[2][4];
-#pragma unroll
-    for (int n = 0; n < 2; n++) { sacc[n][0] = 0.f; sacc[n][1] = 0.f; sacc[n][2] = 0.f; sacc[n][3] = 0.f; }
-    {
-      const int mi = lane >> 3, r = lane & 7;
-      const int tok = wtok + (mi >> 1) * 8 + r;  // matrices 0,1 -> n-tile 0; 2,3 -> n-tile 1
-#pragma unroll
-      for (int ks = 0; ks < KS; ks++) {
-        const int c = ks * 2 + (mi & 1);  // 16-byte chunk of the row
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4(ks_addr + (c >> 3) * Cfg::kHalfBytes + tok * 128 + (((c & 7) ^ (tok & 7)) << 4), b0, b1, b2, b3);
-        mma_bf16_16816(sacc[0], qa[ks][0], 0u, qa[ks][1], 0u, b0, b1);
-        mma_bf16_16816(sacc[1], qa[ks][0], 0u, qa[ks][1], 0u, b2, b3);
+      const int h = h0 + hh;
+      if (whole) {
+        out[((size_t)t * n_heads + h) * D + dd] = float_to_bf16_bits(o / L);
+      } else if constexpr (kShared) {
+        p_o[slot][hh][dd] = o;
+        if (dd == 0) { p_m[slot][hh] = M; p_l[slot][hh] = L; }
+      } else {
+        // scratch: ml [T][n_heads][S][2] then o [T][n_heads][S][D]; m is in the log2 domain
+        float *ml = scratch + (((size_t)t * n_heads + h) * n_splits + rank) * 2;
+        float *op = scratch + (size_t)T * n_heads * n_splits * 2 + (((size_t)t * n_heads + h) * n_splits + rank) * D;
+        op[dd] = o;
+        if (dd == 0) { ml[0] = M; ml[1] = L; }
       }
     }
-    // ---- online softmax on row g (tokens wtok + n*8 + tq*2 + {0,1})
-    float mx = -INFINITY;
-#pragma unroll
-    for (int n = 0; n < 2; n++)
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        const int tok = wtok + n * 8 + tq * 2 + e;
-        const float v = tok < tile_len ? sacc[n][e] * scale_log2 : -INFINITY;
-        sacc[n][e] = v;
-        mx = fmaxf(mx, v);
-      }
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float m_new = fmaxf(m_run, mx);  // finite: token wtok is valid
-    const float corr = exp2f(m_run - m_new);  // 0 on the first tile
-    m_run = m_new;
-    float psum = 0.f;
-    uint32_t pa[2];
-#pragma unroll
-    for (int n = 0; n < 2; n++) {
-      const float p0 = exp2f(sacc[n][0] - m_new), p1 = exp2f(sacc[n][1] - m_new);
-      psum += p0 + p1;
-      pa[n] = float2_to_bf16x2(p0, p1);
+    if (kShared) {
+      fence_proxy_async();  // (plain accesses to a stage that TMA will fill again)
+      sync_compute();
+      if (mine && lane == 0) mbar_arrive(empty_bar(stage));
     }
-    l_run = l_run * corr + psum;
+  });
+  // ---- pieces of one history in several CTAs: the CTA that holds its first piece reads the others' out of their shared memory
+  if constexpr (kShared) {
+    if (pieces) attn_cluster_sync();
+    if (open >= 0) {
+      int end = 0;
+      for (int i = 0; i <= open; i++) end += tiles_of(i);
+      int last = rank + 1;  // the CTAs rank + 1 .. last hold the rest
+      while (bound(last + 1) < end) last++;
+      for (int e = threadIdx.x; e < G * D; e += kAttnThreads) {
+        const int hh = e / D, dd = e - hh * D;
+        float mr2[kAttnMaxCluster], M = p_m[1][hh];
 #pragma unroll
-    for (int n = 0; n < NT; n++) { oacc[n][0] *= corr; oacc[n][1] *= corr; }
-    // ---- O += P V : A = P (rows g; rows g+8 are padding -> zero), B = V^T fragments via ldmatrix.trans
-    {
-      const int mi = lane >> 3, r = lane & 7;
-      const int tok = wtok + (mi & 1) * 8 + r;  // matrices 0,2 -> tokens 0-7; 1,3 -> tokens 8-15
+        for (int r = 1; r < kAttnMaxCluster; r++) {
+          mr2[r] = rank + r <= last ? ld_cluster(&p_m[0][hh], (uint32_t)(rank + r)) : -INFINITY;
+          M = fmaxf(M, mr2[r]);
+        }
+        const float f = exp2f(p_m[1][hh] - M);  // every piece holds a visible key
+        float L = p_l[1][hh] * f, o = p_o[1][hh][dd] * f;
 #pragma unroll
-      for (int n = 0; n < NT; n += 2) {
-        const int c = n + (mi >> 1);
-        uint32_t b0, b1, b2, b3;
-        ldmatrix_x4_trans(vs_addr + (c >> 3) * Cfg::kHalfBytes + tok * 128 + (((c & 7) ^ (tok & 7)) << 4), b0, b1, b2, b3);
-        mma_bf16_16816(oacc[n], pa[0], 0u, pa[1], 0u, b0, b1);
-        mma_bf16_16816(oacc[n + 1], pa[0], 0u, pa[1], 0u, b2, b3);
+        for (int r = 1; r < kAttnMaxCluster; r++)
+          if (rank + r <= last) {
+            const float w = exp2f(mr2[r] - M);
+            L += ld_cluster(&p_l[0][hh], (uint32_t)(rank + r)) * w;
+            o += ld_cluster(&p_o[0][hh][dd], (uint32_t)(rank + r)) * w;
+          }
+        out[((size_t)(t0 + open) * n_heads + h0 + hh) * D + dd] = float_to_bf16_bits(o / L);
       }
     }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(empty_bar(stage));
-  }
-  __syncthreads();  // every warp waited for every load: the stage memory is free
-
-  // ---- merge the four warps' (m, l, O) through the stage memory
-  float *s_o = reinterpret_cast<float *>(smem);        // [4 warps][G][D]
-  float *s_m = s_o + 4 * G * D;                        // [4][G]
-  float *s_l = s_m + 4 * G;                            // [4][G]
-  l_run += __shfl_xor_sync(0xffffffffu, l_run, 1);
-  l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
-  if (g < G) {
-#pragma unroll
-    for (int n = 0; n < NT; n++)
-      *reinterpret_cast<float2 *>(s_o + ((size_t)(warp * G + g) * D + n * 8 + tq * 2)) = make_float2(oacc[n][0], oacc[n][1]);
-    if (tq == 0) { s_m[warp * G + g] = m_run; s_l[warp * G + g] = l_run; }
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < G * D; e += kAttnThreads) {
-    const int hh = e / D, dd = e - hh * D;
-    float M = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < 4; w++) M = fmaxf(M, s_m[w * G + hh]);
-    float L = 0.f, o = 0.f;
-#pragma unroll
-    for (int w = 0; w < 4; w++) {
-      const float mw = s_m[w * G + hh];
-      const float wgt = mw == -INFINITY ? 0.f : exp2f(mw - M);
-      L += s_l[w * G + hh] * wgt;
-      o += s_o[(size_t)(w * G + hh) * D + dd] * wgt;
-    }
-    const int h = h0 + hh;
-    if (n_splits == 1) {
-      out[((size_t)t * n_heads + h) * D + dd] = float_to_bf16_bits(o / L);
-    } else {
-      // scratch: ml [T][n_heads][S][2] then o [T][n_heads][S][D]; m is in the log2 domain
-      float *ml = scratch + (((size_t)t * n_heads + h) * n_splits + split) * 2;
-      float *op = scratch + (size_t)T * n_heads * n_splits * 2 + (((size_t)t * n_heads + h) * n_splits + split) * D;
-      op[dd] = o;
-      if (dd == 0) { ml[0] = M; ml[1] = L; }
-    }
+    // nobody leaves while its pieces are read; without pieces either, so that a cluster of the next launch finds eight places at once
+    // (32 equal histories of 6000: 134 us where each CTA left by itself)
+    attn_cluster_sync();
   }
 }
 
@@ -547,6 +674,17 @@ __global__ void attn_combine_kernel(const float *__restrict__ scratch, uint16_t 
   out[((size_t)t * n_heads + h) * D + dd] = float_to_bf16_bits(o / L);
 }
 
+// Tokens whose histories a cluster of CTAs shares (each history n_splits CTAs' worth), 0: no cluster.  Slices of two to eight per token are
+// merged in shared memory, which saves the merge's launch and its scratch traffic; whole histories are levelled where they can be long: up
+// to kAttnShort keys nothing is gained, and a cluster starts later than a CTA.  Beyond one wave of two CTAs per SM the hardware levels
+// by itself, and whole clusters find room later than single CTAs.
+int attn_tokens_per_cluster(int n_splits, int T, int n_kv, int longest) {
+  if (n_splits > kAttnMaxCluster || (long long)n_splits * T * n_kv > 2 * kNumSMs) return 0;
+  if (n_splits == 1 && (T < 2 || longest <= kAttnShort)) return 0;
+  const int n = kAttnMaxCluster / n_splits;
+  return n < T ? n : T;
+}
+
 size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits) {
   if (n_splits <= 1) return 0;
   return (size_t)T * n_heads * n_splits * (2 + (size_t)d);
@@ -555,10 +693,12 @@ size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits) {
 template <int D, int G>
 static cudaError_t attn_launch(const TmaMap &kv_map, long long row0, const AttnRope &rope, const uint16_t *q, const int *page_table,
                                int max_pages, const int *pt_row, const int *ctx, uint16_t *out, float *scratch,
-                               int n_splits, int T, int n_heads, int n_kv, int page_shift, cudaStream_t st) {
-  dim3 grid(n_splits, n_kv, T);
+                               int n_splits, int T, int n_heads, int n_kv, int page_shift, int longest, cudaStream_t st) {
   static DeviceOnce once;
-  DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(attn_paged_kernel<D, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::kSmemBytes); }));
+  DIS_CUDA_TRY(once.run([&] {
+    cudaError_t e = cudaFuncSetAttribute(attn_paged_kernel<D, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::kSmemBytes);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_paged_kernel<D, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::kSmemBytes);
+  }));
   // ring depth: fewer stages leave shared memory for the NEXT kernel's CTAs to become resident (and prefetch their
   // weights) while this one is still streaming; DIS_ATTN_STAGES overrides (A/B runs), 2 <= stages <= AttnCfg::kStages
   static int stages = 0;
@@ -567,10 +707,17 @@ static cudaError_t attn_launch(const TmaMap &kv_map, long long row0, const AttnR
     stages = e ? atoi(e) : AttnCfg<D>::kStages;
     stages = stages < 2 ? 2 : (stages > AttnCfg<D>::kStages ? AttnCfg<D>::kStages : stages);
   }
-  const int smem = stages * AttnCfg<D>::kStageBytes + 1024 + 64;
-  DIS_CUDA_TRY(launch_k(attn_paged_kernel<D, G>, grid, dim3(kAttnThreads + 32), (size_t)smem, st,
+  const int smem = stages * AttnCfg<D>::kStageBytes + AttnCfg<D>::kExtraBytes;
+  const int per_cluster = attn_tokens_per_cluster(n_splits, T, n_kv, longest);
+  if (per_cluster > 0) {
+    const int ranks = per_cluster * n_splits;
+    return launch_k_cluster(attn_paged_kernel<D, G, true>, dim3(ranks, n_kv, (T + per_cluster - 1) / per_cluster), dim3(kAttnThreads + 32), (size_t)smem, st, ranks,
+                            *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
+                            scratch, n_splits, T, n_heads, n_kv, page_shift, stages, per_cluster);
+  }
+  DIS_CUDA_TRY(launch_k(attn_paged_kernel<D, G, false>, dim3(n_splits, n_kv, T), dim3(kAttnThreads + 32), (size_t)smem, st,
                         *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
-                        scratch, n_splits, T, n_heads, n_kv, page_shift, stages));
+                        scratch, n_splits, T, n_heads, n_kv, page_shift, stages, 0));
   if (n_splits > 1)
     DIS_CUDA_TRY(launch_k(attn_combine_kernel<D>, dim3(n_heads, T), dim3(D), 0, st, (const float *)scratch, out, n_splits, T, n_heads));
   return cudaSuccess;
@@ -584,7 +731,7 @@ cudaError_t make_kv_map(TmaMap *out, const uint16_t *pool, long long total_rows,
 static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const AttnRope &rope, const uint16_t *q,
                                  const int *page_table, int max_pages, const int *pt_row, const int *ctx, uint16_t *out,
                                  float *scratch, int n_splits, int T, int n_heads, int n_kv, int d, int page_size,
-                                 cudaStream_t st) {
+                                 int longest, cudaStream_t st) {
   if (T <= 0) return cudaSuccess;
   if (n_kv <= 0 || n_heads % n_kv != 0) { set_last_error("attn_paged: n_heads must be a multiple of n_kv"); return cudaErrorInvalidValue; }
   if (n_splits < 1 || (n_splits > 1 && !scratch)) { set_last_error("attn_paged: n_splits > 1 needs scratch"); return cudaErrorInvalidValue; }
@@ -596,7 +743,7 @@ static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const Att
 #define DIS_ATTN_CASE(DD, GG)                                                                                        \
   if (d == DD && G == GG)                                                                                            \
     return attn_launch<DD, GG>(kv_map, row0, rope, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, \
-                               n_heads, n_kv, page_shift, st);
+                               n_heads, n_kv, page_shift, longest, st);
   DIS_ATTN_CASE(128, 8) DIS_ATTN_CASE(128, 4) DIS_ATTN_CASE(128, 2) DIS_ATTN_CASE(128, 1)
   DIS_ATTN_CASE(64, 8) DIS_ATTN_CASE(64, 4) DIS_ATTN_CASE(64, 2) DIS_ATTN_CASE(64, 1)
 #undef DIS_ATTN_CASE
@@ -608,8 +755,10 @@ cudaError_t launch_attn_paged(const TmaMap &kv_map, long long row0, const uint16
                               int max_pages, const int *pt_row, const int *ctx, uint16_t *out, float *scratch,
                               int n_splits, int T, int n_heads, int n_kv, int d, int page_size, cudaStream_t st) {
   AttnRope none{};
+  // the page table's width bounds the histories
+  const int longest = (int)std::min<long long>((long long)max_pages * page_size, 1 << 30);
   return attn_dispatch(kv_map, row0, none, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
-                       page_size, st);
+                       page_size, longest, st);
 }
 
 // Decode step: RoPE + KV write of the step's new token (position ctx[t] - 1 == pos[t]) fused in.
@@ -617,10 +766,10 @@ cudaError_t launch_attn_decode_fused(const TmaMap &kv_map, long long row0, uint1
                                      int n_partial, long long partial_stride, const int *pos, const float *rope_cos,
                                      const float *rope_sin, const int *page_table, int max_pages, const int *pt_row,
                                      const int *ctx, uint16_t *out, float *scratch, int n_splits, int T, int n_heads,
-                                     int n_kv, int d, int page_size, cudaStream_t st) {
+                                     int n_kv, int d, int page_size, int longest, cudaStream_t st) {
   AttnRope r{qkv, n_partial, partial_stride, pos, rope_cos, rope_sin, kv_layer_base};
   return attn_dispatch(kv_map, row0, r, nullptr, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
-                       page_size, st);
+                       page_size, longest, st);
 }
 
 template <int D, int G>

@@ -151,21 +151,29 @@ bool &pdl_enabled();
 // are written once; false for a call of the C ABI, whose weight may be what the kernel in front of it writes.
 bool &pdl_weights_settled();
 
+// cluster > 1: clusters of that many CTAs along x (kernels with __cluster_dims__ carry their own size)
 template <class... KArgs, class... Args>
-cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+cudaError_t launch_k_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, int cluster, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
+  cfg.attrs = at;
   if (pdl_enabled()) {
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs++].val.clusterDim = {(unsigned)cluster, 1u, 1u};
   }
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <class... KArgs, class... Args>
+cudaError_t launch_k(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
+  return launch_k_cluster(kern, grid, block, smem, st, 1, args...);
 }
 
 // Gate activation of the products' epilogues, whose result is rounded to bf16 at once: kind 0 = silu(g) = g sigmoid(g), kind 1 =

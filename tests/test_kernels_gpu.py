@@ -349,6 +349,43 @@ def test_attention_full_size_against_torch():
         assert err <= 2 * BF16_ULP * ref.abs().max().item() + 1e-5, (splits, err)
 
 
+@pytest.mark.parametrize("nh,nkv,d,page_size", [(8, 2, 128, 64), (8, 1, 128, 16), (16, 2, 64, 128), (4, 2, 64, 8), (2, 2, 128, 64)])
+@pytest.mark.parametrize("T,n_splits,pattern", [(8, 1, "one-long"), (13, 1, "ragged"), (2, 1, "one-long"), (3, 1, "equal"), (5, 2, "ragged"), (3, 3, "one-long"),
+                                                (2, 4, "one-long"), (1, 5, "equal"), (3, 8, "ragged"), (2, 9, "ragged"), (9, 1, "tiles")])
+def test_attention_of_ragged_histories(nh, nkv, d, page_size, T, n_splits, pattern):
+    """Histories that a cluster of CTAs shares: one long beside short ones, tile edges, batches that leave a cluster part empty, with and
+    without slices, against float64 (weights and outputs in bf16: a relative error of 2^-9 each, 8e-3 of the 2-norm is four times that)."""
+    rng = np.random.default_rng(T * 100 + n_splits + d)
+    ctx = {"one-long": np.where(np.arange(T) == T // 2, 2500, rng.integers(1, 130, T)), "ragged": rng.integers(1, 1800, T), "equal": np.full(T, 1100),
+           "tiles": np.array([1, 63, 64, 65, 127, 128, 129, 1024, 1025])[:T]}[pattern].astype(np.int32)
+    need = [-(-int(c) // page_size) for c in ctx]
+    width = max(max(need), 1040 // page_size + 1)
+    table = np.zeros((T, width), np.int32)
+    order = rng.permutation(sum(need))
+    for t, at in enumerate(np.cumsum([0] + need[:-1])):
+        table[t, :need[t]] = order[at:at + need[t]]
+    g = torch.Generator(device=DEV); g.manual_seed(T + d)
+    pool = torch.randn((sum(need), 2, nkv, page_size, d), device=DEV, generator=g).to(torch.bfloat16)
+    q = (torch.randn((T, nh * d), device=DEV, generator=g) * 1.5).to(torch.bfloat16)
+    rows, dctx, dtab = dev_i32(np.arange(T, dtype=np.int32)), dev_i32(ctx), dev_i32(table)
+    scratch = torch.empty(max(1, lib().dis_k_attn_scratch_elems(T, nh, d, n_splits)), device=DEV)
+    outs = []
+    for _ in range(3):
+        out = torch.full((T, nh * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        check(lib().dis_k_attn_paged(ptr(q), ptr(pool), pool.shape[0], ptr(dtab), width, ptr(rows), ptr(dctx), ptr(out), ptr(scratch), n_splits, T, nh, nkv, d,
+                                     page_size, None))
+        outs.append(out)
+    sync()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])  # the same bits every time
+    for t in range(T):
+        kv = pool[torch.from_numpy(table[t, :need[t]].astype(np.int64)).to(DEV)].double()
+        k, v = (kv[:, c].permute(1, 0, 2, 3).reshape(nkv, -1, d)[:, :int(ctx[t])].repeat_interleave(nh // nkv, 0) for c in (0, 1))
+        w = torch.softmax((k @ q[t].double().view(nh, d, 1))[..., 0] * d ** -0.5, -1)
+        ref = (w[:, None] @ v)[:, 0].flatten()
+        err = (outs[0][t].double() - ref).norm() / ref.norm()
+        assert err <= 8e-3, (t, int(ctx[t]), float(err))
+
+
 def test_attention_long_context_tiles():
     rng = np.random.default_rng(3)
     d, nh, nkv, page_size = 128, 4, 1, 64
