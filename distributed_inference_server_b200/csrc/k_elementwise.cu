@@ -417,7 +417,7 @@ cudaError_t launch_sample(const float *logits, long long ld, int T, int V, const
                           cudaStream_t st) {
   if (T <= 0) return cudaSuccess;
   // A row that a cluster's registers hold takes the kernel that reads it once (k_sample.cu: 32 rows of 128256, three quarters
-  // of them sampled: 701 -> 42 us); longer rows walk through L2 here.
+  // of them sampled: 701 -> 25 us); longer rows walk through L2 here.
   if (V <= kSampleClusterMaxV)
     return launch_sample_cluster(logits, ld, T, V, temperature, top_p, seeds, steps, out_tokens, vocab_offset, out_val, out_sumexp,
                                  out_logprob, st);

@@ -778,6 +778,59 @@ def test_sampler_never_draws_a_masked_token(V, masked, calls):
         assert bool(torch.isfinite(lp).all())
 
 
+@pytest.mark.parametrize("kind,top_p", [("flat", 0.5), ("flat", 0.999), ("below 2^-30", 0.99997), ("below 2^-61", 0.99999988), ("one octave", 0.3), ("steps", 0.0),
+                                        ("steps", 1e-9), ("steps", 0.7), ("steps", 0.99999994)])
+def test_sampler_threshold_in_any_octave(kind, top_p):
+    """The threshold search over rows whose nucleus ends in the first octave, among equal weights, below 2^-30 of the largest weight (a
+    second search over the exponents) and nowhere (nothing below carries mass that fp32 sums see).  Draws with u close to 1 fall to the last kept tokens in index
+    order: they are compared, as running masses, with float64; what fp32 sums of V weights leave open is V^0.5 2^-24 of the mass, below
+    4e-5; where a tail of 7e-5 is looked at, its weights are added to a sum of about 1 and a share of them may be rounded off."""
+    V, T = 131072, 64
+    rng = np.random.default_rng(11)
+    lg = {"flat": np.zeros(V), "one octave": rng.uniform(-0.6, 0.0, V), "steps": -np.floor(np.arange(V) / 1024) * 0.31,
+          "below 2^-30": np.full(V, -21.5), "below 2^-61": np.full(V, -45.0)}[kind].astype(np.float32)
+    if kind.startswith("below"):
+        lg += rng.uniform(-0.5, 0.5, V).astype(np.float32)
+        lg[0] = 0.0
+    seeds, u = [], []
+    k = 0
+    while len(seeds) < T:
+        h = _draw_u(k)
+        if len(seeds) % 2 == 0 or h > 0.9999:
+            seeds.append(k)
+            u.append(h)
+        k += 1
+    ones, tps = dev_f32(np.ones(T)), dev_f32(np.full(T, top_p, np.float32))
+    ds, dst = torch.tensor(seeds, dtype=torch.int64, device=DEV), torch.zeros(T, dtype=torch.int64, device=DEV)
+    out, lp = G.zeros(T, dtype=torch.int32, device=DEV), G.zeros(T, dtype=torch.float32, device=DEV)
+    check(lib().dis_k_sample(ptr(dev_f32(lg)), 0, T, V, ptr(ones), ptr(tps), ptr(ds), ptr(dst), ptr(out), ptr(lp), None))  # (row stride 0: one row)
+    sync()
+    got = out.cpu().numpy()
+    p = np.exp(lg.astype(np.float64) - lg.max())
+    p /= p.sum()
+    order = np.sort(p)[::-1]
+    tp = float(np.float32(top_p))
+    tau = order[min(int((np.cumsum(order) < tp).sum()), V - 1)]
+    run = np.cumsum(np.where(p >= tau * (1 - 1e-6), p, 0.0))
+    for t in range(T):
+        at = run[got[t]] / run[-1]
+        before = (run[got[t]] - p[got[t]]) / run[-1]
+        if top_p <= 0:
+            assert got[t] == int(np.argmax(lg))
+        else:
+            assert before - 4e-5 <= u[t] <= at + 4e-5, (t, u[t], before, at)
+            assert p[got[t]] >= tau * (1 - 1e-3), (t, p[got[t]], tau)
+        assert abs(float(lp[t]) - np.log(p[got[t]])) <= 1e-4 * max(1.0, abs(np.log(p[got[t]])))
+
+
+def _draw_u(seed):
+    m = (1 << 64) - 1
+    z = (seed * 0x9E3779B97F4A7C15 + 0xC0FFEE * 0xD1B54A32D192ED03 + 0x632BE59BD9B4E019) & m
+    z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & m
+    z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & m
+    return ((z ^ (z >> 31)) >> 40) / 16777216.0
+
+
 @pytest.mark.parametrize("tp,T,V", [(1, 48, 4099), (1, 32, 128256), (2, 48, 4100), (3, 20, 4098), (4, 24, 128256), (8, 16, 128256)],
                          ids=["single-rank-ragged-vocab", "single-rank-llama3-vocab", "tp2-small-vocab", "tp3-small-vocab",
                               "tp4-llama3-vocab", "tp8-llama3-vocab"])
