@@ -474,6 +474,68 @@ def test_gemm_slice_count_of_zero(T, N, ok):
         assert not a.any()
 
 
+@pytest.mark.parametrize("nh,nkv,d,BT,page_size", [(32, 8, 128, 32, 64), (64, 8, 128, 16, 16), (32, 4, 64, 16, 8), (32, 8, 64, 32, 128), (16, 4, 128, 32, 32)])
+@pytest.mark.parametrize("kind", ["short", "long", "odd"])
+def test_attention_prefill_of_many_blocks(nh, nkv, d, BT, page_size, kind):
+    """Passes with more blocks than SMs, where a CTA takes pairs of blocks: many prompts of one to three blocks (pairs that are not of
+    one sequence), few long ones beside a portion far behind its cache, and blocks in odd lengths with empty ones between.
+    Eager twice and from a captured graph: the same bits.  Against float64 as in the tests of single blocks."""
+    g = torch.Generator(device=DEV); g.manual_seed(nh + d + page_size)
+    rng = np.random.default_rng(nh + d)
+    per_head = (3 if d == 128 else 6) * 148 // 2 // nkv + 1  # blocks from which pairs are taken
+    lens, past = [], []
+    while sum(-(-n // BT) for n in lens) < per_head + 3:
+        lens.append({"short": int(rng.integers(1, 3 * BT)), "long": int(rng.integers(17 * BT, 30 * BT)), "odd": int(rng.integers(1, 200))}[kind])
+        past.append(1500 if kind == "long" and len(lens) == 2 else int(rng.integers(0, 130)) if kind == "odd" else 0)
+    total = [a + b for a, b in zip(past, lens)]
+    per = [-(-n // page_size) for n in total]
+    perm = rng.permutation(sum(per)).astype(np.int32)
+    pt = np.zeros((len(lens), max(per)), np.int32)
+    for s, at in enumerate(np.cumsum([0] + per[:-1])):
+        pt[s, :per[s]] = perm[at:at + per[s]]
+    pool = torch.randn((sum(per), 2, nkv, page_size, d), device=DEV, generator=g)
+    for s, p in enumerate(per):  # keys grow with their position: the reference has to be raised
+        pool[torch.as_tensor(pt[s, :p].astype(np.int64), device=DEV), 0] *= 0.2 + torch.arange(p * page_size, device=DEV).reshape(p, 1, page_size, 1) / 200.0
+    pool = pool.to(torch.bfloat16)
+    tok0, qlen, pos0, ptrow, t = [], [], [], [], 0
+    for s, n in enumerate(lens):
+        p0 = 0
+        while p0 < n:
+            size = min(int(rng.integers(1, BT + 1)) if kind == "odd" else BT, n - p0)
+            tok0.append(t); qlen.append(size); pos0.append(past[s] + p0); ptrow.append(s); t += size; p0 += size
+            if kind == "odd" and rng.random() < 0.1:
+                tok0.append(t); qlen.append(0); pos0.append(past[s] + p0); ptrow.append(s)
+    assert len(tok0) * nkv > (3 if d == 128 else 6) * 74
+    q = torch.randn((t, nh * d), device=DEV, generator=g).to(torch.bfloat16)
+    args = [dev_i32(a) for a in (pt, tok0, qlen, pos0, ptrow)]
+
+    def run():
+        out = torch.full((t + 1, nh * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        check(lib().dis_k_attn_prefill(ptr(q), ptr(pool), pool.shape[0], ptr(args[0]), pt.shape[1], ptr(args[1]), ptr(args[2]), ptr(args[3]), ptr(args[4]),
+                                       ptr(out), len(tok0), nh, nkv, d, page_size, torch.cuda.current_stream().cuda_stream))
+        return out
+
+    outs = [run(), run()]
+    sync()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        outs.append(run())
+    graph.replay()
+    sync()
+    assert all(torch.equal(o[:t], outs[0][:t]) for o in outs) and bool(torch.isnan(outs[0][t]).all())
+    row = 0
+    for s, n in enumerate(lens):
+        kv = pool[torch.as_tensor(pt[s, :per[s]].astype(np.int64), device=DEV)].double()
+        K, V = (kv[:, c].permute(1, 0, 2, 3).reshape(nkv, -1, d)[:, :total[s]] for c in (0, 1))
+        qs = q[row:row + n].double().reshape(n, nkv, nh // nkv, d).permute(1, 2, 0, 3)
+        sc = qs @ K.transpose(1, 2).unsqueeze(1) / d ** 0.5
+        sc = sc.masked_fill(torch.arange(total[s], device=DEV)[None] > torch.arange(past[s], total[s], device=DEV)[:, None], float("-inf"))
+        ref = (torch.softmax(sc, dim=-1) @ V.unsqueeze(1)).permute(2, 0, 1, 3).reshape(n, nh * d)
+        err = (outs[0][row:row + n].double() - ref).abs().max().item()
+        assert err <= 2 * BF16_ULP * V.abs().max().item() + 1e-5, (s, n, err)
+        row += n
+
+
 @pytest.mark.parametrize("nh,nkv,page_size,BT", [(8, 1, 8, 16), (8, 2, 64, 16), (8, 2, 64, 32), (16, 2, 128, 16), (16, 4, 16, 32)])
 @pytest.mark.parametrize("past", [0, 63, 200])
 def test_attention_prefill_heads_of_64(nh, nkv, page_size, past, BT):
