@@ -127,8 +127,10 @@ int Engine::init(const dis_engine_config *c) {
   attn_scratch_elems = (size_t)(max_batch + 2 * kNumSMs + 64) * nh_l * (2 + m.head_dim);
   ENG_CUDA(dev_alloc(&attn_scratch, attn_scratch_elems, &bytes_allocated));
   // sampler output: [max_batch] token ids, then [max_batch] log-probabilities (fp32) -- one D2H copy per step
-  ENG_CUDA(dev_alloc(&d_out_tokens, (size_t)2 * max_batch, &bytes_allocated));
   ENG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h_out_tokens), (size_t)2 * max_batch * sizeof(uint32_t)));
+  // One GPU: the sampler writes ids and log-probabilities into the pinned block itself.  (The copy behind it took 6 us of every step.)
+  if (tp_size == 1) d_out_tokens = h_out_tokens;
+  else ENG_CUDA(dev_alloc(&d_out_tokens, (size_t)2 * max_batch, &bytes_allocated));
   if (tp_size > 1) {
     ENG_CUDA(dev_alloc(&ar_buf, cap * H, &bytes_allocated));
     ENG_CUDA(dev_alloc(&full_logits, (size_t)max_batch * m.vocab, &bytes_allocated));
@@ -345,7 +347,7 @@ Engine::~Engine() {
   for (int r = 0; r < kTpMaxRanks; r++) if (peer_base[r]) cudaIpcCloseMemHandle(peer_base[r]);
   void *ptrs[] = {embed, wqkv, wo, wgu, wdown, lm_head, attn_norm, mlp_norm, final_norm, x, partial, logits, ar_buf,
                   attn_scratch, full_logits, gather_buf, cand_val, cand_val_all, cand_tok, cand_tok_all, cand_sum, cand_sum_all, xn, q, attn,
-                  act, d_out_tokens, kv_pool, d_page_table, rope_cos, rope_sin, meta_dec.dev, meta_pre.dev, sym};
+                  act, d_out_tokens == h_out_tokens ? nullptr : d_out_tokens, kv_pool, d_page_table, rope_cos, rope_sin, meta_dec.dev, meta_pre.dev, sym};
   for (void *p : ptrs) if (p) cudaFree(p);
   if (h_out_tokens) cudaFreeHost(h_out_tokens);
   if (h_page_table) cudaFreeHost(h_page_table);
@@ -599,7 +601,27 @@ cudaError_t Engine::upload_step(int T, int R) {
   if (((++ar_step) & 0xFFFFFFu) == 0) ++ar_step;  // exchange epochs are (step << 8) + index: never 0, the value of an untouched flag
   cur_meta->h<uint32_t>(cur_meta->o_arstep)[0] = ar_step;
   ar_idx = 0;
+  if (cur_meta == &meta_dec) return cudaSuccess;  // the pass's first kernel reads it (enqueue_meta)
   return cudaMemcpyAsync(cur_meta->dev, cur_meta->host, cur_meta->bytes, cudaMemcpyHostToDevice, stream);
+}
+cudaError_t Engine::fetch_tokens(int rows) {
+  if (d_out_tokens == h_out_tokens) return cudaSuccess;
+  return cudaMemcpyAsync(h_out_tokens, d_out_tokens, (size_t)(max_batch + rows) * 4, cudaMemcpyDeviceToHost, stream);
+}
+
+// The small metadata block of a decode pass: a kernel in front of the others reads it from pinned memory, as a node of the captured pass.  As a
+// copy of its own it stood for a call of the host and 10 to 12 us between its end and the graph's first kernel.  The kernel behind it
+// is launched plainly: attention reads the block in front of its wait for the kernel before it, so it has to be whole before any other starts.
+__global__ void step_meta_kernel(const uint4 *__restrict__ host, uint4 *__restrict__ dev, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) dev[i] = host[i];
+}
+cudaError_t Engine::enqueue_meta() {
+  if (cur_meta != &meta_dec) return cudaSuccess;
+  const int n = (int)(meta_dec.bytes / 16);  // (sections are padded to 16 bytes)
+  step_meta_kernel<<<(n + 127) / 128, 128, 0, stream>>>(reinterpret_cast<const uint4 *>(meta_dec.host), reinterpret_cast<uint4 *>(meta_dec.dev), n);
+  kernel_launches++;
+  return cudaGetLastError();
 }
 
 int Engine::pick_attn_splits(int T, int max_ctx_in_batch) const {
@@ -694,10 +716,11 @@ cudaError_t Engine::enqueue_layers(int T, int n_splits) {
     }
     return cudaSuccess;
   };
+  RET_CUDA(enqueue_meta());
   for (int l = 0; l < m.layers; l++) {
     prof_mark(P_NORM);
     if (l == 0) {
-      pdl_enabled() = false;  // the step's first kernel follows a memcpy
+      pdl_enabled() = false;  // the step's first kernel follows its metadata
       RET_CUDA(launch_add_rmsnorm(x, tokens, embed, nullptr, 0, 0, attn_norm, xn, nullptr, T, H, m.rms_eps, stream));
       kernel_launches++;
     } else {
@@ -918,7 +941,7 @@ int Engine::prefill(int n, const int *slots, uint32_t *out_tokens, int *out_fini
     ENG_CUDA(enqueue_layers(T, 1));
     if (R > 0) {
       ENG_CUDA(enqueue_head(R, all_greedy));
-      ENG_CUDA(cudaMemcpyAsync(h_out_tokens, d_out_tokens, (size_t)(max_batch + R) * 4, cudaMemcpyDeviceToHost, stream));
+      ENG_CUDA(fetch_tokens(R));
     } else if (pend_needs_ar) {
       // A chunk that ends no prompt needs no logits, but its last exchange must still happen: the exchange buffers
       // alternate by the parity of the exchange index, which only lines up across forward passes if every pass
@@ -1055,7 +1078,7 @@ int Engine::step_mixed(int n, const int *slots, int max_prefill_tokens, uint32_t
   ENG_CUDA(enqueue_layers(T, 1));
   if (R > 0) {
     ENG_CUDA(enqueue_head(R, all_greedy));
-    ENG_CUDA(cudaMemcpyAsync(h_out_tokens, d_out_tokens, (size_t)(max_batch + R) * 4, cudaMemcpyDeviceToHost, stream));
+    ENG_CUDA(fetch_tokens(R));
   } else if (pend_needs_ar) {
     ENG_CUDA(consume_pending(final_norm, nullptr, T, T));  // keep the exchange count per pass even (see prefill)
   }
@@ -1195,7 +1218,7 @@ int Engine::decode(int n, const int *slots, uint32_t *out_tokens, int *out_finis
     last_graph = it->second;
     kernel_launches += graph_launches[key];
   }
-  ENG_CUDA(cudaMemcpyAsync(h_out_tokens, d_out_tokens, (size_t)(max_batch + T) * 4, cudaMemcpyDeviceToHost, stream));
+  ENG_CUDA(fetch_tokens(T));
   ENG_CUDA(cudaEventRecord(ev1, stream));
   ENG_CUDA(cudaEventSynchronize(ev1));
   float ms = 0.f;

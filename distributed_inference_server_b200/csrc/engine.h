@@ -221,6 +221,8 @@ struct Engine {
   bool ensure_pages(Sequence &s, int slot, int n_tokens);
   void release_pages(Sequence &s);
   cudaError_t upload_step(int T, int R);
+  cudaError_t enqueue_meta();
+  cudaError_t fetch_tokens(int rows);
   cudaError_t enqueue_layers(int T, int n_splits);
   cudaError_t enqueue_head(int R, bool all_greedy);
   cudaError_t linear_partial(const TmaMap *xmaps, const uint16_t *xptr, const TmaMap &wmap, const uint16_t *wptr,

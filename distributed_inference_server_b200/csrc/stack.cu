@@ -948,8 +948,8 @@ int Engine::init_stack(const dis_engine_config *c, const dis_stack_config *sc) {
       }
     }
   }
-  ENG_CUDA(alloc(reinterpret_cast<void **>(&M.d_out), (size_t)2 * M.max_rows * 4));
   ENG_CUDA(cudaMallocHost(reinterpret_cast<void **>(&M.h_out), (size_t)2 * M.max_rows * 4));
+  M.d_out = M.h_out;  // the sampler writes into the pinned block itself
   ENG_CUDA(stack_meta(meta_pre, cap_tokens, M.max_rows));
   ENG_CUDA(stack_meta(meta_dec, max_batch, M.max_rows));
   use_pdl = !(c->flags & DIS_FLAG_NO_PDL);
@@ -1230,7 +1230,7 @@ int Engine::stack_step(int n, const int *slots, int max_prefill_tokens, uint32_t
     ENG_CUDA(cudaMemcpyAsync(d_page_table, h_page_table, (size_t)max_batch * max_pages * sizeof(int), cudaMemcpyHostToDevice, stream));
     pt_dirty = false;
   }
-  ENG_CUDA(cudaMemcpyAsync(mt.dev, mt.host, mt.bytes, cudaMemcpyHostToDevice, stream));
+  if (&mt != &meta_dec) ENG_CUDA(cudaMemcpyAsync(mt.dev, mt.host, mt.bytes, cudaMemcpyHostToDevice, stream));  // (the small block: enqueue_meta)
   // latent attention: with few query blocks the history is cut into slices so that about two CTAs per SM run
   // (a windowed layer walks at most its window plus the block's own tokens)
   // keys of a slice: whole tiles of the kernel, as few as `want` slices (at most 64) of them need
@@ -1315,7 +1315,6 @@ int Engine::stack_step(int n, const int *slots, int max_prefill_tokens, uint32_t
       ENG_CUDA(cudaGraphLaunch(ex, stream));
     }
   }
-  if (R > 0) ENG_CUDA(cudaMemcpyAsync(M.h_out, M.d_out, (size_t)2 * M.max_rows * 4, cudaMemcpyDeviceToHost, stream));
   ENG_CUDA(cudaEventRecord(ev1, stream));
   ENG_CUDA(cudaEventSynchronize(ev1));
   float ms = 0.f;
@@ -1364,7 +1363,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   long long pend_stride = 0;
   const float *pend_bias = nullptr, *pend_src = nullptr;
   // Programmatic dependent launch: a kernel's CTAs are placed while the one before it drains and wait for its results in their
-  // first instruction (products fill their ring with weights before that).  The pass's first kernel follows a copy and stays plain.
+  // first instruction (products fill their ring with weights before that).  The pass's first kernel follows its metadata and stays plain.
   struct PdlOff { ~PdlOff() { pdl_enabled() = false; } } pdl_off;
   pdl_enabled() = false;
   auto plain = [](auto launch) { const bool on = pdl_enabled(); pdl_enabled() = false; const cudaError_t e = launch(); pdl_enabled() = on; return e; };
@@ -1420,6 +1419,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
   const void *ff_in = two_norms ? M.hc2 : M.hc;  // the feed-forward's input
   StackParBoundary pend_par;                      // parallel layers with two norms: what the next boundary joins
   const int n_streams = std::max(1, M.c.streams);
+  RET_CUDA(enqueue_meta());
   RET_CUDA(launch_stack_embed(M.embed.ptr, f32, sp.tokens, sp.pos, M.pos_freq, M.x, M.x0, M.c.embed_scale, T, W, n_streams, stream)); kl++;
   pdl_enabled() = use_pdl;
   const float *pend_y = nullptr, *pend_post = nullptr, *pend_post_b = nullptr;
