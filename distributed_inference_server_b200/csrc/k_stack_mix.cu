@@ -1132,6 +1132,146 @@ cudaError_t launch_stack_ssm_out(const float *o, const float *buf, long long ld_
              : ssm_out_go<false, false>(o, buf, ld_b, z, ld, D, w, parts, out, T, H, P, eps, st);
 }
 
+// ---- the three steps in one kernel, for passes of single tokens
+// Four kernels of a decode pass (slices of the input projection, convolution, recurrence, gated norm) move 8 MB of state and little else, and
+// took 14.6 us, each waiting for the one before and then for its own first loads.  Here a CTA has one (token, head), the heads of a norm's stretch
+// form a cluster, and whatever does not depend on this token -- state, convolution tails, weights -- is fetched in front of the wait for the
+// projection.  The stretch's mean square is the one thing that the CTAs exchange.  B and C of a group of heads are formed by each of
+// them; their tail moves on when all have read it.  32 heads of 128 x 64, 8 sequences: 14.6 -> 8.1 us.
+constexpr int kSsmStepMax = 128;  // most of N, P
+template <int KR, bool F32>
+__global__ void __launch_bounds__(256) stack_ssm_step_kernel(const float *__restrict__ proj, long long ld, int n_part, long long stride,
+                                                             const float *__restrict__ bias, int x_off, int dt_off, int C, int H, int taps,
+                                                             const float *__restrict__ cw, const float *__restrict__ cb,
+                                                             const float *__restrict__ vec, float *cstate, const int *__restrict__ slots,
+                                                             const int *__restrict__ poss, float *state, const float *__restrict__ w, int N, int P,
+                                                             int hpg, int hu, float eps, void *out) {
+  __shared__ __align__(16) float in[3 * kSsmStepMax], raw[3 * kSsmStepMax], part[4 * 256], zs[kSsmStepMax];  // in: x | B | C of this head
+  __shared__ float sh[32], sums[8], head[2];  // head: step size, decay
+  pdl_launch_dependents();
+  const int h = blockIdx.x, t = blockIdx.y, g = h / hpg, inner = H * P, tid = threadIdx.x;
+  const int slot = slots[t], pos = poss[t];  // (the pass's metadata is whole before any of its kernels starts)
+  // ---- what does not depend on this token
+  const int cols = P >> 2, rows = 256 / cols, col = tid % cols, row0 = tid / cols;  // this thread's state: rows row0 + k rows, columns 4 col ..
+  const bool mine = row0 < rows;
+  float4 *st = reinterpret_cast<float4 *>(state + ((long long)slot * H + h) * N * P);
+  float4 S[KR];
+#pragma unroll
+  for (int k = 0; k < KR; k++) {
+    const int r = row0 + k * rows;
+    S[k] = mine && r < N && pos > 0 ? st[(size_t)r * cols + col] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  // four neighbouring channels of x | B | C: where they are among the C channels of the convolution
+  const int n_ch = (P + 2 * N) >> 2, e = tid * 4;
+  const bool chan = tid < n_ch;
+  const int c = e < P ? h * P + e : e < P + N ? inner + g * N + (e - P) : inner + (H / hpg) * N + g * N + (e - P - N);
+  float *tail = cstate + (long long)slot * (taps - 1) * C + c;
+  auto past = [&](int j) {  // input `taps - 1 - j` tokens back
+    return pos - (taps - 1 - j) >= 0 ? *reinterpret_cast<const float4 *>(tail + (long long)j * C) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  float acc[4], wl[4];
+  if (chan) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) { acc[k] = cb[c + k]; wl[k] = cw[(long long)(c + k) * taps + taps - 1]; }
+    for (int j = 0; j + 1 < taps; j++) {
+      const float4 v = past(j);
+      const float vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; k++) acc[k] = fmaf(cw[(long long)(c + k) * taps + j], vv[k], acc[k]);
+    }
+  }
+  const float dt_bias = vec[h], a_log = vec[H + h], D = vec[2 * H + h], wj = tid < P ? w[h * P + tid] : 0.f;
+  pdl_wait();
+  // ---- the token's row of the projection, its slices added in order
+  const float *row = proj + (long long)t * ld;
+  if (chan) {
+    float4 v = bias ? *reinterpret_cast<const float4 *>(bias + x_off + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    each_slice<8>(0, n_part, [&](int k) { return *reinterpret_cast<const float4 *>(row + x_off + c + (long long)k * stride); },
+                  [&](float4 p) { v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w; });
+    const float vv[4] = {v.x, v.y, v.z, v.w};
+    *reinterpret_cast<float4 *>(raw + e) = v;
+#pragma unroll
+    for (int k = 0; k < 4; k++) in[e + k] = silu_(fmaf(wl[k], vv[k], acc[k]));
+  } else if (tid >= 128 && tid - 128 < P) {
+    const int i = h * P + tid - 128;
+    float v = bias ? bias[i] : 0.f;
+    each_slice<8>(0, n_part, [&](int k) { return row[i + (long long)k * stride]; }, [&](float p) { v += p; });
+    zs[tid - 128] = v;
+  }
+  if (tid == 127) {
+    float v = bias ? bias[dt_off + h] : 0.f;
+    each_slice<8>(0, n_part, [&](int k) { return row[dt_off + h + (long long)k * stride]; }, [&](float p) { v += p; });
+    const float z = v + dt_bias, dt = fmaxf(z, 0.f) + log1pf(expf(-fabsf(z)));
+    head[0] = dt;
+    head[1] = expf(-expf(a_log) * dt);
+  }
+  __syncthreads();
+  // ---- S = a S + B (dt x)^T, o = S^T C
+  const float dt = head[0], a = head[1];
+  if (mine) {
+    const float4 x = *reinterpret_cast<const float4 *>(in + 4 * col);
+    const float4 v = make_float4(x.x * dt, x.y * dt, x.z * dt, x.w * dt);
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < KR; k++) {
+      const int r = row0 + k * rows;
+      if (r < N) {
+        const float b = in[P + r], q = in[P + N + r];
+        S[k].x = fmaf(a, S[k].x, b * v.x); S[k].y = fmaf(a, S[k].y, b * v.y); S[k].z = fmaf(a, S[k].z, b * v.z); S[k].w = fmaf(a, S[k].w, b * v.w);
+        o.x = fmaf(S[k].x, q, o.x); o.y = fmaf(S[k].y, q, o.y); o.z = fmaf(S[k].z, q, o.z); o.w = fmaf(S[k].w, q, o.w);
+        st[(size_t)r * cols + col] = S[k];
+      }
+    }
+    *reinterpret_cast<float4 *>(part + row0 * P + 4 * col) = o;
+  }
+  __syncthreads();
+  float y = 0.f;
+  if (tid < P) {
+    float o = 0.f;
+    for (int r = 0; r < rows; r++) o += part[r * P + tid];
+    y = fmaf(D, in[tid], o) * silu_(zs[tid]);
+  }
+  // ---- the stretch's mean square, its heads' sums added in order
+  float total = block_sum(y * y, sh);
+  if (hu > 1) {
+    if (tid < hu) {
+      uint32_t at;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&sums[h % hu])), "r"(tid));
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(total) : "memory");
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    total = 0.f;
+    for (int r = 0; r < hu; r++) total += sums[r];
+  }
+  if (tid < P) st_el<F32>(out, (long long)t * inner + h * P + tid, y * rsqrtf(total / (float)(hu * P) + eps) * wj);
+  // ---- the tails move on: tail'[i] = tail[i + 1], then the token's input; B and C by the group's first head
+  if (chan && taps > 1 && (e < P || h % hpg == 0)) {
+    for (int j = 1; j + 1 < taps; j++) *reinterpret_cast<float4 *>(tail + (long long)(j - 1) * C) = past(j);
+    *reinterpret_cast<float4 *>(tail + (long long)(taps - 2) * C) = *reinterpret_cast<const float4 *>(raw + e);
+  }
+}
+
+// Passes of single tokens whose layout the kernel above takes: a norm's stretch is whole heads, at most eight (a cluster), and holds whole groups of
+// heads (a group's tail has one owner); sizes and rows in fours, up to 128.
+bool stack_ssm_step_ok(const float *proj, long long ld, const float *cstate, int x_off, int C, int taps, int H, int N, int P, int G, int parts) {
+  if (N > kSsmStepMax || P > kSsmStepMax || N % 4 || P % 4 || (H * P) % parts || taps < 1 || taps > kConvMaxTaps) return false;
+  const int per = H * P / parts;
+  if (per % P || per / P > 8 || (per / P) % (H / G) || H > (1 << 30) / P) return false;
+  return ld % 4 == 0 && x_off % 4 == 0 && C % 4 == 0 && reinterpret_cast<uintptr_t>(proj) % 16 == 0 && (taps == 1 || reinterpret_cast<uintptr_t>(cstate) % 16 == 0);
+}
+cudaError_t launch_stack_ssm_step(const float *proj, long long ld, int n_part, long long stride, const float *bias, int x_off, int dt_off, int C, int H, int taps,
+                                  const float *cw, const float *cb, const float *vec, float *cstate, const StackSpans &sp, float *state, const float *w, int N, int P,
+                                  int G, int parts, float eps, void *out, bool f32, cudaStream_t st) {
+  if (sp.T <= 0) return cudaSuccess;
+  const int hu = H / parts, rows = 256 / (P / 4);
+  auto go = [&](auto kern) {
+    return launch_k_cluster(kern, dim3(H, sp.T), dim3(256), 0, st, hu, proj, ld, n_part, stride, bias, x_off, dt_off, C, H, taps, cw, cb, vec, cstate, sp.slot, sp.pos,
+                            state, w, N, P, H / G, hu, eps, out);
+  };
+  if ((N + rows - 1) / rows <= 8) return f32 ? go(stack_ssm_step_kernel<8, true>) : go(stack_ssm_step_kernel<8, false>);
+  return f32 ? go(stack_ssm_step_kernel<16, true>) : go(stack_ssm_step_kernel<16, false>);
+}
+
 // out[t][off + h*dv + j] = scale * o[t][h][j] / rms(o[t][h]) * w[j] * silu(gate[t][h*dv + j]): the norm runs over one head's dv
 // outputs, its gain vector (null: ones) is shared by the heads.  One warp per (token, head).
 template <bool F32>

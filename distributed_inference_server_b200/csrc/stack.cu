@@ -1671,8 +1671,11 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
     void *ff_act = f32 ? (void *)(reinterpret_cast<float *>(M.act) + L.n_act) : (void *)(reinterpret_cast<uint16_t *>(M.act) + L.n_act);
     const float *in_bias = nullptr;  // minGRU adds its projections' biases itself when the product left them out
     const bool is_attn = lc.mixer == DIS_MIX_ATTENTION || lc.mixer == DIS_MIX_PARALLEL;
-    // the preparation kernels of attention (alone), latent attention and retention sum the slices of a split-K input projection themselves
-    const bool prep_sums = lc.mixer == DIS_MIX_ATTENTION || lc.mixer == DIS_MIX_LATENT || lc.mixer == DIS_MIX_RETENTION || lc.mixer == DIS_MIX_CHANNEL_DELTA;
+    // the preparation kernels of attention (alone), latent attention and retention, and the state-space mixer's step of single tokens, sum the
+    // slices of a split-K input projection themselves
+    const bool ssm_step = lc.mixer == DIS_MIX_SSM && T == sp.n_spans && par_ff == 0 &&
+                          stack_ssm_step_ok(M.proj, N, Rn.conv_state, L.x_off, L.conv_ch, lc.conv_taps, lc.heads, lc.ssm_state, lc.vdim, lc.ssm_groups, lc.ssm_norm_groups);
+    const bool prep_sums = ssm_step || lc.mixer == DIS_MIX_ATTENTION || lc.mixer == DIS_MIX_LATENT || lc.mixer == DIS_MIX_RETENTION || lc.mixer == DIS_MIX_CHANNEL_DELTA;
     if (split_in) RET_CUDA(glu_product(L.w_gu, par_ff, lc.mlp_act, ff_act, L.ld_act));
     RET_CUDA(gemm(M.hc, f32, W, L.w_in, 0, L.b_in.ptr ? reinterpret_cast<const float *>(L.b_in.ptr) : nullptr, M.proj, T, N, W, cap_tokens,
                   lc.mixer == DIS_MIX_MINGRU || is_attn ? &in_bias : nullptr, prep_sums));
@@ -1738,19 +1741,26 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
       const long long ld_b = C;  // x | B | C
       float *dtv = M.dec + (size_t)T * H;  // the step sizes follow the decays
       const float *vec = reinterpret_cast<const float *>(L.ssm_vec.ptr);
-      RET_CUDA(launch_stack_ssm_conv(M.proj, N, L.x_off, L.dt_off, C, H, lc.conv_taps, reinterpret_cast<const float *>(L.conv_w.ptr),
-                                     reinterpret_cast<const float *>(L.conv_b.ptr), vec, Rn.conv_state, sp, M.ssm, ld_b, M.dec, dtv, stream));
-      kl += lc.conv_taps > 1 && T != sp.n_spans ? 2 : 1;
-      const bool segments = M.light_seg && M.light_seg_a && Ns <= 128 && P <= 128 &&
-                            stack_lightning_segmented(sp.n_spans, T, H, max_span,
-                                                      stack_lightning_block(M.ssm, ld_b, inner + G * Ns, inner, 0, M.mix, M.light_seg, Ns, P));
-      RET_CUDA(launch_stack_ssd(M.ssm, ld_b, inner + G * Ns, inner, 0, H / G, M.dec, dtv, Rn.state, sp, M.mix, H, Ns, P, segments ? M.light_seg : nullptr,
-                                segments ? M.light_seg_a : nullptr, max_span, stream));
-      kl += segments ? 3 : 1;
-      RET_CUDA(launch_stack_ssm_out(M.mix, M.ssm, ld_b, M.proj, N, vec + 2 * H, reinterpret_cast<const float *>(L.norm_w.ptr), lc.ssm_norm_groups,
-                                    M.act, f32, T, H, P, eps, stream));
-      kl++;
       n_mix = inner;
+      if (ssm_step) {
+        RET_CUDA(launch_stack_ssm_step(in_src, N, in_parts, in_stride, in_bias, L.x_off, L.dt_off, C, H, lc.conv_taps, reinterpret_cast<const float *>(L.conv_w.ptr),
+                                       reinterpret_cast<const float *>(L.conv_b.ptr), vec, Rn.conv_state, sp, Rn.state, reinterpret_cast<const float *>(L.norm_w.ptr), Ns, P, G,
+                                       lc.ssm_norm_groups, eps, M.act, f32, stream));
+        kl++;
+      } else {
+        RET_CUDA(launch_stack_ssm_conv(M.proj, N, L.x_off, L.dt_off, C, H, lc.conv_taps, reinterpret_cast<const float *>(L.conv_w.ptr),
+                                       reinterpret_cast<const float *>(L.conv_b.ptr), vec, Rn.conv_state, sp, M.ssm, ld_b, M.dec, dtv, stream));
+        kl += lc.conv_taps > 1 && T != sp.n_spans ? 2 : 1;
+        const bool segments = M.light_seg && M.light_seg_a && Ns <= 128 && P <= 128 &&
+                              stack_lightning_segmented(sp.n_spans, T, H, max_span,
+                                                        stack_lightning_block(M.ssm, ld_b, inner + G * Ns, inner, 0, M.mix, M.light_seg, Ns, P));
+        RET_CUDA(launch_stack_ssd(M.ssm, ld_b, inner + G * Ns, inner, 0, H / G, M.dec, dtv, Rn.state, sp, M.mix, H, Ns, P, segments ? M.light_seg : nullptr,
+                                  segments ? M.light_seg_a : nullptr, max_span, stream));
+        kl += segments ? 3 : 1;
+        RET_CUDA(launch_stack_ssm_out(M.mix, M.ssm, ld_b, M.proj, N, vec + 2 * H, reinterpret_cast<const float *>(L.norm_w.ptr), lc.ssm_norm_groups,
+                                      M.act, f32, T, H, P, eps, stream));
+        kl++;
+      }
     } else if (lc.mixer == DIS_MIX_MINGRU) {
       int max_len = 0;
       for (auto &sh : stack_spans_h) max_len = std::max(max_len, sh.len);

@@ -220,6 +220,33 @@ def test_convolution_tail_in_prompts_and_single_tokens(name):
     e.close()
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("heads,vdim,state,groups,taps,norm_groups", [(8, 64, 128, 2, 4, 2), (8, 64, 128, 8, 4, 8), (2, 128, 128, 1, 7, 1), (8, 4, 4, 4, 1, 2), (6, 12, 20, 3, 2, 1),
+                                                                      (4, 8, 8, 1, 16, 2), (6, 36, 68, 6, 3, 3)])
+def test_single_tokens_in_one_kernel(dtype, heads, vdim, state, groups, taps, norm_groups):
+    """Passes of single tokens where the layout lets one kernel do convolution, recurrence and gated norm (a norm's stretch of one to six heads,
+    whole groups in it; sizes from 4 to 128, with threads that own nothing; up to 16 taps) and where a group spans two stretches (not
+    taken): after prompts, from a sequence's first token on, two sequences of unlike positions, a slot with an earlier owner, against the oracle."""
+    cfg = U.config([(U.ssm(heads=heads, vdim=vdim, state=state, groups=groups, conv=taps, norm_groups=norm_groups), None)], width=40)
+    W = U.weights(cfg, seed=6)
+    a, b, c = toks(26, seed=41), toks(21, seed=42), toks(18, seed=43)
+    wa, wb, wc = (U.oracle_logits(cfg, W, x) for x in (a, b, c))
+    e = U.engine(cfg, W, pool_tokens=256, page_size=8, max_batch=2, dtype=dtype)
+    ok = (lambda x, y: U.rel_err(x, y) < F32_TOL) if dtype == "float32" else U.bf16_close
+    f = U.Feeder(e)
+    f.step([("a", a, 6)])
+    for _ in range(3):
+        f.step([("a", a, 1), ("b", b, 1)])
+    f.step([("b", b, 1)])
+    for _ in range(17):
+        f.step([("a", a, 1), ("b", b, 1)])
+    assert ok(f.end("b"), wb) and ok(f.end("a"), wa)
+    for _ in range(18):
+        f.step([("c", c, 1)])
+    assert ok(f.end("c"), wc)
+    e.close()
+
+
 @pytest.mark.parametrize("force", ["1", "2"])
 def test_many_heads_and_sequences_walk_long_spans_whole(monkeypatch, force):
     """Four prompts of 100 tokens over 40 heads fill the GPU span by span, so the pass walks each span in one piece although
