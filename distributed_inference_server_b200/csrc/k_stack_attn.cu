@@ -487,12 +487,12 @@ __device__ __forceinline__ float ex2_(float x) {  // 2^x, flushing results below
 // tanh x = 1 - 2 / (1 + e^(2x)) is formed with one ex2 and one reciprocal (absolute error of the order of 1e-7, times the cap).
 // k0: index of the tile's first key in the walk `wk`; keep: positions below it are always visible.  DIST: the score is lowered by
 // slope2[e] per position of distance (slope in units of log 2).
-template <bool SIG, bool MASKED, bool DIST>
-__device__ __forceinline__ void attn_tile_weights(float (&sacc)[kMmKeys / 8][4], float (&mnew)[2], int k0, int qd, const int (&r_pos)[2],
+template <bool SIG, bool MASKED, bool DIST, int NJ>
+__device__ __forceinline__ void attn_tile_weights(float (&sacc)[NJ][4], float (&mnew)[2], int k0, int qd, const int (&r_pos)[2],
                                                   const int (&r_lo)[2], int k_end, const AttnWalk &wk, int keep, const float (&tmp_h)[2],
                                                   const float (&pb_h)[2], const float (&slope2)[2], float scale2, float cap2) {
 #pragma unroll
-  for (int j = 0; j < kMmKeys / 8; j++)
+  for (int j = 0; j < NJ; j++)
 #pragma unroll
     for (int q4 = 0; q4 < 4; q4++) {
       const int e = q4 >> 1;
@@ -537,7 +537,10 @@ struct AttnKV {
 // DIFF: two maps per head (StackAttn::maps).  Twice the warps: warp w and warp w + kMmWarps own the same rows, the first with map 1, the
 // second with map 2; a key row in shared memory holds both maps, the value rows are shared.  At the end the second map's outputs go
 // through shared memory to the warps of the first, which join, norm and store.  Slice records: maps of a head next to each other.
-template <int DQ, int DV, bool SIG, bool DIST, bool DIFF = false>
+// KS: blocks of at most 16 rows (single tokens), which leave three of four warps nothing to do as above: every warp takes the same rows and 16
+// of a tile's 64 keys, and the four states are joined at the end, a warp a quarter of the columns.  8 sequences of 50 to 80 keys, 8 / 2 heads of 128:
+// BEFOREAFTER.
+template <int DQ, int DV, bool SIG, bool DIST, bool DIFF = false, bool KS = false>
 __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 64 ? 1 : 2) : DQ > 128 ? 2 : 3) stack_attn_mma_kernel(const float *__restrict__ qf, long long ldq, AttnKV kv, const float *temp,
                                                                        const float *pb, const float *sink, StackAttn c, StackSpans sp, const int *qb_tok0,
                                                                        const int *qb_len, const int *page_table, int max_pages,
@@ -567,7 +570,9 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
   // columns d .. 16 nk16 of the K stages are read by the last k-step: zero them once (cp.async never touches them)
   if (d & 15)
     for (int i = threadIdx.x; i < 2 * kMmKeys * 8; i += blockDim.x) Ks[(i >> 3) * KP + krow_d + (i & 7)] = 0;
-  const int rwarp = DIFF ? warp & (kMmWarps - 1) : warp, map = DIFF ? warp / kMmWarps : 0;
+  const int rwarp = KS ? 0 : DIFF ? warp & (kMmWarps - 1) : warp, map = DIFF ? warp / kMmWarps : 0;
+  constexpr int NK = KS ? kMmKeys / kMmWarps : kMmKeys;  // keys of a tile that a warp takes, from kofs on
+  const int kofs = KS ? warp * NK : 0;
   // ---- this thread's rows: r0 = 16 rwarp + gid and r0 + 8
   int r_tok[2], r_head[2], r_pos[2], r_lo[2];
   bool r_ok[2];
@@ -602,7 +607,7 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
 #pragma unroll
   for (int j = 0; j < DV / 8; j++) { oacc[j][0] = oacc[j][1] = oacc[j][2] = oacc[j][3] = 0.f; }
   float mrow[2] = {-INFINITY, -INFINITY}, lrow[2] = {0.f, 0.f};
-  if (!SIG && sink && blockIdx.z == 0) {  // the sink term of the denominator enters as the initial state of the first slice (one lane of the four holds its 1)
+  if (!SIG && sink && blockIdx.z == 0 && (!KS || warp == 0)) {  // the sink term of the denominator enters as the initial state of the first slice (one lane of the four holds its 1)
 #pragma unroll
     for (int e = 0; e < 2; e++) { mrow[e] = sink[r_head[e]] * kLog2e; lrow[e] = qd == 0 ? 1.f : 0.f; }
   }
@@ -667,16 +672,16 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
       // S = Q K^T: k-steps outside, key tiles inside, so that consecutive products go to different accumulators; one ldmatrix
       // brings the fragments of two key tiles (lane l: matrix l / 8 = (tile, column half), row l % 8)
       const uint32_t kt = ks_base + (uint32_t)((stage * kMmKeys * KP + (DIFF ? map * d : 0)) * 2);
-      float sacc[kMmKeys / 8][4];
+      float sacc[NK / 8][4];
 #pragma unroll
-      for (int j = 0; j < kMmKeys / 8; j++) { sacc[j][0] = sacc[j][1] = sacc[j][2] = sacc[j][3] = 0.f; }
+      for (int j = 0; j < NK / 8; j++) { sacc[j][0] = sacc[j][1] = sacc[j][2] = sacc[j][3] = 0.f; }
 #pragma unroll
       for (int ks = 0; ks < DQ / 16; ks++) {
         if (ks < nk16) {
 #pragma unroll
-          for (int j = 0; j < kMmKeys / 8; j += 2) {
+          for (int j = 0; j < NK / 8; j += 2) {
             uint32_t b0, b1, b2, b3;
-            ldsm_x4(kt + (uint32_t)((((j + (lane >> 4)) * 8 + (lane & 7)) * KP + ks * 16 + ((lane >> 3) & 1) * 8) * 2), b0, b1, b2, b3);
+            ldsm_x4(kt + (uint32_t)(((kofs + (j + (lane >> 4)) * 8 + (lane & 7)) * KP + ks * 16 + ((lane >> 3) & 1) * 8) * 2), b0, b1, b2, b3);
             mma_bf16_16816(sacc[j], qa[ks], b0, b1);
             mma_bf16_16816(sacc[j + 1], qa[ks], b2, b3);
           }
@@ -686,8 +691,8 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
       // exponential is one ex2.  Only a tile that reaches past a row's position or the slice's end needs the mask.
       const bool masked = key_z > warp_first_pos || k0 + kMmKeys > k_end || key_a < warp_lo_max;
       float mnew[2] = {mrow[0], mrow[1]};
-      if (masked) attn_tile_weights<SIG, true, DIST>(sacc, mnew, k0, qd, r_pos, r_lo, k_end, wk, c.keep, tmp_h, pb_h, slope2, scale2, cap2);
-      else attn_tile_weights<SIG, false, DIST>(sacc, mnew, k0, qd, r_pos, r_lo, k_end, wk, c.keep, tmp_h, pb_h, slope2, scale2, cap2);
+      if (masked) attn_tile_weights<SIG, true, DIST>(sacc, mnew, k0 + kofs, qd, r_pos, r_lo, k_end, wk, c.keep, tmp_h, pb_h, slope2, scale2, cap2);
+      else attn_tile_weights<SIG, false, DIST>(sacc, mnew, k0 + kofs, qd, r_pos, r_lo, k_end, wk, c.keep, tmp_h, pb_h, slope2, scale2, cap2);
       if (!SIG) {
         float corr[2];
 #pragma unroll
@@ -700,7 +705,7 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
         }
         const float msub[2] = {mnew[0] == -INFINITY ? 0.f : mnew[0], mnew[1] == -INFINITY ? 0.f : mnew[1]};  // a row with nothing visible yet
 #pragma unroll
-        for (int j = 0; j < kMmKeys / 8; j++)
+        for (int j = 0; j < NK / 8; j++)
 #pragma unroll
           for (int q4 = 0; q4 < 4; q4++) {
             const int e = q4 >> 1;
@@ -714,7 +719,7 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
       // ---- O += P V
       const uint32_t vt = vs_base + (uint32_t)(stage * kMmKeys * VP * 2);
 #pragma unroll
-      for (int kk = 0; kk < kMmKeys / 16; kk++) {
+      for (int kk = 0; kk < NK / 16; kk++) {
         uint32_t pa[4];
         pa[0] = pack_bf16(sacc[2 * kk][0], sacc[2 * kk][1]);
         pa[1] = pack_bf16(sacc[2 * kk][2], sacc[2 * kk][3]);
@@ -725,7 +730,7 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
           if (j < nv8) {
             // lanes 0-15: keys 16 kk + lane of columns 8 j; lanes 16-31: the same keys of columns 8 (j + 1)
             uint32_t b0, b1, b2, b3;
-            ldsm_x4_trans(vt + (uint32_t)(((kk * 16 + (lane & 15)) * VP + (j + (lane >> 4)) * 8) * 2), b0, b1, b2, b3);
+            ldsm_x4_trans(vt + (uint32_t)(((kofs + kk * 16 + (lane & 15)) * VP + (j + (lane >> 4)) * 8) * 2), b0, b1, b2, b3);
             mma_bf16_16816(oacc[j], pa, b0, b1);
             mma_bf16_16816(oacc[j + 1], pa, b2, b3);
           }
@@ -739,6 +744,46 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
     for (int e = 0; e < 2; e++) {
       lrow[e] += __shfl_xor_sync(0xffffffffu, lrow[e], 1);
       lrow[e] += __shfl_xor_sync(0xffffffffu, lrow[e], 2);
+    }
+  }
+  constexpr int kOwn = KS ? DV / 8 / kMmWarps : DV / 8;  // n-tiles of the result that a warp stores
+  auto own = [&](int j) { return !KS || j / kOwn == warp; };
+  if constexpr (KS) {
+    float *os = reinterpret_cast<float *>(smem), *ms = os + kMmWarps * 16 * (DV + 4), *ls = ms + kMmWarps * 16;  // [warp][row][DV + 4], [warp][row]
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      const int row = warp * 16 + gid + e * 8;
+#pragma unroll
+      for (int j = 0; j < DV / 8; j++) *reinterpret_cast<float2 *>(os + row * (DV + 4) + j * 8 + qd * 2) = make_float2(oacc[j][e * 2], oacc[j][e * 2 + 1]);
+      if (qd == 0) { ms[row] = mrow[e]; ls[row] = lrow[e]; }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      float f[kMmWarps], mx = -INFINITY, l = 0.f;
+#pragma unroll
+      for (int w = 0; w < kMmWarps; w++) mx = fmaxf(mx, ms[w * 16 + gid + e * 8]);
+#pragma unroll
+      for (int w = 0; w < kMmWarps; w++) {
+        const float m = ms[w * 16 + gid + e * 8];
+        f[w] = SIG ? 1.f : m == -INFINITY ? 0.f : ex2_(m - mx);
+        l = fmaf(ls[w * 16 + gid + e * 8], f[w], l);
+      }
+      mrow[e] = mx;
+      lrow[e] = l;
+#pragma unroll
+      for (int j = 0; j < DV / 8; j++) {
+        if (!own(j)) continue;
+        float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int w = 0; w < kMmWarps; w++) {
+          const float2 v = *reinterpret_cast<const float2 *>(os + (w * 16 + gid + e * 8) * (DV + 4) + j * 8 + qd * 2);
+          a.x = fmaf(v.x, f[w], a.x);
+          a.y = fmaf(v.y, f[w], a.y);
+        }
+        oacc[j][e * 2] = a.x;
+        oacc[j][e * 2 + 1] = a.y;
+      }
     }
   }
   if (DIFF && !part) {  // (the last tile's barrier has passed: the stages are free)
@@ -817,8 +862,8 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
       float *rec = part + (((long long)blockIdx.z * sp.T + r_tok[e]) * c.H + r_head[e]) * (dv + 2) * (DIFF ? 2 : 1) + (DIFF ? map * (dv + 2) : 0);
 #pragma unroll
       for (int j = 0; j < DV / 8; j++)
-        if (j < nv8) { rec[j * 8 + qd * 2] = oacc[j][e * 2]; rec[j * 8 + qd * 2 + 1] = oacc[j][e * 2 + 1]; }
-      if (qd == 0) { rec[dv] = SIG ? 0.f : mrow[e] * kLn2; rec[dv + 1] = lrow[e]; }  // the maximum back in natural units
+        if (j < nv8 && own(j)) { rec[j * 8 + qd * 2] = oacc[j][e * 2]; rec[j * 8 + qd * 2 + 1] = oacc[j][e * 2 + 1]; }
+      if (qd == 0 && (!KS || warp == 0)) { rec[dv] = SIG ? 0.f : mrow[e] * kLn2; rec[dv + 1] = lrow[e]; }  // the maximum back in natural units
       continue;
     }
     const float inv = attn_out_factor(o, r_tok[e], r_head[e]) * (SIG ? 1.f : 1.f / lrow[e]);
@@ -826,7 +871,7 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
     const float *gr = o.gate_full ? o.gate_full + (long long)r_tok[e] * o.ldg + (long long)r_head[e] * dv + qd * 2 : nullptr;
 #pragma unroll
     for (int j = 0; j < DV / 8; j++)
-      if (j < nv8) {
+      if (j < nv8 && own(j)) {
         float a0 = oacc[j][e * 2] * inv, a1 = oacc[j][e * 2 + 1] * inv;
         if (gr) { a0 *= sigmoid_precise(gr[j * 8]); a1 *= sigmoid_precise(gr[j * 8 + 1]); }
         *reinterpret_cast<uint32_t *>(orow + j * 8 + qd * 2) = pack_bf16(a0, a1);
@@ -848,6 +893,12 @@ static cudaError_t attn_mma_go(const float *qf, long long ldq, const AttnKV &kv,
     allow(stack_attn_mma_kernel<128, 128, false, false>);
     allow(stack_attn_mma_kernel<128, 128, false, true>);
     allow(stack_attn_mma_kernel<192, 128, false, false>);
+    allow(stack_attn_mma_kernel<64, 64, true, false, false, true>);
+    allow(stack_attn_mma_kernel<64, 64, false, false, false, true>);
+    allow(stack_attn_mma_kernel<64, 64, false, true, false, true>);
+    allow(stack_attn_mma_kernel<128, 128, true, false, false, true>);
+    allow(stack_attn_mma_kernel<128, 128, false, false, false, true>);
+    allow(stack_attn_mma_kernel<128, 128, false, true, false, true>);
     allow(stack_attn_mma_kernel<64, 64, false, false, true>);
     allow(stack_attn_mma_kernel<64, 128, false, false, true>);
     allow(stack_attn_mma_kernel<128, 128, false, false, true>);
@@ -870,15 +921,21 @@ static cudaError_t attn_mma_go(const float *qf, long long ldq, const AttnKV &kv,
   }
   if (c.d > dq || c.dv > dvp || (dq == 192 && (sig || dist))) return cudaErrorInvalidValue;
   const size_t shm = (size_t)2 * kMmKeys * (dq + dvp + 16) * sizeof(uint16_t);
+  // every span one token: a block's rows are the heads of a group (rotating values back needs whole rows in a warp)
+  const bool ks = sp.T == sp.n_spans && c.H / c.G <= 16 && dq <= 128 && (part || !o.vrot);
 #define DIS_ATTN_MMA(Q, V, S, B) \
-  launch_k(stack_attn_mma_kernel<Q, V, S, B>, dim3(grid), dim3(kMmWarps * 32), (size_t)(shm), st, qf, ldq, kv, temp, pb, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
-  if (dq == 192) DIS_ATTN_MMA(192, 128, false, false);
-  else if (small && sig) DIS_ATTN_MMA(64, 64, true, false);
-  else if (small && dist) DIS_ATTN_MMA(64, 64, false, true);
-  else if (small) DIS_ATTN_MMA(64, 64, false, false);
-  else if (sig) DIS_ATTN_MMA(128, 128, true, false);
-  else if (dist) DIS_ATTN_MMA(128, 128, false, true);
-  else DIS_ATTN_MMA(128, 128, false, false);
+  if (ks) DIS_ATTN_MMA_(Q, V, S, B, true); \
+  else DIS_ATTN_MMA_(Q, V, S, B, false)
+#define DIS_ATTN_MMA_(Q, V, S, B, K) \
+  launch_k(stack_attn_mma_kernel<Q, V, S, B, false, K>, dim3(grid), dim3(kMmWarps * 32), (size_t)(shm), st, qf, ldq, kv, temp, pb, sink, c, sp, qb_tok0, qb_len, page_table, max_pages, page_size, o, keys_per_split, part)
+  if (dq == 192) { DIS_ATTN_MMA_(192, 128, false, false, false); }
+  else if (small && sig) { DIS_ATTN_MMA(64, 64, true, false); }
+  else if (small && dist) { DIS_ATTN_MMA(64, 64, false, true); }
+  else if (small) { DIS_ATTN_MMA(64, 64, false, false); }
+  else if (sig) { DIS_ATTN_MMA(128, 128, true, false); }
+  else if (dist) { DIS_ATTN_MMA(128, 128, false, true); }
+  else { DIS_ATTN_MMA(128, 128, false, false); }
+#undef DIS_ATTN_MMA_
 #undef DIS_ATTN_MMA
   return cudaGetLastError();
 }
