@@ -434,6 +434,14 @@ __global__ void __launch_bounds__(256, 2) stack_light_contrib_kernel(const float
   }
 }
 
+// 16 bytes to shared memory
+__device__ __forceinline__ void light_cp16(float *dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// The incoming state (64 KB of a head of 128 x 128) is the largest input: it comes through shared memory in three chunks under way together, in
+// the room that keys and D take later, while keys and values wait in registers.  (Read from global memory by the thread that multiplies,
+// sixteen times per CTA through L1 and with four loads in flight, it held the kernel at 160 us, a quarter of the fp32 rate.)
+constexpr int kLightChunk = 32;  // rows of the state per chunk
 template <int DT, int DVT, int GATE>
 __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float *__restrict__ proj, long long ld, LightCols col, const float *decay,
                                                                     const float *__restrict__ dec, float qscale, StackSpans sp,
@@ -444,26 +452,92 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
   extern __shared__ __align__(16) float shm[];
   constexpr int kKv = DT * kLbLd > kLightSeg * DVT ? DT * kLbLd : kLightSeg * DVT;
   float *qt = shm, *kv = qt + DT * kLbLd, *at = kv + kKv, *as = at + kLightSeg * kLbLd, *ci = as + kLightSeg;  // [c][tok], [c][tok] then [tok][DVT], [j][i], [tok], [tok]
+  constexpr int kChunkFloats = kLightChunk * DVT, kBufs = (kKv + kLightSeg * kLbLd) / kChunkFloats < 3 ? (kKv + kLightSeg * kLbLd) / kChunkFloats : 3;
+  static_assert(kBufs >= 2, "chunks of the state lie where keys and D go");
   int h;
   LightSpanSeg g;
   if (!light_segment(sp, max_seg, H, h, g)) return;
-  const int tid = threadIdx.x, dv4 = dv >> 2;
+  const int tid = threadIdx.x, dv4 = dv >> 2, n_chunks = (d + kLightChunk - 1) / kLightChunk;
+  const float *sg = seg + g.at * d * dv;
+  auto fetch = [&](int ch) {  // rows of dv floats, one behind the other as they are in memory
+    if (ch < n_chunks) {
+      const int n4 = min(kLightChunk, d - ch * kLightChunk) * dv4;
+      float *dst = kv + (ch % kBufs) * kChunkFloats;
+      const float *src = sg + (size_t)ch * kLightChunk * dv;
+      for (int e = tid; e < n4; e += 256) light_cp16(dst + 4 * e, src + 4 * e);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int ch = 0; ch < kBufs; ch++) fetch(ch);
   if (tid < kLightSeg) as[tid] = tid < g.n ? (GATE == 2 ? dec[(long long)(g.first + tid) * H + h] : decay[h]) : 1.f;
   const float *qp = proj + col.q + (long long)(h / col.hpg) * d, *kp = proj + col.k + (long long)(h / col.hpg) * d, *vp = proj + col.v + (long long)h * dv;
-  {
-    const int t = tid & (kLightSeg - 1);
-    const long long row = (long long)(g.first + t) * ld;
-    for (int c = (tid >> 6) * 4; c < d; c += 16) {  // lanes are tokens: the transposed writes hit different banks
-      float4 q = make_float4(0.f, 0.f, 0.f, 0.f), k = q;
-      if (t < g.n) {
-        q = light_in<GATE>(*reinterpret_cast<const float4 *>(qp + row + c), qscale);
-        k = light_in<GATE>(*reinterpret_cast<const float4 *>(kp + row + c), 1.f);
+  const int t_own = tid & (kLightSeg - 1), c_own = (tid >> 6) * 4;  // lanes are tokens: the transposed writes hit different banks
+  const long long row = (long long)(g.first + t_own) * ld;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  float4 hold[DT / 16];  // this thread's share of the keys, then of the values
+#pragma unroll
+  for (int i = 0; i < DT / 16; i++) {
+    const int c = c_own + 16 * i;
+    hold[i] = zero;
+    if (c < d) {
+      float4 q = zero;
+      if (t_own < g.n) {
+        q = *reinterpret_cast<const float4 *>(qp + row + c);
+        hold[i] = *reinterpret_cast<const float4 *>(kp + row + c);
+        q = light_in<GATE>(q, qscale);
       }
-      qt[(c + 0) * kLbLd + t] = q.x; qt[(c + 1) * kLbLd + t] = q.y; qt[(c + 2) * kLbLd + t] = q.z; qt[(c + 3) * kLbLd + t] = q.w;
-      kv[(c + 0) * kLbLd + t] = k.x; kv[(c + 1) * kLbLd + t] = k.y; kv[(c + 2) * kLbLd + t] = k.z; kv[(c + 3) * kLbLd + t] = k.w;
+      qt[(c + 0) * kLbLd + t_own] = q.x; qt[(c + 1) * kLbLd + t_own] = q.y; qt[(c + 2) * kLbLd + t_own] = q.z; qt[(c + 3) * kLbLd + t_own] = q.w;
     }
   }
-  __syncthreads();
+  const int i0 = (tid >> 4) * 4, tj = (tid & 15) * 4;
+  constexpr int RJ = DVT / 16;
+  float acc[4][RJ];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < RJ; j++) acc[i][j] = 0.f;
+  bool in[RJ / 4];
+#pragma unroll
+  for (int j = 0; j < RJ / 4; j++) in[j] = tj + j * 64 < dv;
+  // ---- q_i S_in
+  for (int ch = 0; ch < n_chunks; ch++) {
+    if (kBufs == 3) asm volatile("cp.async.wait_group 2;" ::: "memory"); else asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const float *sc = kv + (ch % kBufs) * kChunkFloats;
+    const int c0 = ch * kLightChunk, n = min(kLightChunk, d - c0);
+#pragma unroll 4
+    for (int c = 0; c < n; c++) {
+      const float4 q = *reinterpret_cast<const float4 *>(qt + (c0 + c) * kLbLd + i0);
+      const float qv[4] = {q.x, q.y, q.z, q.w};
+      float s[RJ];
+#pragma unroll
+      for (int j = 0; j < RJ; j += 4) *reinterpret_cast<float4 *>(s + j) = in[j / 4] ? *reinterpret_cast<const float4 *>(sc + c * dv + tj + j * 16) : zero;
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(qv[i], s[j], acc[i][j]);
+    }
+    __syncthreads();
+    fetch(ch + kBufs);
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  // ---- keys out of the registers, D, values on their way
+#pragma unroll
+  for (int i = 0; i < DT / 16; i++) {
+    const int c = c_own + 16 * i;
+    if (c < d) {
+      const float4 k = light_in<GATE>(hold[i], 1.f);
+      kv[(c + 0) * kLbLd + t_own] = k.x; kv[(c + 1) * kLbLd + t_own] = k.y; kv[(c + 2) * kLbLd + t_own] = k.z; kv[(c + 3) * kLbLd + t_own] = k.w;
+    }
+  }
+  constexpr int NV = kLightSeg * DVT / 4 / 256;
+  float4 vals[NV];
+#pragma unroll
+  for (int i = 0; i < NV; i++) {
+    const int e = tid + 256 * i, t = e / dv4;
+    vals[i] = e < g.n * dv4 ? *reinterpret_cast<const float4 *>(vp + (long long)(g.first + t) * ld + (e - t * dv4) * 4) : zero;
+  }
   if (tid < kLightSeg) {  // thread j: D_ij times the factor on value j, zero above the diagonal
     const float f = GATE == 2 && tid < g.n ? col.vscale[(long long)(g.first + tid) * H + h] : 1.f;
     float p = 1.f;
@@ -475,7 +549,14 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
     float p = 1.f;
     for (int i = 0; i < kLightSeg; i++) { p *= as[i]; ci[i] = p; }
   }
-  const int i0 = (tid >> 4) * 4, tj = (tid & 15) * 4;
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const float f = ci[i0 + i];
+#pragma unroll
+    for (int j = 0; j < RJ; j++) acc[i][j] *= f;
+  }
+  // ---- q_i k_j
   float a[4][4];
 #pragma unroll
   for (int i = 0; i < 4; i++)
@@ -492,7 +573,7 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
         for (int j = 0; j < 4; j++) a[i][j] = fmaf(qv[i], kw[j], a[i][j]);
     }
   }
-  __syncthreads();  // D is complete and the keys are no longer needed
+  __syncthreads();  // the keys are no longer needed
   // Above the diagonal nothing is multiplied, here and with the values below: zero times a key or value that is not finite would carry a
   // later token into an earlier one's output.
 #pragma unroll
@@ -502,38 +583,10 @@ __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float 
     const int rest = tj + j - i0;  // rows below this one of the four see nothing of token tj + j
     *p = make_float4(rest > 0 ? 0.f : f.x * a[0][j], rest > 1 ? 0.f : f.y * a[1][j], rest > 2 ? 0.f : f.z * a[2][j], rest > 3 ? 0.f : f.w * a[3][j]);
   }
-  for (int e = tid; e < g.n * dv4; e += 256) {
-    const int t = e / dv4, c = (e - t * dv4) * 4;
-    *reinterpret_cast<float4 *>(kv + t * DVT + c) = light_in<GATE>(*reinterpret_cast<const float4 *>(vp + (long long)(g.first + t) * ld + c), 1.f);
-  }
-  constexpr int RJ = DVT / 16;
-  float acc[4][RJ];
 #pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < RJ; j++) acc[i][j] = 0.f;
-  const float *sg = seg + g.at * d * dv;
-  bool in[RJ / 4];
-#pragma unroll
-  for (int j = 0; j < RJ / 4; j++) in[j] = tj + j * 64 < dv;
-#pragma unroll 4
-  for (int c = 0; c < d; c++) {
-    const float4 q = *reinterpret_cast<const float4 *>(qt + c * kLbLd + i0);
-    const float qv[4] = {q.x, q.y, q.z, q.w};
-    float s[RJ];
-#pragma unroll
-    for (int j = 0; j < RJ; j += 4)
-      *reinterpret_cast<float4 *>(s + j) = in[j / 4] ? *reinterpret_cast<const float4 *>(sg + (size_t)c * dv + tj + j * 16) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < RJ; j++) acc[i][j] = fmaf(qv[i], s[j], acc[i][j]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const float f = ci[i0 + i];
-#pragma unroll
-    for (int j = 0; j < RJ; j++) acc[i][j] *= f;
+  for (int i = 0; i < NV; i++) {
+    const int e = tid + 256 * i, t = e / dv4;
+    if (e < g.n * dv4) *reinterpret_cast<float4 *>(kv + t * DVT + (e - t * dv4) * 4) = light_in<GATE>(vals[i], 1.f);
   }
   __syncthreads();
   auto add_token = [&](int t, int first) {  // rows first .. 3 see token t
