@@ -338,7 +338,7 @@ __global__ void stack_lightning_carry_kernel(const float *decay, const float *se
 //                                                                                                  64 (d + dv/2) + d dv per token
 // with both operands of an outer product in registers (8 x 8 or 4 x 8 results per thread).  The decays' products are formed by
 // multiplication, never as quotients or exponentials, so a decay of zero needs no care.
-// Retention, 8 heads of 128 x 128, 6554 tokens of eight spans: contributions 161 -> 55 us, outputs 213 -> 160 us.
+// Retention, 8 heads of 128 x 128, 6554 tokens of eight spans: contributions 161 -> 55 us, outputs 213 -> 160, and 119 with the state staged.
 constexpr int kLbLd = kLightSeg + 4;  // tokens of a transposed row, padded: float4 rows that start on different banks
 
 struct LightSpanSeg { int first, n; size_t at; };
@@ -440,7 +440,8 @@ __device__ __forceinline__ void light_cp16(float *dst, const float *src) {
 }
 // The incoming state (64 KB of a head of 128 x 128) is the largest input: it comes through shared memory in three chunks under way together, in
 // the room that keys and D take later, while keys and values wait in registers.  (Read from global memory by the thread that multiplies,
-// sixteen times per CTA through L1 and with four loads in flight, it held the kernel at 160 us, a quarter of the fp32 rate.)
+// sixteen times per CTA through L1 and with four loads in flight, it held the kernel at 160 us, a quarter of the fp32 rate; now 119.  Two chunks
+// instead of three, with D formed in front of them and only the tiles below the diagonal multiplied: 131, the registers of the queries on top.)
 constexpr int kLightChunk = 32;  // rows of the state per chunk
 template <int DT, int DVT, int GATE>
 __global__ void __launch_bounds__(256, 2) stack_light_output_kernel(const float *__restrict__ proj, long long ld, LightCols col, const float *decay,
