@@ -194,14 +194,17 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     return at + min(n, (r % n_splits) * ((n + n_splits - 1) / n_splits));
   };
   const int lo = bound(rank), hi = bound(rank + 1);
-  // f(history, first tile, end tile, tiles of the history) for every piece in [lo, hi)
+  // f(history, first tile, end tile, tiles of the history) for every piece in [lo, hi); an empty history counts as a tile above, so that it has a
+  // CTA, and as none here: nothing is fetched for it
   auto for_pieces = [&](auto f) {
     if constexpr (!kShared) {
-      f(0, lo, hi, total);  // (an empty slice writes an empty state)
+      const bool some = ctx_0 > 0;
+      f(0, some ? lo : 0, some ? hi : 0, some ? total : 0);  // (an empty slice writes an empty state)
     } else {
       for (int i = 0, at = 0; i < count && at < hi; i++) {
         const int n = tiles_of(i);
-        if (at + n > lo && hi > lo) f(i, max(lo - at, 0), min(hi - at, n), n);
+        const bool some = s_ctx[i] > 0;
+        if (at + n > lo && hi > lo) f(i, some ? max(lo - at, 0) : 0, some ? min(hi - at, n) : 0, some ? n : 0);
         at += n;
       }
     }
