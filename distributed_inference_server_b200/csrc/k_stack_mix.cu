@@ -1202,6 +1202,7 @@ __global__ void __launch_bounds__(256) stack_ssm_step_kernel(const float *__rest
                                                              int hpg, int hu, float eps, void *out) {
   __shared__ __align__(16) float in[3 * kSsmStepMax], raw[3 * kSsmStepMax], part[4 * 256], zs[kSsmStepMax];  // in: x | B | C of this head
   __shared__ float sh[32], sums[8], head[2];  // head: step size, decay
+  if (hu > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (the wait: in front of the stores to the others' shared memory)
   pdl_launch_dependents();
   const int h = blockIdx.x, t = blockIdx.y, g = h / hpg, inner = H * P, tid = threadIdx.x;
   const int slot = slots[t], pos = poss[t];  // (the pass's metadata is whole before any of its kernels starts)
@@ -1288,6 +1289,7 @@ __global__ void __launch_bounds__(256) stack_ssm_step_kernel(const float *__rest
   // ---- the stretch's mean square, its heads' sums added in order
   float total = block_sum(y * y, sh);
   if (hu > 1) {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");  // every CTA of the cluster is running: its shared memory may be written from now on
     if (tid < hu) {
       uint32_t at;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_u32(&sums[h % hu])), "r"(tid));

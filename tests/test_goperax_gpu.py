@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from distributed_inference_server_b200 import ContinuousBatcher, InferenceParams, models
+from distributed_inference_server_b200 import binding as B
 from tests import _goperax_util as U
 from tests import goperax_oracle as GO
 
@@ -244,6 +245,28 @@ def test_single_tokens_in_one_kernel(dtype, heads, vdim, state, groups, taps, no
     for _ in range(18):
         f.step([("c", c, 1)])
     assert ok(f.end("c"), wc)
+    e.close()
+
+
+@pytest.mark.parametrize("width,heads,vdim,state,groups,taps,norm_groups", [(512, 8, 64, 128, 2, 4, 2), (512, 8, 64, 128, 8, 4, 8), (1024, 16, 32, 64, 2, 4, 2)])
+def test_single_tokens_sum_the_slices_of_a_wide_projection(width, heads, vdim, state, groups, taps, norm_groups):
+    """The same kernel where the input projection is cut along K, as it is from a width of 512 on: channels, gate and step size are summed over
+    two to four slices.  A norm's stretch of four, one and eight heads (a cluster each), one and two sequences, against the oracle."""
+    rows = 2 * heads * vdim + 2 * groups * state + heads
+    slices = {T: B.load().dis_k_gemm_pick_split(T, rows, width) for T in (1, 2)}
+    assert min(slices.values()) >= 2
+    cfg = U.config([(U.ssm(heads=heads, vdim=vdim, state=state, groups=groups, conv=taps, norm_groups=norm_groups), None)], width=width)
+    W = U.weights(cfg, seed=7)
+    a, b = toks(24, seed=44), toks(15, seed=45)
+    wa, wb = U.oracle_logits(cfg, W, a), U.oracle_logits(cfg, W, b)
+    e = U.engine(cfg, W, "bfloat16", pool_tokens=128, page_size=8, max_batch=2)
+    f = U.Feeder(e)
+    f.step([("a", a, 5)])
+    for _ in range(4):
+        f.step([("a", a, 1)])
+    for _ in range(15):
+        f.step([("a", a, 1), ("b", b, 1)])
+    assert U.bf16_close(f.end("b"), wb) and U.bf16_close(f.end("a"), wa)
     e.close()
 
 

@@ -41,3 +41,19 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_may_start():
         barrier = body.find("__syncthreads()", alloc.end())
         assert 0 <= barrier < trigger, f"{name}: the trigger stands in front of the barrier that follows the allocation"
     assert seen >= 3
+
+
+def test_shared_memory_of_other_ctas_is_written_only_when_they_run():
+    """CTAs of a cluster are placed together, but only a cluster barrier says that the others have begun: it stands in front of the first
+    store into their shared memory (st.shared::cluster, by itself or in a helper)."""
+    store = re.compile(r"st\.shared::cluster|\bst_cluster\s*\(|\bswap\s*\(\s*s\b")
+    waits = re.compile(r"barrier\.cluster\.wait|\bcluster_wait\s*\(|\bcluster_sync(_all)?\s*\(")
+    seen = 0
+    for name, body in kernels():
+        first = store.search(body)
+        if first is None:
+            continue
+        seen += 1
+        wait = waits.search(body)
+        assert wait is not None and wait.start() < first.start(), f"{name}: stores into another CTA's shared memory before it is known to run"
+    assert seen >= 2
