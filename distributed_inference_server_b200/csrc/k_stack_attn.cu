@@ -567,8 +567,9 @@ __global__ void __launch_bounds__(kMmWarps * 32 * (DIFF ? 2 : 1), DIFF ? (DQ > 6
   constexpr int NTR = DIFF ? 4 : 2;  // threads that copy a key row
   const int krow_d = DIFF ? 2 * d : d;
   const int nk16 = (d + 15) >> 4, nv8 = dv >> 3, dc = krow_d >> 3, vc = dv >> 3;  // k-steps of Q K^T, n-tiles of P V, 16-byte chunks per row
-  // columns d .. 16 nk16 of the K stages are read by the last k-step: zero them once (cp.async never touches them)
-  if (d & 15)
+  // columns d .. 16 nk16 of the K stages are read by the last k-step: zero them once (cp.async never touches them).  Only where a tile follows,
+  // whose barrier orders them: an empty slice has none, and the join of KS lays its states over the stages.
+  if ((d & 15) && k_end > k_begin)
     for (int i = threadIdx.x; i < 2 * kMmKeys * 8; i += blockDim.x) Ks[(i >> 3) * KP + krow_d + (i & 7)] = 0;
   const int rwarp = KS ? 0 : DIFF ? warp & (kMmWarps - 1) : warp, map = DIFF ? warp / kMmWarps : 0;
   constexpr int NK = KS ? kMmKeys / kMmWarps : kMmKeys;  // keys of a tile that a warp takes, from kofs on

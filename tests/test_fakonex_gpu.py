@@ -161,6 +161,32 @@ def test_attention_over_slices_of_the_history():
         assert U.rel_err(got, want) < F32_TOL if dtype == "float32" else U.bf16_close(got, want)
 
 
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim", [(2, 1, 72, 80), (6, 1, 24, 32), (4, 2, 120, 128), (4, 2, 16, 16)])
+def test_ragged_single_tokens_over_slices(heads, kv_heads, dim, vdim):
+    """Single tokens in a batch that is cut into slices for its longest history: a short history leaves most slices without a key, and head
+    sizes of 8 above a multiple of 16 have columns of zeros in the key tiles, in whose place an empty slice's state is joined.  The lengths cross
+    a tile's edge; a sequence starts from nothing beside them.  Against the oracle, and the same bits in a second engine."""
+    cfg = U.config([(U.attention(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, chunk=0), None)], width=40)
+    W = U.weights(cfg, seed=16)
+    a, b, c = toks(680, seed=6), toks(75, seed=7), toks(12, seed=8)
+    wa, wb, wc = (U.oracle_logits(cfg, W, t) for t in (a, b, c))
+    runs = []
+    for _ in range(2):
+        e = U.engine(cfg, W, "bfloat16", max_batch=3, pool_tokens=896, page_size=16)
+        f = U.Feeder(e)
+        f.step([("a", a, 630), ("b", b, 60)])
+        for _ in range(12):
+            f.step([("a", a, 1), ("b", b, 1), ("c", c, 1)])
+        for _ in range(3):
+            f.step([("b", b, 1), ("a", a, 1)])
+        f.step([("a", a, 35)])
+        runs.append([f.end(k) for k in "abc"])
+        e.close()
+    assert all(np.array_equal(x, y) for x, y in zip(*runs))
+    for got, want in zip(runs[0], (wa, wb, wc)):
+        assert U.bf16_close(got, want)
+
+
 def test_large_passes_take_the_tensor_core_expert_products(monkeypatch):
     """A pass of 1280 prompt tokens in bfloat16: per-expert tensor-core products over rows sorted by expert, the shared
     expert's gate-up product with the SiLU epilogue.  Against the oracle, and against the same pass on the tiled fp32-FMA

@@ -57,3 +57,12 @@ def test_shared_memory_of_other_ctas_is_written_only_when_they_run():
         wait = waits.search(body)
         assert wait is not None and wait.start() < first.start(), f"{name}: stores into another CTA's shared memory before it is known to run"
     assert seen >= 2
+
+
+def test_empty_slices_leave_the_stages_alone():
+    """Layer-list attention zeroes the padding columns of its key stages at its start and lays the warps' states over the stages at its end.  The
+    barriers in between are those of the key tiles: a slice without a key has none, so it must not write the columns either."""
+    body = dict(kernels())["stack_attn_mma_kernel"]
+    zero = re.search(r"if\s*\(([^;{]*)\)\s*for\s*\([^;]*;[^;]*;[^)]*\)\s*Ks\[[^;]*\]\s*=\s*0;", body)
+    assert zero is not None and zero.start() < body.find("__syncthreads()")
+    assert "k_end > k_begin" in zero.group(1)
