@@ -8,6 +8,7 @@ import os
 
 import numpy as np
 import pytest
+import torch
 
 from distributed_inference_server_b200 import (BatchedRequest, Engine, FinishReason, InferenceBatch, InferenceParams,
                                                InferenceWorker, ModelShape, WorkerConfig, WorkerError)
@@ -429,6 +430,85 @@ def test_decode_batch_padded_to_graph_bucket_changes_nothing():
     mimic = O.Oracle(shape, act_round=True); mimic.fill_synthetic(77, True)
     got = [[step[b] for step in outs[0][0][:7]] for b in range(13)]
     assert_greedy_matches(got, mimic, prompts, 7, "bucket-padded")
+
+
+def _turn(v, theta):
+    """Rotary embedding of [T][heads][d], coordinates i and i + d/2, positions from 0."""
+    d = v.shape[-1]
+    a = torch.arange(v.shape[0], device=v.device, dtype=torch.float64)[:, None] * theta ** (-2.0 * torch.arange(d // 2, device=v.device, dtype=torch.float64) / d)
+    c, s = torch.cos(a)[:, None], torch.sin(a)[:, None]
+    return torch.cat([v[..., :d // 2] * c - v[..., d // 2:] * s, v[..., d // 2:] * c + v[..., :d // 2] * s], -1)
+
+
+def _logits64(shape, t, tokens, last):
+    """Logits of the last positions of a sequence, in 64 bits."""
+    nh, nkv, d = shape.n_heads, shape.n_kv_heads, shape.head_dim
+    rms = lambda v: v * torch.rsqrt(v.square().mean(-1, keepdim=True) + shape.rms_eps)  # noqa: E731
+    f = lambda v: v.double()  # noqa: E731
+    x = f(t["embed"][tokens])
+    unseen = torch.ones(len(tokens), len(tokens), device=x.device, dtype=torch.bool).triu(1)
+    for w in t["layers"]:
+        h = rms(x) * f(w[B.T_ATTN_NORM])
+        q, k, v = ((h @ f(w[n]).T).view(len(tokens), -1, d) for n in (B.T_WQ, B.T_WK, B.T_WV))
+        q, k = _turn(q, shape.rope_theta), _turn(k, shape.rope_theta)
+        o = [torch.softmax((q[:, a] @ k[:, a // (nh // nkv)].T * d ** -0.5).masked_fill(unseen, float("-inf")), -1) @ v[:, a // (nh // nkv)] for a in range(nh)]
+        x = x + torch.cat(o, -1) @ f(w[B.T_WO]).T
+        h = rms(x) * f(w[B.T_MLP_NORM])
+        x = x + (torch.nn.functional.silu(h @ f(w[B.T_WGATE]).T) * (h @ f(w[B.T_WUP]).T)) @ f(w[B.T_WDOWN]).T
+    return (rms(x[-last:]) * f(t["norm"])) @ f(t["head"]).T
+
+
+@pytest.mark.parametrize("batch,long_ones", [(24, 1), (21, 2), (32, 1)])
+@pytest.mark.parametrize("n_heads,head_dim", [(32, 64), (16, 128)])
+def test_decode_of_one_long_history_beside_short_ones(n_heads, head_dim, batch, long_ones):
+    """Decode steps whose attention forms query and key itself while a cluster's CTAs share the histories of eight requests: one history of
+    about 2000 tokens beside short ones (a CTA holds ends and beginnings of several, and the CTA that holds a history's end is not the one that
+    holds its beginning), lengths around the edges of tiles of 64 and pages, a batch of 21 that the graph pads to 24, whose copied row rewrites
+    its cache row.  30 steps: a wrong cache row would show in every later one.  Logits against 64 bits, graph and eager; the head reads the embedding of a
+    permuted token, so the greedy tokens are known.  Tolerance in the 2-norm: two layers in bf16 are 5e-3 off; a key and value row left as zeros
+    moves the logits of the step that made it by 2e-2 to 1e-1, a lost tile by more."""
+    H, ff, vocab, steps = 256, 256, 384, 30
+    shape = ModelShape(vocab, H, 2, n_heads, 8, head_dim, ff, 2304)
+    g = torch.Generator(device="cuda"); g.manual_seed(n_heads + batch)
+    rnd = lambda *s: (torch.randn(s, device="cuda", generator=g) * s[-1] ** -0.5).to(torch.bfloat16)  # noqa: E731
+    gain = lambda: (1.0 + 0.1 * torch.randn(H, device="cuda", generator=g)).to(torch.bfloat16)  # noqa: E731
+    t = {"embed": torch.randn((vocab, H), device="cuda", generator=g).to(torch.bfloat16), "norm": gain(), "layers": []}
+    perm = torch.randperm(vocab, device="cuda", generator=g)
+    t["head"] = torch.empty_like(t["embed"])
+    t["head"][perm] = (t["embed"].float() * H ** -0.5).to(torch.bfloat16)
+    for _ in range(shape.layers):
+        t["layers"].append({B.T_ATTN_NORM: gain(), B.T_WQ: rnd(n_heads * head_dim, H) * 3, B.T_WK: rnd(8 * head_dim, H), B.T_WV: rnd(8 * head_dim, H), B.T_WO: rnd(H, n_heads * head_dim) * 2,
+                            B.T_MLP_NORM: gain(), B.T_WGATE: rnd(ff, H), B.T_WUP: rnd(ff, H), B.T_WDOWN: rnd(H, ff)})
+    rng = np.random.default_rng(batch)
+    lens = rng.choice([1, 33, 48, 62, 63, 64, 65, 100, 120, 127, 128, 190], batch)
+    lens[rng.choice(batch, long_ones, replace=False)] = [1990, 1300][:long_ones]
+    prompts = [rng.integers(0, vocab, int(n)) for n in lens]
+    whole = []
+    for p in prompts:
+        seq = [int(v) for v in p]
+        for _ in range(steps):
+            seq.append(int(perm[seq[-1]]))
+        whole.append(seq)
+    want = [_logits64(shape, t, torch.tensor(s, device="cuda"), steps + 1).cpu().numpy() for s in whole]
+    host = lambda v: v.contiguous().view(torch.uint16).cpu().numpy()  # noqa: E731
+    for flags in (0, B.FLAG_NO_GRAPH):
+        e = Engine(WorkerConfig(shape, flags=flags, max_batch=32, max_step_tokens=6144, page_size=16, kv_pages=int(sum(-(-(lens + steps + 1) // 16))) + 8))
+        for kind, key in ((B.T_EMBED, "embed"), (B.T_LM_HEAD, "head"), (B.T_FINAL_NORM, "norm")):
+            e.load_tensor(kind, 0, host(t[key]))
+        for i, w in enumerate(t["layers"]):
+            for kind, a in w.items():
+                e.load_tensor(kind, i, host(a))
+        e.finalize()
+        slots = [e.seq_add(p, InferenceParams(max_tokens=1 << 20, temperature=0.0)) for p in prompts]
+        for k in range(steps + 1):
+            tokens = (e.prefill(slots) if k == 0 else e.decode(slots))[0]
+            logits = e.last_logits(batch)
+            for b in range(batch):
+                err = np.linalg.norm(logits[b] - want[b][k]) / np.linalg.norm(want[b][k])
+                assert err <= 2e-2, (flags, k, b, int(lens[b]), err)
+                if k < steps:
+                    assert int(tokens[b]) == whole[b][lens[b] + k]
+        e.close()
 
 
 def test_sampled_rows_of_a_vocabulary_longer_than_the_cluster_sampler_takes():
