@@ -748,8 +748,8 @@ cudaError_t Engine::enqueue_layers(int T, int n_splits) {
       prof_mark(P_ATTN);
       if (!skip(P_ATTN)) RET_CUDA(launch_attn_decode_fused(kv_map, (long long)l * kv_rows_per_layer, pool, partial, s_qkv, (long long)T * nqkv_l,
                                         pos, rope_cos, rope_sin, d_page_table, max_pages, ptrow, ctx, attn, attn_scratch,
-                                        n_splits, T, nh_l, nkv_l, d, page_size, attn_longest, stream));
-      kernel_launches += n_splits > 1 && attn_tokens_per_cluster(n_splits, T, nkv_l, attn_longest) == 0 ? 2 : 1;
+                                        n_splits, T, nh_l, nkv_l, d, page_size, attn_share, stream));
+      kernel_launches += n_splits > 1 ? 2 : 1;
     }
     int s_o = 1;
     prof_mark(P_OPROJ);
@@ -1180,9 +1180,8 @@ int Engine::decode(int n, const int *slots, uint32_t *out_tokens, int *out_finis
     cur_meta->h<unsigned long long>(cur_meta->o_step)[r] = cur_meta->h<unsigned long long>(cur_meta->o_step)[q];
   }
   const int n_splits = pick_attn_splits(T, max_ctx_b);
-  // the attention launch depends on whether any history is long (attn_tokens_per_cluster), and so does the graph
-  const bool long_ctx = max_ctx_b > kAttnShort;
-  attn_longest = long_ctx ? 1 << 30 : kAttnShort;
+  // the attention's launch depends on how unlike the histories are, and so does the graph
+  attn_share = attn_may_share(n_splits, T, nkv_l) && attn_sharing_pays(cur_meta->h<int>(cur_meta->o_ctx), T, nkv_l, m.head_dim);
   last_T = T;
   rowmap_identity = true;
   ENG_CUDA(cudaEventRecord(ev0, stream));
@@ -1192,7 +1191,7 @@ int Engine::decode(int n, const int *slots, uint32_t *out_tokens, int *out_finis
     ENG_CUDA(enqueue_head(T, all_greedy));
     prof_mark(P_COUNT);
   } else {
-    const uint64_t key = ((uint64_t)T << 10) | ((uint64_t)n_splits << 2) | (long_ctx ? 2u : 0u) | (all_greedy ? 1u : 0u);
+    const uint64_t key = ((uint64_t)T << 10) | ((uint64_t)n_splits << 2) | (attn_share ? 2u : 0u) | (all_greedy ? 1u : 0u);
     auto it = graphs.find(key);
     if (it == graphs.end()) {
       const uint64_t before = kernel_launches;

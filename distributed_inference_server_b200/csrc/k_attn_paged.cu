@@ -1,9 +1,10 @@
 // k_attn_paged.cu -- attention of single query tokens over a paged bf16 KV cache.
 //
-// One CTA handles one (query token, kv head, split of the history) for all query heads of the GQA
-// group, so K and V are read from HBM once per group.  64-token K/V tiles are staged by TMA into
+// One CTA handles one (query token, kv head, slice of the history) for all query heads of the GQA
+// group, so K and V are read from HBM once per group; in ragged batches of long histories the CTAs of a
+// cluster share the histories of up to eight tokens instead.  64-token K/V tiles are staged by TMA into
 // 128B-swizzled shared memory through a 3-4 stage mbarrier ring (64-96 KB in flight per CTA, two
-// CTAs per SM); Q K^T and P V run on mma.sync m16n8k16 (bf16 in, fp32 accumulate) with ldmatrix operand
+// or three CTAs per SM); K Q^T and V^T P^T run on mma.sync m16n8k16 (bf16 in, fp32 accumulate) with ldmatrix operand
 // loads -- on CUDA cores the 4 FMA per KV byte of a 4:1 GQA group is issue-bound well below the HBM
 // rate (measured: 56 us vs 5 us per layer at batch 32, ctx 512).  HBM-bound: algorithmic
 // bytes = 2 (K,V) * ctx * n_kv * d * 2 B per query token (+ q and out, negligible).
@@ -11,7 +12,7 @@
 // KV page pool layout, per layer: [page][2 (K,V)][n_kv][page_size][d] bf16 -- each (page, kv head)
 // is one contiguous page_size*d block.
 //
-// With n_splits > 1 every split writes (m, l, unnormalised o) to scratch and a combine pass merges
+// With n_splits > 1 every slice writes (m, l, unnormalised o) to scratch and a combine pass merges
 // them (flash-decoding); that keeps all 148 SMs busy at batch 1.
 #include <algorithm>
 #include <cstdlib>
@@ -23,9 +24,7 @@
 
 namespace dis {
 
-constexpr int kAttnThreads = 256;  // computing threads: two groups of four warps
-constexpr int kAttnWarps = kAttnThreads / 32;
-constexpr int kAttnTile = 64;  // tokens per pipeline stage: 16 per warp of a group
+constexpr int kAttnTile = 64;  // tokens per pipeline stage: 16 per warp of a group of four
 
 template <int D>
 struct AttnCfg {
@@ -59,21 +58,22 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// One CTA = one (query token, kv head, split).  K/V tiles of 64 tokens arrive by TMA (a warp of its own, 128B-swizzled boxes of
-// min(page,64) rows, mbarrier completion) into a 3-4 stage ring.  Two groups of four warps take the tiles in turn, each warp 16 of a
-// tile's 64 tokens, with an online-softmax state (m, l, O) of its own; the eight states are merged once at the end.
+// K/V tiles of 64 tokens arrive by TMA (a warp of its own, 128B-swizzled boxes of min(page,64) rows, mbarrier completion) into a 3-4 stage ring.
+// A group of four warps takes a tile, each warp 16 of its 64 tokens, with an online-softmax state (m, l, O) of its own; the states are merged
+// once at the end.  With two groups the tiles are taken in turn.
 //
 // What bounds it is HBM where the histories are alike; in a ragged batch the longest one, which a single CTA walks: the time of a tile
-// in a warp is a chain of latencies (barrier, ldmatrix, MMAs, shuffles, exponential, MMAs), so what counts is how short the chain is
-// and how many run side by side.  Tokens are therefore the MMAs' rows and the group's query heads (<= 8) their eight columns: S^T = K Q^T and
-// O^T = V^T P^T fill the m16n8k16 shape, half the MMAs and half the accumulators (D / 2 registers) of heads as 16 padded rows, and eight
-// warps fit the registers of two CTAs per SM where four did.  P^T is turned from accumulator to operand by movmatrix.  Batch 32, histories of
-// 500 to 6000 keys, 32 / 8 heads of 128, 318 MB: 74.7 us before, 56 now (5.7 TB/s).
+// in a warp is a chain of latencies (barrier, ldmatrix, MMAs, shuffles, exponential, MMAs).  Tokens are the MMAs' rows and the group's
+// query heads (<= 8) their eight columns: S^T = K Q^T and O^T = V^T P^T fill the m16n8k16 shape, half the MMAs and half the accumulators (D / 2
+// registers) of heads as 16 padded rows.  P^T is turned from accumulator to operand by movmatrix, and two accumulators halve S^T's chain of MMAs.
+// From graphs, against heads as rows (32 / 8 heads of 128): 1 x 8000 keys 15.0 -> 14.7 us, 8 x 512 8.8 -> 8.4, 32 x 512 13.9 -> 13.8, 64 x 575
+// 27.7 -> 28.4, 32 ragged ones of 500 to 6000 77.1 -> 74.8; heads of 64 (32 / 4): 32 x 512 9.0 -> 8.6, 64 x 2000 23.5 -> 24.4.
+// Eight warps in two groups lose nearly everywhere (8 x 512 9.4 us, 32 x 512 14.6, 32 x 100 7.6 against 6.7: more to start, to merge and to
+// keep resident); see attn_dispatch for where they stay.
 //
-// A ragged batch in one wave is as slow as its longest history if every history has a CTA of its own (the eight warps alone moved those 74.7 us
-// to 74: the long CTAs get their share of HBM only when the short ones are done).  So the CTAs of a cluster lay the histories of up to
-// eight tokens end to end and take equal shares; pieces of one history meet in the shared memory of the CTA that has its first.  Clusters of four
-// level less (70 us).  Equal histories pay for it: 32 x 6000 115 -> 117 us, heads of 64, 64 x 2000 24.4 -> 26.
+// A ragged batch in one wave is as slow as its longest history if every history has a CTA of its own.  So (kShared) the CTAs of a cluster lay
+// the histories of up to eight tokens end to end and take equal shares; pieces of one history meet in the shared memory of the CTA that has its
+// first: those 74.8 us are 55.0.  The cluster's start and end cost 2 to 4 us, the pieces 5 more: attn_sharing_pays.
 //
 // P is rounded to bf16 for the P.V MMA (the usual flash-attention choice).
 // Rows past the context inside a box hold stale (finite) cache contents and get probability 0; the
@@ -115,14 +115,16 @@ __device__ __forceinline__ void attn_cluster_sync() {
 
 constexpr int kAttnMaxCluster = 8;  // the portable size
 
-// kShared: a cluster's CTAs share the histories of per_cluster tokens; otherwise a CTA has one slice of one history
-template <int D, int G, bool kShared>
-__global__ void __launch_bounds__(kAttnThreads + 32, 2)
+// kShared: a cluster's CTAs share the histories of as many tokens; otherwise a CTA has one slice of one history.  NG: groups of four computing warps
+template <int D, int G, bool kShared, int NG>
+__global__ void __launch_bounds__(NG * 128 + 32, 2)
 attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, const AttnRope rope, const uint16_t *__restrict__ q,
                   const int *__restrict__ page_table, int max_pages, const int *__restrict__ pt_row,
                   const int *__restrict__ ctx_len, uint16_t *__restrict__ out, float *__restrict__ scratch,
-                  int n_splits, int T, int n_heads, int n_kv, int page_shift, int n_stages, int per_cluster) {
+                  int n_splits, int T, int n_heads, int n_kv, int page_shift, int n_stages) {
   using Cfg = AttnCfg<D>;
+  constexpr int kAttnThreads = NG * 128, kAttnWarps = NG * 4;  // those that compute
+  static_assert(!kShared || NG == 1, "a shared history's stages are counted for one group");
   constexpr int KS = D / 16;  // k-steps of the K Q^T MMA, m-tiles of the V^T P^T MMA
   static_assert(kAttnWarps * G * D * 4 <= Cfg::kStageBytes, "the warps' states are merged in one stage");
 
@@ -130,15 +132,15 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // 128B swizzle atoms are 1024-byte aligned
   uint8_t *smem = smem_raw + (smem_base - smem_u32(smem_raw));
   const uint32_t bar_base = smem_base + n_stages * Cfg::kStageBytes;
-  // A stage has a full barrier for each of the two groups: tile i completes number i % (2 n_stages), whose phases then all belong to the
+  // A stage has a full barrier for each of the groups: tile i completes number i % (NG n_stages), whose phases then all belong to the
   // group that waits for it.  (With one per stage and three stages, a group that runs ahead would take the other group's phase for its own.)
-  auto full_bar = [&](int tile) { return bar_base + 8u * (uint32_t)(tile % (2 * n_stages)); };
+  auto full_bar = [&](int tile) { return bar_base + 8u * (uint32_t)(tile % (NG * n_stages)); };
   auto empty_bar = [&](int s) { return bar_base + 64u + 8u * s; };
 
-  const int t0 = kShared ? (int)blockIdx.z * per_cluster : (int)blockIdx.z;
-  const int count = kShared ? min(per_cluster, T - t0) : 1;
   const int kvh = blockIdx.y;
-  const int rank = blockIdx.x, ranks = gridDim.x;
+  const int rank = blockIdx.x, ranks = gridDim.x;  // kShared: as many histories as CTAs; otherwise the history's slices
+  const int t0 = kShared ? (int)blockIdx.z * ranks : (int)blockIdx.z;
+  const int count = kShared ? min(ranks, T - t0) : 1;
   const int h0 = kvh * G;  // first query head of this CTA (G = n_heads / n_kv)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;  // mma fragment coordinates
@@ -151,7 +153,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&kv_map);
-    for (int s = 0; s < 2 * n_stages; s++) mbar_init(full_bar(s), 1);
+    for (int s = 0; s < NG * n_stages; s++) mbar_init(full_bar(s), 1);
     for (int s = 0; s < n_stages; s++) mbar_init(empty_bar(s), 4);
     fence_barrier_init();
     fence_proxy_async();
@@ -179,19 +181,15 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     total += n;
     if (kShared) most = max(most, n);
   }
-  // A history of its own for every n_splits CTAs, or equal shares of all where that is shorter by more than a piece's start and end cost
+  // A history of its own for every CTA, or equal shares of all where that is shorter by more than a piece's start and end cost
   const int share = kShared ? (total + ranks - 1) / ranks : 0;
-  const bool level = kShared && most > (share + 2) * n_splits;
-  const bool pieces = kShared && (level || n_splits > 1);  // (the same in every CTA of the cluster)
+  const bool level = kShared && most > share + 2;  // (the same in every CTA of the cluster)
   auto bound = [&](int r) {
     if (!kShared) return min(total, r * ((total + n_splits - 1) / n_splits));
     if (level) return min(total, r * share);
-    const int item = r / n_splits;
     int at = 0;
-    for (int i = 0; i < min(item, count); i++) at += tiles_of(i);
-    if (item >= count) return at;
-    const int n = tiles_of(item);
-    return at + min(n, (r % n_splits) * ((n + n_splits - 1) / n_splits));
+    for (int i = 0; i < min(r, count); i++) at += tiles_of(i);
+    return at;
   };
   const int lo = bound(rank), hi = bound(rank + 1);
   // f(history, first tile, end tile, tiles of the history) for every piece in [lo, hi); an empty history counts as a tile above, so that it has a
@@ -211,7 +209,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   };
 
   // The last warp loads and does nothing else, the computing warps free a stage each for themselves: no barrier of the whole block per
-  // tile (with one, the longest history of a ragged batch took 1.04 us per tile, without it and four computing warps 0.83).
+  // tile (with one, the longest history of a ragged batch took 1.04 us per tile, without it 0.83, and 0.79 with tokens as rows).
   if (warp == kAttnWarps) {
     if (lane == 0) {
       int k = 0;  // stages handed out so far
@@ -238,13 +236,15 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
             }
           }
         }
-        next_stage();  // one more, empty: the warps merge their states in it while the next piece's tiles are under way
-        mbar_arrive(full_bar(k));
-        k++;
+        if (kShared) {
+          next_stage();  // one more, empty: the warps merge their states in it while the next piece's tiles are under way
+          mbar_arrive(full_bar(k));
+          k++;
+        }
       });
     }
     __syncwarp();
-    if (pieces) attn_cluster_sync();
+    if (level) attn_cluster_sync();
     if (kShared) attn_cluster_sync();
     return;
   }
@@ -317,9 +317,9 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     for (int m = 0; m < KS; m++) { oacc[m][0] = 0.f; oacc[m][1] = 0.f; oacc[m][2] = 0.f; oacc[m][3] = 0.f; }
     float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};  // heads 2 tq (+ 1); l_run: this thread's tokens (summed at the end)
 
-    for (int tile = a + ((k0 ^ grp) & 1); tile < b; tile += 2) {  // stage number k0 + tile - a: even ones are group 0's
+    for (int tile = a + (NG > 1 ? grp : 0); tile < b; tile += NG) {
       const int k = k0 + tile - a, stage = k % n_stages;
-      mbar_wait(full_bar(k), (uint32_t)(k / (2 * n_stages)) & 1u);
+      mbar_wait(full_bar(k), (uint32_t)(k / (NG * n_stages)) & 1u);
       const uint32_t ks_addr = smem_base + stage * Cfg::kStageBytes;
       const uint32_t vs_addr = ks_addr + Cfg::kHalves * Cfg::kHalfBytes;
       const int tile_len = min(kAttnTile, ctx - tile * kAttnTile);
@@ -345,7 +345,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
           const int c = ks * 2 + (mi >> 1);  // 16-byte chunk of the row
           uint32_t a0, a1, a2, a3;
           ldmatrix_x4(ks_addr + (c >> 3) * Cfg::kHalfBytes + k_tok * 128 + (((c & 7) ^ (k_tok & 7)) << 4), a0, a1, a2, a3);
-          mma_bf16_16816(sacc[0], a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
+          mma_bf16_16816(sacc[ks & 1], a0, a1, a2, a3, qb[ks][0], qb[ks][1]);
         }
         // ---- online softmax of the two heads
         const bool in0 = wtok + g < tile_len, in1 = wtok + g + 8 < tile_len;
@@ -386,11 +386,13 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     }
     k0 += b - a;
 
-    // ---- merge the warps' (m, l, O) in the stage that was handed out empty: [warps][G][D], a pair of heads 8 dims from the next (no bank twice)
-    const int stage = k0 % n_stages;
-    const bool mine = (k0 & 1) == grp;
-    if (mine) mbar_wait(full_bar(k0), (uint32_t)(k0 / (2 * n_stages)) & 1u);
-    k0++;
+    // ---- merge the warps' (m, l, O): [warps][G][D], a pair of heads 8 dims from the next (no bank twice).  Where a piece may follow, in the stage
+    // that was handed out empty; where none does every load has been waited for, and behind the barrier any stage is free
+    const int stage = kShared ? k0 % n_stages : 0;
+    if (kShared) {
+      mbar_wait(full_bar(k0), (uint32_t)(k0 / n_stages) & 1u);
+      k0++;
+    }
     sync_compute();
     float *s_o = reinterpret_cast<float *>(smem + stage * Cfg::kStageBytes);
 #pragma unroll
@@ -440,12 +442,12 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     if (kShared) {
       fence_proxy_async();  // (plain accesses to a stage that TMA will fill again)
       sync_compute();
-      if (mine && lane == 0) mbar_arrive(empty_bar(stage));
+      if (lane == 0) mbar_arrive(empty_bar(stage));
     }
   });
   // ---- pieces of one history in several CTAs: the CTA that holds its first piece reads the others' out of their shared memory
   if constexpr (kShared) {
-    if (pieces) attn_cluster_sync();
+    if (level) attn_cluster_sync();
     if (open >= 0) {
       int end = 0;
       for (int i = 0; i <= open; i++) end += tiles_of(i);
@@ -677,15 +679,28 @@ __global__ void attn_combine_kernel(const float *__restrict__ scratch, uint16_t 
   out[((size_t)t * n_heads + h) * D + dd] = float_to_bf16_bits(o / L);
 }
 
-// Tokens whose histories a cluster of CTAs shares (each history n_splits CTAs' worth), 0: no cluster.  Slices of two to eight per token are
-// merged in shared memory, which saves the merge's launch and its scratch traffic; whole histories are levelled where they can be long: up
-// to kAttnShort keys nothing is gained, and a cluster starts later than a CTA.  Beyond one wave of two CTAs per SM the hardware levels
-// by itself, and whole clusters find room later than single CTAs.
-int attn_tokens_per_cluster(int n_splits, int T, int n_kv, int longest) {
-  if (n_splits > kAttnMaxCluster || (long long)n_splits * T * n_kv > 2 * kNumSMs) return 0;
-  if (n_splits == 1 && (T < 2 || longest <= kAttnShort)) return 0;
-  const int n = kAttnMaxCluster / n_splits;
-  return n < T ? n : T;
+// Whole histories can be shared (slices are a share already; slices merged inside a cluster instead of by the combine pass took 13.0 us for 8 x 512
+// where the two kernels take 8.4, and 22.8 against 16.5 for 8 x 2000: a cluster's start costs more than the launch), in one wave of two CTAs per
+// SM: beyond it the hardware levels by itself, and whole clusters find room later than single CTAs.
+bool attn_may_share(int n_splits, int T, int n_kv) { return n_splits == 1 && T > 1 && (long long)T * n_kv <= 2 * kNumSMs; }
+// Which takes longer, us: the longest history alone or the largest share of a cluster (0.8 us a tile of heads of 128, 0.5 of 64), neither less than
+// the stream of all keys and values at 6.5 TB/s; sharing costs 8 on top.  Of 25 ragged and 19 equal batches (heads of 128: 20 and 32 histories, of
+// 64: 40 and 64; 100 to 7000 keys) it takes the slower form of three, by 3 % at most.
+bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d) {
+  const int n = T < kAttnMaxCluster ? T : kAttnMaxCluster;
+  long long total = 0, most = 0, share = 0;
+  for (int t0 = 0; t0 < T; t0 += n) {
+    long long sum = 0;
+    for (int t = t0; t < std::min(t0 + n, T); t++) {
+      const long long tiles = std::max(1, (ctx[t] + kAttnTile - 1) / kAttnTile);
+      sum += tiles;
+      most = std::max(most, tiles);
+    }
+    total += sum;
+    share = std::max(share, (sum + n - 1) / n);
+  }
+  const double tile = d == 128 ? 0.8 : 0.5, stream = (double)total * n_kv * (kAttnTile * d * 4) / 6.5e6;  // us
+  return std::max(share * tile, stream) + 8.0 < std::max(most * tile, stream);
 }
 
 size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits) {
@@ -693,15 +708,13 @@ size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits) {
   return (size_t)T * n_heads * n_splits * (2 + (size_t)d);
 }
 
-template <int D, int G>
+template <int D, int G, int NG, bool kShared>
 static cudaError_t attn_launch(const TmaMap &kv_map, long long row0, const AttnRope &rope, const uint16_t *q, const int *page_table,
                                int max_pages, const int *pt_row, const int *ctx, uint16_t *out, float *scratch,
-                               int n_splits, int T, int n_heads, int n_kv, int page_shift, int longest, cudaStream_t st) {
+                               int n_splits, int T, int n_heads, int n_kv, int page_shift, cudaStream_t st) {
+  auto kern = attn_paged_kernel<D, G, kShared, NG>;
   static DeviceOnce once;
-  DIS_CUDA_TRY(once.run([&] {
-    cudaError_t e = cudaFuncSetAttribute(attn_paged_kernel<D, G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::kSmemBytes);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_paged_kernel<D, G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::kSmemBytes);
-  }));
+  DIS_CUDA_TRY(once.run([&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AttnCfg<D>::kSmemBytes); }));
   // ring depth: fewer stages leave shared memory for the NEXT kernel's CTAs to become resident (and prefetch their
   // weights) while this one is still streaming; DIS_ATTN_STAGES overrides (A/B runs), 2 <= stages <= AttnCfg::kStages
   static int stages = 0;
@@ -711,16 +724,10 @@ static cudaError_t attn_launch(const TmaMap &kv_map, long long row0, const AttnR
     stages = stages < 2 ? 2 : (stages > AttnCfg<D>::kStages ? AttnCfg<D>::kStages : stages);
   }
   const int smem = stages * AttnCfg<D>::kStageBytes + AttnCfg<D>::kExtraBytes;
-  const int per_cluster = attn_tokens_per_cluster(n_splits, T, n_kv, longest);
-  if (per_cluster > 0) {
-    const int ranks = per_cluster * n_splits;
-    return launch_k_cluster(attn_paged_kernel<D, G, true>, dim3(ranks, n_kv, (T + per_cluster - 1) / per_cluster), dim3(kAttnThreads + 32), (size_t)smem, st, ranks,
-                            *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
-                            scratch, n_splits, T, n_heads, n_kv, page_shift, stages, per_cluster);
-  }
-  DIS_CUDA_TRY(launch_k(attn_paged_kernel<D, G, false>, dim3(n_splits, n_kv, T), dim3(kAttnThreads + 32), (size_t)smem, st,
-                        *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
-                        scratch, n_splits, T, n_heads, n_kv, page_shift, stages, 0));
+  const int ranks = kShared ? std::min(T, kAttnMaxCluster) : n_splits;
+  DIS_CUDA_TRY(launch_k_cluster(kern, dim3(ranks, n_kv, kShared ? (T + ranks - 1) / ranks : T), dim3(NG * 128 + 32), (size_t)smem, st, kShared ? ranks : 1,
+                                *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
+                                scratch, n_splits, T, n_heads, n_kv, page_shift, stages));
   if (n_splits > 1)
     DIS_CUDA_TRY(launch_k(attn_combine_kernel<D>, dim3(n_heads, T), dim3(D), 0, st, (const float *)scratch, out, n_splits, T, n_heads));
   return cudaSuccess;
@@ -734,7 +741,7 @@ cudaError_t make_kv_map(TmaMap *out, const uint16_t *pool, long long total_rows,
 static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const AttnRope &rope, const uint16_t *q,
                                  const int *page_table, int max_pages, const int *pt_row, const int *ctx, uint16_t *out,
                                  float *scratch, int n_splits, int T, int n_heads, int n_kv, int d, int page_size,
-                                 int longest, cudaStream_t st) {
+                                 bool share, cudaStream_t st) {
   if (T <= 0) return cudaSuccess;
   if (n_kv <= 0 || n_heads % n_kv != 0) { set_last_error("attn_paged: n_heads must be a multiple of n_kv"); return cudaErrorInvalidValue; }
   if (n_splits < 1 || (n_splits > 1 && !scratch)) { set_last_error("attn_paged: n_splits > 1 needs scratch"); return cudaErrorInvalidValue; }
@@ -743,13 +750,26 @@ static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const Att
   int page_shift = 0;
   while ((1 << page_shift) < page_size) page_shift++;
   const int G = n_heads / n_kv;  // query heads per kv head, all handled by one CTA
-#define DIS_ATTN_CASE(DD, GG)                                                                                        \
-  if (d == DD && G == GG)                                                                                            \
-    return attn_launch<DD, GG>(kv_map, row0, rope, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, \
-                               n_heads, n_kv, page_shift, longest, st);
+  share = share && attn_may_share(n_splits, T, n_kv);
+  // Heads of 64: three CTAs of four computing warps fit an SM, or two of eight.  Just above three per SM the former leave most of a second round
+  // empty, the latter fill theirs: 512 CTAs, 2000 keys 53.4 -> 45.6 us, 700 22.3 -> 20.2, 200 11.6 -> 11.6; 448 x 2500 58.4 -> 54.0 (200 keys 10.4 -> 11.1).
+  // Elsewhere four warps are ahead: 304 x 700 12.0 against 17.9, 640 x 700 24.1 against 28.5, 1024 x 2500 104.6 against 110.1.
+  const long long ctas = (long long)n_splits * T * n_kv;
+  const bool two_groups = d == 64 && ctas > 3 * kNumSMs && ctas <= 4 * kNumSMs;
+#define DIS_ATTN_GO(DD, GG, NG, SH) \
+  attn_launch<DD, GG, NG, SH>(kv_map, row0, rope, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, page_shift, st)
+#define DIS_ATTN_CASE(DD, GG)                                               \
+  if (d == DD && G == GG) {                                                 \
+    if (share) return DIS_ATTN_GO(DD, GG, 1, true);                         \
+    if constexpr (DD == 64) {                                               \
+      if (two_groups) return DIS_ATTN_GO(DD, GG, 2, false);                 \
+    }                                                                       \
+    return DIS_ATTN_GO(DD, GG, 1, false);                                   \
+  }
   DIS_ATTN_CASE(128, 8) DIS_ATTN_CASE(128, 4) DIS_ATTN_CASE(128, 2) DIS_ATTN_CASE(128, 1)
   DIS_ATTN_CASE(64, 8) DIS_ATTN_CASE(64, 4) DIS_ATTN_CASE(64, 2) DIS_ATTN_CASE(64, 1)
 #undef DIS_ATTN_CASE
+#undef DIS_ATTN_GO
   set_last_error("attn_paged: head_dim must be 64 or 128 and the GQA group 1, 2, 4 or 8");
   return cudaErrorInvalidValue;
 }
@@ -758,10 +778,12 @@ cudaError_t launch_attn_paged(const TmaMap &kv_map, long long row0, const uint16
                               int max_pages, const int *pt_row, const int *ctx, uint16_t *out, float *scratch,
                               int n_splits, int T, int n_heads, int n_kv, int d, int page_size, cudaStream_t st) {
   AttnRope none{};
-  // the page table's width bounds the histories
-  const int longest = (int)std::min<long long>((long long)max_pages * page_size, 1 << 30);
+  // The lengths are on the device; the page table's width bounds them, and from about these on a ragged batch gains (us, whole / shared; heads of 128, 32
+  // histories of up to 1100 17.8 / 19.1, 1500 22.3 / 21.8, 3000 39.6 / 33.4, 7000 86.7 / 63.4; heads of 64, 64 of up to 1500 16.2 / 17.4, 2000
+  // 19.8 / 19.5, 4500 38.7 / 28.7).  Equal histories lose there: 32 x 2000 42.3 / 44.6, 32 x 6000 115.4 / 118.9, heads of 64, 64 x 4000 43.2 / 44.7.
+  const bool share = (long long)max_pages * page_size > (d == 128 ? 1536 : 2048);
   return attn_dispatch(kv_map, row0, none, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
-                       page_size, longest, st);
+                       page_size, share, st);
 }
 
 // Decode step: RoPE + KV write of the step's new token (position ctx[t] - 1 == pos[t]) fused in.
@@ -769,10 +791,10 @@ cudaError_t launch_attn_decode_fused(const TmaMap &kv_map, long long row0, uint1
                                      int n_partial, long long partial_stride, const int *pos, const float *rope_cos,
                                      const float *rope_sin, const int *page_table, int max_pages, const int *pt_row,
                                      const int *ctx, uint16_t *out, float *scratch, int n_splits, int T, int n_heads,
-                                     int n_kv, int d, int page_size, int longest, cudaStream_t st) {
+                                     int n_kv, int d, int page_size, bool share, cudaStream_t st) {
   AttnRope r{qkv, n_partial, partial_stride, pos, rope_cos, rope_sin, kv_layer_base};
   return attn_dispatch(kv_map, row0, r, nullptr, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
-                       page_size, longest, st);
+                       page_size, share, st);
 }
 
 template <int D, int G>

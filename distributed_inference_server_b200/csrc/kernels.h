@@ -82,8 +82,9 @@ cudaError_t launch_gemv_silu(const uint16_t *X, const uint16_t *Wgu, uint16_t *a
                              cudaStream_t st);
 
 // k_attn_paged.cu
-constexpr int kAttnShort = 1024;  // histories up to here need no levelling
-int attn_tokens_per_cluster(int n_splits, int T, int n_kv, int longest);
+// Whether the CTAs of a cluster may share the histories of a decode batch, and whether that pays for these lengths (on the host).
+bool attn_may_share(int n_splits, int T, int n_kv);
+bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d);
 size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits);
 // kv_map: make_kv_map over a pool of d-element rows [..][page][2][n_kv][page_size]; row0 = first row of the
 // layer to read (the engine keeps one map over all layers).
@@ -96,7 +97,7 @@ cudaError_t launch_attn_decode_fused(const TmaMap &kv_map, long long row0, uint1
                                      int n_partial, long long partial_stride, const int *pos, const float *rope_cos,
                                      const float *rope_sin, const int *page_table, int max_pages, const int *pt_row,
                                      const int *ctx, uint16_t *out, float *scratch, int n_splits, int T, int n_heads,
-                                     int n_kv, int d, int page_size, int longest /* no history has more keys */, cudaStream_t st);
+                                     int n_kv, int d, int page_size, bool share, cudaStream_t st);
 cudaError_t launch_attn_prefill(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,
                                 int max_pages, const int *qb_tok0, const int *qb_len, const int *qb_pos0,
                                 const int *qb_ptrow, uint16_t *out, int n_blocks, int n_heads, int n_kv, int d,

@@ -352,16 +352,17 @@ def test_attention_full_size_against_torch():
 @pytest.mark.parametrize("nh,nkv,d,page_size", [(8, 2, 128, 64), (8, 1, 128, 16), (16, 2, 64, 128), (4, 2, 64, 8), (2, 2, 128, 64)])
 @pytest.mark.parametrize("T,n_splits,pattern", [(8, 1, "one-long"), (13, 1, "ragged"), (2, 1, "one-long"), (3, 1, "equal"), (5, 2, "ragged"), (3, 3, "one-long"),
                                                 (2, 4, "one-long"), (1, 5, "equal"), (3, 8, "ragged"), (2, 9, "ragged"), (9, 1, "tiles"),
-                                                (9, 1, "holes"), (4, 2, "holes"), (2, 9, "holes")])
+                                                (9, 1, "holes"), (4, 2, "holes"), (2, 9, "holes"), (230, 1, "short")])
 def test_attention_of_ragged_histories(nh, nkv, d, page_size, T, n_splits, pattern):
-    """Histories that a cluster of CTAs shares: one long beside short ones, tile edges, batches that leave a cluster part empty, with and
-    without slices, against float64 (weights and outputs in bf16: a relative error of 2^-9 each, 8e-3 of the 2-norm is four times that)."""
+    """Histories that a cluster of CTAs shares (the page table's width says that they may be long): one long beside short ones, tile edges, batches
+    that leave a cluster part empty; slices; more CTAs than fit at once, for heads of 64 as many as take eight computing warps each.  Against
+    float64 (weights and outputs in bf16: a relative error of 2^-9 each, 8e-3 of the 2-norm is four times that)."""
     rng = np.random.default_rng(T * 100 + n_splits + d)
     ctx = {"one-long": np.where(np.arange(T) == T // 2, 2500, rng.integers(1, 130, T)), "ragged": rng.integers(1, 1800, T), "equal": np.full(T, 1100),
-           "tiles": np.array([1, 63, 64, 65, 127, 128, 129, 1024, 1025])[:T],
+           "tiles": np.array([1, 63, 64, 65, 127, 128, 129, 1024, 1025])[:T], "short": np.random.default_rng(T).integers(1, 300, T),
            "holes": np.array([0, 700, 0, 2200, 0, 0, 65, 1, 0])[:T]}[pattern].astype(np.int32)
     need = [-(-int(c) // page_size) for c in ctx]
-    width = max(max(need), 1040 // page_size + 1)
+    width = max(max(need), 2100 // page_size + 1)
     table = np.zeros((T, width), np.int32)
     order = rng.permutation(sum(need))
     for t, at in enumerate(np.cumsum([0] + need[:-1])):
