@@ -419,14 +419,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
 // ---------------------------------------------------------------------------------------- two query blocks per CTA
 // attn_prefill_pair_kernel: the form for passes that fill the GPU.  A CTA per SM stays, takes a pair of query blocks, and while it works on
 // it asks the hardware for the next pair that no CTA has begun (cluster launch control: a dynamic schedule without a counter in memory).
-// The two blocks, if they are of one sequence, share every K and V tile, and each has a softmax group, an O and a softmax reference of its own:
-// nothing is handed from group to group, S is double-buffered (2 x 2 x 64 columns, O 2 x D), and the next pair's first tiles, scores and
-// query rows are under way while the output of this one is read out.
+// The two blocks, if they are of one sequence, share every K and V tile, and each has a softmax group, an O and a softmax reference of its own
+// (D = 64: one of each for even and for odd tiles, as above and with the same bits): nothing is handed from group to group, S is
+// double-buffered (2 x 2 x 64 columns, O 2 x 128), and the next pair's first tiles, scores and query rows are under way while the output of this
+// one is read out.
 //
 //   warp 0       page numbers (32 at a time), K and V tiles of 64 keys into a ring of six, the list of passes
 //   warps 1, 2   the MMAs of group 0 and 1, S two tiles ahead of P V
 //   warp 3       query rows, two slots for each group
-//   warps 4-11   softmax of the two groups, one thread per row; the rounded maximum of D = 64 and the lazy reference of D = 128 as above
+//   warps 4-11   softmax of the two groups, one thread per row; the running maxima of D = 64 and the lazy reference of D = 128 as above
 //
 // What bounds it, stamped per pair of 64-key tiles (D = 128): 1280 clocks of the tensor pipe (a product with N = 64 reads Q at shared memory's rate:
 // 48 clocks where it computes 32) beside 1024 of exponentials; a group's own chain is 1800 (scores 200-400, maximum 250, exponentials 850-1100,
@@ -504,7 +505,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
                          uint16_t *__restrict__ out, int n_heads, int n_kv, int page_shift, int n_blocks) {
   constexpr int QT = 128 / G, kHalves = D / 64, kRing = kPpRing;
   constexpr uint32_t kQBytes = kHalves * kPfQHalf, kSlot = kHalves * kPfHalf;
-  constexpr bool kLazy = D == 128;
+  constexpr bool kOwn = D == 64;  // even and odd tiles each with an O and a reference of their own; D = 128: one of each, the reference lazy
+  constexpr uint32_t kOCols = 128;  // columns of a group's O
   extern __shared__ __align__(1024) uint8_t smem_al[];
   const uint32_t smem_base = smem_u32(smem_al);
   if (smem_base & 1023u) __trap();  // the 128B-swizzle atoms need 1024-byte alignment and there is no room for slack
@@ -651,7 +653,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
       constexpr uint32_t idesc_s = umma_idesc<kPpTile>();
       constexpr uint32_t idesc_o = umma_idesc<D>() | (1u << 16);  // B (= V) MN-major
       const uint32_t q_lo = umma_lo(q_base) + 2 * g * (kQBytes >> 4), k_lo0 = umma_lo(ring_base), v_off = umma_lo_mn(ring_base, kPfHalf) - k_lo0;
-      const uint32_t s_col = s_base + 2 * g * kPpTile, o_col = o_base + g * D;
+      const uint32_t s_col = s_base + 2 * g * kPpTile, o_col = o_base + g * kOCols;
       uint32_t slot = 0, phase = 0, lo = k_lo0;                     // the ring's next tile
       uint32_t steps = 0, scores = 0, passes = 0, tiles_q = 0;      // the group's P V products, S products, passes, query tiles so far
       auto step_ring = [&] {
@@ -709,7 +711,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
             if (elect_one()) {
               const uint32_t a = s_col + w * kPpTile, b = lo + v_off;
 #pragma unroll
-              for (uint32_t k = 0; k < kPpTile / 16; k++) umma_ts(o_col, a + 8 * k, b + k * 128, idesc_o, k > 0 ? 1u : (uint32_t)(j > 0));
+              for (uint32_t k = 0; k < kPpTile / 16; k++)
+                umma_ts(o_col + (kOwn ? ((uint32_t)j & 1u) * D : 0u), a + 8 * k, b + k * 128, idesc_o, k > 0 ? 1u : (uint32_t)(j > (kOwn ? 1 : 0)));
               umma_commit(pv_done(g, w));
               umma_commit(empty(slot));
             }
@@ -763,7 +766,7 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
     const int g = (warp - 4) >> 2;
     const int row = quarter * 32 + lane, hl = row / QT, t = row % QT;
     const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-    const uint32_t s_addr0 = s_base + lane_off + 2 * g * kPpTile, o_addr = o_base + lane_off + g * D;
+    const uint32_t s_addr0 = s_base + lane_off + 2 * g * kPpTile, o_addr = o_base + lane_off + g * kOCols;
     const float scale_log2 = rsqrtf((float)D) * 1.4426950408889634f;
     const float2 scale2 = make_float2(scale_log2, scale_log2);
     // The two warps of a quarter share an SM partition and its exponential unit, and left to themselves they run in step: both at the
@@ -776,7 +779,8 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
     for (PfPass p = next_pass(); p.n[0] >= 0; p = next_pass()) {
       const int n = g ? p.n[1] : p.n[0], tok0 = g ? p.tok0[1] : p.tok0[0], len = g ? p.len[1] : p.len[0], qp = (g ? p.pos0[1] : p.pos0[0]) + t;
       const int tiles = max(p.n[0], p.n[1]);
-      float m_ref = 0.f, l_run = 0.f;
+      float m_ref = kOwn ? -FLT_MAX : 0.f, l_run = 0.f;   // kOwn: of this tile's parity (finite where its first tile may hide every key of a row)
+      float m_other = -FLT_MAX, l_other = 0.f;            // of the other parity
 #pragma unroll 1
       for (int j = 0; j < n; j++, step++) {
         const uint32_t w = step & 1u, s_addr = s_addr0 + w * kPpTile;
@@ -800,10 +804,16 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
         const float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3])) * scale_log2;  // scale > 0: it commutes with the maximum
         float f = 1.0f;
         bool rescale = false;
-        if (j == 0) {
+        if (kOwn) {
+          const float m_now = fmaxf(m_ref, mx);
+          rescale = j >= 2 && __any_sync(0xffffffffu, mx > m_ref);
+          f = ex2_approx(m_ref - m_now);
+          m_ref = m_now;
+          l_run *= f;
+        } else if (j == 0) {
           m_ref = mx;  // finite: key 0 is visible to every query; O is first written by P_0 V_0 (accumulate off)
         } else {
-          const bool need = mx > m_ref + (kLazy ? kPfLazy : 0.f);
+          const bool need = mx > m_ref + kPfLazy;
           rescale = __any_sync(0xffffffffu, need);  // tcgen05.ld / st are warp-collective: decide per warp, scale per lane
           if (need) {
             f = ex2_approx(m_ref - mx);
@@ -828,18 +838,27 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
           tmem_st_32x16(s_addr + 16 * c, pk);
         }
         if (kTurns) named_arrive_64(its_turn);
-        if (rescale) {  // behind the weights: the P V before this has had their time to end
-          mbar_wait(pv_done(g, w ^ 1u), ((step - 1) >> 1) & 1u);
-          tc_fence_after();
+        if (rescale) {
+          if (kOwn) {  // S was issued behind the P V of two tiles before: this parity's O is complete
+            rescale_64(o_addr + ((uint32_t)j & 1u) * D, f);
+          } else {  // behind the weights: the P V before this has had their time to end
+            mbar_wait(pv_done(g, w ^ 1u), ((step - 1) >> 1) & 1u);
+            tc_fence_after();
 #pragma unroll
-          for (int c = 0; c < D; c += 64) rescale_64(o_addr + c, f);
-          l_run *= f;
+            for (int c = 0; c < D; c += 64) rescale_64(o_addr + c, f);
+            l_run *= f;
+          }
         }
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(p_full(g, w));
         l_run += (ps[0].x + ps[0].y) + (ps[1].x + ps[1].y);
+        if (kOwn) {
+          const float m = m_ref, l = l_run;
+          m_ref = m_other; l_run = l_other;
+          m_other = m; l_other = l;
+        }
       }
       if (kTurns)
         for (int j = max(n, 0); j < tiles; j++) {  // nothing to do while the other group works on
@@ -847,7 +866,19 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
           named_arrive_64(its_turn);
         }
       if (n <= 0) continue;
-      const float inv = 1.0f / l_run;
+      float inv, f0 = 1.f, f1 = 1.f;  // kOwn: what the even and the odd tiles' O are weighted with
+      if (kOwn) {
+        const bool last_odd = (n & 1) == 0;
+        const float m0 = last_odd ? m_ref : m_other, m1 = last_odd ? m_other : m_ref, l0 = last_odd ? l_run : l_other, l1 = last_odd ? l_other : l_run;
+        const float m = fmaxf(m0, m1);
+        f0 = ex2_approx(m0 - m);
+        f1 = ex2_approx(m1 - m);
+        inv = 1.0f / (l0 * f0 + l1 * f1);
+        f0 *= inv;
+        f1 *= inv;
+      } else {
+        inv = 1.0f / l_run;
+      }
       mbar_wait(pv_done(g, (step - 1) & 1u), ((step - 1) >> 1) & 1u);
       tc_fence_after();
       uint16_t *o = out + ((size_t)(tok0 + t) * n_heads + p.kvh * G + hl) * D;
@@ -857,6 +888,21 @@ attn_prefill_pair_kernel(const __grid_constant__ CUtensorMap kv_map, long long r
         tmem_ld_32x32(o_addr + c, v[0]);
         tmem_ld_32x32(o_addr + c + 32, v[1]);
         tmem_ld_wait();
+        if (kOwn) {
+#pragma unroll
+          for (int i = 0; i < 64; i++) v[i >> 5][i & 31] = __float_as_uint(__uint_as_float(v[i >> 5][i & 31]) * f0);
+          if (n > 1) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+              uint32_t u[32];
+              tmem_ld_32x32(o_addr + D + 32 * h, u);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; i++) v[h][i] = __float_as_uint(fmaf(__uint_as_float(u[i]), f1, __uint_as_float(v[h][i])));
+            }
+          }
+          inv = 1.f;
+        }
         if (c == D - 64) {  // everything is in registers: the next pass may write O
           tc_fence_before();
           __syncwarp();

@@ -543,6 +543,49 @@ def test_attention_prefill_of_many_blocks(nh, nkv, d, BT, page_size, kind):
         row += n
 
 
+@pytest.mark.parametrize("nh,nkv,BT", [(32, 8, 32), (32, 4, 16)])
+def test_attention_prefill_heads_of_64_bits_in_pairs_and_alone(nh, nkv, BT):
+    """Heads of 64: a query block has the same bits whether it is one of a pair or alone in its CTA, so the number of blocks of a pass does
+    not move its error (even and odd key tiles have a maximum of their own in both forms).  Prompts of 1 to 40 tiles, some behind a cache,
+    keys that grow with their position, one block of an odd sequence left over."""
+    d, page_size = 64, 64
+    g = torch.Generator(device=DEV); g.manual_seed(nh + nkv)
+    rng = np.random.default_rng(nkv)
+    lens, past = [2500, 65, 700, 1, 1300], [0, 200, 0, 0, 64]
+    while sum(-(-n // BT) for n in lens) * nkv <= 6 * 148 // 2 + nkv:
+        lens.append(int(rng.integers(1, 900))); past.append(int(rng.choice([0, 100])))
+    total = [a + b for a, b in zip(past, lens)]
+    per = [-(-n // page_size) for n in total]
+    pt = np.zeros((len(lens), max(per)), np.int32)
+    perm = rng.permutation(sum(per))
+    for s, at in enumerate(np.cumsum([0] + per[:-1])):
+        pt[s, :per[s]] = perm[at:at + per[s]]
+    pool = torch.randn((sum(per), 2, nkv, page_size, d), device=DEV, generator=g)
+    for s, p in enumerate(per):
+        pool[torch.as_tensor(pt[s, :p].astype(np.int64), device=DEV), 0] *= 0.3 + torch.arange(p * page_size, device=DEV).reshape(p, 1, page_size, 1) / 600.0
+    pool = pool.to(torch.bfloat16)
+    tok0, qlen, pos0, ptrow, t = [], [], [], [], 0
+    for s, n in enumerate(lens):
+        for k in range(0, n, BT):
+            tok0.append(t + k); qlen.append(min(BT, n - k)); pos0.append(past[s] + k); ptrow.append(s)
+        t += n
+    q = torch.randn((t, nh * d), device=DEV, generator=g).to(torch.bfloat16)
+    dpt, args = dev_i32(pt), [np.asarray(a, np.int32) for a in (tok0, qlen, pos0, ptrow)]
+
+    def run(step):
+        out = torch.full((t, nh * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        for at in range(0, len(tok0), step):
+            part = [dev_i32(a[at:at + step]) for a in args]
+            check(lib().dis_k_attn_prefill(ptr(q), ptr(pool), pool.shape[0], ptr(dpt), pt.shape[1], *[ptr(p) for p in part], ptr(out), len(tok0[at:at + step]), nh, nkv, d, page_size,
+                                           torch.cuda.current_stream().cuda_stream))
+        return out
+
+    together, alone = run(len(tok0)), run(6 * 148 // 2 // nkv)
+    sync()
+    assert len(tok0) * nkv > 6 * 148 // 2 and not bool(torch.isnan(alone.float()).any())
+    assert torch.equal(together, alone)
+
+
 @pytest.mark.parametrize("nh,nkv,page_size,BT", [(8, 1, 8, 16), (8, 2, 64, 16), (8, 2, 64, 32), (16, 2, 128, 16), (16, 4, 16, 32)])
 @pytest.mark.parametrize("past", [0, 63, 200])
 def test_attention_prefill_heads_of_64(nh, nkv, page_size, past, BT):
