@@ -66,16 +66,19 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 // in a warp is a chain of latencies (barrier, ldmatrix, MMAs, shuffles, exponential, MMAs).  Tokens are the MMAs' rows and the group's
 // query heads (<= 8) their eight columns: S^T = K Q^T and O^T = V^T P^T fill the m16n8k16 shape, half the MMAs and half the accumulators (D / 2
 // registers) of heads as 16 padded rows.  P^T is turned from accumulator to operand by movmatrix, and two accumulators halve S^T's chain of MMAs.
-// From graphs, against heads as rows (32 / 8 heads of 128): 1 x 8000 keys 15.0 -> 14.7 us, 8 x 512 8.8 -> 8.4, 32 x 512 13.9 -> 13.8, 64 x 575
-// 27.7 -> 28.4, 32 ragged ones of 500 to 6000 77.1 -> 74.8; heads of 64 (32 / 4): 32 x 512 9.0 -> 8.6, 64 x 2000 23.5 -> 24.4.
-// Eight warps in two groups lose nearly everywhere (8 x 512 9.4 us, 32 x 512 14.6, 32 x 100 7.6 against 6.7: more to start, to merge and to
-// keep resident); see attn_dispatch for where they stay.
+// From graphs, against heads as rows with weights in one half (32 / 8 heads of 128): 1 x 8000 keys 15.0 -> 14.7 us, 8 x 512 8.7 -> 8.5, 32 x 512
+// 13.8 -> 14.0, 64 x 575 27.9 -> 28.8, 32 ragged ones of 500 to 6000 76.9 -> 76.8; heads of 64 (32 / 4): 32 x 512 9.0 -> 8.8, 64 x 2000 23.5 -> 24.4.
+// Eight warps in two groups lose nearly everywhere (weights in one half: 8 x 512 9.4 us against 8.4, 32 x 512 14.6 / 13.8, 32 x 100 7.6 / 6.7: more to
+// start, to merge and to keep resident); see attn_dispatch for where they stay.
+//
+// A weight goes into the V^T P^T product as two bf16, its upper half and the rest: rounded to one it was most of the error, the more so the fewer
+// warps have a maximum (a weight of exactly 1) of their own.  Error of 32 ragged histories against 64 bits, 2-norm: 1.91e-3 with one half and four warps,
+// 1.87e-3 with eight, 1.66e-3 with two halves, which is the rounding of the output; 1 to 2.5 % of the time (one CTA per SM: 7 %).
 //
 // A ragged batch in one wave is as slow as its longest history if every history has a CTA of its own.  So (kShared) the CTAs of a cluster lay
 // the histories of up to eight tokens end to end and take equal shares; pieces of one history meet in the shared memory of the CTA that has its
-// first: those 74.8 us are 55.0.  The cluster's start and end cost 2 to 4 us, the pieces 5 more: attn_sharing_pays.
+// first: those 76.8 us are 56.2.  The cluster's start and end cost 2 to 4 us, the pieces 5 more: attn_sharing_pays.
 //
-// P is rounded to bf16 for the P.V MMA (the usual flash-attention choice).
 // Rows past the context inside a box hold stale (finite) cache contents and get probability 0; the
 // engine zero-fills the pool once so that they can never be NaN.
 // Decode steps fuse the RoPE + KV-write stage into this kernel (rope.qkv != nullptr): the CTA sums the split-K
@@ -209,7 +212,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   };
 
   // The last warp loads and does nothing else, the computing warps free a stage each for themselves: no barrier of the whole block per
-  // tile (with one, the longest history of a ragged batch took 1.04 us per tile, without it 0.83, and 0.79 with tokens as rows).
+  // tile (with one, the longest history of a ragged batch took 1.04 us per tile, without it 0.83).
   if (warp == kAttnWarps) {
     if (lane == 0) {
       int k = 0;  // stages handed out so far
@@ -364,21 +367,27 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
           p[e] = exp2f(fmaf(p[e], scale_log2, -m_new));
           p[2 + e] = exp2f(fmaf(p[2 + e], scale_log2, -m_new));
         }
-        // the sums take the weights as P V takes them, rounded: the weights of a row then add up to one
+        l_run[0] = l_run[0] * corr[0] + (p[0] + p[2]);
+        l_run[1] = l_run[1] * corr[1] + (p[1] + p[3]);
         const uint32_t p01 = float2_to_bf16x2(p[0], p[1]), p23 = float2_to_bf16x2(p[2], p[3]);
         const float2 r01 = bf16x2_to_float2(p01), r23 = bf16x2_to_float2(p23);
-        l_run[0] = l_run[0] * corr[0] + (r01.x + r23.x);
-        l_run[1] = l_run[1] * corr[1] + (r01.y + r23.y);
         const uint32_t pb0 = movmatrix(p01), pb1 = movmatrix(p23);
+        const uint32_t pl0 = movmatrix(float2_to_bf16x2(p[0] - r01.x, p[1] - r01.y)), pl1 = movmatrix(float2_to_bf16x2(p[2] - r23.x, p[3] - r23.y));
 #pragma unroll
         for (int m = 0; m < KS; m++) { oacc[m][0] *= corr[0]; oacc[m][1] *= corr[1]; oacc[m][2] *= corr[0]; oacc[m][3] *= corr[1]; }
         // ---- O^T += V^T P^T : A = V^T by ldmatrix.trans of the [tokens][dims] tile
 #pragma unroll
-        for (int m = 0; m < KS; m++) {
-          const int c = m * 2 + (mi & 1);
-          uint32_t a0, a1, a2, a3;
-          ldmatrix_x4_trans(vs_addr + (c >> 3) * Cfg::kHalfBytes + v_tok * 128 + (((c & 7) ^ (v_tok & 7)) << 4), a0, a1, a2, a3);
-          mma_bf16_16816(oacc[m], a0, a1, a2, a3, pb0, pb1);
+        for (int m = 0; m < KS; m += 2) {  // two at a time: neighbouring products go to different accumulators
+          uint32_t v[2][4];
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int c = (m + h) * 2 + (mi & 1);
+            ldmatrix_x4_trans(vs_addr + (c >> 3) * Cfg::kHalfBytes + v_tok * 128 + (((c & 7) ^ (v_tok & 7)) << 4), v[h][0], v[h][1], v[h][2], v[h][3]);
+          }
+#pragma unroll
+          for (int h = 0; h < 2; h++) mma_bf16_16816(oacc[m + h], v[h][0], v[h][1], v[h][2], v[h][3], pb0, pb1);
+#pragma unroll
+          for (int h = 0; h < 2; h++) mma_bf16_16816(oacc[m + h], v[h][0], v[h][1], v[h][2], v[h][3], pl0, pl1);
         }
       }
       __syncwarp();
@@ -685,7 +694,7 @@ __global__ void attn_combine_kernel(const float *__restrict__ scratch, uint16_t 
 bool attn_may_share(int n_splits, int T, int n_kv) { return n_splits == 1 && T > 1 && (long long)T * n_kv <= 2 * kNumSMs; }
 // Which takes longer, us: the longest history alone or the largest share of a cluster (0.8 us a tile of heads of 128, 0.5 of 64), neither less than
 // the stream of all keys and values at 6.5 TB/s; sharing costs 8 on top.  Of 25 ragged and 19 equal batches (heads of 128: 20 and 32 histories, of
-// 64: 40 and 64; 100 to 7000 keys) it takes the slower form of three, by 3 % at most.
+// 64: 40 and 64; 100 to 7000 keys) it takes the slower form of two, by 0.2 and 8 %.
 bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d) {
   const int n = T < kAttnMaxCluster ? T : kAttnMaxCluster;
   long long total = 0, most = 0, share = 0;
@@ -752,8 +761,8 @@ static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const Att
   const int G = n_heads / n_kv;  // query heads per kv head, all handled by one CTA
   share = share && attn_may_share(n_splits, T, n_kv);
   // Heads of 64: three CTAs of four computing warps fit an SM, or two of eight.  Just above three per SM the former leave most of a second round
-  // empty, the latter fill theirs: 512 CTAs, 2000 keys 53.4 -> 45.6 us, 700 22.3 -> 20.2, 200 11.6 -> 11.6; 448 x 2500 58.4 -> 54.0 (200 keys 10.4 -> 11.1).
-  // Elsewhere four warps are ahead: 304 x 700 12.0 against 17.9, 640 x 700 24.1 against 28.5, 1024 x 2500 104.6 against 110.1.
+  // empty, the latter fill theirs: 512 CTAs, 2500 keys 67.0 -> 56.4 us, 700 23.0 -> 20.6, 200 11.9 -> 11.8; 448 x 2500 59.9 -> 55.4 (200 keys 10.8 -> 11.2).
+  // Elsewhere four warps are ahead: 304 x 700 12.3 against 18.0, 640 x 700 24.5 against 28.9, 1024 x 2500 106.5 against 111.5.
   const long long ctas = (long long)n_splits * T * n_kv;
   const bool two_groups = d == 64 && ctas > 3 * kNumSMs && ctas <= 4 * kNumSMs;
 #define DIS_ATTN_GO(DD, GG, NG, SH) \
@@ -779,9 +788,10 @@ cudaError_t launch_attn_paged(const TmaMap &kv_map, long long row0, const uint16
                               int n_splits, int T, int n_heads, int n_kv, int d, int page_size, cudaStream_t st) {
   AttnRope none{};
   // The lengths are on the device; the page table's width bounds them, and from about these on a ragged batch gains (us, whole / shared; heads of 128, 32
-  // histories of up to 1100 17.8 / 19.1, 1500 22.3 / 21.8, 3000 39.6 / 33.4, 7000 86.7 / 63.4; heads of 64, 64 of up to 1500 16.2 / 17.4, 2000
-  // 19.8 / 19.5, 4500 38.7 / 28.7).  Equal histories lose there: 32 x 2000 42.3 / 44.6, 32 x 6000 115.4 / 118.9, heads of 64, 64 x 4000 43.2 / 44.7.
-  const bool share = (long long)max_pages * page_size > (d == 128 ? 1536 : 2048);
+  // histories of up to 1100 18.3 / 20.2, 1500 23.0 / 22.9, 2000 29.1 / 27.2, 7000 89.0 / 64.1, 20 of up to 2000 24.9 / 24.1; heads of 64, 64 of up
+  // to 1500 16.7 / 17.7, 2000 20.6 / 19.7, 4500 39.9 / 29.3).  Equal histories lose there: 32 x 2000 42.9 / 44.3, 32 x 6000 114.7 / 116.1,
+  // 20 x 2000 29.5 / 33.7, heads of 64, 64 x 4000 42.8 / 44.6.
+  const bool share = (long long)max_pages * page_size > (d == 128 ? 1792 : 2048);
   return attn_dispatch(kv_map, row0, none, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
                        page_size, share, st);
 }

@@ -393,6 +393,38 @@ def test_attention_of_ragged_histories(nh, nkv, d, page_size, T, n_splits, patte
         assert err <= 8e-3, (t, int(ctx[t]), float(err))
 
 
+@pytest.mark.parametrize("nh,nkv,d", [(32, 8, 128), (32, 4, 64)])
+@pytest.mark.parametrize("T,n_splits,most", [(2, 4, 900), (24, 1, 600), (40, 1, 3000), (130, 1, 300)])
+def test_attention_is_as_close_as_its_output_s_type(nh, nkv, d, T, n_splits, most):
+    """Decode attention's error against 64 bits is that of rounding the result to bf16 (weights go into the product as two halves: in one, the
+    error is 10 % larger): slices, whole histories, histories that a cluster shares, more CTAs than fit at once."""
+    rng = np.random.default_rng(T + d)
+    page_size = 64
+    ctx = np.exp(rng.uniform(np.log(most / 12), np.log(most), T)).astype(np.int32)
+    ctx[T // 2] = most
+    need = [-(-int(c) // page_size) for c in ctx]
+    table = np.zeros((T, max(need)), np.int32)
+    order = rng.permutation(sum(need))
+    for t, at in enumerate(np.cumsum([0] + need[:-1])):
+        table[t, :need[t]] = order[at:at + need[t]]
+    g = torch.Generator(device=DEV); g.manual_seed(T + d)
+    pool = torch.randn((sum(need), 2, nkv, page_size, d), device=DEV, generator=g).to(torch.bfloat16)
+    q = (torch.randn((T, nh * d), device=DEV, generator=g) * 1.5).to(torch.bfloat16)
+    out = torch.empty_like(q)
+    scratch = torch.empty(max(1, lib().dis_k_attn_scratch_elems(T, nh, d, n_splits)), device=DEV)
+    rows, dctx, dtab = dev_i32(np.arange(T, dtype=np.int32)), dev_i32(ctx), dev_i32(table)
+    check(lib().dis_k_attn_paged(ptr(q), ptr(pool), pool.shape[0], ptr(dtab), table.shape[1], ptr(rows), ptr(dctx), ptr(out), ptr(scratch), n_splits, T, nh, nkv, d, page_size, None))
+    sync()
+    ref = torch.empty(q.shape, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        kv = pool[torch.from_numpy(table[t, :need[t]].astype(np.int64)).to(DEV)].double()
+        k, v = (kv[:, c].permute(1, 0, 2, 3).reshape(nkv, -1, d)[:, :int(ctx[t])].repeat_interleave(nh // nkv, 0) for c in (0, 1))
+        w = torch.softmax((k @ q[t].double().view(nh, d, 1))[..., 0] * d ** -0.5, -1)
+        ref[t] = (w[:, None] @ v)[:, 0].flatten()
+    err, rounding = (out.double() - ref).norm(), (ref.to(torch.bfloat16).double() - ref).norm()
+    assert err <= 1.03 * rounding, float(err / rounding)
+
+
 def test_attention_long_context_tiles():
     rng = np.random.default_rng(3)
     d, nh, nkv, page_size = 128, 4, 1, 64
