@@ -1309,11 +1309,11 @@ __global__ void __launch_bounds__(256) stack_ssm_step_kernel(const float *__rest
 
 // Passes of single tokens whose layout the kernel above takes: a norm's stretch is whole heads, at most eight (a cluster), and holds whole groups of
 // heads (a group's tail has one owner); sizes and rows in fours, up to 128.
-bool stack_ssm_step_ok(const float *proj, long long ld, const float *cstate, int x_off, int C, int taps, int H, int N, int P, int G, int parts) {
+bool stack_ssm_step_ok(const float *proj, const float *slices, long long ld, const float *cstate, int x_off, int C, int taps, int H, int N, int P, int G, int parts) {
   if (N > kSsmStepMax || P > kSsmStepMax || N % 4 || P % 4 || (H * P) % parts || taps < 1 || taps > kConvMaxTaps) return false;
   const int per = H * P / parts;
   if (per % P || per / P > 8 || (per / P) % (H / G) || H > (1 << 30) / P) return false;
-  return ld % 4 == 0 && x_off % 4 == 0 && C % 4 == 0 && reinterpret_cast<uintptr_t>(proj) % 16 == 0 && (taps == 1 || reinterpret_cast<uintptr_t>(cstate) % 16 == 0);
+  return ld % 4 == 0 && x_off % 4 == 0 && C % 4 == 0 && (reinterpret_cast<uintptr_t>(proj) | reinterpret_cast<uintptr_t>(slices)) % 16 == 0 && (taps == 1 || reinterpret_cast<uintptr_t>(cstate) % 16 == 0);
 }
 cudaError_t launch_stack_ssm_step(const float *proj, long long ld, int n_part, long long stride, const float *bias, int x_off, int dt_off, int C, int H, int taps,
                                   const float *cw, const float *cb, const float *vec, float *cstate, const StackSpans &sp, float *state, const float *w, int N, int P,
