@@ -44,6 +44,12 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t &r0, u
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr));
 }
+// 2^x; results below 2^-126 are zero (as weights they are lost beside one of 1)
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // an 8x8 matrix of bf16 pairs transposed across the warp
 __device__ __forceinline__ uint32_t movmatrix(uint32_t v) {
   uint32_t r;
@@ -67,17 +73,19 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 // query heads (<= 8) their eight columns: S^T = K Q^T and O^T = V^T P^T fill the m16n8k16 shape, half the MMAs and half the accumulators (D / 2
 // registers) of heads as 16 padded rows.  P^T is turned from accumulator to operand by movmatrix, and two accumulators halve S^T's chain of MMAs.
 // From graphs, against heads as rows with weights in one half (32 / 8 heads of 128): 1 x 8000 keys 15.0 -> 14.7 us, 8 x 512 8.7 -> 8.5, 32 x 512
-// 13.8 -> 14.0, 64 x 575 27.9 -> 28.8, 32 ragged ones of 500 to 6000 76.9 -> 76.8; heads of 64 (32 / 4): 32 x 512 9.0 -> 8.8, 64 x 2000 23.5 -> 24.4.
+// 13.7 -> 13.9, 64 x 575 27.7 -> 28.4, 32 ragged ones of 500 to 6000 77.1 -> 74.9; heads of 64 (32 / 4): 32 x 512 9.1 -> 8.7, 64 x 2000 23.4 -> 24.4.
 // Eight warps in two groups lose nearly everywhere (weights in one half: 8 x 512 9.4 us against 8.4, 32 x 512 14.6 / 13.8, 32 x 100 7.6 / 6.7: more to
 // start, to merge and to keep resident); see attn_dispatch for where they stay.
 //
 // A weight goes into the V^T P^T product as two bf16, its upper half and the rest: rounded to one it was most of the error, the more so the fewer
-// warps have a maximum (a weight of exactly 1) of their own.  Error of 32 ragged histories against 64 bits, 2-norm: 1.91e-3 with one half and four warps,
-// 1.87e-3 with eight, 1.66e-3 with two halves, which is the rounding of the output; 1 to 2.5 % of the time (one CTA per SM: 7 %).
+// warps have a maximum (a weight of exactly 1) of their own.  Groups of up to four heads leave columns free, so a head has two: K Q^T forms its
+// scores in both, and V^T P^T multiplies the halves in one product, to be added at the end.  Groups of eight take a second product (1 to 2 % of the
+// time, 6 % where an SM has one CTA).  Error of 32 ragged histories against 64 bits, 2-norm: 1.91e-3 with one half and four warps, 1.87e-3 with
+// eight, 1.66e-3 with two halves, which is the rounding of the output.
 //
 // A ragged batch in one wave is as slow as its longest history if every history has a CTA of its own.  So (kShared) the CTAs of a cluster lay
 // the histories of up to eight tokens end to end and take equal shares; pieces of one history meet in the shared memory of the CTA that has its
-// first: those 76.8 us are 56.2.  The cluster's start and end cost 2 to 4 us, the pieces 5 more: attn_sharing_pays.
+// first: those 74.9 us are 55.4.  The cluster's start and end cost 2 to 4 us, the pieces 5 more: attn_sharing_pays.
 //
 // Rows past the context inside a box hold stale (finite) cache contents and get probability 0; the
 // engine zero-fills the pool once so that they can never be NaN.
@@ -128,6 +136,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   using Cfg = AttnCfg<D>;
   constexpr int kAttnThreads = NG * 128, kAttnWarps = NG * 4;  // those that compute
   static_assert(!kShared || NG == 1, "a shared history's stages are counted for one group");
+  constexpr bool kTwice = G <= 4;  // a head has two columns: the weights' upper halves go through one, the rest through the other
   constexpr int KS = D / 16;  // k-steps of the K Q^T MMA, m-tiles of the V^T P^T MMA
   static_assert(kAttnWarps * G * D * 4 <= Cfg::kStageBytes, "the warps' states are merged in one stage");
 
@@ -303,13 +312,14 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
       }
     }
 
-    // ---- Q^T as the B operand: column g = head g (g < G), everything else zero
+    // ---- Q^T as the B operand: column g = head g; where the group leaves columns free, the next G repeat it (kTwice)
     uint32_t qb[KS][2];
 #pragma unroll
     for (int ks = 0; ks < KS; ks++) {
       qb[ks][0] = 0u; qb[ks][1] = 0u;
-      if (g < G) {
-        const uint16_t *qp = fused ? s_q[g] + ks * 16 + tq * 2 : q + ((size_t)t * n_heads + h0 + g) * D + ks * 16 + tq * 2;
+      if (g < (kTwice ? 2 * G : G)) {
+        const int hq = kTwice ? g % G : g;
+        const uint16_t *qp = fused ? s_q[hq] + ks * 16 + tq * 2 : q + ((size_t)t * n_heads + h0 + hq) * D + ks * 16 + tq * 2;
         qb[ks][0] = *reinterpret_cast<const uint32_t *>(qp);
         qb[ks][1] = *reinterpret_cast<const uint32_t *>(qp + 8);
       }
@@ -362,32 +372,30 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
           mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
           const float m_new = fmaxf(m_run[e], mx * scale_log2);  // finite: token wtok is valid
-          corr[e] = exp2f(m_run[e] - m_new);        // 0 on the first tile
+          corr[e] = ex2_ftz(m_run[e] - m_new);      // 0 on the first tile
           m_run[e] = m_new;
-          p[e] = exp2f(fmaf(p[e], scale_log2, -m_new));
-          p[2 + e] = exp2f(fmaf(p[2 + e], scale_log2, -m_new));
+          p[e] = ex2_ftz(fmaf(p[e], scale_log2, -m_new));
+          p[2 + e] = ex2_ftz(fmaf(p[2 + e], scale_log2, -m_new));
         }
         l_run[0] = l_run[0] * corr[0] + (p[0] + p[2]);
         l_run[1] = l_run[1] * corr[1] + (p[1] + p[3]);
         const uint32_t p01 = float2_to_bf16x2(p[0], p[1]), p23 = float2_to_bf16x2(p[2], p[3]);
         const float2 r01 = bf16x2_to_float2(p01), r23 = bf16x2_to_float2(p23);
-        const uint32_t pb0 = movmatrix(p01), pb1 = movmatrix(p23);
-        const uint32_t pl0 = movmatrix(float2_to_bf16x2(p[0] - r01.x, p[1] - r01.y)), pl1 = movmatrix(float2_to_bf16x2(p[2] - r23.x, p[3] - r23.y));
+        const uint32_t q01 = float2_to_bf16x2(p[0] - r01.x, p[1] - r01.y), q23 = float2_to_bf16x2(p[2] - r23.x, p[3] - r23.y);
+        // kTwice: columns G .. 2 G take the rest
+        const bool rest = kTwice && tq * 2 >= G;
+        const uint32_t pb0 = movmatrix(G == 1 ? (p01 & 0xffffu) | (q01 << 16) : rest ? q01 : p01), pb1 = movmatrix(G == 1 ? (p23 & 0xffffu) | (q23 << 16) : rest ? q23 : p23);
+        const uint32_t pl0 = kTwice ? 0u : movmatrix(q01), pl1 = kTwice ? 0u : movmatrix(q23);
 #pragma unroll
         for (int m = 0; m < KS; m++) { oacc[m][0] *= corr[0]; oacc[m][1] *= corr[1]; oacc[m][2] *= corr[0]; oacc[m][3] *= corr[1]; }
         // ---- O^T += V^T P^T : A = V^T by ldmatrix.trans of the [tokens][dims] tile
 #pragma unroll
-        for (int m = 0; m < KS; m += 2) {  // two at a time: neighbouring products go to different accumulators
-          uint32_t v[2][4];
-#pragma unroll
-          for (int h = 0; h < 2; h++) {
-            const int c = (m + h) * 2 + (mi & 1);
-            ldmatrix_x4_trans(vs_addr + (c >> 3) * Cfg::kHalfBytes + v_tok * 128 + (((c & 7) ^ (v_tok & 7)) << 4), v[h][0], v[h][1], v[h][2], v[h][3]);
-          }
-#pragma unroll
-          for (int h = 0; h < 2; h++) mma_bf16_16816(oacc[m + h], v[h][0], v[h][1], v[h][2], v[h][3], pb0, pb1);
-#pragma unroll
-          for (int h = 0; h < 2; h++) mma_bf16_16816(oacc[m + h], v[h][0], v[h][1], v[h][2], v[h][3], pl0, pl1);
+        for (int m = 0; m < KS; m++) {
+          const int c = m * 2 + (mi & 1);
+          uint32_t a0, a1, a2, a3;
+          ldmatrix_x4_trans(vs_addr + (c >> 3) * Cfg::kHalfBytes + v_tok * 128 + (((c & 7) ^ (v_tok & 7)) << 4), a0, a1, a2, a3);
+          mma_bf16_16816(oacc[m], a0, a1, a2, a3, pb0, pb1);
+          if (!kTwice) mma_bf16_16816(oacc[m], a0, a1, a2, a3, pl0, pl1);
         }
       }
       __syncwarp();
@@ -403,6 +411,18 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
       k0++;
     }
     sync_compute();
+    if (kTwice) {
+#pragma unroll
+      for (int m = 0; m < KS; m++) {
+        if (G == 1) {
+          oacc[m][0] += oacc[m][1];
+          oacc[m][2] += oacc[m][3];
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; i++) oacc[m][i] += __shfl_xor_sync(0xffffffffu, oacc[m][i], G / 2);
+        }
+      }
+    }
     float *s_o = reinterpret_cast<float *>(smem + stage * Cfg::kStageBytes);
 #pragma unroll
     for (int e = 0; e < 2; e++) {
@@ -689,16 +709,21 @@ __global__ void attn_combine_kernel(const float *__restrict__ scratch, uint16_t 
 }
 
 // Whole histories can be shared (slices are a share already; slices merged inside a cluster instead of by the combine pass took 13.0 us for 8 x 512
-// where the two kernels take 8.4, and 22.8 against 16.5 for 8 x 2000: a cluster's start costs more than the launch), in one wave of two CTAs per
-// SM: beyond it the hardware levels by itself, and whole clusters find room later than single CTAs.
-bool attn_may_share(int n_splits, int T, int n_kv) { return n_splits == 1 && T > 1 && (long long)T * n_kv <= 2 * kNumSMs; }
-// Which takes longer, us: the longest history alone or the largest share of a cluster (0.8 us a tile of heads of 128, 0.5 of 64), neither less than
-// the stream of all keys and values at 6.5 TB/s; sharing costs 8 on top.  Of 25 ragged and 19 equal batches (heads of 128: 20 and 32 histories, of
-// 64: 40 and 64; 100 to 7000 keys) it takes the slower form of two, by 0.2 and 8 %.
+// where the two kernels take 8.5, and 22.8 against 16.5 for 8 x 2000: a cluster's start costs more than the launch), as far as the clusters that
+// have eight tokens run at once (33 of two CTAs per SM by the occupancy query of one B200): 36 of them in two rounds take 33.0 us where single CTAs
+// take 23.8 (heads of 64, 72 histories of up to 2500).
+constexpr int kAttnClusters = 32;
+bool attn_may_share(int n_splits, int T, int n_kv) {
+  const long long full = T >= kAttnMaxCluster ? (long long)(T / kAttnMaxCluster) * n_kv : ((long long)T * n_kv + kAttnMaxCluster - 1) / kAttnMaxCluster;
+  return n_splits == 1 && T > 1 && full <= kAttnClusters && (long long)T * n_kv <= 2 * kNumSMs;
+}
+// Which takes longer, us: the longest history alone or the largest share of a cluster (0.8 us a tile of heads of 128, 0.5 of 64), the largest of the
+// clusters that have to wait on top, neither less than the stream of all keys and values at 6.5 TB/s; sharing costs 8.  Of 25 ragged and 19 equal
+// batches (heads of 128: 20 and 32 histories, of 64: 40 and 64; 100 to 7000 keys) it takes the slower form of two, by 1 and 5 %.
 bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d) {
-  const int n = T < kAttnMaxCluster ? T : kAttnMaxCluster;
-  long long total = 0, most = 0, share = 0;
-  for (int t0 = 0; t0 < T; t0 += n) {
+  const int n = T < kAttnMaxCluster ? T : kAttnMaxCluster, at_once = std::max(1, kAttnClusters / n_kv);
+  long long total = 0, most = 0, share = 0, later = 0;
+  for (int t0 = 0, k = 0; t0 < T; t0 += n, k++) {
     long long sum = 0;
     for (int t = t0; t < std::min(t0 + n, T); t++) {
       const long long tiles = std::max(1, (ctx[t] + kAttnTile - 1) / kAttnTile);
@@ -706,10 +731,11 @@ bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d) {
       most = std::max(most, tiles);
     }
     total += sum;
-    share = std::max(share, (sum + n - 1) / n);
+    long long &round = T >= kAttnMaxCluster && k >= at_once ? later : share;
+    round = std::max(round, (sum + n - 1) / n);
   }
   const double tile = d == 128 ? 0.8 : 0.5, stream = (double)total * n_kv * (kAttnTile * d * 4) / 6.5e6;  // us
-  return std::max(share * tile, stream) + 8.0 < std::max(most * tile, stream);
+  return std::max((share + later) * tile, stream) + 8.0 < std::max(most * tile, stream);
 }
 
 size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits) {
@@ -761,8 +787,8 @@ static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const Att
   const int G = n_heads / n_kv;  // query heads per kv head, all handled by one CTA
   share = share && attn_may_share(n_splits, T, n_kv);
   // Heads of 64: three CTAs of four computing warps fit an SM, or two of eight.  Just above three per SM the former leave most of a second round
-  // empty, the latter fill theirs: 512 CTAs, 2500 keys 67.0 -> 56.4 us, 700 23.0 -> 20.6, 200 11.9 -> 11.8; 448 x 2500 59.9 -> 55.4 (200 keys 10.8 -> 11.2).
-  // Elsewhere four warps are ahead: 304 x 700 12.3 against 18.0, 640 x 700 24.5 against 28.9, 1024 x 2500 106.5 against 111.5.
+  // empty, the latter fill theirs: 512 CTAs, 2500 keys 64.3 -> 55.3 us, 700 22.0 -> 20.2, 200 11.6 -> 11.7; 448 x 2500 58.2 -> 54.2 (200 keys 10.5 -> 11.1).
+  // Elsewhere four warps are ahead: 304 x 700 12.1 against 17.8, 640 x 700 23.9 against 28.5, 1024 x 2500 103.8 against 110.1.
   const long long ctas = (long long)n_splits * T * n_kv;
   const bool two_groups = d == 64 && ctas > 3 * kNumSMs && ctas <= 4 * kNumSMs;
 #define DIS_ATTN_GO(DD, GG, NG, SH) \
@@ -788,10 +814,11 @@ cudaError_t launch_attn_paged(const TmaMap &kv_map, long long row0, const uint16
                               int n_splits, int T, int n_heads, int n_kv, int d, int page_size, cudaStream_t st) {
   AttnRope none{};
   // The lengths are on the device; the page table's width bounds them, and from about these on a ragged batch gains (us, whole / shared; heads of 128, 32
-  // histories of up to 1100 18.3 / 20.2, 1500 23.0 / 22.9, 2000 29.1 / 27.2, 7000 89.0 / 64.1, 20 of up to 2000 24.9 / 24.1; heads of 64, 64 of up
-  // to 1500 16.7 / 17.7, 2000 20.6 / 19.7, 4500 39.9 / 29.3).  Equal histories lose there: 32 x 2000 42.9 / 44.3, 32 x 6000 114.7 / 116.1,
-  // 20 x 2000 29.5 / 33.7, heads of 64, 64 x 4000 42.8 / 44.6.
-  const bool share = (long long)max_pages * page_size > (d == 128 ? 1792 : 2048);
+  // histories of up to 1100 17.9 / 19.4, 1500 22.5 / 22.3, 2000 28.5 / 26.7, 7000 87.0 / 63.8, 20 of up to 2000 24.1 / 22.3; heads of 64, 64 of up
+  // to 1500 16.5 / 17.5, 2000 20.2 / 19.6, 4500 38.9 / 29.1).  Where clusters have to wait, those of the last tokens, only long ones do: 36 of up to 2500
+  // 34.0 / 36.8, 6000 73.7 / 61.4.  Equal histories lose: 32 x 2000 42.2 / 44.7, 32 x 6000 115.1 / 119.1, heads of 64, 64 x 4000 42.7 / 44.5.
+  const bool waits = (long long)((T + kAttnMaxCluster - 1) / kAttnMaxCluster) * n_kv > kAttnClusters && T >= kAttnMaxCluster;
+  const bool share = (long long)max_pages * page_size > (waits ? 4096 : d == 128 ? 1792 : 2048);
   return attn_dispatch(kv_map, row0, none, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
                        page_size, share, st);
 }
