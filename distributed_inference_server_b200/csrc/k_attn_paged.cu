@@ -85,7 +85,8 @@ __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint3
 //
 // A ragged batch in one wave is as slow as its longest history if every history has a CTA of its own.  So (kShared) the CTAs of a cluster lay
 // the histories of up to eight tokens end to end and take equal shares; pieces of one history meet in the shared memory of the CTA that has its
-// first: those 74.9 us are 55.4.  The cluster's start and end cost 2 to 4 us, the pieces 5 more: attn_sharing_pays.
+// first: those 74.9 us are 53.8.  The cluster's start and end cost 2 to 3 us, the pieces as much again: attn_sharing_pays.  (Fetched one after the
+// other, a load and a branch at a time, the pieces cost 5: 55.4.)
 //
 // Rows past the context inside a box hold stale (finite) cache contents and get probability 0; the
 // engine zero-fills the pool once so that they can never be NaN.
@@ -113,11 +114,19 @@ __device__ __forceinline__ float4 attn_sum_slices(const float *p, int n, long lo
   return a;
 }
 
-__device__ __forceinline__ float ld_cluster(const float *p, uint32_t rank) {
+// From another CTA's shared memory.  No memory clobber: several are in flight; they keep their order with the cluster barriers, which are volatile too.
+__device__ __forceinline__ float2 ld_cluster2(const float2 *p, uint32_t rank) {
   uint32_t a;
-  float v;
+  float2 v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ float4 ld_cluster4(const float *p, uint32_t rank) {
+  uint32_t a;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
   return v;
 }
 __device__ __forceinline__ void attn_cluster_sync() {
@@ -150,9 +159,9 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   auto empty_bar = [&](int s) { return bar_base + 64u + 8u * s; };
 
   const int kvh = blockIdx.y;
-  const int rank = blockIdx.x, ranks = gridDim.x;  // kShared: as many histories as CTAs; otherwise the history's slices
-  const int t0 = kShared ? (int)blockIdx.z * ranks : (int)blockIdx.z;
-  const int count = kShared ? min(ranks, T - t0) : 1;
+  const int rank = blockIdx.x, ranks = gridDim.x, per_cluster = kShared ? ranks / n_splits : 1;
+  const int t0 = (int)blockIdx.z * per_cluster;
+  const int count = kShared ? min(per_cluster, T - t0) : 1;
   const int h0 = kvh * G;  // first query head of this CTA (G = n_heads / n_kv)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, tq = lane & 3;  // mma fragment coordinates
@@ -160,7 +169,8 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   __shared__ __align__(16) uint16_t s_q[G][D];
   __shared__ __align__(16) uint16_t s_kvnew[2][D];
   __shared__ float s_m[kAttnWarps][G], s_l[kAttnWarps][G];
-  __shared__ float p_o[kShared ? 2 : 1][G][kShared ? D : 1], p_m[2][G], p_l[2][G];  // pieces of a history: one begun by a CTA before, one that goes on in the next
+  __shared__ __align__(16) float p_o[kShared ? 2 : 1][G][kShared ? D : 1];
+  __shared__ float2 p_ml[2][G];  // pieces of a history: one begun by a CTA before, one that goes on in the next
   __shared__ int s_ctx[kAttnMaxCluster], s_row[kAttnMaxCluster];
 
   if (threadIdx.x == 0) {
@@ -193,15 +203,19 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
     total += n;
     if (kShared) most = max(most, n);
   }
-  // A history of its own for every CTA, or equal shares of all where that is shorter by more than a piece's start and end cost
+  // A history of its own for every n_splits CTAs, or equal shares of all where that is shorter by more than a piece's start and end cost
   const int share = kShared ? (total + ranks - 1) / ranks : 0;
-  const bool level = kShared && most > share + 2;  // (the same in every CTA of the cluster)
+  const bool level = kShared && most > (share + 2) * n_splits;
+  const bool pieces = kShared && (level || n_splits > 1);  // (the same in every CTA of the cluster)
   auto bound = [&](int r) {
     if (!kShared) return min(total, r * ((total + n_splits - 1) / n_splits));
     if (level) return min(total, r * share);
+    const int item = r / n_splits;
     int at = 0;
-    for (int i = 0; i < min(r, count); i++) at += tiles_of(i);
-    return at;
+    for (int i = 0; i < min(item, count); i++) at += tiles_of(i);
+    if (item >= count) return at;
+    const int n = tiles_of(item);
+    return at + min(n, (r % n_splits) * ((n + n_splits - 1) / n_splits));
   };
   const int lo = bound(rank), hi = bound(rank + 1);
   // f(history, first tile, end tile, tiles of the history) for every piece in [lo, hi); an empty history counts as a tile above, so that it has a
@@ -256,7 +270,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
       });
     }
     __syncwarp();
-    if (level) attn_cluster_sync();
+    if (pieces) attn_cluster_sync();
     if (kShared) attn_cluster_sync();
     return;
   }
@@ -459,7 +473,7 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
         out[((size_t)t * n_heads + h) * D + dd] = float_to_bf16_bits(o / L);
       } else if constexpr (kShared) {
         p_o[slot][hh][dd] = o;
-        if (dd == 0) { p_m[slot][hh] = M; p_l[slot][hh] = L; }
+        if (dd == 0) p_ml[slot][hh] = make_float2(M, L);
       } else {
         // scratch: ml [T][n_heads][S][2] then o [T][n_heads][S][D]; m is in the log2 domain
         float *ml = scratch + (((size_t)t * n_heads + h) * n_splits + rank) * 2;
@@ -476,30 +490,36 @@ attn_paged_kernel(const __grid_constant__ CUtensorMap kv_map, long long row0, co
   });
   // ---- pieces of one history in several CTAs: the CTA that holds its first piece reads the others' out of their shared memory
   if constexpr (kShared) {
-    if (level) attn_cluster_sync();
+    if (pieces) attn_cluster_sync();
     if (open >= 0) {
       int end = 0;
       for (int i = 0; i <= open; i++) end += tiles_of(i);
       int last = rank + 1;  // the CTAs rank + 1 .. last hold the rest
       while (bound(last + 1) < end) last++;
-      for (int e = threadIdx.x; e < G * D; e += kAttnThreads) {
+      for (int e = threadIdx.x * 4; e < G * D; e += kAttnThreads * 4) {
         const int hh = e / D, dd = e - hh * D;
-        float mr2[kAttnMaxCluster], M = p_m[1][hh];
+        // all of them at once (the last one again where there are fewer): one after the other they took 0.2 us each
+        float2 ml[kAttnMaxCluster];
+        float4 po[kAttnMaxCluster];
+        ml[0] = p_ml[1][hh];
+        po[0] = *reinterpret_cast<const float4 *>(&p_o[1][hh][dd]);
 #pragma unroll
-        for (int r = 1; r < kAttnMaxCluster; r++) {
-          mr2[r] = rank + r <= last ? ld_cluster(&p_m[0][hh], (uint32_t)(rank + r)) : -INFINITY;
-          M = fmaxf(M, mr2[r]);
+        for (int r = 1; r < kAttnMaxCluster; r++) ml[r] = ld_cluster2(&p_ml[0][hh], (uint32_t)min(rank + r, last));
+#pragma unroll
+        for (int r = 1; r < kAttnMaxCluster; r++) po[r] = ld_cluster4(&p_o[0][hh][dd], (uint32_t)min(rank + r, last));
+        float M = ml[0].x;
+#pragma unroll
+        for (int r = 1; r < kAttnMaxCluster; r++) M = fmaxf(M, ml[r].x);
+        float L = 0.f;
+        float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < kAttnMaxCluster; r++) {
+          const float w = rank + r <= last ? exp2f(ml[r].x - M) : 0.f;  // every piece holds a visible key
+          L = fmaf(ml[r].y, w, L);
+          o.x = fmaf(po[r].x, w, o.x); o.y = fmaf(po[r].y, w, o.y); o.z = fmaf(po[r].z, w, o.z); o.w = fmaf(po[r].w, w, o.w);
         }
-        const float f = exp2f(p_m[1][hh] - M);  // every piece holds a visible key
-        float L = p_l[1][hh] * f, o = p_o[1][hh][dd] * f;
-#pragma unroll
-        for (int r = 1; r < kAttnMaxCluster; r++)
-          if (rank + r <= last) {
-            const float w = exp2f(mr2[r] - M);
-            L += ld_cluster(&p_l[0][hh], (uint32_t)(rank + r)) * w;
-            o += ld_cluster(&p_o[0][hh][dd], (uint32_t)(rank + r)) * w;
-          }
-        out[((size_t)(t0 + open) * n_heads + h0 + hh) * D + dd] = float_to_bf16_bits(o / L);
+        uint16_t *to = out + ((size_t)(t0 + open) * n_heads + h0 + hh) * D + dd;  // (out may start on any element)
+        to[0] = float_to_bf16_bits(o.x / L); to[1] = float_to_bf16_bits(o.y / L); to[2] = float_to_bf16_bits(o.z / L); to[3] = float_to_bf16_bits(o.w / L);
       }
     }
     // nobody leaves while its pieces are read; without pieces either, so that a cluster of the next launch finds eight places at once
@@ -708,18 +728,22 @@ __global__ void attn_combine_kernel(const float *__restrict__ scratch, uint16_t 
   out[((size_t)t * n_heads + h) * D + dd] = float_to_bf16_bits(o / L);
 }
 
-// Whole histories can be shared (slices are a share already; slices merged inside a cluster instead of by the combine pass took 13.0 us for 8 x 512
-// where the two kernels take 8.5, and 22.8 against 16.5 for 8 x 2000: a cluster's start costs more than the launch), as far as the clusters that
-// have eight tokens run at once (33 of two CTAs per SM by the occupancy query of one B200): 36 of them in two rounds take 33.0 us where single CTAs
-// take 23.8 (heads of 64, 72 histories of up to 2500).
+// Whole histories can be shared as far as the clusters that have eight tokens run at once (33 of two CTAs per SM by the occupancy query of one
+// B200): 36 of them in two rounds take 30.2 us where single CTAs take 23.8 (heads of 64, 72 histories of up to 2500).
 constexpr int kAttnClusters = 32;
 bool attn_may_share(int n_splits, int T, int n_kv) {
   const long long full = T >= kAttnMaxCluster ? (long long)(T / kAttnMaxCluster) * n_kv : ((long long)T * n_kv + kAttnMaxCluster - 1) / kAttnMaxCluster;
   return n_splits == 1 && T > 1 && full <= kAttnClusters && (long long)T * n_kv <= 2 * kNumSMs;
 }
+// A history's two to eight slices in one cluster, which joins them itself: no combine pass, but from graphs it takes longer (1 x 512 keys 6.2 -> 7.9 us, 8 x
+// 512 8.5 -> 11.1, 8 x 2000 15.7 -> 18.3: a cluster starts and ends later than its CTAs alone).  A call of its own saves its caller a launch, 2 us.
+static bool attn_may_join(int n_splits, int T, int n_kv) {
+  const int per = kAttnMaxCluster / n_splits;
+  return n_splits <= kAttnMaxCluster && (long long)((T + per - 1) / per) * n_kv <= kAttnClusters;
+}
 // Which takes longer, us: the longest history alone or the largest share of a cluster (0.8 us a tile of heads of 128, 0.5 of 64), the largest of the
-// clusters that have to wait on top, neither less than the stream of all keys and values at 6.5 TB/s; sharing costs 8.  Of 25 ragged and 19 equal
-// batches (heads of 128: 20 and 32 histories, of 64: 40 and 64; 100 to 7000 keys) it takes the slower form of two, by 1 and 5 %.
+// clusters that have to wait on top, neither less than the stream of all keys and values at 6.5 TB/s; sharing costs 6.  Of 29 ragged and 19 equal
+// batches (heads of 128: 20 and 32 histories, of 64: 40 and 64; 100 to 7000 keys) it takes the slower form of two, by 3 and 7 %.
 bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d) {
   const int n = T < kAttnMaxCluster ? T : kAttnMaxCluster, at_once = std::max(1, kAttnClusters / n_kv);
   long long total = 0, most = 0, share = 0, later = 0;
@@ -735,7 +759,7 @@ bool attn_sharing_pays(const int *ctx, int T, int n_kv, int d) {
     round = std::max(round, (sum + n - 1) / n);
   }
   const double tile = d == 128 ? 0.8 : 0.5, stream = (double)total * n_kv * (kAttnTile * d * 4) / 6.5e6;  // us
-  return std::max((share + later) * tile, stream) + 8.0 < std::max(most * tile, stream);
+  return std::max((share + later) * tile, stream) + 6.0 < std::max(most * tile, stream);
 }
 
 size_t attn_scratch_elems(int T, int n_heads, int d, int n_splits) {
@@ -759,11 +783,11 @@ static cudaError_t attn_launch(const TmaMap &kv_map, long long row0, const AttnR
     stages = stages < 2 ? 2 : (stages > AttnCfg<D>::kStages ? AttnCfg<D>::kStages : stages);
   }
   const int smem = stages * AttnCfg<D>::kStageBytes + AttnCfg<D>::kExtraBytes;
-  const int ranks = kShared ? std::min(T, kAttnMaxCluster) : n_splits;
-  DIS_CUDA_TRY(launch_k_cluster(kern, dim3(ranks, n_kv, kShared ? (T + ranks - 1) / ranks : T), dim3(NG * 128 + 32), (size_t)smem, st, kShared ? ranks : 1,
+  const int per_cluster = kShared ? std::min(T, kAttnMaxCluster / n_splits) : 1, ranks = per_cluster * n_splits;
+  DIS_CUDA_TRY(launch_k_cluster(kern, dim3(ranks, n_kv, (T + per_cluster - 1) / per_cluster), dim3(NG * 128 + 32), (size_t)smem, st, kShared ? ranks : 1,
                                 *reinterpret_cast<const CUtensorMap *>(&kv_map), row0, rope, q, page_table, max_pages, pt_row, ctx, out,
                                 scratch, n_splits, T, n_heads, n_kv, page_shift, stages));
-  if (n_splits > 1)
+  if (n_splits > 1 && !kShared)
     DIS_CUDA_TRY(launch_k(attn_combine_kernel<D>, dim3(n_heads, T), dim3(D), 0, st, (const float *)scratch, out, n_splits, T, n_heads));
   return cudaSuccess;
 }
@@ -785,7 +809,7 @@ static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const Att
   int page_shift = 0;
   while ((1 << page_shift) < page_size) page_shift++;
   const int G = n_heads / n_kv;  // query heads per kv head, all handled by one CTA
-  share = share && attn_may_share(n_splits, T, n_kv);
+  share = share && (n_splits > 1 ? attn_may_join(n_splits, T, n_kv) : attn_may_share(n_splits, T, n_kv));
   // Heads of 64: three CTAs of four computing warps fit an SM, or two of eight.  Just above three per SM the former leave most of a second round
   // empty, the latter fill theirs: 512 CTAs, 2500 keys 64.3 -> 55.3 us, 700 22.0 -> 20.2, 200 11.6 -> 11.7; 448 x 2500 58.2 -> 54.2 (200 keys 10.5 -> 11.1).
   // Elsewhere four warps are ahead: 304 x 700 12.1 against 17.8, 640 x 700 23.9 against 28.5, 1024 x 2500 103.8 against 110.1.
@@ -809,16 +833,26 @@ static cudaError_t attn_dispatch(const TmaMap &kv_map, long long row0, const Att
   return cudaErrorInvalidValue;
 }
 
+static bool captured(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) == cudaSuccess) return cs != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();  // (another thread captures what the legacy stream would have to wait for: the launch says so)
+  return true;
+}
 cudaError_t launch_attn_paged(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,
                               int max_pages, const int *pt_row, const int *ctx, uint16_t *out, float *scratch,
                               int n_splits, int T, int n_heads, int n_kv, int d, int page_size, cudaStream_t st) {
   AttnRope none{};
   // The lengths are on the device; the page table's width bounds them, and from about these on a ragged batch gains (us, whole / shared; heads of 128, 32
-  // histories of up to 1100 17.9 / 19.4, 1500 22.5 / 22.3, 2000 28.5 / 26.7, 7000 87.0 / 63.8, 20 of up to 2000 24.1 / 22.3; heads of 64, 64 of up
-  // to 1500 16.5 / 17.5, 2000 20.2 / 19.6, 4500 38.9 / 29.1).  Where clusters have to wait, those of the last tokens, only long ones do: 36 of up to 2500
-  // 34.0 / 36.8, 6000 73.7 / 61.4.  Equal histories lose: 32 x 2000 42.2 / 44.7, 32 x 6000 115.1 / 119.1, heads of 64, 64 x 4000 42.7 / 44.5.
+  // histories of up to 1100 17.9 / 17.9, 1500 22.3 / 20.5, 2000 28.3 / 25.0, 7000 87.1 / 62.3, 20 of up to 1100 15.2 / 16.4, 1500 19.2 / 18.3; heads of
+  // 64, 64 of up to 1100 13.1 / 14.5, 1500 16.4 / 16.0, 4500 39.1 / 27.1, 40 of up to 1500 14.6 / 15.5, 2000 18.2 / 16.9).  Where clusters have to wait,
+  // those of the last tokens, it takes longer ones: 36 of up to 2500 33.8 / 33.7, 6000 74.1 / 57.9.  Equal histories lose: 32 x 2000 42.6 / 45.0, 32 x 6000
+  // 115.1 / 119.7, heads of 64, 64 x 4000 43.0 / 45.1.
   const bool waits = (long long)((T + kAttnMaxCluster - 1) / kAttnMaxCluster) * n_kv > kAttnClusters && T >= kAttnMaxCluster;
-  const bool share = (long long)max_pages * page_size > (waits ? 4096 : d == 128 ? 1792 : 2048);
+  const long long keys = (long long)max_pages * page_size;
+  bool share = keys > (waits ? 2560 : d == 128 ? 1280 : 1664);
+  // Slices are joined in their cluster where the call is not captured and so short that its caller's time counts: up to 16 MB of keys and values
+  if (n_splits > 1) share = T * keys * n_kv * d * 4 <= (16ll << 20) && !captured(st);
   return attn_dispatch(kv_map, row0, none, q, page_table, max_pages, pt_row, ctx, out, scratch, n_splits, T, n_heads, n_kv, d,
                        page_size, share, st);
 }

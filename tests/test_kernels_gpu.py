@@ -394,10 +394,11 @@ def test_attention_of_ragged_histories(nh, nkv, d, page_size, T, n_splits, patte
 
 
 @pytest.mark.parametrize("nh,nkv,d", [(32, 8, 128), (32, 4, 64)])
-@pytest.mark.parametrize("T,n_splits,most", [(2, 4, 900), (24, 1, 600), (40, 1, 3000), (130, 1, 300)])
+@pytest.mark.parametrize("T,n_splits,most", [(2, 4, 900), (1, 8, 1500), (5, 3, 700), (4, 2, 130), (24, 1, 600), (40, 1, 3000), (130, 1, 300)])
 def test_attention_is_as_close_as_its_output_s_type(nh, nkv, d, T, n_splits, most):
     """Decode attention's error against 64 bits is that of rounding the result to bf16 (weights go into the product as two halves: in one, the
-    error is 10 % larger): slices, whole histories, histories that a cluster shares, more CTAs than fit at once."""
+    error is 10 % larger): slices, whole histories, histories that a cluster shares, more CTAs than fit at once.  The same bits from a graph, where
+    a small call's slices are joined by a kernel of its own and not in a cluster."""
     rng = np.random.default_rng(T + d)
     page_size = 64
     ctx = np.exp(rng.uniform(np.log(most / 12), np.log(most), T)).astype(np.int32)
@@ -413,8 +414,20 @@ def test_attention_is_as_close_as_its_output_s_type(nh, nkv, d, T, n_splits, mos
     out = torch.empty_like(q)
     scratch = torch.empty(max(1, lib().dis_k_attn_scratch_elems(T, nh, d, n_splits)), device=DEV)
     rows, dctx, dtab = dev_i32(np.arange(T, dtype=np.int32)), dev_i32(ctx), dev_i32(table)
-    check(lib().dis_k_attn_paged(ptr(q), ptr(pool), pool.shape[0], ptr(dtab), table.shape[1], ptr(rows), ptr(dctx), ptr(out), ptr(scratch), n_splits, T, nh, nkv, d, page_size, None))
+
+    def run():
+        check(lib().dis_k_attn_paged(ptr(q), ptr(pool), pool.shape[0], ptr(dtab), table.shape[1], ptr(rows), ptr(dctx), ptr(out), ptr(scratch), n_splits, T, nh, nkv, d, page_size,
+                                     torch.cuda.current_stream().cuda_stream))
+
+    run()
+    eager = out.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run()
+    out.fill_(float("nan"))
+    graph.replay()
     sync()
+    assert torch.equal(eager, out)
     ref = torch.empty(q.shape, dtype=torch.float64, device=DEV)
     for t in range(T):
         kv = pool[torch.from_numpy(table[t, :need[t]].astype(np.int64)).to(DEV)].double()
