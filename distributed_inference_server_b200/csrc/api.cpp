@@ -288,9 +288,11 @@ int dis_k_attn_prefill(const uint16_t *q, const uint16_t *kv_pool, int64_t n_pag
   // Heads of 64 off a 16-byte boundary: the mma.sync kernel moves q and out in words of 4 bytes and takes the 16-token blocks that this
   // entry point promises for them.  (Blocks of heads of 128 are longer: those are refused.)
   const bool tc = dis::attn_prefill_uses_tc(n_heads, n_kv, d) && (d != 64 || dis::attn_prefill_tc_aligned(q, out));
-  auto fn = tc ? dis::launch_attn_prefill_tc : dis::launch_attn_prefill;
-  return k_ret(fn(map, 0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_blocks, n_heads, n_kv, d, page_size,
-                  (cudaStream_t)stream));
+  // The lengths are on the device.  Blocks of ragged prompts see about a quarter of the longest on average, which the page table's width bounds.
+  if (tc) return k_ret(dis::launch_attn_prefill_tc(map, 0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_blocks, n_heads, n_kv, d,
+                                                   page_size, (long long)max_pages * page_size * 24 / 100, (cudaStream_t)stream));
+  return k_ret(dis::launch_attn_prefill(map, 0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_blocks, n_heads, n_kv, d, page_size,
+                                        (cudaStream_t)stream));
 }
 int dis_k_attn_prefill_block_tokens(int32_t n_heads, int32_t n_kv, int32_t d) {
   return dis::attn_prefill_block_tokens(n_heads, n_kv, d);

@@ -717,6 +717,8 @@ cudaError_t Engine::enqueue_layers(int T, int n_splits) {
     return cudaSuccess;
   };
   RET_CUDA(enqueue_meta());
+  long long block_keys = 0;  // keys that the query blocks see, all together
+  for (int b = 0; b < n_qblocks; b++) block_keys += cur_meta->h<int>(cur_meta->o_qb_pos0)[b] + cur_meta->h<int>(cur_meta->o_qb_len)[b];
   for (int l = 0; l < m.layers; l++) {
     prof_mark(P_NORM);
     if (l == 0) {
@@ -738,10 +740,12 @@ cudaError_t Engine::enqueue_layers(int T, int n_splits) {
       RET_CUDA(launch_rope_kv_write(partial, s_qkv, (long long)T * nqkv_l, q, pool, d_page_table, max_pages, ptrow, pos,
                                     rope_cos, rope_sin, T, nh_l, nkv_l, d, page_size, stream));
       prof_mark(P_ATTN);
-      RET_CUDA((pf_tc ? launch_attn_prefill_tc : launch_attn_prefill)(kv_map, (long long)l * kv_rows_per_layer, q, d_page_table, max_pages,
-                                   cur_meta->d<int>(cur_meta->o_qb_tok0), cur_meta->d<int>(cur_meta->o_qb_len),
-                                   cur_meta->d<int>(cur_meta->o_qb_pos0), cur_meta->d<int>(cur_meta->o_qb_ptrow), attn,
-                                   n_qblocks, nh_l, nkv_l, d, page_size, stream));
+      const int *qb_tok0 = cur_meta->d<int>(cur_meta->o_qb_tok0), *qb_len = cur_meta->d<int>(cur_meta->o_qb_len);
+      const int *qb_pos0 = cur_meta->d<int>(cur_meta->o_qb_pos0), *qb_row = cur_meta->d<int>(cur_meta->o_qb_ptrow);
+      if (pf_tc) RET_CUDA(launch_attn_prefill_tc(kv_map, (long long)l * kv_rows_per_layer, q, d_page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_row, attn,
+                                                 n_qblocks, nh_l, nkv_l, d, page_size, block_keys / n_qblocks, stream));
+      else RET_CUDA(launch_attn_prefill(kv_map, (long long)l * kv_rows_per_layer, q, d_page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_row, attn,
+                                        n_qblocks, nh_l, nkv_l, d, page_size, stream));
       kernel_launches += 2;
     } else {
       // decode: RoPE + KV write live inside the attention kernel (one kernel boundary less per layer)

@@ -152,8 +152,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
   float *l_row = reinterpret_cast<float *>(smem + (bar_base - smem_base) + 256);  // [group][row]: at the end
   float *m_row = l_row + 256;  // one O: [row], the softmax reference, handed from tile to tile; two: [group][row], at the end
 
-  // later query blocks of a sequence have more key tiles: launch them first, so that the longest CTAs do not form the tail
-  const int qb = (int)gridDim.x - 1 - (int)blockIdx.x, kvh = blockIdx.y;
+  // Later query blocks of a sequence have more key tiles: launch them first, so that the longest CTAs do not form the tail.  D = 64, whose passes of
+  // more than a round stay here where histories are long: a block's kv heads one after the other, or the tail would be whole heads (one prompt of
+  // 3000 tokens, 32 / 4 heads, 75.5 -> 63.6 us).
+  const unsigned long long at = (unsigned long long)blockIdx.y * gridDim.x + blockIdx.x;
+  const int qb = (int)(gridDim.x - 1 - (D == 64 ? at / n_kv : blockIdx.x)), kvh = D == 64 ? (int)(at % n_kv) : blockIdx.y;
   const int warp = uniform_warp(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -973,18 +976,22 @@ static cudaError_t prefill_tc_launch(K kern, dim3 grid, int threads, int smem, D
 }
 
 // A pair of blocks on an SM of its own pays where the GPU has more blocks than SMs to spread them on: us of one block per CTA / of pairs, by blocks
-// times kv heads, heads of 128: 152 16.2 / 15.9, 208 12.9 / 13.6, 216 16.9 / 15.6, 304 25.8 / 24.8, 328 17.6 / 15.0, 560 39.5 / 30.4, 672 39.5 / 28.1;
-// heads of 64, whose single blocks run two to an SM with less between them: 316 10.8 / 10.8, 320 27.6 / 35.4, 548 25.7 / 22.2, 664 23.3 / 20.0.
-static bool prefill_in_pairs(int n_blocks, int n_kv, int d) {
+// times kv heads, heads of 128: 152 16.2 / 15.9, 208 12.9 / 13.6, 216 16.9 / 15.6, 304 25.8 / 24.8, 328 17.6 / 15.0, 560 39.5 / 30.4, 672 39.5 / 28.1.
+// (Equal blocks that fill a little more than one round lose 5 to 14 %: 20 prompts of 33 tokens, 320, 10.8 / 12.0; blocks whose pairs are of two
+// sequences likewise: 5 of 100 behind 700, 280, 22.0 / 25.4.)
+// Heads of 64, whose single blocks run two to an SM with four softmax groups between them: 316 10.8 / 10.8, 320 27.6 / 35.4, and beyond that by the
+// history that a block sees on average, up to which starts and ends weigh more: 80 prompts of 17 tokens 13.1 / 11.0, behind 700 35.2 / 41.2; ragged
+// prompts (a quarter of the longest on average), eight to 700 tokens 20.9 / 19.9, six to 1900 69.2 / 66.4, three to 3333 134 / 140; one of 8000 364 / 405.
+static bool prefill_in_pairs(int n_blocks, int n_kv, int d, long long mean_keys) {
   const long long n = (long long)n_blocks * n_kv;
-  return n > (d == 128 ? 3 : 6) * kNumSMs / 2 && n < (1ll << 31);
+  return n > (d == 128 ? 3 : 6) * kNumSMs / 2 && n < (1ll << 31) && (d == 128 || mean_keys <= 720);
 }
 
 // Same contract as launch_attn_prefill (k_attn_paged.cu) with query blocks of up to 128 / G tokens.
 cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,
                                    int max_pages, const int *qb_tok0, const int *qb_len, const int *qb_pos0,
                                    const int *qb_ptrow, uint16_t *out, int n_blocks, int n_heads, int n_kv, int d,
-                                   int page_size, cudaStream_t st) {
+                                   int page_size, long long mean_keys, cudaStream_t st) {
   if (n_blocks <= 0) return cudaSuccess;
   if (n_kv <= 0 || n_heads % n_kv != 0 || n_kv > 65535) { set_last_error("attn_prefill_tc: bad head geometry"); return cudaErrorInvalidValue; }
   if (!attn_prefill_tc_aligned(q, out)) { set_last_error("attn_prefill_tc: q and out must start on 16 bytes"); return cudaErrorInvalidValue; }
@@ -995,7 +1002,7 @@ cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const u
 #define DIS_PF_TC_CASE(DD, GG)                                                                                                   \
   if (d == DD && G == GG) {                                                                                                      \
     static DeviceOnce once, once_pair;                                                                                           \
-    if (prefill_in_pairs(n_blocks, n_kv, DD))                                                                                        \
+    if (prefill_in_pairs(n_blocks, n_kv, DD, mean_keys))                                                                             \
       return prefill_tc_launch(attn_prefill_pair_kernel<DD, GG>, dim3((n_blocks + 1) / 2 * n_kv), kPpThreads, pp_smem_bytes<DD>(), once_pair, st, kv_map, \
                                row0, q, page_table, max_pages, qb_tok0, qb_len, qb_pos0, qb_ptrow, out, n_heads, n_kv, page_shift, n_blocks); \
     return prefill_tc_launch(attn_prefill_tc_kernel<DD, GG>, dim3(n_blocks, n_kv), kPfThreads, pf_smem_bytes<DD>(), once, st, kv_map, row0, q,        \

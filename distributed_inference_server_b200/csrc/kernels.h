@@ -112,7 +112,7 @@ int attn_prefill_full_block(int n_heads, int n_kv, int d);
 cudaError_t launch_attn_prefill_tc(const TmaMap &kv_map, long long row0, const uint16_t *q, const int *page_table,
                                    int max_pages, const int *qb_tok0, const int *qb_len, const int *qb_pos0,
                                    const int *qb_ptrow, uint16_t *out, int n_blocks, int n_heads, int n_kv, int d,
-                                   int page_size, cudaStream_t st);
+                                   int page_size, long long mean_keys /* keys in front of and in a block, on average */, cudaStream_t st);
 
 // k_gemm_tcgen05.cu
 cudaError_t make_tma_map_2d(TmaMap *out, const void *base, uint64_t rows, uint64_t cols, uint32_t box_rows);

@@ -589,14 +589,16 @@ def test_attention_prefill_of_many_blocks(nh, nkv, d, BT, page_size, kind):
 
 
 @pytest.mark.parametrize("nh,nkv,BT", [(32, 8, 32), (32, 4, 16)])
-def test_attention_prefill_heads_of_64_bits_in_pairs_and_alone(nh, nkv, BT):
+@pytest.mark.parametrize("longest", [2300, 4200])
+def test_attention_prefill_heads_of_64_bits_in_pairs_and_alone(nh, nkv, BT, longest):
     """Heads of 64: a query block has the same bits whether it is one of a pair or alone in its CTA, so the number of blocks of a pass does
     not move its error (even and odd key tiles have a maximum of their own in both forms).  Prompts of 1 to 40 tiles, some behind a cache,
-    keys that grow with their position, one block of an odd sequence left over."""
+    keys that grow with their position, one block of an odd sequence left over.  With the longer prompt a pass of any size keeps its blocks
+    alone, more of them than run at once."""
     d, page_size = 64, 64
     g = torch.Generator(device=DEV); g.manual_seed(nh + nkv)
     rng = np.random.default_rng(nkv)
-    lens, past = [2500, 65, 700, 1, 1300], [0, 200, 0, 0, 64]
+    lens, past = [longest, 65, 700, 1, 1300], [0, 200, 0, 0, 64]
     while sum(-(-n // BT) for n in lens) * nkv <= 6 * 148 // 2 + nkv:
         lens.append(int(rng.integers(1, 900))); past.append(int(rng.choice([0, 100])))
     total = [a + b for a, b in zip(past, lens)]
