@@ -1309,7 +1309,10 @@ __global__ void __launch_bounds__(256) stack_ssm_step_kernel(const float *__rest
 
 // Passes of single tokens whose layout the kernel above takes: a norm's stretch is whole heads, at most eight (a cluster), and holds whole groups of
 // heads (a group's tail has one owner); sizes and rows in fours, up to 128.
-bool stack_ssm_step_ok(const float *proj, const float *slices, long long ld, const float *cstate, int x_off, int C, int taps, int H, int N, int P, int G, int parts) {
+// Beyond three rounds of two CTAs per SM the four kernels are ahead, which hold more of their state in flight: steps of a model of four layers, 32 heads of
+// 128 x 64, one kernel / four: 24 sequences 215 / 225 us, 32 239 / 235, 48 300 / 276, 96 448 / 383; 16 heads: 48 sequences 218 / 224, 64 246 / 235.
+bool stack_ssm_step_ok(const float *proj, const float *slices, long long ld, const float *cstate, int x_off, int C, int taps, int T, int H, int N, int P, int G, int parts) {
+  if ((long long)T * H > 6 * kNumSMs) return false;
   if (N > kSsmStepMax || P > kSsmStepMax || N % 4 || P % 4 || (H * P) % parts || taps < 1 || taps > kConvMaxTaps) return false;
   const int per = H * P / parts;
   if (per % P || per / P > 8 || (per / P) % (H / G) || H > (1 << 30) / P) return false;

@@ -1674,7 +1674,7 @@ cudaError_t Engine::stack_forward(int T, int n_spans, int n_qb, int R, bool all_
     // the preparation kernels of attention (alone), latent attention and retention, and the state-space mixer's step of single tokens, sum the
     // slices of a split-K input projection themselves
     const bool ssm_step = lc.mixer == DIS_MIX_SSM && T == sp.n_spans && par_ff == 0 &&
-                          stack_ssm_step_ok(M.proj, cur_scratch, N, Rn.conv_state, L.x_off, L.conv_ch, lc.conv_taps, lc.heads, lc.ssm_state, lc.vdim, lc.ssm_groups, lc.ssm_norm_groups);
+                          stack_ssm_step_ok(M.proj, cur_scratch, N, Rn.conv_state, L.x_off, L.conv_ch, lc.conv_taps, T, lc.heads, lc.ssm_state, lc.vdim, lc.ssm_groups, lc.ssm_norm_groups);
     const bool prep_sums = ssm_step || lc.mixer == DIS_MIX_ATTENTION || lc.mixer == DIS_MIX_LATENT || lc.mixer == DIS_MIX_RETENTION || lc.mixer == DIS_MIX_CHANNEL_DELTA;
     if (split_in) RET_CUDA(glu_product(L.w_gu, par_ff, lc.mlp_act, ff_act, L.ld_act));
     RET_CUDA(gemm(M.hc, f32, W, L.w_in, 0, L.b_in.ptr ? reinterpret_cast<const float *>(L.b_in.ptr) : nullptr, M.proj, T, N, W, cap_tokens,

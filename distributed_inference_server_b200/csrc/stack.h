@@ -139,7 +139,7 @@ cudaError_t launch_stack_ssm_out(const float *o, const float *buf, long long ld_
                                  const float *w, int parts, void *out, bool f32, int T, int H, int P, float eps, cudaStream_t st);
 // All three at once for a pass of single tokens, straight from the projection's slices (n_part of them, stride apart, a multiple
 // of ld; bias or null).  slices: the buffer that they are in when there are several; both start on 16 bytes.
-bool stack_ssm_step_ok(const float *proj, const float *slices, long long ld, const float *cstate, int x_off, int C, int taps, int H, int N, int P, int G, int parts);
+bool stack_ssm_step_ok(const float *proj, const float *slices, long long ld, const float *cstate, int x_off, int C, int taps, int T, int H, int N, int P, int G, int parts);
 cudaError_t launch_stack_ssm_step(const float *proj, long long ld, int n_part, long long stride, const float *bias, int x_off, int dt_off, int C, int H, int taps,
                                   const float *cw, const float *cb, const float *vec, float *cstate, const StackSpans &sp, float *state, const float *w, int N, int P,
                                   int G, int parts, float eps, void *out, bool f32, cudaStream_t st);

@@ -248,6 +248,23 @@ def test_single_tokens_in_one_kernel(dtype, heads, vdim, state, groups, taps, no
     e.close()
 
 
+def test_single_tokens_on_both_sides_of_the_line():
+    """40 heads: passes of 22 sequences take the one kernel, of 23 the four (more than three rounds of CTAs).  Sequences go from one form
+    to the other and back, their state and convolution tail with them; against the oracle."""
+    cfg = U.config([(U.ssm(heads=40, vdim=4, state=8, groups=5, conv=3, norm_groups=5), None)], width=24, streams=0)
+    W = U.weights(cfg, seed=35)
+    seqs = {k: toks(14, seed=70 + k) for k in range(23)}
+    e = U.engine(cfg, W, pool_tokens=23 * 24, page_size=8, max_batch=23, max_step_tokens=200)
+    f = U.Feeder(e)
+    f.step([(k, v, 3) for k, v in seqs.items()])
+    for n in (22, 23, 23, 22, 23):
+        f.step([(k, seqs[k], 1) for k in range(n)])
+    for k, v in seqs.items():
+        got = f.end(k)
+        assert U.rel_err(got, U.oracle_logits(cfg, W, v[:len(got)])) < F32_TOL
+    e.close()
+
+
 @pytest.mark.parametrize("width,heads,vdim,state,groups,taps,norm_groups", [(512, 8, 64, 128, 2, 4, 2), (512, 8, 64, 128, 8, 4, 8), (1024, 16, 32, 64, 2, 4, 2)])
 def test_single_tokens_sum_the_slices_of_a_wide_projection(width, heads, vdim, state, groups, taps, norm_groups):
     """The same kernel where the input projection is cut along K, as it is from a width of 512 on: channels, gate and step size are summed over
