@@ -436,7 +436,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap kv_map, long long row
 // 48 clocks where it computes 32) beside 1024 of exponentials; a group's own chain is 1800 (scores 200-400, maximum 250, exponentials 850-1100,
 // hand-over).  A run of such passes draws 1000 W: 244 us cold, 281 under the power cap.  D = 64: the chain, 640 tensor, 1024 exponentials.
 // Measured against the kernel above: heads of 128, six prompts of 437 to 3000 tokens, 32 / 8 heads: 335 -> 281 us (cold 312 -> 244); eight of up to
-// 700: 39.5 -> 28.1; 64 / 8 heads, six of up to 1900: 202 -> 152; heads of 64, six of 276 to 1900 tokens, 32 / 4 heads: 76 -> 69.4.
+// 700: 39.5 -> 28.1; 64 / 8 heads, six of up to 1900: 202 -> 152; heads of 64, six of 276 to 1900 tokens, 32 / 4 heads: 76 -> 69.1.
 // On the way: a page lookup in front of each TMA load cost 580 clocks a tile, one MMA warp for both groups 100 to 170 clocks per wait; tiles of 128 keys
 // with one score buffer (a wait for S in every step) 335 us, four blocks per CTA for heads of 64 (96 registers, all in step) 79 to 84 us.
 constexpr int kPpTile = kPfTile;             // keys per tile
